@@ -23,11 +23,22 @@
 // breakpoints: each max picks one side, so over the year the sum is
 // sum_h [ |U_h| (sum of |cos| over days with c < |U_h|) + |z| (sum of
 // |cos| |tan| over the other days) ], both inner sums read from prefix /
-// suffix sums over the days sorted by |tan tau| (built once per block), at
-// a count found through a bucket index: twelve lookups per vertex for a
-// year of hourly positions.  Longer schedules sum day by day (paired lanes,
-// groups of 8 days, Kahan across groups), so the result tracks the binary64
-// sum either way.
+// suffix sums over the days sorted by |tan tau| (built once per block).  A
+// pair's value is a convex piecewise linear function of |U_h|, so a bucket
+// table of line pairs gives it as the larger of two lines: twelve table
+// reads per vertex for a year of hourly positions.  Longer schedules sum day
+// by day (paired lanes, groups of 8 days, Kahan across groups).
+//
+// Schedules of many rotations (a day in one-degree steps) are summed by
+// arcs: U(theta) + const > 0 holds on one arc of rotation angles, so a tilt
+// costs one arc (an arc cosine, two searches in the sorted angles) and the
+// difference of two prefix sums of (cos, sin) instead of a max per rotation.
+//
+// The vertices come in binary64; GB300 issues two binary64 operations per
+// SM and cycle, so the kernels split them into binary32 pairs with integer
+// operations and test ||v|^2 - r^2| in pairs: with the test in binary64 (8
+// operations and 3 conversions per vertex) it alone took longer than the
+// reading of the vertices.
 #include "nx_common.cuh"
 
 namespace nx {
@@ -41,6 +52,8 @@ struct InsoArgs {
     int64_t n;
     double r;
     float inv_r;
+    float r2h, r2l;        // r^2 as a pair; r2h = 0: r outside [2^-20, 2^60] (binary64 test)
+    float zmin;            // 1e-20 r: |z| of the breakpoint form is kept off 0
     const float2 *tilt;    // (cos tau, sin tau) per tilt
     int n_tilt;
     const float2 *rot;     // (cos theta, sin theta): all rotations, or the first half in pair mode
@@ -49,6 +62,71 @@ struct InsoArgs {
     float *out;
     int accumulate;
 };
+
+__host__ __device__ __forceinline__ void radius_pair(double r, float &h, float &l)
+{
+    h = l = 0.0f;
+    if (!(r >= 0x1p-20 && r <= 0x1p60)) return;
+    const double r2 = r * r;
+    h = (float)r2;
+    l = (float)(r2 - (double)h);
+}
+
+// |v| as h + l2 / 2, binary32s, by integer operations, for 2^-40 <= |v| <
+// 2^61: h = the top 24 bits (truncated), l2 / 2 the next 23.  ah = the high
+// word of |v|.
+__device__ __forceinline__ void split_abs(uint32_t ah, uint32_t lw, float &h, float &l2)
+{
+    h = __uint_as_float(__funnelshift_l(lw, ah - (896u << 20), 3));
+    const float i = __fsub_rn(__uint_as_float(0x4B000000u | ((lw >> 6) & 0x7FFFFFu)), 8388608.0f);
+    l2 = __fmul_rn(i, __uint_as_float(((ah & 0x7FF00000u) - (941u << 20)) << 3));
+}
+
+__device__ __forceinline__ float signed_sum(float h, float l2, uint32_t hw)
+{
+    return __uint_as_float(__float_as_uint(__fmaf_rn(0.5f, l2, h)) | (hw & 0x80000000u));
+}
+
+// s + e == a + b exactly.
+__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e)
+{
+    s = __fadd_rn(a, b);
+    const float bb = __fsub_rn(s, a);
+    e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+}
+
+// A vertex in binary32 and whether it lies on the sphere of radius r
+// (| |v|^2 - r^2 | <= 1e-12 r^2): the difference in pairs, within 2^-44 r^2;
+// in binary64 for a radius or coordinate outside the pairs' range (a
+// coordinate of 0 among them).
+__device__ __forceinline__ bool load_vertex(double X, double Y, double Z, double r, float r2h, float r2l, float &x,
+                                            float &y, float &z)
+{
+    const uint32_t hx = (uint32_t)__double2hiint(X), hy = (uint32_t)__double2hiint(Y), hz = (uint32_t)__double2hiint(Z);
+    const uint32_t ax = hx & 0x7FFFFFFFu, ay = hy & 0x7FFFFFFFu, az = hz & 0x7FFFFFFFu;
+    if (min(ax, min(ay, az)) >= (983u << 20) && max(ax, max(ay, az)) < (1084u << 20) && r2h > 0.0f) {
+        float xh, xl, yh, yl, zh, zl;
+        split_abs(ax, (uint32_t)__double2loint(X), xh, xl);
+        split_abs(ay, (uint32_t)__double2loint(Y), yh, yl);
+        split_abs(az, (uint32_t)__double2loint(Z), zh, zl);
+        const float px = __fmul_rn(xh, xh), py = __fmul_rn(yh, yh), pz = __fmul_rn(zh, zh);
+        const float ex = __fmaf_rn(xh, xl, __fmaf_rn(xh, xh, -px)), ey = __fmaf_rn(yh, yl, __fmaf_rn(yh, yh, -py)),
+                    ez = __fmaf_rn(zh, zl, __fmaf_rn(zh, zh, -pz));
+        float s1, e1, s2, e2;
+        two_sum(px, py, s1, e1);
+        two_sum(s1, pz, s2, e2);
+        const float low = __fsub_rn(__fadd_rn(__fadd_rn(e1, e2), __fadd_rn(__fadd_rn(ex, ey), ez)), r2l);
+        x = signed_sum(xh, xl, hx);
+        y = signed_sum(yh, yl, hy);
+        z = signed_sum(zh, zl, hz);
+        return fabsf(__fadd_rn(__fsub_rn(s2, r2h), low)) <= 1e-12f * r2h;
+    }
+    x = (float)X;
+    y = (float)Y;
+    z = (float)Z;
+    const double rho2 = X * X + Y * Y + Z * Z, r2 = r * r;
+    return fabs(rho2 - r2) <= 1e-12 * r2;
+}
 
 // climate.py:419-442 for a vertex off the sphere of radius r (binary32).
 __device__ __forceinline__ float general_term(float x, float y, float z, float inv_r, float ct, float st, float cr, float sr)
@@ -65,7 +143,20 @@ __device__ __forceinline__ float general_term(float x, float y, float z, float i
     return clat * fmaxf(clon, 0.0f);
 }
 
-// Sum over the schedule for one vertex.
+__device__ __forceinline__ float approx_sqrt(float v)
+{
+    float w;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(w) : "f"(v));
+    return w;
+}
+
+__device__ __forceinline__ float approx_rcp(float v)
+{
+    float w;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(w) : "f"(v));
+    return w;
+}
+
 // Tilts whose per-day constants a block stages in shared memory (16 B each).
 constexpr int TILT_STAGE_MAX = 2048;
 
@@ -73,8 +164,9 @@ constexpr int TILT_STAGE_MAX = 2048;
 // tau|, HP sin tau, 0); days with |cos tau| < 2^-20 (the direct form) get
 // zeros, which add nothing to the factored sum, and are listed after the
 // days (day indices as ints, their count in entry n_tilt.y); entry n_tilt.x
-// holds the sum of HP sin tau over the factored days (day order, binary64,
-// rounded once), so a vertex adds its days' C terms as one product.
+// holds the sum of HP sin tau over the factored days (binary64, rounded
+// once; a lane per 32nd day, so that a block is not held up by one thread's
+// chain of additions), so a vertex adds its days' C terms as one product.
 // Shared memory: tilt_smem(a).
 template <int HP>
 __device__ __forceinline__ void stage_tilts(const InsoArgs &a, float4 *tt)
@@ -86,16 +178,23 @@ __device__ __forceinline__ void stage_tilts(const InsoArgs &a, float4 *tt)
                                : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    // warp 0: the sum and, in day order, the list of direct days
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
         int *direct = reinterpret_cast<int *>(tt + a.n_tilt + 1);
         double sc = 0.0;
         int nd = 0;
-        for (int d = 0; d < a.n_tilt; ++d) {
-            const float4 k = tt[d];
-            if (k.x > 0.0f) sc += (double)k.z;
-            else direct[nd++] = d;
+        for (int d0 = 0; d0 < a.n_tilt; d0 += 32) {
+            const int d = d0 + lane;
+            const float4 k = d < a.n_tilt ? tt[d] : make_float4(1.0f, 0.0f, 0.0f, 0.0f);
+            const bool dir = !(k.x > 0.0f);
+            if (!dir) sc += (double)k.z;
+            const unsigned m = __ballot_sync(0xFFFFFFFFu, dir);
+            if (dir) direct[nd + __popc(m & ((1u << lane) - 1u))] = d;
+            nd += __popc(m);
         }
-        tt[a.n_tilt] = make_float4((float)sc, __int_as_float(nd), 0.0f, 0.0f);
+        for (int o = 16; o > 0; o >>= 1) sc += __shfl_xor_sync(0xFFFFFFFFu, sc, o);
+        if (lane == 0) tt[a.n_tilt] = make_float4((float)sc, __int_as_float(nd), 0.0f, 0.0f);
     }
     __syncthreads();
 }
@@ -111,18 +210,28 @@ constexpr int DAY_GROUP = 8;
 //     = sum_h [ a_h sum_{d: c_d < a_h} cos_d + |z| sum_{d: c_d >= a_h} cos_d tan_d ],
 // exactly (each max picks one side).  With the days sorted by tan_d, both
 // inner sums are a prefix sum P0 and a suffix sum Q1 of the sorted days,
-// read at the count B_h of days with tan_d < a_h / |z|; a vertex then needs
-// twelve searches instead of a max and an add per pair and day.
-// Shared memory after the staged constants (floats): T[SP] the sorted tan_d
-// padded with +inf to a power of two SP > factored days (at least one +inf
-// sentinel), P0[nf + 1] and Q1[nf + 1] (binary64 sums rounded once), the
-// cos_d in sorted order, and a bucket index of SP + 1 ints: with tmax the
-// largest tan_d and NB = SP buckets of width tmax / NB, F[b] = the count of
-// days with tan_d < b tmax / NB (F[NB] = nf).  A search for t > tmax is nf;
-// otherwise it starts at F[b] for b = floor(t NB / tmax) and steps down
-// while the day below is not below t and up while the next day is below t
-// (a step or two: the buckets hold under one day on average), which ends
-// at the exact count whatever the rounding of b.
+// read at the count B_h of days with tan_d < a_h / |z|.  As a function of
+// a_h this is the line P0[B] a_h + Q1[B] |z|, its slope P0 growing with B at
+// the breakpoints T: convex, so near a breakpoint it is the larger of the
+// two lines that meet there, and no comparison with T is needed.  With t =
+// a_h / |z| a value is |z| (P0 t + Q1).
+// Shared memory after the staged constants: the bucket table of SP + 1
+// float4s (SP a power of two > the days), the lines L[nf + 1] = (P0,
+// Q1) (exact sums rounded once), K[SP] the sorted tan_d, padded with +inf,
+// with their cos_d.  Bucket b holds the t nearest to tmax (1 - (b /
+// SP)^2), tmax the largest tan_d: seasonal tilts go as a sine, so the
+// breakpoints crowd at tmax as those t do, and hardly a bucket gets two
+// (with buckets of equal width in t the crowded ones held up to 14, and the
+// walk through them was a third of the instructions).  Bucket 0 takes all t
+// beyond tmax.  An entry is the lines of the bucket's two ends (p0, p0', q1,
+// q1') where its breakpoints lie within 2e-6 of each other; otherwise p0 is
+// NaN, the two ends' line numbers follow, and a vertex takes the largest of
+// the lines between.  A bucket number one off by rounding changes a value by
+// no more than its rounding does, as the lines meet there.
+// Measured (GB300, a year of hourly positions, 10,000,002 vertices): 289 ->
+// 137 us (2.0 TB/s of the 28 B per vertex; issue-bound, 66 % of the issue
+// slots, 340 instructions per vertex with the search and the binary64 test
+// at 507); 9,002 vertices 63.6 -> 16.6 us (the blocks' start).
 constexpr int SORT_MAX = 512;
 
 __host__ __device__ __forceinline__ int sort_pad(int n)
@@ -132,91 +241,319 @@ __host__ __device__ __forceinline__ int sort_pad(int n)
     return p;
 }
 
-// Builds T, P0, Q1 from the staged constants (after stage_tilts); returns
-// the number of factored days.  Called by the whole block.
-__device__ __forceinline__ int stage_breakpoints(const InsoArgs &a, const float4 *tt, float *T, float *P0, float *Q1,
-                                                 float *CS, int *F, float &scale, float &tmax)
+// Exclusive prefix sums over the block of 64-bit integers (two per thread),
+// and their totals.  Sums of cosines are kept as integers of 2^-44: exact,
+// and without chains of binary64 additions, which took most of a block's
+// start (40 of 64 us from launch to end on a sphere of 9,002 vertices).
+__device__ __forceinline__ void block_scan2(long long &u, long long &v, long long &tu, long long &tv)
 {
-    const int nd = __float_as_int(tt[a.n_tilt].y);
-    const int nf = a.n_tilt - nd;
-    const int sp = sort_pad(nf + 1);
-    // rank sort of the factored days by (tan, day): position = how many
-    // factored days come before
-    for (int d = threadIdx.x; d < a.n_tilt; d += blockDim.x) {
-        const float4 k = tt[d];
-        if (!(k.x > 0.0f)) continue;
-        int rank = 0;
-        for (int e = 0; e < a.n_tilt; ++e) {
-            const float4 o = tt[e];
-            rank += (o.x > 0.0f && (o.y < k.y || (o.y == k.y && e < d))) ? 1 : 0;
-        }
-        T[rank] = k.y;
-        CS[rank] = k.x;
+    __shared__ long long s_sum[2][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const long long u0 = u, v0 = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long a = __shfl_up_sync(0xFFFFFFFFu, u, o), b = __shfl_up_sync(0xFFFFFFFFu, v, o);
+        if (lane >= o) { u += a; v += b; }
     }
-    for (int j = nf + threadIdx.x; j < sp; j += blockDim.x) T[j] = __int_as_float(0x7F800000);
+    if (lane == 31) { s_sum[0][w] = u; s_sum[1][w] = v; }
     __syncthreads();
-    // prefix sums of cos and suffix sums of cos * tan, binary64, one warp:
-    // a lane sums its run of days, the runs are scanned across the warp
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        const int per = (nf + 31) / 32;
-        const int j0 = min(nf, lane * per), j1 = min(nf, j0 + per);
-        double s0 = 0.0, s1 = 0.0;
-        for (int j = j0; j < j1; ++j) {
-            s0 += (double)CS[j];
-            s1 += (double)CS[j] * (double)T[j];
-        }
-        double e0 = s0, e1 = s1;                  // inclusive scan over the lanes
-        for (int o = 1; o < 32; o <<= 1) {
-            const double u0 = __shfl_up_sync(0xFFFFFFFFu, e0, o), u1 = __shfl_up_sync(0xFFFFFFFFu, e1, o);
-            if (lane >= o) { e0 += u0; e1 += u1; }
-        }
-        const double tot1 = __shfl_sync(0xFFFFFFFFu, e1, 31);
-        const double tot0 = __shfl_sync(0xFFFFFFFFu, e0, 31);
-        e0 -= s0;                                 // exclusive
-        e1 -= s1;
-        for (int j = j0; j < j1; ++j) {
-            P0[j] = (float)e0;
-            Q1[j] = (float)(tot1 - e1);
-            e0 += (double)CS[j];
-            e1 += (double)CS[j] * (double)T[j];
-        }
-        if (lane == 0) {
-            P0[nf] = (float)tot0;
-            Q1[nf] = 0.0f;
-        }
-    }
-    // the bucket index: F[b] by a binary search per bucket
-    tmax = nf > 0 ? T[nf - 1] : 0.0f;
-    scale = tmax > 0.0f ? (float)sp / tmax : 0.0f;
-    const float width = tmax / (float)sp;
-    for (int b = threadIdx.x; b <= sp; b += blockDim.x) {
-        if (b == sp) { F[b] = nf; continue; }
-        const float edge = (float)b * width;
-        int c = 0;
-        for (int step = sp >> 1; step > 0; step >>= 1) c += T[c + step - 1] < edge ? step : 0;
-        F[b] = c;
+    u -= u0;
+    v -= v0;
+    tu = tv = 0;
+    for (int k = 0; k < nw; ++k) {
+        if (k == w) { u += tu; v += tv; }
+        tu += s_sum[0][k];
+        tv += s_sum[1][k];
     }
     __syncthreads();
-    return nf;
 }
+
+__device__ __forceinline__ long long to_fixed(float v) { return __float2ll_rn(v * 0x1p44f); }
+__device__ __forceinline__ float from_fixed(long long v) { return __ll2float_rn(v) * 0x1p-44f; }
 
 // Breakpoint tables of a block (stage_breakpoints), or nf < 0 for none.
 struct Breaks {
-    const float *T = nullptr, *P0 = nullptr, *Q1 = nullptr;
-    const int *F = nullptr;
-    int nf = -1, sp = 0;       // factored days, buckets
-    float scale = 0.0f, tmax = 0.0f;
+    const float2 *L = nullptr;
+    const float4 *rot = nullptr;   // the rotations, two to an entry
+    uint32_t bucket = 0;       // shared address of the table less what a bucket number's binary32 exponent adds
+    int nf = -1;               // factored days
+    float sp = 0.0f;           // buckets
+    float inv = 0.0f;          // 1 / tmax
+    bool crowded = false;      // some bucket holds distinct breakpoints
 };
 
-template <int HP>
-__device__ __forceinline__ float inso_vertex(const InsoArgs &a, double X, double Y, double Z, double r, float inv_r,
-                                             const float4 *tt = nullptr, const Breaks &bk = Breaks())
+// Builds the tables from the staged constants (after stage_tilts).  Called
+// by the whole block.
+__device__ __forceinline__ Breaks stage_breakpoints(const InsoArgs &a, const float4 *tt, uint2 *K, float2 *L,
+                                                    float4 *bucket)
 {
-    const double rho2 = X * X + Y * Y + Z * Z;
-    const double r2 = r * r;
-    const bool on_sphere = fabs(rho2 - r2) <= 1e-12 * r2;
-    const float x = (float)X, y = (float)Y, z = (float)Z;
+    const int nd = __float_as_int(tt[a.n_tilt].y);
+    const int nf = a.n_tilt - nd;
+    const int sp = sort_pad(a.n_tilt + 1);
+    // bitonic sort of the factored days by tan (direct days, padding: +inf),
+    // the cosine alongside
+    for (int d = threadIdx.x; d < sp; d += blockDim.x) {
+        const bool day = d < a.n_tilt && tt[d].x > 0.0f;
+        K[d] = day ? make_uint2(__float_as_uint(tt[d].y), __float_as_uint(tt[d].x)) : make_uint2(0x7F800000u, 0u);
+    }
+    __syncthreads();
+    for (int size = 2; size <= sp; size <<= 1)
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            for (int q = threadIdx.x; q < sp / 2; q += blockDim.x) {
+                const int i = 2 * q - (q & (stride - 1)), j = i + stride;
+                const uint2 u = K[i], v = K[j];
+                if ((u.x > v.x) == ((i & size) == 0)) { K[i] = v; K[j] = u; }
+            }
+            __syncthreads();
+        }
+    // prefix sums of cos and of cos * tan: each thread a run of the days
+    const int per = (sp + (int)blockDim.x - 1) / (int)blockDim.x;
+    const int j0 = min(nf, (int)threadIdx.x * per), j1 = min(nf, j0 + per);
+    auto term = [&](int j, long long &u, long long &v) {
+        const float c = __uint_as_float(K[j].y), t = __uint_as_float(K[j].x), p = __fmul_rn(c, t);
+        u += to_fixed(c);
+        v += to_fixed(p) + to_fixed(__fmaf_rn(c, t, -p));
+    };
+    long long u = 0, v = 0, tu, tv;
+    for (int j = j0; j < j1; ++j) term(j, u, v);
+    block_scan2(u, v, tu, tv);
+    for (int j = j0; j < j1; ++j) {
+        L[j] = make_float2(from_fixed(u), from_fixed(tv - v));
+        term(j, u, v);
+    }
+    if (threadIdx.x == 0) L[nf] = make_float2(from_fixed(tu), 0.0f);
+    __syncthreads();
+    Breaks bk;
+    bk.L = L;
+    bk.bucket = (uint32_t)__cvta_generic_to_shared(bucket) - (0x4B000000u << 4);
+    bk.nf = nf;
+    bk.sp = (float)sp;
+    auto tan_of = [&](int j) { return __uint_as_float(K[j].x); };
+    const float tmax = nf > 0 ? tan_of(nf - 1) : 0.0f;
+    bk.inv = tmax > 0.0f ? 1.0f / tmax : 0.0f;
+    auto below = [&](float t) {
+        int c = 0;
+        for (int step = sp >> 1; step > 0; step >>= 1) c += tan_of(c + step - 1) < t ? step : 0;
+        return c;
+    };
+    bool crowded = false;
+    for (int b = threadIdx.x; b <= sp; b += blockDim.x) {
+        const float w0 = ((float)b - 0.5f) / bk.sp, w1 = ((float)b + 0.5f) / bk.sp;
+        const int k0 = below(tmax * (1.0f - w1 * w1)), k1 = b > 0 && tmax > 0.0f ? below(tmax * (1.0f - w0 * w0)) : nf;
+        const float2 l0 = L[k0], l1 = L[k1];
+        const bool simple = k1 - k0 <= 1 || tan_of(k1 - 1) - tan_of(k0) <= 2e-6f * tan_of(k1 - 1);
+        bucket[b] = simple ? make_float4(l0.x, l1.x, l0.y, l1.y)
+                           : make_float4(__int_as_float(0x7FFFFFFF), __int_as_float(k0), __int_as_float(k1), 0.0f);
+        crowded = crowded || !simple;
+    }
+    // (the rotations from shared memory: read through the global pointer they
+    // cost each vertex twelve loads, as its result might overwrite them)
+    __shared__ float4 s_rot[8];
+    if (threadIdx.x < a.n_rot && threadIdx.x < 16) reinterpret_cast<float2 *>(s_rot)[threadIdx.x] = a.rot[threadIdx.x];
+    bk.rot = s_rot;
+    bk.crowded = __syncthreads_or(crowded) != 0;
+    return bk;
+}
+
+// The year's sum of the factored days for one rotation pair of a = |U|, c =
+// |z|: the larger of the two lines of the bucket of a / c (ti = 1 / (c
+// tmax), rounded).
+template <bool CROWDED>
+__device__ __forceinline__ float pair_value(const Breaks &bk, float a, float c, float ti)
+{
+    // the bucket number, rounded to nearest, in the low bits of a binary32
+    const float w = approx_sqrt(__saturatef(fmaf(-a, ti, 1.0f)));
+    const uint32_t at = (__float_as_uint(fmaf(w, bk.sp, 8388608.0f)) << 4) + bk.bucket;
+    float4 e;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(e.x), "=f"(e.y), "=f"(e.z), "=f"(e.w) : "r"(at));
+    const float2 v2 = __ffma2_rn(make_float2(a, a), make_float2(e.x, e.y),
+                                 __fmul2_rn(make_float2(c, c), make_float2(e.z, e.w)));
+    float v = fmaxf(v2.x, v2.y);
+    if (CROWDED && e.x != e.x) {
+        const int k1 = __float_as_int(e.z);
+        v = 0.0f;
+        for (int k = __float_as_int(e.y); k <= k1; ++k) {
+            const float2 l = bk.L[k];
+            v = fmaxf(v, fmaf(a, l.x, c * l.y));
+        }
+    }
+    return v;
+}
+
+template <int HP, bool CROWDED>
+__device__ __forceinline__ float pair_sum(const Breaks &bk, float x, float y, float c, float ti)
+{
+    float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll
+    for (int h = 0; h < HP; h += 2) {
+        const float4 q = bk.rot[h / 2];
+        s0 += pair_value<CROWDED>(bk, fabsf(fmaf(x, q.x, -(y * q.y))), c, ti);
+        s1 += pair_value<CROWDED>(bk, fabsf(fmaf(x, q.z, -(y * q.w))), c, ti);
+    }
+    return s0 + s1;
+}
+
+// Arcs (HP = ARCS).  x cos(theta) - y sin(theta) = rho cos(theta + phi), phi
+// = atan2(y, x), so a tilt's terms max(k rho cos(theta + phi) + C, 0), k =
+// cos tau, are positive on the arc of half width acos(-C / (|k| rho)) about
+// -phi (about -phi + pi for k < 0), and their sum over it is k (x sum cos -
+// y sum sin) + C count: a difference of prefix sums of the rotations sorted
+// by angle.  A rotation put on the wrong side of an end of the arc by
+// rounding has a term of that rounding's size, so the searches need not be
+// exact.  Rotations come in any order; up to ARC_MAX of them.
+// Shared memory: the prefix sums P[n + 1] (exact sums rounded once), the
+// angles less the smallest one, ascending, an index F of NB = a power of two
+// >= n buckets (F[b] = angles below b 2 pi / NB), the rotations' order.
+// Measured (GB300, one tilt, 360 rotations): 110.8 -> 37.8 us for 2,500,002
+// vertices, 420 -> 111 us for 10,000,002 (2.5 TB/s of the 28 B per vertex;
+// instruction issue and the two gathers bound it).
+// From ARC_MIN rotations on, and only for ARC_VERTICES vertices or
+// ARC_TERMS positions: below 128 rotations the maxima are as fast or faster
+// (30 tilts of 48 rotations, 625,002 vertices: 113 us against 131 us by
+// arcs; of 96: 205 against 131 us, but 22.6 against 35 us for 9,002
+// vertices), and on a small sphere a block's sorting and prefix sums show
+// (128 rotations, 9,002 vertices: 6.3 against 8.3 us; 625,002: 14.5 us both).
+constexpr int ARCS = -1;
+constexpr int ARC_MIN = 128;
+constexpr int64_t ARC_VERTICES = 1 << 18;
+constexpr int ARC_TERMS = 360;
+constexpr int ARC_MAX = 1024;
+constexpr float TWO_PI = 6.28318531f;
+
+struct Arcs {
+    const float2 *P = nullptr;
+    const float *ang = nullptr;
+    const int *F = nullptr;
+    int n = 0, nb = 0;
+    float base = 0.0f, scale = 0.0f;
+};
+
+__host__ __device__ __forceinline__ size_t arc_smem(int n)
+{
+    return sizeof(float2) * ((size_t)n + 1) + sizeof(float) * (2 * (size_t)n + 1) + sizeof(int) * (size_t)(sort_pad(n) + n + 1);
+}
+
+__device__ __forceinline__ Arcs stage_arcs(const InsoArgs &a, void *smem)
+{
+    Arcs A;
+    const int n = a.pairs ? 2 * a.n_rot : a.n_rot, nb = sort_pad(n);
+    float2 *P = reinterpret_cast<float2 *>(smem);
+    float *ang = reinterpret_cast<float *>(P + n + 1), *raw = ang + n;
+    int *order = reinterpret_cast<int *>(raw + n + 1), *F = order + n;
+    auto rot = [&](int i) {
+        const float2 q = a.rot[i < a.n_rot ? i : i - a.n_rot];
+        return i < a.n_rot ? q : make_float2(-q.x, -q.y);
+    };
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const float2 q = rot(i);
+        raw[i] = atan2f(q.y, q.x);
+    }
+    __syncthreads();
+    bool ascending = true;
+    for (int i = threadIdx.x; i + 1 < n; i += blockDim.x) ascending = ascending && raw[i] <= raw[i + 1];
+    if (__syncthreads_and(ascending)) {
+        for (int i = threadIdx.x; i < n; i += blockDim.x) order[i] = i;
+    } else {
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            const float v = raw[i];
+            int rank = 0;
+            for (int j = 0; j < n; ++j) rank += raw[j] < v || (raw[j] == v && j < i) ? 1 : 0;
+            order[rank] = i;
+        }
+    }
+    __syncthreads();
+    const float base = raw[order[0]];
+    for (int i = threadIdx.x; i < n; i += blockDim.x) ang[i] = raw[order[i]] - base;
+    const int per = (n + (int)blockDim.x - 1) / (int)blockDim.x;
+    const int j0 = min(n, (int)threadIdx.x * per), j1 = min(n, j0 + per);
+    long long u = 0, v = 0, tu, tv;
+    for (int j = j0; j < j1; ++j) {
+        const float2 q = rot(order[j]);
+        u += to_fixed(q.x);
+        v += to_fixed(q.y);
+    }
+    block_scan2(u, v, tu, tv);
+    for (int j = j0; j < j1; ++j) {
+        const float2 q = rot(order[j]);
+        P[j] = make_float2(from_fixed(u), from_fixed(v));
+        u += to_fixed(q.x);
+        v += to_fixed(q.y);
+    }
+    if (threadIdx.x == 0) P[n] = make_float2(from_fixed(tu), from_fixed(tv));
+    __syncthreads();
+    for (int b = threadIdx.x; b <= nb; b += blockDim.x) {
+        const float edge = (float)b * (TWO_PI / (float)nb);
+        int lo = 0, hi = n;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (ang[mid] < edge) lo = mid + 1;
+            else hi = mid;
+        }
+        F[b] = lo;
+    }
+    __syncthreads();
+    A.P = P;
+    A.ang = ang;
+    A.F = F;
+    A.n = n;
+    A.nb = nb;
+    A.base = base;
+    A.scale = (float)nb / TWO_PI;
+    return A;
+}
+
+// How many of the sorted angles lie below v (0 <= v <= 2 pi).
+__device__ __forceinline__ int arc_find(const Arcs &A, float v)
+{
+    int c = A.F[min((int)(v * A.scale), A.nb)];
+    while (c < A.n && A.ang[c] < v) ++c;
+    return c;
+}
+
+__device__ __forceinline__ float arc_sum(const InsoArgs &a, const Arcs &A, float x, float y, float z)
+{
+    const float phi = atan2f(-y, x), rho = sqrtf(fmaf(x, x, y * y));
+    float tot = 0.0f, comp = 0.0f;          // Kahan over tilts
+    for (int d = 0; d < a.n_tilt; ++d) {
+        const float2 t = a.tilt[d];
+        const float C = z * t.y, den = fabsf(t.x) * rho;
+        float2 S = make_float2(0.0f, 0.0f);
+        int cnt = 0;
+        if (C >= den) {
+            S = A.P[A.n];
+            cnt = A.n;
+        } else if (C > -den) {
+            const float alpha = acosf(__fdividef(-C, den));
+            float a0 = (t.x < 0.0f ? phi + 0.5f * TWO_PI : phi) - alpha - A.base;
+            a0 -= TWO_PI * floorf(a0 * (1.0f / TWO_PI));
+            const float a1 = a0 + 2.0f * alpha;
+            const int lo = arc_find(A, a0), hi = arc_find(A, a1 < TWO_PI ? a1 : a1 - TWO_PI);
+            const float2 l = A.P[lo], h = A.P[hi];
+            S = make_float2(h.x - l.x, h.y - l.y);
+            cnt = hi - lo;
+            if (a1 >= TWO_PI) {
+                const float2 w = A.P[A.n];
+                S.x += w.x;
+                S.y += w.y;
+                cnt += A.n;
+            }
+        }
+        const float s = fmaxf(fmaf(t.x, fmaf(x, S.x, -(y * S.y)), C * (float)cnt), 0.0f);
+        const float yk = s - comp;
+        const float tk = tot + yk;
+        comp = (tk - tot) - yk;
+        tot = tk;
+    }
+    return tot;
+}
+
+template <int HP>
+__device__ __forceinline__ float inso_vertex(const InsoArgs &a, double X, double Y, double Z, double r, float r2h,
+                                             float r2l, float zmin, float inv_r, const float4 *tt = nullptr,
+                                             const Breaks &bk = Breaks(), const Arcs &arc = Arcs())
+{
+    float x, y, z;
+    const bool on_sphere = load_vertex(X, Y, Z, r, r2h, r2l, x, y, z);
+    if (HP == ARCS && on_sphere) return arc_sum(a, arc, x, y, z) * inv_r;
     float tot = 0.0f, comp = 0.0f;          // Kahan over tilts
     const int nr = HP > 0 ? HP : a.n_rot;
     if (on_sphere && HP > 0 && (HP & 1) == 0 && a.pairs) {
@@ -227,10 +564,12 @@ __device__ __forceinline__ float inso_vertex(const InsoArgs &a, double X, double
         // day costs a max and an add per rotation pair.  Days with |k| near 0
         // take the direct form.
         float au[HP > 0 ? HP : 2];
+        if (!tt || bk.nf < 0) {
 #pragma unroll
-        for (int h = 0; h < (HP > 0 ? HP : 2); ++h) {
-            const float2 q = a.rot[h];
-            au[h] = fabsf(fmaf(x, q.x, -(y * q.y)));
+            for (int h = 0; h < (HP > 0 ? HP : 2); ++h) {
+                const float2 q = a.rot[h];
+                au[h] = fabsf(fmaf(x, q.x, -(y * q.y)));
+            }
         }
         if (tt) {
             // constants staged by the block: per day a shared load, one
@@ -246,36 +585,11 @@ __device__ __forceinline__ float inso_vertex(const InsoArgs &a, double X, double
                 tot = tk;
             };
             if (bk.nf >= 0) {
-                // B_h = number of sorted days with tan_d < a_h / |z|
-                // (|z| = 0: every day for a_h > 0, none for a_h = 0)
-                const float iz = 1.0f / az;
-                float th[HP > 0 ? HP : 2];
-                int B[HP > 0 ? HP : 2];
-#pragma unroll
-                for (int h = 0; h < (HP > 0 ? HP : 2); ++h) {
-                    th[h] = au[h] > 0.0f ? au[h] * iz : 0.0f;
-                    B[h] = 0;
-                }
-#pragma unroll
-                for (int h = 0; h < (HP > 0 ? HP : 2); ++h) {
-                    if (th[h] > bk.tmax) {
-                        B[h] = bk.nf;
-                    } else {
-                        const int b = min((int)(th[h] * bk.scale), bk.sp - 1);
-                        int c = bk.F[b];
-                        while (c > 0 && !(bk.T[c - 1] < th[h])) --c;
-                        while (c < bk.nf && bk.T[c] < th[h]) ++c;
-                        B[h] = c;
-                    }
-                }
-                float s0 = 0.0f, s1 = 0.0f;
-#pragma unroll
-                for (int h = 0; h < (HP > 0 ? HP : 2); h += 2) {
-                    const int b0 = min(B[h], bk.nf), b1 = min(B[h + 1], bk.nf);
-                    s0 = fmaf(au[h], bk.P0[b0], fmaf(az, bk.Q1[b0], s0));
-                    s1 = fmaf(au[h + 1], bk.P0[b1], fmaf(az, bk.Q1[b1], s1));
-                }
-                tot = s0 + s1;
+                // each pair's line pair from its bucket of t = a_h / |z|
+                // (|z| kept off 0: 1e-20 r in its place changes no value)
+                const float ti = approx_rcp(fmaxf(az, zmin)) * bk.inv;
+                tot = (bk.crowded ? pair_sum<(HP > 0 ? HP : 2), true>(bk, x, y, az, ti)
+                                  : pair_sum<(HP > 0 ? HP : 2), false>(bk, x, y, az, ti));
             } else {
             auto day = [&](int d, float2 g) {
                 const float4 k = tt[d];
@@ -406,30 +720,37 @@ __device__ __forceinline__ Breaks stage_all(const InsoArgs &a, float4 *s_tilt)
     Breaks bk;
     stage_tilts<HP>(a, s_tilt);
     if (a.n_tilt <= SORT_MAX) {
-        float *base = reinterpret_cast<float *>(reinterpret_cast<int *>(s_tilt + a.n_tilt + 1) + a.n_tilt);
+        // 16-byte units: the bucket table first, then the lines, then the rest
         const int sp = sort_pad(a.n_tilt + 1);
-        float *T = base, *P0 = T + sp, *Q1 = P0 + a.n_tilt + 1, *CS = Q1 + a.n_tilt + 1;
-        int *F = reinterpret_cast<int *>(CS + a.n_tilt + 1);
-        bk.nf = stage_breakpoints(a, s_tilt, T, P0, Q1, CS, F, bk.scale, bk.tmax);
-        bk.sp = sort_pad(bk.nf + 1);
-        bk.F = F;
-        bk.T = T;
-        bk.P0 = P0;
-        bk.Q1 = Q1;
+        float4 *bucket = s_tilt + a.n_tilt + 1 + (a.n_tilt + 3) / 4;
+        float2 *L = reinterpret_cast<float2 *>(bucket + sp + 1);
+        uint2 *K = reinterpret_cast<uint2 *>(L + a.n_tilt + 1);
+        bk = stage_breakpoints(a, s_tilt, K, L, bucket);
     }
     return bk;
 }
 
 template <int HP>
-__global__ void __launch_bounds__(256, 3) insolation_kernel(InsoArgs a)
+__global__ void __launch_bounds__(256, 4) insolation_kernel(InsoArgs a)
 {
     extern __shared__ float4 s_tilt[];
     const bool staged = HP > 0 && a.pairs && a.n_tilt <= TILT_STAGE_MAX;
     Breaks bk;
+    Arcs arc;
     if (staged) bk = stage_all<HP>(a, s_tilt);
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += (int64_t)gridDim.x * blockDim.x) {
-        float tot = inso_vertex<HP>(a, a.xyz[3 * i], a.xyz[3 * i + 1], a.xyz[3 * i + 2], a.r, a.inv_r,
-                                    staged ? s_tilt : nullptr, bk);
+    if (HP == ARCS) arc = stage_arcs(a, s_tilt);
+    // the next vertex is read while this one is summed (32 warps' 768 bytes
+    // each are too few in flight per SM for the memory's latency)
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    double X = 0.0, Y = 0.0, Z = 0.0;
+    if (i < a.n) { X = a.xyz[3 * i]; Y = a.xyz[3 * i + 1]; Z = a.xyz[3 * i + 2]; }
+    for (; i < a.n; i += step) {
+        const double cx = X, cy = Y, cz = Z;
+        const int64_t j = i + step;
+        if (j < a.n) { X = a.xyz[3 * j]; Y = a.xyz[3 * j + 1]; Z = a.xyz[3 * j + 2]; }
+        const float tot = inso_vertex<HP>(a, cx, cy, cz, a.r, a.r2h, a.r2l, a.zmin, a.inv_r, staged ? s_tilt : nullptr,
+                                          bk, arc);
         a.out[i] = a.accumulate ? a.out[i] + tot : tot;
     }
 }
@@ -443,21 +764,32 @@ __global__ void __launch_bounds__(256, 3) insolation_batch_kernel(InsoArgs a, co
     extern __shared__ float4 s_tilt[];
     const bool staged = HP > 0 && a.pairs && a.n_tilt <= TILT_STAGE_MAX;
     Breaks bk;
+    Arcs arc;
     if (staged) bk = stage_all<HP>(a, s_tilt);
+    if (HP == ARCS) arc = stage_arcs(a, s_tilt);
+    // rows only go up: walk to the next planet, and form a planet's radius
+    // constants (binary64) once
+    int p = -1;
+    int64_t beg = 0, next = 0;
+    double r = 1.0;
+    float r2h = 0.0f, r2l = 0.0f, zmin = 0.0f, inv_r = 1.0f;
     for (int64_t blk = blockIdx.x; blk * 256 < total_rows; blk += gridDim.x) {
-        const int64_t row = blk * 256 + threadIdx.x;
-        int lo = 0, hi = np - 1;
-        while (lo < hi) {
-            int mid = (lo + hi + 1) >> 1;
-            if (P[mid].vbeg <= blk * 256) lo = mid; else hi = mid - 1;
+        if (p < 0 || blk * 256 >= next) {
+            do {
+                ++p;
+                next = p + 1 < np ? P[p + 1].vbeg : INT64_MAX;
+            } while (blk * 256 >= next);
+            beg = P[p].vbeg;
+            r = P[p].radius;
+            radius_pair(r, r2h, r2l);
+            inv_r = (float)(1.0 / r);
+            zmin = (float)(1e-20 * r);
         }
-        const nx_inso_planet &pl = P[lo];
-        const int64_t i = row - pl.vbeg;
-        if (i < 0 || i >= pl.n) continue;
-        const double r = pl.radius;
-        float tot = inso_vertex<HP>(a, pl.xyz[3 * i], pl.xyz[3 * i + 1], pl.xyz[3 * i + 2], r, (float)(1.0 / r),
-                                    staged ? s_tilt : nullptr, bk);
-        a.out[row] = tot;
+        const int64_t i = blk * 256 + threadIdx.x - beg;
+        if (i < 0 || i >= P[p].n) continue;
+        const double *xyz = P[p].xyz;
+        a.out[beg + i] = inso_vertex<HP>(a, xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], r, r2h, r2l, zmin, inv_r,
+                                         staged ? s_tilt : nullptr, bk, arc);
     }
 }
 
@@ -590,9 +922,10 @@ size_t tilt_smem(const InsoArgs &a)
 {
     if (!a.pairs || a.n_tilt > TILT_STAGE_MAX) return 0;
     size_t b = sizeof(float4) * ((size_t)a.n_tilt + 1) + sizeof(int) * (size_t)a.n_tilt;
-    if (a.n_tilt <= SORT_MAX)      // T (padded), P0, Q1, the sorted cosines, the bucket index
-        b += sizeof(float) * ((size_t)sort_pad(a.n_tilt + 1) + 3 * ((size_t)a.n_tilt + 1)) +
-             sizeof(int) * ((size_t)sort_pad(a.n_tilt + 1) + 1);
+    if (a.n_tilt <= SORT_MAX) {    // the list rounded to 16 bytes, bucket table, lines, sorted days
+        const size_t sp = (size_t)sort_pad(a.n_tilt + 1), nt = (size_t)a.n_tilt;
+        b = sizeof(float4) * (nt + 1 + (nt + 3) / 4 + sp + 1) + sizeof(float2) * (nt + 1 + sp);
+    }
     return b;
 }
 
@@ -605,11 +938,18 @@ int grid_for(int64_t n, int per_sm = 8)
 }
 
 // Blocks of a 12-pair launch: a block that sums by breakpoints sorts the
-// schedule first, so the grid is the resident blocks (3 per SM) and each
+// schedule first, so the grid is the resident blocks (4 per SM) and each
 // block takes many vertices.
 int grid_staged(int64_t n, const InsoArgs &a)
 {
-    return grid_for(n, a.pairs && a.n_tilt <= SORT_MAX ? 3 : 8);
+    return grid_for(n, a.pairs && a.n_tilt <= SORT_MAX ? 4 : 8);
+}
+
+// Whether a schedule is summed by arcs.
+bool use_arcs(const InsoArgs &a, int64_t vertices)
+{
+    const int n = a.pairs ? 2 * a.n_rot : a.n_rot;
+    return n >= ARC_MIN && n <= ARC_MAX && (vertices >= ARC_VERTICES || n * a.n_tilt >= ARC_TERMS);
 }
 
 }  // namespace
@@ -665,6 +1005,8 @@ NX_EXPORT int nx_insolation(const double *xyz_dev, int64_t n, double radius, con
     a.n = n;
     a.r = radius;
     a.inv_r = (float)(1.0 / radius);
+    radius_pair(radius, a.r2h, a.r2l);
+    a.zmin = (float)(1e-20 * radius);
     a.rot = (const float2 *)table_dev;
     a.n_rot = n_rot_entries;
     a.pairs = pairs ? 1 : 0;
@@ -674,6 +1016,8 @@ NX_EXPORT int nx_insolation(const double *xyz_dev, int64_t n, double radius, con
     a.accumulate = accumulate;
     if (a.pairs && n_rot_entries == 12)
         insolation_kernel<12><<<grid_staged(n, a), 256, tilt_smem(a), s>>>(a);
+    else if (use_arcs(a, n))
+        insolation_kernel<ARCS><<<grid_for(n, 4), 256, arc_smem(a.pairs ? 2 * a.n_rot : a.n_rot), s>>>(a);
     else
         insolation_kernel<0><<<grid_for(n), 256, 0, s>>>(a);
     NX_CHECK_LAUNCH("insolation_kernel");
@@ -700,6 +1044,7 @@ NX_EXPORT int nx_insolation_batch(const nx_inso_planet *planets_dev, const nx_in
     a.n = 0;
     a.r = 1.0;
     a.inv_r = 1.0f;
+    a.r2h = a.r2l = a.zmin = 0.0f;
     a.rot = (const float2 *)table_dev;
     a.n_rot = n_rot_entries;
     a.pairs = pairs ? 1 : 0;
@@ -708,11 +1053,13 @@ NX_EXPORT int nx_insolation_batch(const nx_inso_planet *planets_dev, const nx_in
     a.out = out_dev;
     a.accumulate = 0;
     cudaStream_t s = (cudaStream_t)stream;
-    int grid = a.pairs && n_rot_entries == 12 ? grid_staged(total, a) : grid_for(total);
     if (a.pairs && n_rot_entries == 12)
-        insolation_batch_kernel<12><<<grid, 256, tilt_smem(a), s>>>(a, planets_dev, nplanets, total);
+        insolation_batch_kernel<12><<<grid_staged(total, a), 256, tilt_smem(a), s>>>(a, planets_dev, nplanets, total);
+    else if (use_arcs(a, total))
+        insolation_batch_kernel<ARCS><<<grid_for(total, 4), 256, arc_smem(a.pairs ? 2 * a.n_rot : a.n_rot), s>>>(
+            a, planets_dev, nplanets, total);
     else
-        insolation_batch_kernel<0><<<grid, 256, 0, s>>>(a, planets_dev, nplanets, total);
+        insolation_batch_kernel<0><<<grid_for(total), 256, 0, s>>>(a, planets_dev, nplanets, total);
     NX_CHECK_LAUNCH("insolation_batch_kernel");
     nx::note_launch(1);
     return NX_OK;

@@ -1,0 +1,58 @@
+"""Insolation schedules summed by arcs and by breakpoints, against the terms summed one by one in binary64.
+
+Tolerance (stated): 2e-6 of the largest sum.  By arcs a tilt's sum over n rotations is a difference of prefix sums of up
+to n/pi, each rounded once (4 roundings of 2^-25), three products (2^-24 each) and at most one rotation misplaced at
+either end of the arc, whose term is then within 1e-6 of 0; by breakpoints the lines' sums are rounded once and 12 values
+of a few roundings each are added.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROTATIONS = {
+    "degrees": [-180.0 + i for i in range(360)],                            # pairs, ascending
+    "shuffled": list(np.random.default_rng(1).permutation(360) - 180.0),
+    "uneven": list(np.random.default_rng(2).uniform(-400.0, 400.0, 129)),   # no pairs, beyond one turn
+    "most": [-90.0 + 0.3515625 * i for i in range(1024)],
+    "hourly": [-180.0 + 15.0 * i for i in range(24)],                       # by breakpoints
+}
+
+
+@pytest.mark.parametrize("tilts", [[0.0], [23.44, -7.5, 90.0, 135.0, 10.0]])
+@pytest.mark.parametrize("name", list(ROTATIONS))
+@pytest.mark.parametrize("radius", [1.0, 6378100.0])
+def test_sums_equal_the_terms_in_binary64(name, tilts, radius):
+    import torch
+    from nixis_gb300 import climate, mesh
+    xyz = mesh.icosphere(17, with_tris=False)[0]
+    poles = torch.tensor([[0, 0, 1], [0, 0, -1], [1, 0, 0], [0, -1, 0], [1e-13, 0, 1]], dtype=torch.float64, device="cuda")
+    xyz = torch.cat([xyz, poles / poles.norm(dim=1, keepdim=True)]) * radius
+    if name == "uneven" and len(tilts) == 1:
+        tilts = tilts * 3
+    got = climate.insolation_sum(xyz, radius, ROTATIONS[name], tilts).double()
+    rot, tilt = (torch.deg2rad(torch.tensor(v, dtype=torch.float64, device="cuda")) for v in (ROTATIONS[name], tilts))
+    want = torch.zeros_like(got)
+    x, y, z = (xyz / radius).unbind(1)
+    for t in tilt:
+        u = x[:, None] * torch.cos(rot) - y[:, None] * torch.sin(rot)
+        want += (u * torch.cos(t) + (z * torch.sin(t))[:, None]).clamp(min=0.0).sum(1)
+    assert (got - want).abs().max() <= 2e-6 * want.max()
+
+
+def test_large_sphere_and_batch_rows_take_the_same_values():
+    import torch
+    from nixis_gb300 import climate, mesh
+    from nixis_gb300.planets import PlanetBatch, PlanetRequest
+    m = mesh.PlanetMesh(170)                                                # over 2^18 vertices: one tilt by arcs
+    rot = [-180.0 + 2.0 * i for i in range(180)]
+    one = climate.insolation_sum(m.xyz, 1.0, rot, [12.0])
+    part = climate.insolation_sum(m.xyz[:5000], 1.0, rot, [12.0])           # rotation by rotation
+    assert (one[:5000] - part).abs().max() <= 2e-6 * one.max()
+    reqs = [PlanetRequest(seed=1, divisions=k, octaves=2, insolation=True, days=3, hours=h) for k, h in ((9, 360), (14, 360), (11, 24))]
+    b = PlanetBatch(reqs)
+    b.run()
+    for r, got in zip(reqs, b.results()):
+        rot, tilts = climate.annual_schedule(r.axial_tilt, r.days, r.days, r.hours)
+        want = climate.insolation_sum(mesh.PlanetMesh(r.divisions).xyz, 1.0, rot, tilts) * (climate.SOLAR_CONSTANT / (r.days * r.hours))
+        assert torch.equal(got.insolation, want)
