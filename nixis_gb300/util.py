@@ -110,7 +110,7 @@ def make_bool_elevation_mask(height, mask_elevation, stream=None):
     n = hd.numel()
     m = torch.empty(n, dtype=torch.uint8, device="cuda")
     call("nx_elevation_mask", _dev.ptr(hd), n, float(mask_elevation), _dev.ptr(m), _dev.stream_handle(stream))
-    return m.cpu().numpy().astype(bool) if host else m.bool()
+    return m.cpu().numpy().view(bool) if host else m.view(torch.bool)
 
 
 def shape_heights(height, min_alt=-4000.0, max_alt=8850.0, ocean_percent=55.0, stream=None):
@@ -129,8 +129,8 @@ def shape_heights(height, min_alt=-4000.0, max_alt=8850.0, ocean_percent=55.0, s
     call("nx_shape_heights", _dev.ptr(hd), n, float(min_alt), float(max_alt), float(ocean_percent), _dev.ptr(out),
          _dev.ptr(tmp), _dev.ptr(mask), _dev.ptr(level), _dev.ptr(ws), ws.numel(), _dev.stream_handle(stream))
     if host:
-        return out.cpu().numpy(), mask.cpu().numpy().astype(bool), float(level.item())
-    return out, mask.bool(), level
+        return out.cpu().numpy(), mask.cpu().numpy().view(bool), float(level.item())
+    return out, mask.view(torch.bool), level
 
 
 # ---------------------------------------------------------------------------
