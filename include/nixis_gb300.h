@@ -173,6 +173,12 @@ int nx_icosphere_tables(const double *corners, const int32_t *faces, const int32
  * NULL).  Corners are vertices 0-11; layout in nixis_gb300/icosphere.py. */
 int nx_icosphere(int k, double *xyz_dev, int32_t *tris_dev, void *stream);
 
+/* The icosphere's own neighbour rows (the table that nx_build_adjacency and
+ * nx_sort_adjacency give for its triangles) in nbr_dev, (10 k^2 + 2) x 6
+ * int32, without its triangles; k >= 2.  With edge_dev also the edge length
+ * pairs (as nx_edge_lengths) of the vertices xyz_dev. */
+int nx_icosphere_rows(int k, const double *xyz_dev, int32_t *nbr_dev, float *edge_dev, void *stream);
+
 /* Workspace bytes for nx_build_adjacency. */
 size_t nx_adjacency_workspace_size(int64_t nv);
 

@@ -95,8 +95,37 @@ __device__ __forceinline__ bool settle(unsigned long long &g, float h, float c, 
     return ok;
 }
 
-__device__ __noinline__ double div_slow(double a, double b) { return __ddiv_rn(a, b); }
-__device__ __noinline__ double sqrt_slow(double s) { return __dsqrt_rn(s); }
+// a * w, rounded to nearest even, for an integer 0 <= w < 2^31 and |a| in
+// [2^-900, 2^900] or 0: the product of the 53-bit significand and w as an
+// integer of at most 84 bits, rounded by hand (a binary64 product costs as
+// many issue slots as three of these).
+__device__ __forceinline__ double times(double a, int w)
+{
+    const uint2 x = words(a);
+    const uint32_t sign = x.y & 0x80000000u;
+    if (w == 0 || ((x.y << 1) | x.x) == 0u) return __hiloint2double((int)sign, 0);
+    const unsigned long long lo = (unsigned long long)x.x * (uint32_t)w;
+    const unsigned long long hi = (unsigned long long)((x.y & 0xFFFFFu) | 0x100000u) * (uint32_t)w + (lo >> 32);
+    // p = hi : low word of lo, with its top bit at 52 + d, d = that of w (or one more)
+    const int d = 43 - __clzll((long long)hi);              // shift of the significand, 0 .. 31
+    const uint32_t l = (uint32_t)lo;
+    unsigned long long m;
+    if (d == 0) {
+        m = (hi << 32) | l;
+    } else {
+        m = (hi << (32 - d)) | (l >> d);
+        const uint32_t rest = l << (32 - d);
+        m += rest > 0x80000000u || (rest == 0x80000000u && (m & 1ull)) ? 1ull : 0ull;
+    }
+    // (the implicit bit adds 1 to the exponent field; a carry out of the
+    // rounding adds one more)
+    const uint32_t e = ((x.y >> 20) & 0x7FFu) + (uint32_t)d - 1u;
+    const unsigned long long b = m + ((unsigned long long)e << 52);
+    return __longlong_as_double((long long)(b | ((unsigned long long)sign << 32)));
+}
+
+static __device__ __noinline__ double div_slow(double a, double b) { return __ddiv_rn(a, b); }
+static __device__ __noinline__ double sqrt_slow(double s) { return __dsqrt_rn(s); }
 
 // 1 / b as a pair y1 + y2 (relative error below 2^-44); y1 = 0 for b outside
 // [2^-28, 2^28).

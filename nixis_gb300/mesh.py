@@ -121,32 +121,35 @@ def edge_lengths(xyz, nbr, stream=None):
 
 class PlanetMesh:
     """A subdivision's resident mesh: xyz float64 (N,3), nbr int32 (N,6),
-    edge float32 (N,6,2) pairs; triangles are dropped after the adjacency is
-    built.  With defer_checks the build only enqueues work on the stream
+    edge float32 (N,6,2) pairs.  With defer_checks the build only enqueues work on the stream
     (no host wait); check() reads the error flags later."""
 
     def __init__(self, divisions, stream=None, defer_checks=False):
         self.k = ico.check_divisions(divisions)
         self.n = ico.counts(self.k)[0]
         s = stream if stream is not None else torch.cuda.current_stream()
-        xyz, tris = icosphere(self.k, stream=stream)
+        # (one division: the twelve corners' rows need the general functions)
+        xyz, tris = icosphere(self.k, with_tris=self.k < 2, stream=stream)
         # the vertices alone are ready here (work that needs only them, like
         # the noise, can start on another stream while the rest is built)
         self.xyz_ready = torch.cuda.Event()
         self.xyz_ready.record(s)
-        adj, aerr = _adjacency(tris, stream)
-        del tris
-        nbr = torch.empty_like(adj)
-        call("nx_sort_adjacency", _dev.ptr(adj), _dev.ptr(nbr), self.n, _dev.stream_handle(stream))
-        del adj
         self.xyz = xyz
-        self.nbr = nbr
-        self.edge, eerr = edge_lengths(xyz, nbr, stream=stream)
+        if tris is None:
+            self.nbr = torch.empty((self.n, 6), dtype=torch.int32, device="cuda")
+            self.edge = torch.empty((self.n, 6, 2), dtype=torch.float32, device="cuda")
+            call("nx_icosphere_rows", self.k, _dev.ptr(xyz), _dev.ptr(self.nbr), _dev.ptr(self.edge), _dev.stream_handle(stream))
+            self._errs = None
+        else:
+            adj, aerr = _adjacency(tris, stream)
+            self.nbr = torch.empty_like(adj)
+            call("nx_sort_adjacency", _dev.ptr(adj), _dev.ptr(self.nbr), self.n, _dev.stream_handle(stream))
+            self.edge, eerr = edge_lengths(xyz, self.nbr, stream=stream)
+            self._errs = (aerr, eerr)
         # the whole mesh is ready here (an event of its own, so a later user
         # need not wait for whatever else its stream has queued since)
         self.built = torch.cuda.Event()
         self.built.record(s)
-        self._errs = (aerr, eerr)
         self._tilings = {}
         if not defer_checks:
             self.check()

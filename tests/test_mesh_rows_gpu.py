@@ -1,0 +1,56 @@
+"""The icosphere's vertices, neighbour rows and edge lengths made directly, bit for bit against the general functions
+(adjacency of its triangles) and the oracle."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 7, 33, 64, 129])
+def test_rows_equal_the_adjacency_of_the_triangles(k):
+    import torch
+    from nixis_gb300 import mesh
+    m = mesh.PlanetMesh(k)
+    xyz, tris = mesh.icosphere(k)
+    nbr = mesh.sort_adjacency(mesh.build_adjacency(tris))
+    assert torch.equal(m.xyz.view(torch.int64), xyz.view(torch.int64))
+    assert torch.equal(m.nbr, nbr)
+    edge, err = mesh.edge_lengths(xyz, nbr)
+    assert int(err.item()) == 0 and torch.equal(m.edge, edge)
+
+
+@pytest.mark.parametrize("k", [257, 640])
+def test_large_meshes_equal_the_oracle(k):
+    from nixis_gb300 import mesh
+    m = mesh.PlanetMesh(k)
+    pts, tris = O.icosphere(k)
+    adj = O.build_adjacency(tris)
+    O.sort_adjacency(adj)
+    assert np.array_equal(m.xyz.cpu().numpy().view(np.uint64), pts.view(np.uint64))
+    assert np.array_equal(m.nbr.cpu().numpy(), adj)
+    e = pts[adj.clip(0)] - pts[:, None, :]
+    d = np.sqrt((e[..., 0] * e[..., 0] + e[..., 1] * e[..., 1]) + e[..., 2] * e[..., 2]) * (adj >= 0)
+    hi = d.astype(np.float32)
+    got = m.edge.cpu().numpy()
+    assert np.array_equal(got[..., 0], hi) and np.array_equal(got[..., 1], (d - hi).astype(np.float32))
+
+
+def test_scaled_and_shuffled_vertices_have_exact_lengths():
+    """Edge lengths of radii and orders that no icosphere here has: the binary64 lengths' pairs exactly."""
+    import torch
+    from nixis_gb300 import mesh
+    rng = np.random.default_rng(4)
+    m = mesh.PlanetMesh(24)
+    for radius in (6378100.0, 1e-7, 3e11, 1e25):
+        perm = torch.from_numpy(rng.permutation(m.n)).cuda()
+        inv = torch.empty_like(perm)
+        inv[perm] = torch.arange(m.n, device="cuda")
+        xyz = (m.xyz * radius)[perm]
+        nbr = torch.where(m.nbr[perm] >= 0, inv[m.nbr[perm].clamp(min=0).long()].int(), m.nbr[perm]).int()
+        e = xyz[nbr.clamp(min=0).long()] - xyz[:, None, :]
+        d = torch.sqrt((e[..., 0] * e[..., 0] + e[..., 1] * e[..., 1]) + e[..., 2] * e[..., 2]) * (nbr >= 0)
+        edge, _ = mesh.edge_lengths(xyz, nbr)
+        hi = d.float()
+        assert torch.equal(edge[..., 0], hi) and torch.equal(edge[..., 1], (d - hi.double()).float())
