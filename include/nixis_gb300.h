@@ -175,9 +175,20 @@ int nx_icosphere(int k, double *xyz_dev, int32_t *tris_dev, void *stream);
 
 /* The icosphere's own neighbour rows (the table that nx_build_adjacency and
  * nx_sort_adjacency give for its triangles) in nbr_dev, (10 k^2 + 2) x 6
- * int32, without its triangles; k >= 2.  With edge_dev also the edge length
- * pairs (as nx_edge_lengths) of the vertices xyz_dev. */
-int nx_icosphere_rows(int k, const double *xyz_dev, int32_t *nbr_dev, float *edge_dev, void *stream);
+ * int32, without its triangles; k >= 2. */
+int nx_icosphere_rows(int k, int32_t *nbr_dev, void *stream);
+
+/* Sets *differ_dev (device int, caller zeroes it) to 1 if a row of a
+ * face-interior vertex in nbr_dev is not the icosphere's own. */
+int nx_icosphere_like(int k, const int32_t *nbr_dev, int *differ_dev, void *stream);
+
+/* Edge length pairs (as nx_edge_lengths) for a table whose face-interior rows
+ * are the icosphere's own, each distance computed once; the vertices may be
+ * any.  info_dev (may be NULL; two device ints, caller zeroes them) gets bit 0
+ * of the first for an id outside [-1, nv), the longest length's binary32 bits
+ * in the second. */
+int nx_icosphere_edges(int k, const double *xyz_dev, const int32_t *nbr_dev, float *edge_dev, int *info_dev,
+                       void *stream);
 
 /* Workspace bytes for nx_build_adjacency. */
 size_t nx_adjacency_workspace_size(int64_t nv);

@@ -26,7 +26,9 @@ SIGNATURES = {
     "nx_noise3d_trace": (_i32, [_p, _i64, _p, _p, _d, _p, _p, _p, _p, _p]),
     "nx_icosphere_tables": (_i32, [_p, _p, _p, _p]),
     "nx_icosphere": (_i32, [_i32, _p, _p, _p]),
-    "nx_icosphere_rows": (_i32, [_i32, _p, _p, _p, _p]),
+    "nx_icosphere_rows": (_i32, [_i32, _p, _p]),
+    "nx_icosphere_like": (_i32, [_i32, _p, _p, _p]),
+    "nx_icosphere_edges": (_i32, [_i32, _p, _p, _p, _p, _p]),
     "nx_adjacency_workspace_size": (ctypes.c_size_t, [_i64]),
     "nx_build_adjacency": (_i32, [_p, _i64, _i64, _p, _p, ctypes.c_size_t, _p, _p]),
     "nx_sort_adjacency": (_i32, [_p, _p, _i64, _p]),

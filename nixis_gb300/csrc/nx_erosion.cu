@@ -29,6 +29,7 @@
 // that prefix.  Each planet alternates its two buffers so that its last
 // iteration writes buffer 0.
 #include "nx_common.cuh"
+#include "nx_f64.cuh"
 
 #include <mutex>
 
@@ -752,17 +753,32 @@ __global__ void erosion_rebase_kernel(const nx_erosion_planet *__restrict__ P, i
 __global__ void erosion_maxabs64_kernel(const double *__restrict__ h, const double *__restrict__ w,
                                         const double *__restrict__ s, int64_t n, unsigned long long *__restrict__ mbits)
 {
-    double m = 0.0;
+    // magnitudes compared as integers, NaN left out as fmax leaves it out
+    unsigned long long m = 0;
+    auto take = [&](double v) {
+        const unsigned long long b = nxf::bits(v) & 0x7FFFFFFFFFFFFFFFull;
+        m = b > m && b <= 0x7FF0000000000000ull ? b : m;
+    };
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double a = fabs(h[i]);
-        if (w) a = fmax(a, fabs(w[i]));
-        if (s) a = fmax(a, fabs(s[i]));
-        m = fmax(m, a);
+        take(h[i]);
+        if (w) take(w[i]);
+        if (s) take(s[i]);
     }
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(mbits, (unsigned long long)__double_as_longlong(m));
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long b = __shfl_xor_sync(0xFFFFFFFFu, m, o);
+        m = b > m ? b : m;
+    }
+    if ((threadIdx.x & 31) == 0) atomicMax(mbits, m);
 }
 
+// v * 2^-K as a pair: for K = 0, the common case, without the binary64 pipe
+// (nx_f64.cuh).
+__device__ __forceinline__ float2 scaled_pair(double v, int K)
+{
+    return K == 0 ? nxf::pair(v) : nxf::pair(ldexp(v, -K));
+}
+
+// Measured (GB300, 10,000,002 heights): 154 -> 78 us (400 MB).
 __global__ void erosion_load64_kernel(const double *__restrict__ h, const double *__restrict__ w,
                                       const double *__restrict__ s, int64_t n, const unsigned long long *__restrict__ mbits,
                                       float4 *__restrict__ st, nx_erosion_ctl *__restrict__ ctl)
@@ -770,11 +786,11 @@ __global__ void erosion_load64_kernel(const double *__restrict__ h, const double
     double m = __longlong_as_double((long long)*mbits);
     int K = 0;
     if (m > 0x1p64) K = ilogb(m) - 64;
+    const float2 none = make_float2(0.0f, 0.0f);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double hv = ldexp(h[i], -K), wv = w ? ldexp(w[i], -K) : 0.0, sv = s ? ldexp(s[i], -K) : 0.0;
-        const float hh = (float)hv, wh = (float)wv, sh = (float)sv;
-        st[2 * i] = make_float4(hh, (float)(hv - (double)hh), wh, (float)(wv - (double)wh));
-        st[2 * i + 1] = make_float4(sh, (float)(sv - (double)sh), 0.0f, 0.0f);
+        const float2 hp = scaled_pair(h[i], K), wp = w ? scaled_pair(w[i], K) : none, sp = s ? scaled_pair(s[i], K) : none;
+        st[2 * i] = make_float4(hp.x, hp.y, wp.x, wp.y);
+        st[2 * i + 1] = make_float4(sp.x, sp.y, 0.0f, 0.0f);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         float mf = (float)ldexp(m, -K);
@@ -788,15 +804,26 @@ __global__ void erosion_load64_kernel(const double *__restrict__ h, const double
     }
 }
 
+// (hi + lo) * 2^K: both parts scaled by integer operations (f32_scaled), one
+// binary64 sum; the same bits as scaling the sum.
 __global__ void erosion_store64_kernel(const float4 *__restrict__ st, int64_t n, const nx_erosion_ctl *__restrict__ ctl,
                                        double *__restrict__ h, double *__restrict__ w, double *__restrict__ so)
 {
     const int K = ctl->K[0];
+    auto value = [&](float a, float b) {
+        // a result below 2^-968 would be rounded twice: scaled as a whole
+        const int e = (int)((__float_as_uint(a) >> 23) & 0xFFu) - 127 + K;
+        if (e > -900 && e < 1000) return __dadd_rn(f32_scaled(a, K), b == 0.0f ? 0.0 : f32_scaled(b, K));
+        return ldexp((double)a + (double)b, K);
+    };
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float4 v = st[2 * i], b = st[2 * i + 1];
-        h[i] = ldexp((double)v.x + (double)v.y, K);
-        if (w) w[i] = ldexp((double)v.z + (double)v.w, K);
-        if (so) so[i] = ldexp((double)b.x + (double)b.y, K);
+        const float4 v = st[2 * i];
+        h[i] = value(v.x, v.y);
+        if (w) w[i] = value(v.z, v.w);
+        if (so) {
+            const float2 b = reinterpret_cast<const float2 *>(st + 2 * i + 1)[0];
+            so[i] = value(b.x, b.y);
+        }
     }
 }
 

@@ -192,19 +192,19 @@ __device__ __forceinline__ double sqrt(double s)
     return sqrt_slow(s);
 }
 
-// d as a pair hi + lo of binary32s, both rounded to nearest (d > 0 in
-// [2^-60, 2^60), else by conversion): hi by integer rounding of the top 24
-// bits, lo = the rest, an integer of at most 29 bits times its last place.
+// d as a pair hi + lo of binary32s, both rounded to nearest (|d| in [2^-60,
+// 2^60), else by conversion): hi by integer rounding of the top 24 bits, lo =
+// the rest, an integer of at most 29 bits times its last place.
 __device__ __forceinline__ float2 pair(double d)
 {
     const uint2 w = words(d);
-    const uint32_t hw = w.y, lw = w.x;
+    const uint32_t sign = w.y & 0x80000000u, hw = w.y & 0x7FFFFFFFu, lw = w.x;
     if (hw - (963u << 20) < (120u << 20)) {
         const uint32_t t = __funnelshift_l(lw, hw - (896u << 20), 3), rem = lw & 0x1FFFFFFFu;
         const bool up = rem > 0x10000000u || (rem == 0x10000000u && (t & 1u));
         const int r = up ? (int)rem - 0x20000000 : (int)rem;
-        return make_float2(__uint_as_float(t + (up ? 1u : 0u)),
-                           __fmul_rn(__int2float_rn(r), __uint_as_float((((hw >> 20) & 0x7FFu) - 948u) << 23)));
+        return make_float2(__uint_as_float((t + (up ? 1u : 0u)) | sign),
+                           __fmul_rn(__int2float_rn(sign ? -r : r), __uint_as_float((((hw >> 20) & 0x7FFu) - 948u) << 23)));
     }
     const float h = (float)d;
     return make_float2(h, (float)(d - (double)h));

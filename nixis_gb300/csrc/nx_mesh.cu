@@ -451,14 +451,20 @@ __global__ void __launch_bounds__(256) ico_neighbours_kernel(int k, int64_t nv, 
 // 359 us, against ~880 us for the general pair of passes before (the binary64
 // operations alone take 227 us).
 __global__ void __launch_bounds__(256) ico_edges_kernel(int k, int64_t nv, const double *__restrict__ xyz,
-                                                        const int32_t *__restrict__ nbr, float2 *__restrict__ el)
+                                                        const int32_t *__restrict__ nbr, float2 *__restrict__ el,
+                                                        int *__restrict__ info)
 {
     const int64_t inner = 12 + (int64_t)30 * (k - 1);
+    float longest = 0.0f;
     for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += (int64_t)gridDim.x * blockDim.x) {
         if (v < inner) {
             for (int s = 0; s < 6; ++s) {
                 const int32_t j = nbr[6 * v + s];
-                el[6 * v + s] = j >= 0 ? edge_pair(edge_len(xyz, v, j)) : make_float2(0.0f, 0.0f);
+                const bool on = j >= 0 && (int64_t)j < nv;
+                if (!on && j != -1 && info) atomicOr(info, 1);
+                const float2 d = on ? edge_pair(edge_len(xyz, v, j)) : make_float2(0.0f, 0.0f);
+                longest = fmaxf(longest, d.x);
+                el[6 * v + s] = d;
             }
             continue;
         }
@@ -469,6 +475,7 @@ __global__ void __launch_bounds__(256) ico_edges_kernel(int k, int64_t nv, const
 #pragma unroll
         for (int s = 2; s < 5; ++s) {
             const float2 d = edge_pair(edge_len(xyz, v, row[s]));
+            longest = fmaxf(longest, d.x);
             el[6 * v + s] = d;
             if (in & (1u << s)) el[6 * (int64_t)row[s] + (s + 3) % 6] = d;
         }
@@ -478,6 +485,27 @@ __global__ void __launch_bounds__(256) ico_edges_kernel(int k, int64_t nv, const
             if (!(in & 32u)) el[6 * v + 5] = edge_pair(edge_len(xyz, v, row[5]));
         }
     }
+    if (!info) return;
+    for (int o = 16; o > 0; o >>= 1) longest = fmaxf(longest, __shfl_xor_sync(0xFFFFFFFFu, longest, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(info + 1, __float_as_int(longest));     // (not negative: ordered as integers)
+}
+
+// Whether a table's rows of face-interior vertices are the icosphere's own
+// (differ: set to 1 where not).
+__global__ void __launch_bounds__(256) ico_like_kernel(int k, int64_t nv, const int32_t *__restrict__ nbr, int *__restrict__ differ)
+{
+    const int64_t inner = 12 + (int64_t)30 * (k - 1);
+    bool same = true;
+    for (int64_t v = inner + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += (int64_t)gridDim.x * blockDim.x) {
+        int f, i, j;
+        interior_fij(v - inner, k, f, i, j);
+        int32_t row[6];
+        interior_row(v, f, i, j, k, row);
+        const int2 *o = reinterpret_cast<const int2 *>(nbr + 6 * v);
+        const int2 a = o[0], b = o[1], c = o[2];
+        same = same && a.x == row[0] && a.y == row[1] && b.x == row[2] && b.y == row[3] && c.x == row[4] && c.y == row[5];
+    }
+    if (!same) *differ = 1;
 }
 
 int grid1d(int64_t n, int block = 256)
@@ -579,26 +607,51 @@ NX_EXPORT int nx_icosphere(int k, double *xyz_dev, int32_t *tris_dev, void *stre
     return NX_OK;
 }
 
-NX_EXPORT int nx_icosphere_rows(int k, const double *xyz_dev, int32_t *nbr_dev, float *edge_dev, void *stream)
+static int check_rows(int k, const void *nbr, const void *edge, const char *who)
 {
-    if (k < 2 || (int64_t)10 * k * k + 2 > 0x7FFFFFFFLL) return nx::fail(NX_EINVAL, "nx_icosphere_rows: bad divisions %d", k);
-    if (!nbr_dev || (edge_dev && !xyz_dev)) return nx::fail(NX_EINVAL, "nx_icosphere_rows: null pointer");
-    if (((uintptr_t)nbr_dev & 7u) || ((uintptr_t)edge_dev & 7u))
-        return nx::fail(NX_EINVAL, "nx_icosphere_rows: rows must be 8-byte aligned");
+    if (k < 2 || (int64_t)10 * k * k + 2 > 0x7FFFFFFFLL) return nx::fail(NX_EINVAL, "%s: bad divisions %d", who, k);
+    if (!nbr) return nx::fail(NX_EINVAL, "%s: null pointer", who);
+    if (((uintptr_t)nbr & 7u) || ((uintptr_t)edge & 7u)) return nx::fail(NX_EINVAL, "%s: rows must be 8-byte aligned", who);
     int dev = 0;
     NX_CHECK_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !g_tables_ready[dev])
-        return nx::fail(NX_EINVAL, "nx_icosphere_rows: call nx_icosphere_tables first on this device");
+        return nx::fail(NX_EINVAL, "%s: call nx_icosphere_tables first on this device", who);
+    return NX_OK;
+}
+
+NX_EXPORT int nx_icosphere_rows(int k, int32_t *nbr_dev, void *stream)
+{
+    int rc = check_rows(k, nbr_dev, nullptr, "nx_icosphere_rows");
+    if (rc) return rc;
     const int64_t nv = (int64_t)10 * k * k + 2;
-    cudaStream_t s = (cudaStream_t)stream;
-    ico_neighbours_kernel<<<grid1d(nv), 256, 0, s>>>(k, nv, nbr_dev);
+    ico_neighbours_kernel<<<grid1d(nv), 256, 0, (cudaStream_t)stream>>>(k, nv, nbr_dev);
     NX_CHECK_LAUNCH("ico_neighbours_kernel");
     nx::note_launch(1);
-    if (edge_dev) {
-        ico_edges_kernel<<<grid1d(nv), 256, 0, s>>>(k, nv, xyz_dev, nbr_dev, (float2 *)edge_dev);
-        NX_CHECK_LAUNCH("ico_edges_kernel");
-        nx::note_launch(1);
-    }
+    return NX_OK;
+}
+
+NX_EXPORT int nx_icosphere_like(int k, const int32_t *nbr_dev, int *differ_dev, void *stream)
+{
+    int rc = check_rows(k, nbr_dev, nullptr, "nx_icosphere_like");
+    if (rc) return rc;
+    if (!differ_dev) return nx::fail(NX_EINVAL, "nx_icosphere_like: null pointer");
+    const int64_t nv = (int64_t)10 * k * k + 2;
+    ico_like_kernel<<<grid1d(nv), 256, 0, (cudaStream_t)stream>>>(k, nv, nbr_dev, differ_dev);
+    NX_CHECK_LAUNCH("ico_like_kernel");
+    nx::note_launch(1);
+    return NX_OK;
+}
+
+NX_EXPORT int nx_icosphere_edges(int k, const double *xyz_dev, const int32_t *nbr_dev, float *edge_dev, int *info_dev,
+                                 void *stream)
+{
+    int rc = check_rows(k, nbr_dev, edge_dev, "nx_icosphere_edges");
+    if (rc) return rc;
+    if (!xyz_dev || !edge_dev) return nx::fail(NX_EINVAL, "nx_icosphere_edges: null pointer");
+    const int64_t nv = (int64_t)10 * k * k + 2;
+    ico_edges_kernel<<<grid1d(nv), 256, 0, (cudaStream_t)stream>>>(k, nv, xyz_dev, nbr_dev, (float2 *)edge_dev, info_dev);
+    NX_CHECK_LAUNCH("ico_edges_kernel");
+    nx::note_launch(1);
     return NX_OK;
 }
 

@@ -138,7 +138,9 @@ class PlanetMesh:
         if tris is None:
             self.nbr = torch.empty((self.n, 6), dtype=torch.int32, device="cuda")
             self.edge = torch.empty((self.n, 6, 2), dtype=torch.float32, device="cuda")
-            call("nx_icosphere_rows", self.k, _dev.ptr(xyz), _dev.ptr(self.nbr), _dev.ptr(self.edge), _dev.stream_handle(stream))
+            call("nx_icosphere_rows", self.k, _dev.ptr(self.nbr), _dev.stream_handle(stream))
+            call("nx_icosphere_edges", self.k, _dev.ptr(xyz), _dev.ptr(self.nbr), _dev.ptr(self.edge), None,
+                 _dev.stream_handle(stream))
             self._errs = None
         else:
             adj, aerr = _adjacency(tris, stream)
