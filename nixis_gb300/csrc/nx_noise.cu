@@ -68,18 +68,31 @@ static_assert(sizeof(nx_fbm_planet) == 960, "fBm planet descriptor layout");
 constexpr int TABLE_WORDS = 256 * 32;
 constexpr int TABLE_BYTES = TABLE_WORDS * 4;
 
+// A warp fills runs of 32 entries: each lane forms one entry's word (two
+// global reads a lane, all in flight together), then the 32 words go out one
+// by one to their 32 replicas, a conflict-free store each.
+template <typename F>
+__device__ __forceinline__ void fill_table(uint32_t *T, const int32_t *__restrict__ perm, const int32_t *__restrict__ pgi,
+                                           F word)
+{
+    const int lane = threadIdx.x & 31;
+    for (int k0 = (threadIdx.x >> 5) * 32; k0 < 256; k0 += blockDim.x) {
+        const uint32_t p = (uint32_t)perm[k0 + lane] & 255u;
+        int g = pgi[k0 + lane];
+        g = g < 0 ? 0 : (g > 69 ? 69 : g);
+        const uint32_t w = word(p, g);
+#pragma unroll 8
+        for (int j = 0; j < 32; ++j) T[32 * (k0 + j) + lane] = __shfl_sync(0xFFFFFFFFu, w, j);
+    }
+}
+
 __device__ __forceinline__ void build_table(uint32_t *T, const int32_t *__restrict__ perm,
                                             const int32_t *__restrict__ pgi)
 {
-    for (int i = threadIdx.x; i < TABLE_WORDS; i += blockDim.x) {
-        int k = i >> 5;
-        uint32_t p = (uint32_t)perm[k] & 255u;
-        int g = pgi[k];
-        g = g < 0 ? 0 : (g > 69 ? 69 : g);
-        uint32_t w = ((uint32_t)(c_grad3[g + 2] + 16) & 0x7Fu) | (p << 7) |
-                     ((uint32_t)(c_grad3[g] + 16) << 16) | ((uint32_t)(c_grad3[g + 1] + 16) << 24);
-        T[i] = w;
-    }
+    fill_table(T, perm, pgi, [](uint32_t p, int g) {
+        return ((uint32_t)(c_grad3[g + 2] + 16) & 0x7Fu) | (p << 7) | ((uint32_t)(c_grad3[g] + 16) << 16) |
+               ((uint32_t)(c_grad3[g + 1] + 16) << 24);
+    });
 }
 
 // The pair path's table: the same layout with the gradient's index (0-23,
@@ -88,13 +101,7 @@ __device__ __forceinline__ void build_table(uint32_t *T, const int32_t *__restri
 __device__ __forceinline__ void build_table_pair(uint32_t *T, const int32_t *__restrict__ perm,
                                                  const int32_t *__restrict__ pgi)
 {
-    for (int i = threadIdx.x; i < TABLE_WORDS; i += blockDim.x) {
-        int k = i >> 5;
-        uint32_t p = (uint32_t)perm[k] & 255u;
-        int g = pgi[k];
-        g = g < 0 ? 0 : (g > 69 ? 69 : g);
-        T[i] = (uint32_t)(g / 3) | (p << 7);
-    }
+    fill_table(T, perm, pgi, [](uint32_t p, int g) { return (uint32_t)(g / 3) | (p << 7); });
 }
 
 // GRADIENTS_3D as binary32 (x, y, z, 0), and as sign masks (bit 31 of each
@@ -103,9 +110,9 @@ __device__ __forceinline__ void build_table_pair(uint32_t *T, const int32_t *__r
 __shared__ float4 s_grad[24];
 __shared__ uint4 s_gsign[24];
 
-__device__ __forceinline__ void init_grad_table()
+__device__ __forceinline__ void init_grad_table(int i)
 {
-    for (int i = threadIdx.x; i < 24; i += blockDim.x) {
+    if (i >= 0 && i < 24) {
         const int gx = c_grad3[3 * i], gy = c_grad3[3 * i + 1], gz = c_grad3[3 * i + 2];
         s_grad[i] = make_float4((float)gx, (float)gy, (float)gz, 0.0f);
         const uint32_t a = (gx == 11 || gx == -11) ? 0u : ((gy == 11 || gy == -11) ? 1u : 2u);
@@ -778,9 +785,9 @@ __device__ __forceinline__ void anchored_offsets(uint32_t w, float *H, float *L)
     }
 }
 
-__device__ __forceinline__ void init_extra_table_pair()
+__device__ __forceinline__ void init_extra_table_pair(int i)
 {
-    for (int i = threadIdx.x; i < 192; i += blockDim.x) {
+    if (i >= 0 && i < 192) {
         const uint32_t w = i < 64 ? octa_case(i) : tetra_case(i - 64);
         float H[6], L[6];
         anchored_offsets(w, H, L);
@@ -815,8 +822,11 @@ __device__ __forceinline__ void slot_disp(float X0H, float X0L2, float2 K, float
 
 // Two lattice contributions (slots a, b in the lanes) in pair arithmetic,
 // added to the pair accumulator (AH, AL).  X0H, X0L2: the anchored dx0 (hi,
-// 2 lo); KX/KXL2 the slots' anchored offsets (hi, 2 lo); ON 1/0 masks.
-template <bool NORM>
+// 2 lo); KX/KXL2 the slots' anchored offsets (hi, 2 lo); MASK: ON 1/0 masks.
+// Without NORM the accumulator starts at ACC_BIAS, which keeps it larger than
+// any contribution, so that fast two-sums do.
+constexpr float ACC_BIAS = 48.0f;      // a contribution's quarter is below 14.7, four of them below 26
+template <bool NORM, bool MASK>
 __device__ __forceinline__ void contrib2_pair(uint32_t wa, uint32_t wb, float X0H, float X0L2, float Y0H, float Y0L2,
                                               float Z0H, float Z0L2, float2 KX, float2 KXL2, float2 KY, float2 KYL2,
                                               float2 KZ, float2 KZL2, float2 ON, float2 &AH, float2 &AL)
@@ -825,28 +835,51 @@ __device__ __forceinline__ void contrib2_pair(uint32_t wa, uint32_t wb, float X0
     slot_disp<NORM>(X0H, X0L2, KX, KXL2, Xh, X2);
     slot_disp<NORM>(Y0H, Y0L2, KY, KYL2, Yh, Y2);
     slot_disp<NORM>(Z0H, Z0L2, KZ, KZL2, Zh, Z2);
-    // attn = 2 - |d|^2: squares of the hi parts exact as p + pe, plus the
-    // cross terms 2 hi lo
-    const float2 px = mul2(Xh, Xh), py = mul2(Yh, Yh), pz = mul2(Zh, Zh);
-    const float2 pxe = fma2(Xh, Xh, f2(-px.x, -px.y)), pye = fma2(Yh, Yh, f2(-py.x, -py.y)),
-                 pze = fma2(Zh, Zh, f2(-pz.x, -pz.y));
-    float2 L = add2(pxe, add2(pye, pze));
-    L = fma2(Xh, X2, L);
-    L = fma2(Yh, Y2, L);
-    L = fma2(Zh, Z2, L);
-    const float2 two = f2(2.0f, 2.0f);
-    const float2 r1 = sub2(two, px), r2 = sub2(r1, py), r3 = sub2(r2, pz);
-    const float2 e1 = sub2(sub2(two, r1), px), e2 = sub2(sub2(r1, r2), py), e3 = sub2(sub2(r2, r3), pz);
-    const float2 al = sub2(add2(add2(e1, e2), e3), L);
+    // attn = 2 - |d|^2 = r3 + al
+    float2 r3, al;
+    if (NORM) {
+        // squares of the hi parts exact as p + pe, plus the cross terms 2 hi lo
+        const float2 px = mul2(Xh, Xh), py = mul2(Yh, Yh), pz = mul2(Zh, Zh);
+        const float2 pxe = fma2(Xh, Xh, f2(-px.x, -px.y)), pye = fma2(Yh, Yh, f2(-py.x, -py.y)),
+                     pze = fma2(Zh, Zh, f2(-pz.x, -pz.y));
+        float2 L = add2(pxe, add2(pye, pze));
+        L = fma2(Xh, X2, L);
+        L = fma2(Yh, Y2, L);
+        L = fma2(Zh, Z2, L);
+        const float2 r0 = f2(2.0f, 2.0f);
+        const float2 r1 = sub2(r0, px), r2 = sub2(r1, py);
+        r3 = sub2(r2, pz);
+        const float2 e1 = sub2(sub2(r0, r1), px), e2 = sub2(sub2(r1, r2), py), e3 = sub2(sub2(r2, r3), pz);
+        al = sub2(add2(add2(e1, e2), e3), L);
+    } else {
+        // the squares added to 2 one by one: while the sum stays below 4 (where
+        // attn > 0) each step rounds to the 2^-22 grid, its increment is exact
+        // and the square's rest (below 2^-22, on the 2^-42 grid) comes exact
+        // from one fma; 15 operations against 23 above, and no less exact
+        // beside the cross terms, which reach 2^-19 without NORM
+        const float2 t0 = f2(2.0f, 2.0f), t1 = fma2(Xh, Xh, t0), t2 = fma2(Yh, Yh, t1), t3 = fma2(Zh, Zh, t2);
+        const float2 d1 = sub2(t1, t0), d2 = sub2(t2, t1), d3 = sub2(t3, t2);
+        const float2 e1 = fma2(Xh, Xh, f2(-d1.x, -d1.y)), e2 = fma2(Yh, Yh, f2(-d2.x, -d2.y)),
+                     e3 = fma2(Zh, Zh, f2(-d3.x, -d3.y));
+        float2 L = add2(add2(e1, e2), e3);
+        L = fma2(Xh, X2, L);
+        L = fma2(Yh, Y2, L);
+        L = fma2(Zh, Z2, L);
+        r3 = sub2(f2(4.0f, 4.0f), t3);
+        al = f2(-L.x, -L.y);
+    }
     // only attn > 0 counts, and only in the region (ah = 0 zeroes the rest)
-    const float2 ah = mul2(f2(fmaxf(r3.x, 0.0f), fmaxf(r3.y, 0.0f)), ON);
-    // attn^2, attn^4 as pairs
+    float2 ah = f2(fmaxf(r3.x, 0.0f), fmaxf(r3.y, 0.0f));
+    if (MASK) ah = mul2(ah, ON);
+    // attn^2, attn^4 as pairs (with the squares of the low parts: without NORM
+    // al reaches 2^-19, and its square would show)
+    const float2 two = f2(2.0f, 2.0f);
     const float2 h2 = mul2(ah, ah);
     float2 l2 = fma2(ah, ah, f2(-h2.x, -h2.y));
-    l2 = fma2(add2(ah, ah), al, l2);
+    l2 = fma2(fma2(two, ah, al), al, l2);
     const float2 h4 = mul2(h2, h2);
     float2 l4 = fma2(h2, h2, f2(-h4.x, -h4.y));
-    l4 = fma2(add2(h2, h2), l2, l4);
+    l4 = fma2(fma2(two, h2, l2), l2, l4);
     // grad . d as a pair (dh, dl), times DSC (see below)
     const float4 ga = s_grad[wa & 31u], gb = s_grad[wb & 31u];
     const float2 gx = f2(ga.x, gb.x), gy = f2(ga.y, gb.y), gz = f2(ga.z, gb.z);
@@ -873,19 +906,58 @@ __device__ __forceinline__ void contrib2_pair(uint32_t wa, uint32_t wb, float X0
         const float2 s_a = f2(sa.w == 0u ? sx.x : (sa.w == 1u ? sy.x : sz.x), sb.w == 0u ? sx.y : (sb.w == 1u ? sy.y : sz.y));
         const float2 U = fma2(f2(2.0f, 2.0f), s_a, add2(add2(sx, sy), sz));
         const float2 V = mul2(f2(-0.25f, -0.25f), s_a);
-        float2 e;
-        two_sum2(U, V, dh, e);
+        // a fast two-sum: where |U| < |V| (below 3/8) the sum, on the 2^-23
+        // grid and below 1, is exact
+        dh = add2(U, V);
+        const float2 e = sub2(V, sub2(dh, U));
         const float2 gl = fma2(gx, X2, fma2(gy, Y2, mul2(gz, Z2)));     // 2 (grad . lo)
         dl = fma2(f2(0.125f, 0.125f), gl, e);
     }
     // attn^4 * (grad . d)
     const float2 ch = mul2(h4, dh);
     float2 cl = fma2(h4, dh, f2(-ch.x, -ch.y));
-    cl = fma2(h4, dl, fma2(l4, dh, cl));
+    cl = fma2(add2(h4, l4), dl, fma2(l4, dh, cl));
     float2 s, e;
-    two_sum2(AH, ch, s, e);
+    if (NORM) {
+        two_sum2(AH, ch, s, e);
+    } else {
+        s = add2(AH, ch);
+        e = sub2(ch, sub2(s, AH));
+    }
     AH = s;
     AL = add2(AL, add2(e, cl));
+}
+
+// Offsets of the fixed corners that a lane of each region evaluates (slots
+// X1..X4 of noise_pair), anchored: entry 4 q + region, q = 0: (X1x, X2x, X1y,
+// X2y), 1: (X1z, X2z, X1 2lo, X2 2lo), 2 and 3 the same of X3, X4.  Four
+// shared loads (the regions' entries on different banks) instead of 27
+// selects per vertex and octave.
+__shared__ float4 s_corner[16];
+
+__device__ __forceinline__ void init_corner_table(int i)
+{
+    // X1..X4 per region in thirds m / 3 (hi), and the sign of the lo part
+    if (i >= 0 && i < 12) {
+        const int q = i / 3, g = i % 3;
+        // corner 0 | A1, A2, A3 | B1, B2, B3: region 0 (0, A1, A2, A3), region 1
+        // (corner (1,1,1) = 6/3, B1, B2, B3), octahedron (A1, A2, A3, B1)
+        float v[2][4];
+        for (int u = 0; u < 2; ++u) {
+            const int x = 2 * (q / 2) + u;                   // slot X1..X4
+            const int c = g == 2 ? x + 1 : (x == 0 ? 0 : (g == 1 ? 3 + x : x));   // 0, A1-A3 = 1-3, B1-B3 = 4-6
+            for (int a = 0; a < 3; ++a) {
+                int m = 0;
+                if (c == 0) m = g == 1 ? 6 : 0;
+                else if (c <= 3) m = a == c - 1 ? 4 : 1;     // (4,1,1), (1,4,1), (1,1,4)
+                else m = a == 6 - c ? 2 : 5;                 // (5,5,2), (5,2,5), (2,5,5)
+                v[u][a] = m == 6 ? 2.0f : (m == 5 ? T5H : (m == 4 ? T4H : (m == 2 ? T2H : (m == 1 ? T1H : 0.0f))));
+            }
+            v[u][3] = c == 0 ? 0.0f : (c <= 3 ? -C3L2 : C3L2);
+        }
+        s_corner[4 * q + g] = (q & 1) ? make_float4(v[0][2], v[1][2], v[0][3], v[1][3])
+                                      : make_float4(v[0][0], v[1][0], v[0][1], v[1][1]);
+    }
 }
 
 // x*scale = A + a1 + a2 + a3 for one axis: x = x1 + x2 + x3 and scale =
@@ -1021,31 +1093,26 @@ __device__ __forceinline__ void noise_pair(float x1, float x2, float x3, float y
     // (1,0,0) -> (4,1,1)/3, A2 (1,4,1)/3, A3 (1,1,4)/3, B1 = (1,1,0) ->
     // (5,5,2)/3, B2 (5,2,5)/3, B3 (2,5,5)/3; corner 0: (0,0,0) or (2,2,2));
     // A-corners' anchored lo is -C3L, B-corners' +C3L, the corner's 0
-    const float k0 = r1 ? 2.0f : 0.0f;
-    const float nL2 = -C3L2, pL2 = C3L2;
+    const float pL2 = C3L2;
     //   X1: r2 ? A1 : corner 0       X2: r2 ? A2 : (r1 ? B1 : A1)
     //   X3: r2 ? A3 : (r1 ? B2 : A2) X4: r2 ? B1 : (r1 ? B3 : A3)
     //   X5: B2, X6: B3 (octahedron only)
     const uint32_t wX1 = r2 ? w100 : w0, wX2 = r2 ? w010 : (r1 ? w110 : w100);
     const uint32_t wX3 = r2 ? w001 : (r1 ? w101 : w010), wX4 = r2 ? w110 : (r1 ? w011 : w001);
-    const float2 X1X2x = f2(r2 ? T4H : k0, r2 ? T1H : (r1 ? T5H : T4H));
-    const float2 X1X2y = f2(r2 ? T1H : k0, r2 ? T4H : (r1 ? T5H : T1H));
-    const float2 X1X2z = f2(r2 ? T1H : k0, r2 ? T1H : (r1 ? T2H : T1H));
-    const float2 X1X2l = f2(r2 ? nL2 : 0.0f, r1 ? pL2 : nL2);
-    const float2 X3X4x = f2(r2 ? T1H : (r1 ? T5H : T1H), r2 ? T5H : (r1 ? T2H : T1H));
-    const float2 X3X4y = f2(r2 ? T1H : (r1 ? T2H : T4H), r2 ? T5H : (r1 ? T5H : T1H));
-    const float2 X3X4z = f2(r2 ? T4H : (r1 ? T5H : T1H), r2 ? T2H : (r1 ? T5H : T4H));
-    const float2 X3X4l = f2(r1 ? pL2 : nL2, (r1 || r2) ? pL2 : nL2);
+    const float4 c0 = s_corner[region], c1 = s_corner[4 + region], c2 = s_corner[8 + region], c3 = s_corner[12 + region];
     const float fr2 = r2 ? 1.0f : 0.0f;
-    float2 AH = f2(0.0f, 0.0f), AL = f2(0.0f, 0.0f);
-    contrib2_pair<NORM>(wX1, wX2, X0H, X0L2, Y0H, Y0L2, Z0H, Z0L2, X1X2x, X1X2l, X1X2y, X1X2l, X1X2z, X1X2l, f2(1.0f, 1.0f),
-                  AH, AL);
-    contrib2_pair<NORM>(wX3, wX4, X0H, X0L2, Y0H, Y0L2, Z0H, Z0L2, X3X4x, X3X4l, X3X4y, X3X4l, X3X4z, X3X4l, f2(1.0f, 1.0f),
-                  AH, AL);
-    contrib2_pair<NORM>(w101, w011, X0H, X0L2, Y0H, Y0L2, Z0H, Z0L2, f2(T5H, T2H), f2(pL2, pL2), f2(T2H, T5H), f2(pL2, pL2),
-                  f2(T5H, T5H), f2(pL2, pL2), f2(fr2, fr2), AH, AL);
-    contrib2_pair<NORM>(we0, we1, X0H, X0L2, Y0H, Y0L2, Z0H, Z0L2, f2(EH[0], EH[3]), f2(EL2[0], EL2[3]), f2(EH[1], EH[4]),
-                  f2(EL2[1], EL2[4]), f2(EH[2], EH[5]), f2(EL2[2], EL2[5]), f2(1.0f, 1.0f), AH, AL);
+    const float bias = NORM ? 0.0f : ACC_BIAS;
+    float2 AH = f2(bias, bias), AL = f2(0.0f, 0.0f);
+    const float2 none = f2(1.0f, 1.0f), l12 = f2(c1.z, c1.w), l34 = f2(c3.z, c3.w);
+    contrib2_pair<NORM, false>(wX1, wX2, X0H, X0L2, Y0H, Y0L2, Z0H, Z0L2, f2(c0.x, c0.y), l12, f2(c0.z, c0.w), l12,
+                               f2(c1.x, c1.y), l12, none, AH, AL);
+    contrib2_pair<NORM, false>(wX3, wX4, X0H, X0L2, Y0H, Y0L2, Z0H, Z0L2, f2(c2.x, c2.y), l34, f2(c2.z, c2.w), l34,
+                               f2(c3.x, c3.y), l34, none, AH, AL);
+    contrib2_pair<NORM, true>(w101, w011, X0H, X0L2, Y0H, Y0L2, Z0H, Z0L2, f2(T5H, T2H), f2(pL2, pL2), f2(T2H, T5H),
+                              f2(pL2, pL2), f2(T5H, T5H), f2(pL2, pL2), f2(fr2, fr2), AH, AL);
+    contrib2_pair<NORM, false>(we0, we1, X0H, X0L2, Y0H, Y0L2, Z0H, Z0L2, f2(EH[0], EH[3]), f2(EL2[0], EL2[3]),
+                               f2(EH[1], EH[4]), f2(EL2[1], EL2[4]), f2(EH[2], EH[5]), f2(EL2[2], EL2[5]), none, AH, AL);
+    if (!NORM) AH = f2(__fsub_rn(AH.x, ACC_BIAS), __fsub_rn(AH.y, ACC_BIAS));     // exact
     float e;
     two_sum1(AH.x, AH.y, vh, e);
     vl = __fadd_rn(e, __fadd_rn(AL.x, AL.y));
@@ -1208,19 +1275,45 @@ __device__ __forceinline__ int chunk_planet(const nx_fbm_planet *P, int np, int 
     return lo;
 }
 
-// Chunk ranges of a batched launch: block b takes chunks [first[b],
-// first[b + 1]) in order, the ranges cut so that each block gets an equal
-// share of the estimated cost (vertices x octaves, renormalised octaves
-// weighted 9/8).
+// Threads of a pair block: one block of 512 per SM (128 registers a thread).
+// Measured (GB300, 12 octaves of 10,000,002 vertices): 3.13 ms, against 3.38
+// ms for two blocks of 256 (each with a table of its own), 3.63 ms for three
+// of 192, 3.74 ms for one of 640 and 3.90 ms for two of 320 (96 registers:
+// more warps, but longer dependent stretches).
+constexpr int PAIR_THREADS = 512;
+constexpr int PAIR_WARPS = PAIR_THREADS / 32;
+
+// A block's step: PAIR_THREADS / S vertices, their octaves dealt out to S
+// groups of warps (S a power of two up to 16).  S = 1 where there are vertices
+// for every warp; small spheres and the remainder of large ones are split, so
+// that they fill the GPU with fewer octaves each: a warp's octave takes ~6 us
+// however few there are.
+constexpr int SPLIT_MAX = 16;
+
+// Shared memory of the octaves' values of a split step.
+static size_t split_bytes(int S, int n_oct) { return S > 1 ? sizeof(float2) * (size_t)(PAIR_THREADS / S) * (size_t)n_oct : 0; }
+
+// The largest split with which `vertices` make no more than `blocks` steps.
+static int split_for(int64_t vertices, int blocks, int n_oct)
+{
+    int S = 1;
+    while (2 * S <= SPLIT_MAX && S < n_oct && (vertices * 2 * S + PAIR_THREADS - 1) / PAIR_THREADS <= blocks) S *= 2;
+    return S;
+}
+
+// Steps of a batched launch: block b takes steps [first[b], first[b + 1]) in
+// order, the ranges cut so that each block gets an equal share of the
+// estimated cost (vertices x octaves, renormalised octaves weighted 9/8).
 constexpr int FBM_SPLIT_MAX = 2048;
 struct FbmSplit {
+    int S;                              // octave split
     int first[FBM_SPLIT_MAX + 1];
 };
 
 // Fold the ordered keys (kmn, kmx) of the block's sums of planet P into its
 // min/max (a block barrier; the whole block calls it).
 __device__ __forceinline__ void fold_minmax(const nx_fbm_planet &P, unsigned long long kmn, unsigned long long kmx,
-                                            unsigned long long (*s_mm)[8])
+                                            unsigned long long (*s_mm)[PAIR_WARPS])
 {
     for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long a = __shfl_xor_sync(0xFFFFFFFFu, kmn, o);
@@ -1243,27 +1336,113 @@ __device__ __forceinline__ void fold_minmax(const nx_fbm_planet &P, unsigned lon
     __syncthreads();
 }
 
-// Many planets in one persistent launch: work items are chunks of CHUNK
-// vertices of one planet; each block walks its contiguous range of chunks
+// One vertex's binary32 triples.
+struct Triples {
+    float x1, x2, x3, y1, y2, y3, z1, z2, z3;
+};
+
+__device__ __forceinline__ Triples load_triples(const double *__restrict__ xyz, int64_t i)
+{
+    Triples t;
+    split3_f64(xyz[3 * i], t.x1, t.x2, t.x3);
+    split3_f64(xyz[3 * i + 1], t.y1, t.y2, t.y3);
+    split3_f64(xyz[3 * i + 2], t.z1, t.z2, t.z3);
+    return t;
+}
+
+__device__ __forceinline__ void octave_value(const Triples &t, const OctP &O, bool norm, bool pow2, uint32_t lb,
+                                             unsigned &nfb, float &vh, float &vl)
+{
+    if (norm) noise_pair<true>(t.x1, t.x2, t.x3, t.y1, t.y2, t.y3, t.z1, t.z2, t.z3, O, pow2, lb, nfb, vh, vl);
+    else noise_pair<false>(t.x1, t.x2, t.x3, t.y1, t.y2, t.y3, t.z1, t.z2, t.z3, O, pow2, lb, nfb, vh, vl);
+}
+
+// The block's constant tables, by its upper warps (the hash table's words are
+// filled by the lower ones meanwhile).
+__device__ __forceinline__ void init_pair_tables()
+{
+    static_assert(PAIR_THREADS == 512, "threads 256-447, 448-459 and 480-503 fill the tables");
+    init_extra_table_pair((int)threadIdx.x - 256);
+    init_corner_table((int)threadIdx.x - 448);
+    init_grad_table((int)threadIdx.x - 480);
+}
+
+// Octave o's constants of a planet descriptor or a launch's parameters.
+__device__ __forceinline__ OctP oct_of(const nx_fbm_planet &P, int o)
+{
+    OctP O;
+    O.s1 = P.s1[o]; O.s2 = P.s2[o]; O.s3 = P.s3[o];
+    O.amph = P.amp_hi[o]; O.ampl = P.amp_lo[o]; O.s = P.s[o];
+    return O;
+}
+
+// The sum over P's octaves at vertex i, added to (rh, rl).  SPLIT: the block
+// evaluates one step's PAIR_THREADS / S vertices from `first` on; the sum is
+// valid in threads below PAIR_THREADS / S (vertex first + thread), the octaves
+// summed there in order, so the bits do not depend on S.
+template <typename P_t>
+__device__ __forceinline__ void sum_octaves(const P_t &P, int n_oct, const Triples &t, bool pow2, uint32_t lb,
+                                            unsigned &nfb, float &rh, float &rl)
+{
+    for (int o = 0; o < n_oct; ++o) {
+        const OctP O = oct_of(P, o);
+        float vh, vl;
+        octave_value(t, O, (P.norm_mask >> o) & 1u, pow2, lb, nfb, vh, vl);
+        octave_accumulate(vh, vl, O.amph, O.ampl, rh, rl);
+    }
+}
+
+template <typename P_t>
+__device__ __forceinline__ void sum_split(const P_t &P, int n_oct, const double *__restrict__ xyz, int64_t first,
+                                          int64_t last, int S, bool pow2, uint32_t lb, float2 *part, unsigned &nfb,
+                                          float &rh, float &rl)
+{
+    const int U = PAIR_THREADS / S, q = threadIdx.x % U;
+    const int64_t i = first + q;
+    // (past the end: the last vertex again, so that warps stay whole)
+    const Triples t = load_triples(xyz, i < last ? i : last - 1);
+    unsigned extra = 0;
+    for (int o = threadIdx.x / U; o < n_oct; o += S) {
+        const OctP O = oct_of(P, o);
+        float vh, vl;
+        octave_value(t, O, (P.norm_mask >> o) & 1u, pow2, lb, extra, vh, vl);
+        part[o * U + q] = make_float2(vh, vl);
+    }
+    if (i < last) nfb += extra;
+    __syncthreads();
+    if ((int)threadIdx.x < U)
+        for (int o = 0; o < n_oct; ++o) {
+            const OctP O = oct_of(P, o);
+            const float2 v = part[o * U + q];
+            octave_accumulate(v.x, v.y, O.amph, O.ampl, rh, rl);
+        }
+    __syncthreads();
+}
+
+// Many planets in one persistent launch: work items are steps of
+// PAIR_THREADS / S vertices of one planet (CHUNK vertices hold S CHUNK /
+// PAIR_THREADS of them); each block walks its contiguous range of steps
 // (so it meets few planets), rebuilding its shared table when the planet
 // changes.  Sums are pairs (pair path above); the ordered keys of a block's
 // sums of a planet are folded into the planet's min/max once, when the
 // block leaves the planet (for the rescale to metres that follows).
-__global__ void __launch_bounds__(256) fbm_batch_kernel(const nx_fbm_planet *__restrict__ planets, int np,
-                                                        const __grid_constant__ FbmSplit split,
-                                                        unsigned long long *nfb_out)
+__global__ void __launch_bounds__(PAIR_THREADS, 1) fbm_batch_kernel(const nx_fbm_planet *__restrict__ planets, int np,
+                                                                    const __grid_constant__ FbmSplit split,
+                                                                    unsigned long long *nfb_out)
 {
     extern __shared__ __align__(16) uint32_t smem[];
-    __shared__ unsigned long long s_mm[2][8];
-    init_extra_table_pair();
-    init_grad_table();
+    __shared__ unsigned long long s_mm[2][PAIR_WARPS];
+    init_pair_tables();
     __syncthreads();
     const uint32_t lb = lane_base(smem);
-    const int c0 = split.first[blockIdx.x], c1 = split.first[blockIdx.x + 1];
+    float2 *part = reinterpret_cast<float2 *>(smem + TABLE_WORDS);
+    const int S = split.S, U = PAIR_THREADS / S, per = CHUNK / U;
+    const int u0 = split.first[blockIdx.x], u1 = split.first[blockIdx.x + 1];
     int cur = -1;
     unsigned nfb = 0;
     unsigned long long kmn = ~0ull, kmx = 0ull;
-    for (int c = c0; c < c1; ++c) {
+    for (int u = u0; u < u1; ++u) {
+        const int c = u / per;
         int p = cur < 0 ? chunk_planet(planets, np, c) : cur;
         while (p + 1 < np && planets[p + 1].chunk0 <= c) ++p;
         if (p != cur) {
@@ -1276,26 +1455,19 @@ __global__ void __launch_bounds__(256) fbm_batch_kernel(const nx_fbm_planet *__r
             cur = p;
         }
         const nx_fbm_planet &P = planets[p];
-        const int64_t base = (int64_t)(c - P.chunk0) * CHUNK;
+        const int64_t first = (int64_t)(c - P.chunk0) * CHUNK + (int64_t)(u - c * per) * U;
+        if (first >= P.n) continue;
         const bool pow2 = P.pow2 != 0;
-        for (int64_t i = base + threadIdx.x; i < base + CHUNK && i < P.n; i += blockDim.x) {
-            const double X = P.xyz[3 * i], Y = P.xyz[3 * i + 1], Z = P.xyz[3 * i + 2];
-            float x1, x2, x3, y1, y2, y3, z1, z2, z3;
-            split3_f64(X, x1, x2, x3);
-            split3_f64(Y, y1, y2, y3);
-            split3_f64(Z, z1, z2, z3);
-            float rh = 0.0f, rl = 0.0f;
-            for (int o = 0; o < P.n_octaves; ++o) {
-                OctP O;
-                O.s1 = P.s1[o]; O.s2 = P.s2[o]; O.s3 = P.s3[o];
-                O.amph = P.amp_hi[o]; O.ampl = P.amp_lo[o]; O.s = P.s[o];
-                float vh, vl;
-                if ((P.norm_mask >> o) & 1u)
-                    noise_pair<true>(x1, x2, x3, y1, y2, y3, z1, z2, z3, O, pow2, lb, nfb, vh, vl);
-                else
-                    noise_pair<false>(x1, x2, x3, y1, y2, y3, z1, z2, z3, O, pow2, lb, nfb, vh, vl);
-                octave_accumulate(vh, vl, O.amph, O.ampl, rh, rl);
-            }
+        float rh = 0.0f, rl = 0.0f;
+        const int64_t i = first + threadIdx.x;
+        bool mine = i < P.n;
+        if (S == 1) {
+            if (mine) sum_octaves(P, P.n_octaves, load_triples(P.xyz, i), pow2, lb, nfb, rh, rl);
+        } else {
+            sum_split(P, P.n_octaves, P.xyz, first, P.n, S, pow2, lb, part, nfb, rh, rl);
+            mine = mine && (int)threadIdx.x < U;
+        }
+        if (mine) {
             reinterpret_cast<float2 *>(P.out)[i] = make_float2(rh, rl);
             const unsigned long long k = pair_key(rh, rl);
             kmn = k < kmn ? k : kmn;
@@ -1324,46 +1496,37 @@ struct FbmPairParams {
 // the first) added to the running pair sums in out2 (float2 per vertex),
 // and/or written as binary64 (out64, = hi + lo exactly; accumulate adds to
 // it).  minmax (optional): ordered keys of the resulting pair sums.
-__global__ void __launch_bounds__(256) fbm_pair_kernel(const double *__restrict__ xyz, int64_t n,
-                                                       const int32_t *__restrict__ perm,
-                                                       const int32_t *__restrict__ pgi, FbmPairParams P,
-                                                       float2 *__restrict__ out2, double *__restrict__ out64,
-                                                       int accumulate, unsigned long long *minmax,
-                                                       unsigned long long *nfb_out)
+//
+// Vertices [0, main) in whole rounds of the grid, a thread a vertex; the
+// remainder split over its octaves, a step to a block (split_for).
+__device__ __forceinline__ OctP oct_of(const FbmPairParams &P, int o)
+{
+    OctP O;
+    O.s1 = P.s1[o]; O.s2 = P.s2[o]; O.s3 = P.s3[o];
+    O.amph = P.amph[o]; O.ampl = P.ampl[o]; O.s = P.s[o];
+    return O;
+}
+
+__global__ void __launch_bounds__(PAIR_THREADS, 1) fbm_pair_kernel(const double *__restrict__ xyz, int64_t n, int64_t main,
+                                                                   int S, const int32_t *__restrict__ perm,
+                                                                   const int32_t *__restrict__ pgi,
+                                                                   const __grid_constant__ FbmPairParams P,
+                                                                   float2 *__restrict__ out2,
+                                                                   double *__restrict__ out64, int accumulate,
+                                                                   unsigned long long *minmax,
+                                                                   unsigned long long *nfb_out)
 {
     extern __shared__ __align__(16) uint32_t smem[];
-    __shared__ unsigned long long s_mm[2][8];
+    __shared__ unsigned long long s_mm[2][PAIR_WARPS];
     build_table_pair(smem, perm, pgi);
-    init_extra_table_pair();
-    init_grad_table();
+    init_pair_tables();
     __syncthreads();
     const uint32_t lb = lane_base(smem);
+    float2 *part = reinterpret_cast<float2 *>(smem + TABLE_WORDS);
     unsigned nfb = 0;
     unsigned long long kmn = ~0ull, kmx = 0ull;
     const bool pow2 = P.pow2 != 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double X = xyz[3 * i], Y = xyz[3 * i + 1], Z = xyz[3 * i + 2];
-        float x1, x2, x3, y1, y2, y3, z1, z2, z3;
-        split3_f64(X, x1, x2, x3);
-        split3_f64(Y, y1, y2, y3);
-        split3_f64(Z, z1, z2, z3);
-        float rh = 0.0f, rl = 0.0f;
-        if (accumulate && out2) {
-            const float2 v = out2[i];
-            rh = v.x;
-            rl = v.y;
-        }
-        for (int o = 0; o < P.n_oct; ++o) {
-            OctP O;
-            O.s1 = P.s1[o]; O.s2 = P.s2[o]; O.s3 = P.s3[o];
-            O.amph = P.amph[o]; O.ampl = P.ampl[o]; O.s = P.s[o];
-            float vh, vl;
-            if ((P.norm_mask >> o) & 1u)
-                noise_pair<true>(x1, x2, x3, y1, y2, y3, z1, z2, z3, O, pow2, lb, nfb, vh, vl);
-            else
-                noise_pair<false>(x1, x2, x3, y1, y2, y3, z1, z2, z3, O, pow2, lb, nfb, vh, vl);
-            octave_accumulate(vh, vl, O.amph, O.ampl, rh, rl);
-        }
+    auto put = [&](int64_t i, float rh, float rl) {
         if (out2) out2[i] = make_float2(rh, rl);
         if (out64) {
             const double v = (double)rh + (double)rl;
@@ -1372,26 +1535,29 @@ __global__ void __launch_bounds__(256) fbm_pair_kernel(const double *__restrict_
         const unsigned long long k = pair_key(rh, rl);
         kmn = k < kmn ? k : kmn;
         kmx = k > kmx ? k : kmx;
+    };
+    const bool running = accumulate && out2;
+    for (int64_t i = (int64_t)blockIdx.x * PAIR_THREADS + threadIdx.x; i < main; i += (int64_t)gridDim.x * PAIR_THREADS) {
+        const float2 v = running ? out2[i] : make_float2(0.0f, 0.0f);
+        float rh = v.x, rl = v.y;
+        sum_octaves(P, P.n_oct, load_triples(xyz, i), pow2, lb, nfb, rh, rl);
+        put(i, rh, rl);
+    }
+    const int U = PAIR_THREADS / S;
+    const int64_t first = main + (int64_t)blockIdx.x * U;
+    if (first < n) {
+        const int64_t i = first + threadIdx.x;
+        const bool mine = i < n && (int)threadIdx.x < U;
+        const float2 v = running && mine ? out2[i] : make_float2(0.0f, 0.0f);
+        float rh = v.x, rl = v.y;
+        if (S > 1) sum_split(P, P.n_oct, xyz, first, n, S, pow2, lb, part, nfb, rh, rl);
+        else if (mine) sum_octaves(P, P.n_oct, load_triples(xyz, i), pow2, lb, nfb, rh, rl);
+        if (mine) put(i, rh, rl);
     }
     if (minmax) {
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long a = __shfl_xor_sync(0xFFFFFFFFu, kmn, o);
-            const unsigned long long b = __shfl_xor_sync(0xFFFFFFFFu, kmx, o);
-            kmn = a < kmn ? a : kmn;
-            kmx = b > kmx ? b : kmx;
-        }
-        const int w = threadIdx.x >> 5;
-        if ((threadIdx.x & 31) == 0) { s_mm[0][w] = kmn; s_mm[1][w] = kmx; }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned long long a0 = s_mm[0][0], a1 = s_mm[1][0];
-            for (int k = 1; k < (int)(blockDim.x >> 5); ++k) {
-                a0 = s_mm[0][k] < a0 ? s_mm[0][k] : a0;
-                a1 = s_mm[1][k] > a1 ? s_mm[1][k] : a1;
-            }
-            atomicMin(&minmax[0], a0);
-            atomicMax(&minmax[1], a1);
-        }
+        nx_fbm_planet out;
+        out.minmax = minmax;
+        fold_minmax(out, kmn, kmx, s_mm);
     }
     if (nfb_out) {
         unsigned tot = __reduce_add_sync(0xFFFFFFFFu, nfb);
@@ -1417,8 +1583,9 @@ int configure_smem()
     if (smem_configured) return NX_OK;
     NX_CHECK_CUDA(cudaFuncSetAttribute(fbm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TABLE_BYTES));
     NX_CHECK_CUDA(cudaFuncSetAttribute(trace_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TABLE_BYTES));
-    NX_CHECK_CUDA(cudaFuncSetAttribute(fbm_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TABLE_BYTES));
-    NX_CHECK_CUDA(cudaFuncSetAttribute(fbm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TABLE_BYTES));
+    const int pair_bytes = TABLE_BYTES + (int)split_bytes(2, NX_MAX_OCTAVES);
+    NX_CHECK_CUDA(cudaFuncSetAttribute(fbm_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_bytes));
+    NX_CHECK_CUDA(cudaFuncSetAttribute(fbm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_bytes));
     smem_configured = true;
     return NX_OK;
 }
@@ -1592,10 +1759,15 @@ NX_EXPORT int nx_fbm_pair(const double *xyz_dev, int64_t n, const int32_t *perm_
     P.norm_mask = norm_mask(n_octaves, strength, radius, amp_ref);
     rc = configure_smem();
     if (rc) return rc;
-    int grid = grid_for(n, 256, (const void *)fbm_pair_kernel, TABLE_BYTES);
-    fbm_pair_kernel<<<grid, 256, TABLE_BYTES, (cudaStream_t)stream>>>(xyz_dev, n, perm_dev, pgi_dev, P,
-                                                                      (float2 *)pair_dev, elev_f64_dev, accumulate,
-                                                                      minmax_dev, n_fallback_dev);
+    // whole rounds of one block per SM, then the remainder, one step a block
+    const int sms = nx::sm_count();
+    const int64_t round = (int64_t)sms * PAIR_THREADS, main = n / round * round, rest = n - main;
+    const int S = split_for(rest, sms, n_octaves);
+    const int64_t steps = (rest * S + PAIR_THREADS - 1) / PAIR_THREADS;
+    const int grid = main > 0 ? sms : (int)(steps < 1 ? 1 : steps);
+    fbm_pair_kernel<<<grid, PAIR_THREADS, TABLE_BYTES + split_bytes(S, n_octaves), (cudaStream_t)stream>>>(
+        xyz_dev, n, main, S, perm_dev, pgi_dev, P, (float2 *)pair_dev, elev_f64_dev, accumulate, minmax_dev,
+        n_fallback_dev);
     NX_CHECK_LAUNCH("fbm_pair_kernel");
     nx::note_launch(1);
     return NX_OK;
@@ -1621,10 +1793,21 @@ NX_EXPORT int nx_fbm_batch(const nx_fbm_planet *planets_dev, const nx_fbm_planet
     if (total == 0) return NX_OK;
     int rc = configure_smem();
     if (rc) return rc;
-    int grid = grid_for((int64_t)total * 256, 256, (const void *)fbm_batch_kernel, TABLE_BYTES);
-    if (grid > FBM_SPLIT_MAX) grid = FBM_SPLIT_MAX;
-    // cut the chunks into grid ranges of equal estimated cost: a planet's
-    // chunk costs its vertices x (8 per octave + 1 per renormalised octave)
+    int64_t vertices = 0;
+    int max_oct = 0;
+    for (int p = 0; p < nplanets; ++p) {
+        vertices += planets_host[p].n;
+        if (planets_host[p].n > 0 && planets_host[p].n_octaves > max_oct) max_oct = planets_host[p].n_octaves;
+    }
+    const int sms = nx::sm_count() < FBM_SPLIT_MAX ? nx::sm_count() : FBM_SPLIT_MAX;
+    FbmSplit split;
+    split.S = split_for(vertices, sms, max_oct);
+    const int U = PAIR_THREADS / split.S, per_chunk = CHUNK / U;
+    if ((int64_t)total * per_chunk > 0x7FFFFFFF) return nx::fail(NX_EINVAL, "nx_fbm_batch: too many vertices");
+    const int steps = total * per_chunk;
+    const int grid = steps < sms ? steps : sms;
+    // cut the steps into grid ranges of equal estimated cost: a planet's
+    // step costs its vertices x (8 per octave + 1 per renormalised octave)
     std::vector<int64_t> wchunk(nplanets), cum(nplanets + 1, 0);
     for (int p = 0; p < nplanets; ++p) {
         const nx_fbm_planet &P = planets_host[p];
@@ -1632,25 +1815,25 @@ NX_EXPORT int nx_fbm_batch(const nx_fbm_planet *planets_dev, const nx_fbm_planet
         wchunk[p] = 8 * (int64_t)P.n_octaves + (int64_t)__builtin_popcount(P.norm_mask & live);
         cum[p + 1] = cum[p] + wchunk[p] * P.n;
     }
-    FbmSplit split;
     const int64_t tot = cum[nplanets];
     int p = 0;
     split.first[0] = 0;
     for (int b = 1; b <= grid; ++b) {
-        if (b == grid || tot == 0) { split.first[b] = total; continue; }
-        // first chunk whose cost prefix reaches b * tot / grid
+        if (b == grid || tot == 0) { split.first[b] = steps; continue; }
+        // first step whose cost prefix reaches b * tot / grid
         const int64_t t = (int64_t)((__int128)tot * b / grid);
         while (p + 1 < nplanets && cum[p + 1] <= t) ++p;
         const nx_fbm_planet &P = planets_host[p];
-        const int64_t per = wchunk[p] * CHUNK;
+        const int64_t per = wchunk[p] * U;
         int64_t k = per > 0 ? (t - cum[p] + per - 1) / per : 0;
-        const int64_t nch = (P.n + CHUNK - 1) / CHUNK;
-        if (k > nch) k = nch;
-        int c = P.chunk0 + (int)k;
+        const int64_t nst = (P.n + CHUNK - 1) / CHUNK * per_chunk;
+        if (k > nst) k = nst;
+        int c = P.chunk0 * per_chunk + (int)k;
         if (c < split.first[b - 1]) c = split.first[b - 1];
         split.first[b] = c;
     }
-    fbm_batch_kernel<<<grid, 256, TABLE_BYTES, (cudaStream_t)stream>>>(planets_dev, nplanets, split, n_fallback_dev);
+    fbm_batch_kernel<<<grid, PAIR_THREADS, TABLE_BYTES + split_bytes(split.S, max_oct), (cudaStream_t)stream>>>(
+        planets_dev, nplanets, split, n_fallback_dev);
     NX_CHECK_LAUNCH("fbm_batch_kernel");
     nx::note_launch(1);
     return NX_OK;

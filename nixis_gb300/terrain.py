@@ -44,7 +44,7 @@ def fbm(verts, perm, pgi, scale, strength, radius, out=None, accumulate=False, o
     p = _dev.to_device(perm, np.int32, (256,), "perm")
     g = _dev.to_device(pgi, np.int32, (256,), "pgi")
     if out is None:
-        out = torch.zeros(n, dtype=out_dtype, device="cuda")
+        out = torch.empty(n, dtype=out_dtype, device="cuda")     # written whole
         accumulate = False
     if out.shape != (n,) or not out.is_cuda or not out.is_contiguous():
         raise ValueError("out must be a contiguous CUDA tensor of shape (N,)")
