@@ -722,6 +722,12 @@ __device__ __forceinline__ float noise_raw(float xh, float xl, float yh, float y
 //    transforms (fma-exact products, two-sums; the running 2 - dx^2 - dy^2
 //    - dz^2 uses fast two-sums, exact whenever attn > 0), two slots at a
 //    time in paired binary32 lanes;
+//  * for the octaves below 1/8 of the largest amplitude, whose displacements
+//    are not renormalised, the squares are summed on a fixed grid and the
+//    two-sums ordered by a bias, 50 paired operations per two slots instead
+//    of 64; attn^2, attn^4 and the product keep the low parts' squares, which
+//    puts the error below that of the longer form without them (12 octaves:
+//    1.16e-14 of the field's norm against 1.44e-14);
 //  * the contributions, the division by 103 and the octave's
 //    (noise + 1) * 0.5 * strength * radius term are summed in pairs; the
 //    running sum over octaves is renormalised after every octave, so a
@@ -1287,7 +1293,8 @@ constexpr int PAIR_WARPS = PAIR_THREADS / 32;
 // groups of warps (S a power of two up to 16).  S = 1 where there are vertices
 // for every warp; small spheres and the remainder of large ones are split, so
 // that they fill the GPU with fewer octaves each: a warp's octave takes ~6 us
-// however few there are.
+// however few there are.  Measured (GB300, 12 octaves): 1,442 vertices 47.5
+// -> 14.9 us, 19,456 48.4 -> 21.7 us, 77,824 59.2 -> 55.3 us.
 constexpr int SPLIT_MAX = 16;
 
 // Shared memory of the octaves' values of a split step.
@@ -1426,6 +1433,7 @@ __device__ __forceinline__ void sum_split(const P_t &P, int n_oct, const double 
 // changes.  Sums are pairs (pair path above); the ordered keys of a block's
 // sums of a planet are folded into the planet's min/max once, when the
 // block leaves the planet (for the rescale to metres that follows).
+template <bool SPLIT>
 __global__ void __launch_bounds__(PAIR_THREADS, 1) fbm_batch_kernel(const nx_fbm_planet *__restrict__ planets, int np,
                                                                     const __grid_constant__ FbmSplit split,
                                                                     unsigned long long *nfb_out)
@@ -1436,7 +1444,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) fbm_batch_kernel(const nx_fbm
     __syncthreads();
     const uint32_t lb = lane_base(smem);
     float2 *part = reinterpret_cast<float2 *>(smem + TABLE_WORDS);
-    const int S = split.S, U = PAIR_THREADS / S, per = CHUNK / U;
+    const int S = SPLIT ? split.S : 1, U = PAIR_THREADS / S, per = CHUNK / U;
     const int u0 = split.first[blockIdx.x], u1 = split.first[blockIdx.x + 1];
     int cur = -1;
     unsigned nfb = 0;
@@ -1461,7 +1469,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) fbm_batch_kernel(const nx_fbm
         float rh = 0.0f, rl = 0.0f;
         const int64_t i = first + threadIdx.x;
         bool mine = i < P.n;
-        if (S == 1) {
+        if (!SPLIT) {
             if (mine) sum_octaves(P, P.n_octaves, load_triples(P.xyz, i), pow2, lb, nfb, rh, rl);
         } else {
             sum_split(P, P.n_octaves, P.xyz, first, P.n, S, pow2, lb, part, nfb, rh, rl);
@@ -1497,8 +1505,8 @@ struct FbmPairParams {
 // and/or written as binary64 (out64, = hi + lo exactly; accumulate adds to
 // it).  minmax (optional): ordered keys of the resulting pair sums.
 //
-// Vertices [0, main) in whole rounds of the grid, a thread a vertex; the
-// remainder split over its octaves, a step to a block (split_for).
+// Vertices [begin, n): a thread a vertex, or (SPLIT) a step of S octave
+// groups to a block.
 __device__ __forceinline__ OctP oct_of(const FbmPairParams &P, int o)
 {
     OctP O;
@@ -1507,8 +1515,9 @@ __device__ __forceinline__ OctP oct_of(const FbmPairParams &P, int o)
     return O;
 }
 
-__global__ void __launch_bounds__(PAIR_THREADS, 1) fbm_pair_kernel(const double *__restrict__ xyz, int64_t n, int64_t main,
-                                                                   int S, const int32_t *__restrict__ perm,
+template <bool SPLIT>
+__global__ void __launch_bounds__(PAIR_THREADS, 1) fbm_pair_kernel(const double *__restrict__ xyz, int64_t begin,
+                                                                   int64_t n, int S, const int32_t *__restrict__ perm,
                                                                    const int32_t *__restrict__ pgi,
                                                                    const __grid_constant__ FbmPairParams P,
                                                                    float2 *__restrict__ out2,
@@ -1537,21 +1546,20 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) fbm_pair_kernel(const double 
         kmx = k > kmx ? k : kmx;
     };
     const bool running = accumulate && out2;
-    for (int64_t i = (int64_t)blockIdx.x * PAIR_THREADS + threadIdx.x; i < main; i += (int64_t)gridDim.x * PAIR_THREADS) {
-        const float2 v = running ? out2[i] : make_float2(0.0f, 0.0f);
-        float rh = v.x, rl = v.y;
-        sum_octaves(P, P.n_oct, load_triples(xyz, i), pow2, lb, nfb, rh, rl);
-        put(i, rh, rl);
-    }
-    const int U = PAIR_THREADS / S;
-    const int64_t first = main + (int64_t)blockIdx.x * U;
-    if (first < n) {
-        const int64_t i = first + threadIdx.x;
+    if (!SPLIT) {
+        for (int64_t i = begin + (int64_t)blockIdx.x * PAIR_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * PAIR_THREADS) {
+            const float2 v = running ? out2[i] : make_float2(0.0f, 0.0f);
+            float rh = v.x, rl = v.y;
+            sum_octaves(P, P.n_oct, load_triples(xyz, i), pow2, lb, nfb, rh, rl);
+            put(i, rh, rl);
+        }
+    } else {
+        const int U = PAIR_THREADS / S;
+        const int64_t first = begin + (int64_t)blockIdx.x * U, i = first + threadIdx.x;
         const bool mine = i < n && (int)threadIdx.x < U;
         const float2 v = running && mine ? out2[i] : make_float2(0.0f, 0.0f);
         float rh = v.x, rl = v.y;
-        if (S > 1) sum_split(P, P.n_oct, xyz, first, n, S, pow2, lb, part, nfb, rh, rl);
-        else if (mine) sum_octaves(P, P.n_oct, load_triples(xyz, i), pow2, lb, nfb, rh, rl);
+        if (first < n) sum_split(P, P.n_oct, xyz, first, n, S, pow2, lb, part, nfb, rh, rl);
         if (mine) put(i, rh, rl);
     }
     if (minmax) {
@@ -1584,8 +1592,10 @@ int configure_smem()
     NX_CHECK_CUDA(cudaFuncSetAttribute(fbm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TABLE_BYTES));
     NX_CHECK_CUDA(cudaFuncSetAttribute(trace_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TABLE_BYTES));
     const int pair_bytes = TABLE_BYTES + (int)split_bytes(2, NX_MAX_OCTAVES);
-    NX_CHECK_CUDA(cudaFuncSetAttribute(fbm_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_bytes));
-    NX_CHECK_CUDA(cudaFuncSetAttribute(fbm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_bytes));
+    NX_CHECK_CUDA(cudaFuncSetAttribute(fbm_batch_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_bytes));
+    NX_CHECK_CUDA(cudaFuncSetAttribute(fbm_batch_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TABLE_BYTES));
+    NX_CHECK_CUDA(cudaFuncSetAttribute(fbm_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_bytes));
+    NX_CHECK_CUDA(cudaFuncSetAttribute(fbm_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TABLE_BYTES));
     smem_configured = true;
     return NX_OK;
 }
@@ -1759,17 +1769,29 @@ NX_EXPORT int nx_fbm_pair(const double *xyz_dev, int64_t n, const int32_t *perm_
     P.norm_mask = norm_mask(n_octaves, strength, radius, amp_ref);
     rc = configure_smem();
     if (rc) return rc;
-    // whole rounds of one block per SM, then the remainder, one step a block
+    // whole rounds of one block per SM, then the remainder by octaves (a
+    // round of its own, however few its vertices, would take as long as a
+    // warp's octaves one after the other)
     const int sms = nx::sm_count();
-    const int64_t round = (int64_t)sms * PAIR_THREADS, main = n / round * round, rest = n - main;
+    const int64_t round = (int64_t)sms * PAIR_THREADS, rest = n % round;
     const int S = split_for(rest, sms, n_octaves);
-    const int64_t steps = (rest * S + PAIR_THREADS - 1) / PAIR_THREADS;
-    const int grid = main > 0 ? sms : (int)(steps < 1 ? 1 : steps);
-    fbm_pair_kernel<<<grid, PAIR_THREADS, TABLE_BYTES + split_bytes(S, n_octaves), (cudaStream_t)stream>>>(
-        xyz_dev, n, main, S, perm_dev, pgi_dev, P, (float2 *)pair_dev, elev_f64_dev, accumulate, minmax_dev,
-        n_fallback_dev);
-    NX_CHECK_LAUNCH("fbm_pair_kernel");
-    nx::note_launch(1);
+    const int64_t main = S > 1 ? n - rest : n;
+    if (main > 0) {
+        const int64_t blocks = (main + PAIR_THREADS - 1) / PAIR_THREADS;
+        fbm_pair_kernel<false><<<(int)(blocks < sms ? blocks : sms), PAIR_THREADS, TABLE_BYTES, (cudaStream_t)stream>>>(
+            xyz_dev, 0, main, 1, perm_dev, pgi_dev, P, (float2 *)pair_dev, elev_f64_dev, accumulate, minmax_dev,
+            n_fallback_dev);
+        NX_CHECK_LAUNCH("fbm_pair_kernel");
+        nx::note_launch(1);
+    }
+    if (main < n) {
+        const int64_t steps = (rest * S + PAIR_THREADS - 1) / PAIR_THREADS;
+        fbm_pair_kernel<true><<<(int)steps, PAIR_THREADS, TABLE_BYTES + split_bytes(S, n_octaves), (cudaStream_t)stream>>>(
+            xyz_dev, main, n, S, perm_dev, pgi_dev, P, (float2 *)pair_dev, elev_f64_dev, accumulate, minmax_dev,
+            n_fallback_dev);
+        NX_CHECK_LAUNCH("fbm_pair_kernel");
+        nx::note_launch(1);
+    }
     return NX_OK;
 }
 
@@ -1832,7 +1854,8 @@ NX_EXPORT int nx_fbm_batch(const nx_fbm_planet *planets_dev, const nx_fbm_planet
         if (c < split.first[b - 1]) c = split.first[b - 1];
         split.first[b] = c;
     }
-    fbm_batch_kernel<<<grid, PAIR_THREADS, TABLE_BYTES + split_bytes(split.S, max_oct), (cudaStream_t)stream>>>(
+    const auto kernel = split.S > 1 ? fbm_batch_kernel<true> : fbm_batch_kernel<false>;
+    kernel<<<grid, PAIR_THREADS, TABLE_BYTES + split_bytes(split.S, max_oct), (cudaStream_t)stream>>>(
         planets_dev, nplanets, split, n_fallback_dev);
     NX_CHECK_LAUNCH("fbm_batch_kernel");
     nx::note_launch(1);
