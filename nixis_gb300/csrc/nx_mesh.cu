@@ -1365,32 +1365,93 @@ NX_EXPORT int nx_tiling_build(int k, int tile, int rings, const int32_t *nbr_dev
 // nearest vertices of a point are always among them (checked against brute
 // force in the tests).  Distances sqrt((dx*dx + dy*dy) + dz*dz), ascending,
 // ties by vertex id.
+//
+// Binary64 bounds a direct evaluation (180 operations for the faces, 16 for
+// each of 21 candidates, on a pipe of two per SM and cycle).  The location
+// needs no more than binary32: a point within its error of another face or
+// triangle has the same three among either's candidates.  The candidates are
+// ranked in binary32 as well; the four best are compared exactly, and only
+// where a fifth is not clearly farther than the third (the poles' rows, whose
+// neighbours are all alike) all of them.  Measured (GB300, 1024 x 512 queries,
+// 256,002 vertices): 636 -> 107 us.
 
 namespace {
+
+struct Best {
+    double d[3];
+    int64_t i[3];
+};
+
+__device__ __forceinline__ void best_take(Best &b, const double *xyz, int64_t v, double qx, double qy, double qz)
+{
+    if (v == b.i[0] || v == b.i[1] || v == b.i[2]) return;
+    const double dx = __dsub_rn(qx, xyz[3 * v]), dy = __dsub_rn(qy, xyz[3 * v + 1]), dz = __dsub_rn(qz, xyz[3 * v + 2]);
+    const double d = nxf::sqrt(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+        if (!(d < b.d[m] || (d == b.d[m] && v < b.i[m]))) continue;
+#pragma unroll
+        for (int r = 2; r > m; --r) { b.d[r] = b.d[r - 1]; b.i[r] = b.i[r - 1]; }
+        b.d[m] = d;
+        b.i[m] = v;
+        return;
+    }
+}
+
+__device__ __noinline__ void best_of_all(Best &b, const int32_t *tri, const double *xyz, const int32_t *nbr, int64_t nv, double qx,
+                                         double qy, double qz)
+{
+    for (int m = 0; m < 3; ++m) { b.d[m] = INFINITY; b.i[m] = -1; }
+    for (int c = 0; c < 21; ++c) {
+        const int32_t v = c < 3 ? tri[c] : nbr[6 * (int64_t)tri[(c - 3) / 6] + (c - 3) % 6];
+        if (v < 0 || (int64_t)v >= nv) continue;
+        best_take(b, xyz, v, qx, qy, qz);
+    }
+}
+
+// v * 2^-e as a binary32 (truncated), e the exponent that brings the query to
+// [1, 2); 0 below 2^-60 of it.
+__device__ __forceinline__ float scaled_chop(double v, uint32_t e20)
+{
+    const uint2 w = nxf::words(v);
+    const uint32_t a = (w.y & 0x7FFFFFFFu);
+    if (a + (60u << 20) < e20) return 0.0f;
+    if (a > e20 + (60u << 20)) return __int_as_float(0x7F800000);
+    const uint32_t s = a + (1023u << 20) - e20;
+    return __uint_as_float(__funnelshift_l(w.x, s - (896u << 20), 3) | (w.y & 0x80000000u));
+}
 
 __global__ void __launch_bounds__(256) nearest3_kernel(int k, const double *__restrict__ xyz,
                                                        const int32_t *__restrict__ nbr, int64_t nv,
                                                        const double *__restrict__ q, int64_t nq,
                                                        double *__restrict__ dist, int64_t *__restrict__ idx)
 {
+    __shared__ float s_inv[20][9];
+    for (int x = threadIdx.x; x < 180; x += blockDim.x) s_inv[x / 9][x % 9] = (float)c_ico.inv[x / 9][x % 9 / 3][x % 3];
+    __syncthreads();
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nq; p += (int64_t)gridDim.x * blockDim.x) {
         const double qx = q[3 * p], qy = q[3 * p + 1], qz = q[3 * p + 2];
+        // the query scaled to its largest component's binade
+        const uint32_t ex = nxf::words(qx).y & 0x7FF00000u, ey = nxf::words(qy).y & 0x7FF00000u, ez = nxf::words(qz).y & 0x7FF00000u;
+        const uint32_t e20 = max(ex, max(ey, ez));
+        const float x = scaled_chop(qx, e20), y = scaled_chop(qy, e20), z = scaled_chop(qz, e20);
         int bf = 0;
-        double bw[3] = {0, 0, 0}, bs = -INFINITY;
+        float bw0 = 0.0f, bw1 = 0.0f, bw2 = 0.0f, bs = -INFINITY;
         for (int f = 0; f < 20; ++f) {
-            double w[3];
-            for (int r = 0; r < 3; ++r) w[r] = c_ico.inv[f][r][0] * qx + c_ico.inv[f][r][1] * qy + c_ico.inv[f][r][2] * qz;
-            const double sc = fmin(w[0], fmin(w[1], w[2]));
-            if (sc > bs) { bs = sc; bf = f; bw[0] = w[0]; bw[1] = w[1]; bw[2] = w[2]; }
+            const float *m = s_inv[f];
+            const float w0 = fmaf(m[0], x, fmaf(m[1], y, m[2] * z)), w1 = fmaf(m[3], x, fmaf(m[4], y, m[5] * z)),
+                        w2 = fmaf(m[6], x, fmaf(m[7], y, m[8] * z));
+            const float sc = fminf(w0, fminf(w1, w2));
+            if (sc > bs) { bs = sc; bf = f; bw0 = w0; bw1 = w1; bw2 = w2; }
         }
-        const double tot = bw[0] + bw[1] + bw[2];
-        const double fi = fmin(fmax(bw[1] / tot, 0.0), 1.0) * k, fj = fmin(fmax(bw[2] / tot, 0.0), 1.0) * k;
-        int i0 = (int)floor(fi), j0 = (int)floor(fj);
+        const float tot = bw0 + bw1 + bw2;
+        const float fi = fminf(fmaxf(bw1 / tot, 0.0f), 1.0f) * (float)k, fj = fminf(fmaxf(bw2 / tot, 0.0f), 1.0f) * (float)k;
+        int i0 = (int)floorf(fi), j0 = (int)floorf(fj);
         if (i0 > k - 1) i0 = k - 1;
         if (i0 < 0) i0 = 0;
         if (j0 > k - 1 - i0) j0 = k - 1 - i0;
         if (j0 < 0) j0 = 0;
-        const bool up = (fi - i0) + (fj - j0) <= 1.0 || i0 + j0 == k - 1;
+        const bool up = (fi - i0) + (fj - j0) <= 1.0f || i0 + j0 == k - 1;
         int32_t tri[3];
         if (up) {
             tri[0] = face_vid(bf, i0, j0, k); tri[1] = face_vid(bf, i0 + 1, j0, k); tri[2] = face_vid(bf, i0, j0 + 1, k);
@@ -1398,26 +1459,44 @@ __global__ void __launch_bounds__(256) nearest3_kernel(int k, const double *__re
             tri[0] = face_vid(bf, i0 + 1, j0, k); tri[1] = face_vid(bf, i0 + 1, j0 + 1, k);
             tri[2] = face_vid(bf, i0, j0 + 1, k);
         }
-        double bd[3] = {INFINITY, INFINITY, INFINITY};
-        int64_t bi[3] = {-1, -1, -1};
+        // the four smallest binary32 squared distances, and the smallest left out
+        float a[4] = {INFINITY, INFINITY, INFINITY, INFINITY}, out = INFINITY;
+        int32_t id[4] = {-1, -1, -1, -1};
         for (int c = 0; c < 21; ++c) {
-            const int32_t v = c < 3 ? tri[c] : nbr[6 * (int64_t)tri[(c - 3) / 6] + (c - 3) % 6];
-            if (v < 0 || (int64_t)v >= nv) continue;
-            if (v == bi[0] || v == bi[1] || v == bi[2]) continue;
-            const double dx = __dsub_rn(qx, xyz[3 * (int64_t)v]), dy = __dsub_rn(qy, xyz[3 * (int64_t)v + 1]),
-                         dz = __dsub_rn(qz, xyz[3 * (int64_t)v + 2]);
-            const double d = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
-            int m = 3;
-            while (m > 0 && (d < bd[m - 1] || (d == bd[m - 1] && v < bi[m - 1]))) --m;
-            if (m < 3) {
-                for (int r = 2; r > m; --r) { bd[r] = bd[r - 1]; bi[r] = bi[r - 1]; }
-                bd[m] = d;
-                bi[m] = v;
-            }
+            const int t = (c - 3) / 6;
+            const int32_t v = c < 3 ? (c == 0 ? tri[0] : (c == 1 ? tri[1] : tri[2]))
+                                    : nbr[6 * (int64_t)(t == 0 ? tri[0] : (t == 1 ? tri[1] : tri[2])) + (c - 3) % 6];
+            if (v < 0 || (int64_t)v >= nv || v == id[0] || v == id[1] || v == id[2] || v == id[3]) continue;
+            const float dx = x - scaled_chop(xyz[3 * (int64_t)v], e20), dy = y - scaled_chop(xyz[3 * (int64_t)v + 1], e20),
+                        dz = z - scaled_chop(xyz[3 * (int64_t)v + 2], e20);
+            float d = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+            int32_t w = v;
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+                if (d < a[m]) {
+                    const float td = a[m];
+                    const int32_t ti = id[m];
+                    a[m] = d; id[m] = w;
+                    d = td; w = ti;
+                }
+            // (a vertex pushed out earlier may come again: it only lowers out to
+            // what it was)
+            out = fminf(out, d);
+        }
+        // a component is off by its truncation, below 2^-22 of the query: a
+        // distance by less than 2^-20
+        const float d3 = sqrtf(a[2]), d5 = sqrtf(out);
+        Best b;
+        if (d5 > d3 + 4e-6f && a[3] < INFINITY) {
+            for (int m = 0; m < 3; ++m) { b.d[m] = INFINITY; b.i[m] = -1; }
+#pragma unroll
+            for (int m = 0; m < 4; ++m) best_take(b, xyz, id[m], qx, qy, qz);
+        } else {
+            best_of_all(b, tri, xyz, nbr, nv, qx, qy, qz);
         }
         for (int m = 0; m < 3; ++m) {
-            dist[3 * p + m] = bd[m];
-            idx[3 * p + m] = bi[m];
+            dist[3 * p + m] = b.d[m];
+            idx[3 * p + m] = b.i[m];
         }
     }
 }
