@@ -59,6 +59,18 @@ unsigned long long nx_launch_count(void);
 int nx_perm_init(int64_t seed, int32_t *perm, int32_t *pgi);
 
 /* ------------------------------------------------------------------ */
+/* Small host tables                                                   */
+/* ------------------------------------------------------------------ */
+
+#define NX_UPLOAD_MAX 16000
+
+/* dst_dev[0, bytes) = src_host[0, bytes), at most NX_UPLOAD_MAX bytes, as
+ * kernel arguments on `stream`: src_host may be reused as soon as the call
+ * returns, the stream is not waited for, and under capture the bytes become
+ * part of the graph. */
+int nx_upload(void *dst_dev, const void *src_host, int64_t bytes, void *stream);
+
+/* ------------------------------------------------------------------ */
 /* Noise                                                               */
 /* ------------------------------------------------------------------ */
 
@@ -557,6 +569,20 @@ int nx_insolation_plan(const double *rot_deg, int n_rot, const double *tilt_deg,
  * a compensated total. */
 int nx_insolation(const double *xyz_dev, int64_t n, double radius, const float *table_dev, int n_rot_entries,
                   int pairs, int n_tilt, float *out_dev, int accumulate, void *stream);
+
+#define NX_MAX_POSITIONS 2000
+
+/* nx_insolation for a schedule on the host (degrees; n_rot + n_tilt <=
+ * NX_MAX_POSITIONS): the plan, its upload into table_dev (scratch, 2*(n_rot +
+ * n_tilt) floats, in use until the stream has passed this call) and the sums,
+ * each times (float)scale. */
+int nx_insolation_positions(const double *xyz_dev, int64_t n, double radius, const double *rot_deg, int n_rot,
+                            const double *tilt_deg, int n_tilt, double scale, float *table_dev, float *out_dev,
+                            int accumulate, void *stream);
+
+/* Host: tilt_deg[d] = climate.calculate_seasonal_tilt(axial_tilt,
+ * climate.day2deg(year_length, d)) (climate.py:167-201) for d < days. */
+int nx_seasonal_tilts(double axial_tilt, double year_length, int days, double *tilt_deg);
 
 /* One planet of a batched insolation launch: its vertices and radius; its
  * sums go to packed output rows [vbeg, vbeg + n) (vbeg a multiple of 256). */

@@ -20,6 +20,7 @@ SIGNATURES = {
     "nx_last_error": (ctypes.c_char_p, []),
     "nx_version": (_i32, []),
     "nx_launch_count": (_u64, []),
+    "nx_upload": (_i32, [_p, _p, _i64, _p]),
     "nx_perm_init": (_i32, [_i64, _p, _p]),
     "nx_fbm": (_i32, [_p, _i64, _p, _p, _i32, _p, _p, _d, _p, _p, _i32, _p, _p]),
     "nx_sample_octaves": (_i32, [_p, _i64, _p, _p, _i32, _d, _d, _d, _d, _d, _p, _p, _i32, _p]),
@@ -41,6 +42,8 @@ SIGNATURES = {
     "nx_erosion_store": (_i32, [_p, _i64, _p, _p, _p, _p, _p]),
     "nx_steepest_descent": (_i32, [_p, _p, _i64, _p, _p, _p]),
     "nx_insolation_plan": (_i32, [_p, _i32, _p, _i32, _p, _p, _p]),
+    "nx_insolation_positions": (_i32, [_p, _i64, _d, _p, _i32, _p, _i32, _d, _p, _p, _i32, _p]),
+    "nx_seasonal_tilts": (_i32, [_d, _d, _i32, _p]),
     "nx_insolation": (_i32, [_p, _i64, _d, _p, _i32, _i32, _i32, _p, _i32, _p]),
     "nx_insolation_batch": (_i32, [_p, _p, _i32, _p, _i32, _i32, _i32, _p, _p]),
     "nx_fbm_planet_fill": (_i32, [_p, _i32, _p, _p, _d]),

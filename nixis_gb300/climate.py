@@ -43,24 +43,50 @@ def _plan(rot_deg, tilt_deg):
     return tab[:used], nre.value, pairs.value
 
 
-def insolation_sum(verts, radius, rotations, tilts, out=None, accumulate=False, stream=None):
-    """Sum over every (tilt, rotation) of sample_insolation's term.
+# Schedules up to this many positions go to the device as kernel arguments
+# (nx_insolation_positions); longer ones as a table of their own.
+MAX_POSITIONS = 2000
 
-    verts float64 (N,3) (CUDA tensor or numpy); rotations/tilts in degrees.
-    Returns a float32 CUDA tensor (N,) (or adds into `out`)."""
+
+def _sum(verts, radius, rotations, tilts, out, accumulate, stream, scale=None):
+    """insolation_sum, each sum times binary32 `scale`."""
     xyz = _dev.to_device(verts, np.float64, name="verts")
     _dev.check_vertices(xyz)
     n = xyz.shape[0]
-    tab, nre, pairs = _plan(rotations, tilts)
-    tdev = _dev.to_device(tab, np.float32, name="table")
+    rot = np.ascontiguousarray(rotations, np.float64)
+    tilt = np.ascontiguousarray(tilts, np.float64)
+    short = len(rot) + len(tilt) <= MAX_POSITIONS
+    if short:
+        tdev = torch.empty(2 * (len(rot) + len(tilt)), dtype=torch.float32, device="cuda")
+    else:
+        tab, nre, pairs = _plan(rot, tilt)
+        tdev = _dev.to_device(tab, np.float32, name="table")
     if out is None:
         out = torch.empty(n, dtype=torch.float32, device="cuda")
         accumulate = False
     if out.dtype != torch.float32 or out.shape != (n,) or not out.is_cuda:
         raise ValueError("out must be a float32 CUDA tensor of shape (N,)")
-    call("nx_insolation", _dev.ptr(xyz), n, float(radius), _dev.ptr(tdev), nre, pairs, len(tilts), _dev.ptr(out),
-         1 if accumulate else 0, _dev.stream_handle(stream))
+    if stream is not None:
+        tdev.record_stream(stream)
+    if short:
+        vp = ctypes.c_void_p
+        call("nx_insolation_positions", _dev.ptr(xyz), n, float(radius), vp(rot.ctypes.data), len(rot),
+             vp(tilt.ctypes.data), len(tilt), 1.0 if scale is None else float(scale), _dev.ptr(tdev), _dev.ptr(out),
+             1 if accumulate else 0, _dev.stream_handle(stream))
+    else:
+        call("nx_insolation", _dev.ptr(xyz), n, float(radius), _dev.ptr(tdev), nre, pairs, len(tilt), _dev.ptr(out),
+             1 if accumulate else 0, _dev.stream_handle(stream))
+        if scale is not None:
+            out.mul_(scale)
     return out
+
+
+def insolation_sum(verts, radius, rotations, tilts, out=None, accumulate=False, stream=None):
+    """Sum over every (tilt, rotation) of sample_insolation's term.
+
+    verts float64 (N,3) (CUDA tensor or numpy); rotations/tilts in degrees.
+    Returns a float32 CUDA tensor (N,) (or adds into `out`)."""
+    return _sum(verts, radius, rotations, tilts, out, accumulate, stream)
 
 
 def sample_insolation(arr, verts, radius, rotation, tilt):
@@ -72,7 +98,7 @@ def sample_insolation(arr, verts, radius, rotation, tilt):
             raise ValueError("arr must be a C-contiguous float32 array")
         dev = _dev.to_device(arr, np.float32)
         insolation_sum(verts, radius, [float(rotation)], [float(tilt)], out=dev, accumulate=True)
-        arr[...] = dev.cpu().numpy()
+        _dev.to_host(arr, dev)
         return
     insolation_sum(verts, radius, [float(rotation)], [float(tilt)], out=arr, accumulate=True)
 
@@ -83,8 +109,7 @@ def brute_daily_insolation(verts, altitudes, radius, tilt, snapshot=False):
     if snapshot:
         raise NotImplementedError("insolation snapshots (PNG export) are not provided by nixis_gb300")
     host = _dev.is_host(verts)
-    rot = [-180.0 + i * 1.0 for i in range(360)]
-    out = insolation_sum(verts, radius, rot, [float(tilt)])
+    out = insolation_sum(verts, radius, np.arange(-180.0, 180.0), [float(tilt)])
     return out.cpu().numpy() if host else out
 
 
@@ -104,8 +129,18 @@ def annual_schedule(axial_tilt=23.44, year_length=365, days=365, hours=24):
     for _ in range(hours):
         rot.append(r)
         r += rot_amt
-    tilts = [calculate_seasonal_tilt(axial_tilt, day2deg(year_length, d)) for d in range(days)]
-    return rot, tilts
+    return rot, _seasonal_tilts(axial_tilt, year_length, days)
+
+
+def _seasonal_tilts(axial_tilt, year_length, days):
+    # plain numbers of ordinary size: the same sums and sines, natively (365
+    # days: 60 us in Python)
+    if (type(days) is int and 0 < days < 1 << 24 and type(axial_tilt) in (int, float) and abs(axial_tilt) < 1e15
+            and type(year_length) in (int, float) and 1e-9 < abs(year_length) < 1e15):
+        t = np.empty(days, np.float64)
+        call("nx_seasonal_tilts", float(axial_tilt), float(year_length), days, ctypes.c_void_p(t.ctypes.data))
+        return t.tolist()
+    return [calculate_seasonal_tilt(axial_tilt, day2deg(year_length, d)) for d in range(days)]
 
 
 def annual_insolation(verts, radius, axial_tilt=23.44, year_length=365, days=365, hours=24, mean_wm2=False,
@@ -114,10 +149,8 @@ def annual_insolation(verts, radius, axial_tilt=23.44, year_length=365, days=365
     (float32 CUDA tensor).  With mean_wm2, converted to the mean top-of-
     atmosphere flux: SOLAR_CONSTANT * sum / (days * hours)."""
     rot, tilts = annual_schedule(axial_tilt, year_length, days, hours)
-    s = insolation_sum(verts, radius, rot, tilts, out=out, stream=stream)
-    if mean_wm2:
-        s.mul_(SOLAR_CONSTANT / (days * hours))
-    return s
+    scale = SOLAR_CONSTANT / (days * hours) if mean_wm2 else None
+    return _sum(verts, radius, rot, tilts, out, False, stream, scale)
 
 
 _tables = {}
@@ -160,7 +193,7 @@ def interpolate_insolation(verts, lookup_table, insolation, radius):
     call("nx_interpolate_insolation", _dev.ptr(xyz), n, float(radius), _dev.ptr(tab), 1, _dev.ptr(out), 0,
          _dev.stream_handle())
     if host:
-        insolation[...] = out.cpu().numpy()
+        _dev.to_host(insolation, out)
 
 
 def calc_daily_insolation(verts, altitudes, radius, tilt):

@@ -61,6 +61,7 @@ struct InsoArgs {
     int pairs;             // 1: each rot entry stands for theta and theta + 180
     float *out;
     int accumulate;
+    float scale;           // of the sums (1: none)
 };
 
 __host__ __device__ __forceinline__ void radius_pair(double r, float &h, float &l)
@@ -751,7 +752,10 @@ __global__ void __launch_bounds__(256, 4) insolation_kernel(InsoArgs a)
         if (j < a.n) { X = a.xyz[3 * j]; Y = a.xyz[3 * j + 1]; Z = a.xyz[3 * j + 2]; }
         const float tot = inso_vertex<HP>(a, cx, cy, cz, a.r, a.r2h, a.r2l, a.zmin, a.inv_r, staged ? s_tilt : nullptr,
                                           bk, arc);
-        a.out[i] = a.accumulate ? a.out[i] + tot : tot;
+        // the scale here instead of in a pass of its own over the sums (10 M
+        // vertices: 11 us of 137)
+        const float v = __fmul_rn(tot, a.scale);
+        a.out[i] = a.accumulate ? a.out[i] + v : v;
     }
 }
 
@@ -987,8 +991,8 @@ NX_EXPORT int nx_insolation_plan(const double *rot_deg, int n_rot, const double 
     return NX_OK;
 }
 
-NX_EXPORT int nx_insolation(const double *xyz_dev, int64_t n, double radius, const float *table_dev, int n_rot_entries,
-                            int pairs, int n_tilt, float *out_dev, int accumulate, void *stream)
+static int insolation_sums(const double *xyz_dev, int64_t n, double radius, const float *table_dev, int n_rot_entries,
+                           int pairs, int n_tilt, float scale, float *out_dev, int accumulate, void *stream)
 {
     if (n < 0 || n_rot_entries < 0 || n_tilt < 0) return nx::fail(NX_EINVAL, "nx_insolation: negative size");
     if (n == 0) return NX_OK;
@@ -1014,6 +1018,7 @@ NX_EXPORT int nx_insolation(const double *xyz_dev, int64_t n, double radius, con
     a.n_tilt = n_tilt;
     a.out = out_dev;
     a.accumulate = accumulate;
+    a.scale = scale;
     if (a.pairs && n_rot_entries == 12)
         insolation_kernel<12><<<grid_staged(n, a), 256, tilt_smem(a), s>>>(a);
     else if (use_arcs(a, n))
@@ -1022,6 +1027,45 @@ NX_EXPORT int nx_insolation(const double *xyz_dev, int64_t n, double radius, con
         insolation_kernel<0><<<grid_for(n), 256, 0, s>>>(a);
     NX_CHECK_LAUNCH("insolation_kernel");
     nx::note_launch(1);
+    return NX_OK;
+}
+
+NX_EXPORT int nx_insolation(const double *xyz_dev, int64_t n, double radius, const float *table_dev, int n_rot_entries,
+                            int pairs, int n_tilt, float *out_dev, int accumulate, void *stream)
+{
+    return insolation_sums(xyz_dev, n, radius, table_dev, n_rot_entries, pairs, n_tilt, 1.0f, out_dev, accumulate, stream);
+}
+
+NX_EXPORT int nx_insolation_positions(const double *xyz_dev, int64_t n, double radius, const double *rot_deg, int n_rot,
+                                      const double *tilt_deg, int n_tilt, double scale, float *table_dev, float *out_dev,
+                                      int accumulate, void *stream)
+{
+    if (n < 0 || n_rot < 0 || n_tilt < 0 || n_rot + (int64_t)n_tilt > NX_MAX_POSITIONS)
+        return nx::fail(NX_EINVAL, "nx_insolation_positions: bad sizes");
+    if (n == 0) return NX_OK;
+    if (n_rot && n_tilt && !table_dev) return nx::fail(NX_EINVAL, "nx_insolation_positions: null pointer");
+    float table[2 * NX_MAX_POSITIONS];
+    int entries = 0, pairs = 0;
+    int rc = nx_insolation_plan(rot_deg, n_rot, tilt_deg, n_tilt, table, &entries, &pairs);
+    if (rc) return rc;
+    if (n_rot && n_tilt) {
+        rc = nx_upload(table_dev, table, (int64_t)sizeof(float) * 2 * (entries + n_tilt), stream);
+        if (rc) return rc;
+    }
+    return insolation_sums(xyz_dev, n, radius, table_dev, entries, pairs, n_tilt, (float)scale, out_dev, accumulate, stream);
+}
+
+// climate.calculate_seasonal_tilt(axial, climate.day2deg(year, d)) for days
+// d = 0..days-1, in the reference's order of operations (climate.py:171,
+// 201) with the C library's sine, the one Python's math.sin calls.
+NX_EXPORT int nx_seasonal_tilts(double axial_tilt, double year_length, int days, double *tilt_deg)
+{
+    if (days < 0 || (days && !tilt_deg)) return nx::fail(NX_EINVAL, "nx_seasonal_tilts: bad arguments");
+    const double PI = 3.141592653589793;
+    for (int d = 0; d < days; ++d) {
+        const double deg = (double)d / year_length * 360.0;
+        tilt_deg[d] = sin(deg * PI / 180) * axial_tilt;
+    }
     return NX_OK;
 }
 
@@ -1052,6 +1096,7 @@ NX_EXPORT int nx_insolation_batch(const nx_inso_planet *planets_dev, const nx_in
     a.n_tilt = n_tilt;
     a.out = out_dev;
     a.accumulate = 0;
+    a.scale = 1.0f;
     cudaStream_t s = (cudaStream_t)stream;
     if (a.pairs && n_rot_entries == 12)
         insolation_batch_kernel<12><<<grid_staged(total, a), 256, tilt_smem(a), s>>>(a, planets_dev, nplanets, total);

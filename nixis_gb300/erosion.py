@@ -203,10 +203,10 @@ def _run_inplace(verts, neighbors, h, w, s, iters, rain, with_fields):
     else:
         run.store(hd)
     if host:
-        h[...] = hd.cpu().numpy()
+        _dev.to_host(h, hd)
         if w is not None:
-            w[...] = wd.cpu().numpy()
-            s[...] = sd.cpu().numpy()
+            _dev.to_host(w, wd)
+            _dev.to_host(s, sd)
     else:
         for dst, src in ((h, hd), (w, wd), (s, sd)):
             if dst is not None and dst.data_ptr() != src.data_ptr():

@@ -99,7 +99,7 @@ def sort_adjacency(adj, stream=None):
     out = torch.empty_like(a)
     call("nx_sort_adjacency", _dev.ptr(a), _dev.ptr(out), a.shape[0], _dev.stream_handle(stream))
     if host:
-        adj[...] = out.cpu().numpy()
+        _dev.to_host(adj, out)
     else:
         adj.copy_(out)
     return adj

@@ -466,8 +466,7 @@ def generate_plain(request, meshes=None, sync=True, out=None, blocked=False):
     ins = None
     if r.insolation:
         rot, tilts = _climate.annual_schedule(r.axial_tilt, r.days, r.days, r.hours)
-        ins = _climate.insolation_sum(m.xyz, r.radius, rot, tilts)
-        ins.mul_(_climate.SOLAR_CONSTANT / (r.days * r.hours))
+        ins = _climate._sum(m.xyz, r.radius, rot, tilts, None, False, None, _climate.SOLAR_CONSTANT / (r.days * r.hours))
     if sync:
         torch.cuda.synchronize()
     return PlanetResult(r, heights, ins, 0)

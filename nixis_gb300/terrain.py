@@ -88,7 +88,7 @@ def sample_octaves(verts, elevations, perm, pgi, n_octaves=1, n_init_roughness=1
             raise ValueError("elevations must be a C-contiguous float64 array")
         dev = _dev.to_device(elevations, np.float64)
         fbm(verts, perm, pgi, scale, strength, world_radius, out=dev, accumulate=True)
-        elevations[...] = dev.cpu().numpy()
+        _dev.to_host(elevations, dev)
         return elevations
     fbm(verts, perm, pgi, scale, strength, world_radius, out=elevations, accumulate=True)
     return elevations

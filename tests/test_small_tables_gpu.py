@@ -1,0 +1,78 @@
+"""Host tables as kernel arguments, schedules by one native call, and results written straight into host arrays.
+
+Everything here is copied or computed by the same operations as on the general path, so every comparison is exact."""
+import ctypes
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from nixis_gb300 import _dev, _lib, climate, mesh  # noqa: E402
+
+gpu = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("axial, year, days", [(23.44, 365, 365), (-7.5, 88.25, 1), (0, 3, 40), (97, -12.5, 700)])
+def test_seasonal_tilts_are_the_reference_sums(axial, year, days):
+    want = [climate.calculate_seasonal_tilt(axial, climate.day2deg(year, d)) for d in range(days)]
+    assert climate.annual_schedule(axial, year, days, 24)[1] == want
+
+
+@pytest.mark.parametrize("axial, year", [(np.float32(23.44), 365), (23.44, np.int64(12)), (23.44, 1e-300)])
+def test_other_number_types_keep_pythons_arithmetic(axial, year):
+    want = [climate.calculate_seasonal_tilt(axial, climate.day2deg(year, d)) for d in range(1)]
+    assert climate.annual_schedule(axial, year, 1, 2)[1] == want
+    with pytest.raises(ZeroDivisionError):
+        climate.annual_schedule(23.44, 0, 2, 2)
+
+
+@gpu
+@pytest.mark.parametrize("off", [0, 1, 4])
+@pytest.mark.parametrize("n", [0, 1, 3, 4, 255, 3999, 4000, 4001, 8000, 15999, 16000])
+def test_upload_sizes_and_alignments(n, off):
+    src = np.random.default_rng(n).integers(0, 256, n, np.uint8)
+    want = src.copy()
+    dst = torch.full((n + 16,), 77, dtype=torch.uint8, device="cuda")
+    torch.cuda._sleep(1000)
+    _lib.call("nx_upload", ctypes.c_void_p(dst.data_ptr() + off), ctypes.c_void_p(src.ctypes.data), n, _dev.stream_handle())
+    src[:] = 0                                   # the bytes were taken by the call
+    got = dst.cpu().numpy()
+    assert np.array_equal(got[off:off + n], want)
+    assert (got[:off] == 77).all() and (got[off + n:] == 77).all()
+    with pytest.raises(_lib.NxError):
+        _lib.call("nx_upload", ctypes.c_void_p(dst.data_ptr()), ctypes.c_void_p(got.ctypes.data), 16001, None)
+
+
+@gpu
+@pytest.mark.parametrize("n", [1999, 2000, 2001, 2500])
+def test_arrays_around_the_upload_limit(n):
+    a = np.random.default_rng(n).random(2 * n)[::2]          # strided
+    b = a.copy()
+    t = _dev.to_device(a, np.float64)
+    a[:] = 0.0
+    assert np.array_equal(t.cpu().numpy(), b)
+    for out in (np.zeros(n), np.zeros(2 * n)[::2], np.zeros(n, np.float32), np.zeros(2 * n)[::-2]):
+        _dev.to_host(out, t)
+        assert np.array_equal(out, b.astype(out.dtype))
+    ro = np.zeros(n)
+    ro.flags.writeable = False
+    with pytest.raises(ValueError):
+        _dev.to_host(ro, t)
+
+
+@gpu
+@pytest.mark.parametrize("n_rot, n_tilt", [(24, 365), (7, 3), (0, 4), (1600, 400), (1601, 400)])
+def test_schedules_by_arguments_and_by_table(n_rot, n_tilt):
+    m = mesh.PlanetMesh(9)
+    rot, tilt = [-180.0 + 360.0 / max(n_rot, 1) * i for i in range(n_rot)], list(np.linspace(-30.0, 31.0, n_tilt))
+    tab, nre, pairs = climate._plan(rot, tilt)
+    tdev = torch.from_numpy(tab).cuda()
+    want = torch.empty(m.n, dtype=torch.float32, device="cuda")
+    _lib.call("nx_insolation", _dev.ptr(m.xyz), m.n, 1.0, _dev.ptr(tdev), nre, pairs, n_tilt, _dev.ptr(want), 0,
+              _dev.stream_handle())
+    assert torch.equal(climate.insolation_sum(m.xyz, 1.0, rot, tilt), want)
+    assert torch.equal(climate._sum(m.xyz, 1.0, rot, tilt, None, False, torch.cuda.current_stream(), 1361.0 / 77), want * (1361.0 / 77))
+    out = want.clone()
+    climate.insolation_sum(m.xyz, 1.0, rot, tilt, out=out, accumulate=True)
+    assert torch.equal(out, want + want)
