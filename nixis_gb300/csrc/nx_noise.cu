@@ -7,9 +7,10 @@
 //  * One thread per vertex, all octaves in registers; persistent grid of
 //    (#SM x resident CTAs) walking the vertex range.
 //  * The seeded tables live in shared memory as one packed word per entry
-//    [bits 0-6: gz+16 | bits 7-14: perm | bits 16-23: gx+16 | 24-31: gy+16],
-//    replicated 32 times (entry k of lane l at word 32*k + l) so the three
-//    dependent hash loads of a warp never conflict on a bank.
+//    (perm in bits 7-14, the gradient's byte offset above), replicated 32
+//    times (entry k of lane l at word 32*k + l) so the three dependent hash
+//    loads of a warp never conflict on a bank; the gradients are binary32,
+//    one copy per lane too.
 //  * Arithmetic is binary32.  The lattice cell, the region and the two extra
 //    lattice points must equal what binary64 decides.  The large-magnitude
 //    part of the skew is removed exactly: x*scale is formed as a float pair,
@@ -20,13 +21,23 @@
 //    |x*scale| < 2^16 (the bound is worked through at decide_f32).  Every
 //    comparison that decides the cell or region records its margin; the
 //    compared quantities combine up to three such terms with a few more
-//    roundings (errors below 1.3e-6), and when the smallest margin is below
-//    TAU = 4e-6 (> 3x that), or |x*scale| >= 2^16, that lane recomputes the
+//    roundings (errors below 1.6e-6), and when the smallest margin is below
+//    TAU = 4e-6 (2.5x that), or |x*scale| >= 2^16, that lane recomputes the
 //    decisions in binary64 with the reference's operation order
 //    (decide_f64), so the decisions always equal the reference's.
-//  * The 6 or 8 contributions are evaluated branch-free as 9 slots: the
-//    corner (0,0,0)|(1,1,1), the six mixed corners, and the two extra points,
-//    with masks per region; hash prefixes of the fixed slots are shared.
+//  * The 6 or 8 contributions are evaluated branch-free as four pairs of
+//    slots: a region's first four fixed corners (offsets from a table by
+//    region), the octahedron's other two (masked), the two extra points
+//    (offsets and hash steps from a table by case); hash prefixes of the
+//    fixed slots are shared.
+//  * Both kernels are bound by instruction issue (binary32: 81 % of the slots,
+//    320 instructions per vertex and octave) and, in pairs, as much by the FMA
+//    pipe (68 %).  Measured on 10,000,002 vertices x 12 octaves: case numbers
+//    from sign bits and cases SoA 1570 -> 1385 us in binary32 and 3131 -> 2969
+//    in pairs, slots by region 1385 -> 1299 (binary32), gradients by single
+//    loads, tables in operand order and the rest of the shorter chain 1299 ->
+//    1184 and 2965 -> 2750.  Skipping the octahedron's pair where no lane
+//    needs it: 1226 and 2750 (nearly every warp has one).
 #include "nx_common.cuh"
 
 #include <vector>
@@ -41,7 +52,6 @@ constexpr float TAU = 4.0e-6f;         // decision margin below which binary64 d
 constexpr float PMAX = 65536.0f;       // |x*scale| bound of the binary32 decision path
 constexpr float THIRD = 1.0f / 3.0f;
 constexpr float SIXTH = 1.0f / 6.0f;
-constexpr float GBIAS = 8388624.0f;    // 2^23 + 16: removes the byte bias of a packed gradient
 
 // opensimplex.py:51-60 (GRADIENTS_3D), used only to build the packed table.
 __constant__ int c_grad3[72] = {
@@ -59,7 +69,8 @@ struct FbmParams {
     int n_oct;
     float s_hi[NX_MAX_OCTAVES];   // scale[o] as a binary32 pair
     float s_lo[NX_MAX_OCTAVES];
-    float amp[NX_MAX_OCTAVES];    // 0.5 * strength[o] * radius
+    float amp[NX_MAX_OCTAVES];    // 0.5 * strength[o] * radius / 103
+    float base;                   // sum over octaves of 0.5 * strength[o] * radius
     double s[NX_MAX_OCTAVES];     // scale[o] (binary64 decision path)
 };
 
@@ -68,66 +79,56 @@ static_assert(sizeof(nx_fbm_planet) == 960, "fBm planet descriptor layout");
 constexpr int TABLE_WORDS = 256 * 32;
 constexpr int TABLE_BYTES = TABLE_WORDS * 4;
 
-// A warp fills runs of 32 entries: each lane forms one entry's word (two
-// global reads a lane, all in flight together), then the 32 words go out one
-// by one to their 32 replicas, a conflict-free store each.
-template <typename F>
-__device__ __forceinline__ void fill_table(uint32_t *T, const int32_t *__restrict__ perm, const int32_t *__restrict__ pgi,
-                                           F word)
+// GRADIENTS_3D as binary32, per component and lane (entry 32 i + lane of
+// component c at s_gr[768 c + 32 i + lane]: no bank conflicts), in the order
+// of the component that is +-11: i = 8 axis + (0-7) (every gradient has one
+// +-11 and two +-4 components).  Three single loads a slot go straight into
+// the halves of the paired operands; one 16-byte load took moves to get there.
+__shared__ float s_gr[3 * 768];
+
+__device__ __forceinline__ void init_grad_table()
 {
-    const int lane = threadIdx.x & 31;
-    for (int k0 = (threadIdx.x >> 5) * 32; k0 < 256; k0 += blockDim.x) {
-        const uint32_t p = (uint32_t)perm[k0 + lane] & 255u;
-        int g = pgi[k0 + lane];
-        g = g < 0 ? 0 : (g > 69 ? 69 : g);
-        const uint32_t w = word(p, g);
-#pragma unroll 8
-        for (int j = 0; j < 32; ++j) T[32 * (k0 + j) + lane] = __shfl_sync(0xFFFFFFFFu, w, j);
+    for (int j = threadIdx.x; j < 768; j += blockDim.x) {
+        const int i = j >> 5, row = 3 * (i & 7) + (i >> 3);
+        for (int c = 0; c < 3; ++c) s_gr[768 * c + j] = (float)c_grad3[3 * row + c];
     }
 }
 
-__device__ __forceinline__ void build_table(uint32_t *T, const int32_t *__restrict__ perm,
-                                            const int32_t *__restrict__ pgi)
-{
-    fill_table(T, perm, pgi, [](uint32_t p, int g) {
-        return ((uint32_t)(c_grad3[g + 2] + 16) & 0x7Fu) | (p << 7) | ((uint32_t)(c_grad3[g] + 16) << 16) |
-               ((uint32_t)(c_grad3[g + 1] + 16) << 24);
-    });
-}
+// The hash table (TABLE_WORDS), at the start of the block's dynamic memory.
+// A lane's word of an entry: perm in bits 7-14, and from bit 18 on the byte
+// offset of the entry's gradient in s_gr for this lane, 128 i + 4 lane (so
+// the gradient's axis is bits 26-27).
+extern __shared__ __align__(16) uint32_t smem[];
 
-// The pair path's table: the same layout with the gradient's index (0-23,
-// perm_grad_index_3D / 3) in bits 0-4 instead of the gradient bytes; the
-// gradients themselves come as binary32 from s_grad.
-__device__ __forceinline__ void build_table_pair(uint32_t *T, const int32_t *__restrict__ perm,
-                                                 const int32_t *__restrict__ pgi)
+// A warp fills runs of 32 entries: each lane forms one entry's word (two
+// global reads a lane, all in flight together), then the 32 words go out one
+// by one to their 32 replicas, a conflict-free store each.
+__device__ __forceinline__ void build_table(const int32_t *__restrict__ perm, const int32_t *__restrict__ pgi)
 {
-    fill_table(T, perm, pgi, [](uint32_t p, int g) { return (uint32_t)(g / 3) | (p << 7); });
-}
-
-// GRADIENTS_3D as binary32 (x, y, z, 0), and as sign masks (bit 31 of each
-// component) with the axis of the +-11 component (every gradient has one
-// +-11 and two +-4 components), filled per block.
-__shared__ float4 s_grad[24];
-__shared__ uint4 s_gsign[24];
-
-__device__ __forceinline__ void init_grad_table(int i)
-{
-    if (i >= 0 && i < 24) {
-        const int gx = c_grad3[3 * i], gy = c_grad3[3 * i + 1], gz = c_grad3[3 * i + 2];
-        s_grad[i] = make_float4((float)gx, (float)gy, (float)gz, 0.0f);
-        const uint32_t a = (gx == 11 || gx == -11) ? 0u : ((gy == 11 || gy == -11) ? 1u : 2u);
-        s_gsign[i] = make_uint4(gx < 0 ? 0x80000000u : 0u, gy < 0 ? 0x80000000u : 0u, gz < 0 ? 0x80000000u : 0u, a);
+    const uint32_t lane = threadIdx.x & 31;
+    for (int k0 = (threadIdx.x >> 5) * 32; k0 < 256; k0 += blockDim.x) {
+        const uint32_t p = (uint32_t)perm[k0 + lane] & 255u;
+        int g = pgi[k0 + lane];
+        g = (g < 0 ? 0 : (g > 69 ? 69 : g)) / 3;
+        const uint32_t w = p << 7 | (uint32_t)(8 * (g % 3) + g / 3) << 23;
+#pragma unroll 8
+        for (int j = 0; j < 32; ++j) smem[32 * (k0 + j) + lane] = __shfl_sync(0xFFFFFFFFu, w, j) | lane << 18;
     }
 }
 
 // Hash table load: bits 7-14 of a select the entry; lb = this lane's byte
-// offset of replica 0 in shared memory.
+// offset in an entry's 32 words.  The table's own address goes into the
+// load, so an address is one three-input logic operation (19 lookups per
+// vertex and octave).
 __device__ __forceinline__ uint32_t lk(uint32_t lb, int a)
 {
-    uint32_t v;
-    uint32_t addr = lb + ((uint32_t)a & 0x7F80u);
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
-    return v;
+    return *reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(smem) + (((uint32_t)a & 0x7F80u) | lb));
+}
+
+// Component c of the gradient of a table word.
+__device__ __forceinline__ float grad_of(uint32_t w, int c)
+{
+    return *reinterpret_cast<const float *>(reinterpret_cast<const char *>(s_gr + 768 * c) + (w >> 16));
 }
 
 // Split a binary64 into hi + lo binary32 with integer operations (no FP64
@@ -159,43 +160,29 @@ __device__ __forceinline__ void split_f64(double v, float &hi, float &lo)
 struct Decision {
     int region;
     float e0x, e0y, e0z, e1x, e1y, e1z;   // decide() only
-    uint32_t w;                           // the offsets + 1, two bits each (e0x, e0y, e0z, e1x, e1y, e1z)
+    uint32_t w0, w1;                      // step words of the two extra points (pack_step)
     float E[6];                           // displacement offsets e + (ex + ey + ez) / 3 of both points
 };
 
-template <typename T, bool TRACK>
-struct Cmp {
-    float m;
-    __device__ __forceinline__ void note(T a, T b)
-    {
-        if (TRACK) m = fminf(m, fabsf((float)(a - b)));
-    }
-    __device__ __forceinline__ bool gt(T a, T b) { note(a, b); return a > b; }
-    __device__ __forceinline__ bool ge(T a, T b) { note(a, b); return a >= b; }
-    __device__ __forceinline__ bool lt(T a, T b) { note(a, b); return a < b; }
-    __device__ __forceinline__ bool le(T a, T b) { note(a, b); return a <= b; }
-};
-
-template <typename T, bool TRACK>
-__device__ __forceinline__ void decide(T xins, T yins, T zins, T in_sum, Cmp<T, TRACK> &C,
-                                       Decision &D)
+__device__ __forceinline__ void decide(double xins, double yins, double zins, double in_sum, Decision &D)
 {
+    using T = double;
     const T one = (T)1, two = (T)2, three = (T)3;
-    if (C.le(in_sum, one)) {
+    if (in_sum <= one) {
         // tetrahedron at (0,0,0): closest two of (1,0,0), (0,1,0), (0,0,1)
         D.region = 0;
         int ap = 1, bp = 2;
         T as = xins, bs = yins;
-        if (C.ge(as, bs)) {
-            if (C.gt(zins, bs)) { bs = zins; bp = 4; }
+        if (as >= bs) {
+            if (zins > bs) { bs = zins; bp = 4; }
         } else {
-            if (C.gt(zins, as)) { as = zins; ap = 4; }
+            if (zins > as) { as = zins; ap = 4; }
         }
         T wins = one - in_sum;
-        bool near0 = C.gt(wins, as);
-        if (!near0) near0 = C.gt(wins, bs);
+        bool near0 = wins > as;
+        if (!near0) near0 = wins > bs;
         if (near0) {
-            int c = C.gt(bs, as) ? bp : ap;
+            int c = (bs > as) ? bp : ap;
             if ((c & 1) == 0) { D.e0x = -1.f; D.e1x = 0.f; } else { D.e0x = 1.f; D.e1x = 1.f; }
             if ((c & 2) == 0) {
                 D.e0y = 0.f; D.e1y = 0.f;
@@ -208,21 +195,21 @@ __device__ __forceinline__ void decide(T xins, T yins, T zins, T in_sum, Cmp<T, 
             if ((c & 2) == 0) { D.e0y = 0.f; D.e1y = -1.f; } else { D.e0y = 1.f; D.e1y = 1.f; }
             if ((c & 4) == 0) { D.e0z = 0.f; D.e1z = -1.f; } else { D.e0z = 1.f; D.e1z = 1.f; }
         }
-    } else if (C.ge(in_sum, two)) {
+    } else if (in_sum >= two) {
         // tetrahedron at (1,1,1): closest two of (1,1,0), (1,0,1), (0,1,1)
         D.region = 1;
         int ap = 6, bp = 5;
         T as = xins, bs = yins;
-        if (C.le(as, bs)) {
-            if (C.lt(zins, bs)) { bs = zins; bp = 3; }
+        if (as <= bs) {
+            if (zins < bs) { bs = zins; bp = 3; }
         } else {
-            if (C.lt(zins, as)) { as = zins; ap = 3; }
+            if (zins < as) { as = zins; ap = 3; }
         }
         T wins = three - in_sum;
-        bool near1 = C.lt(wins, as);
-        if (!near1) near1 = C.lt(wins, bs);
+        bool near1 = wins < as;
+        if (!near1) near1 = wins < bs;
         if (near1) {
-            int c = C.lt(bs, as) ? bp : ap;
+            int c = (bs < as) ? bp : ap;
             if ((c & 1) != 0) { D.e0x = 2.f; D.e1x = 1.f; } else { D.e0x = 0.f; D.e1x = 0.f; }
             if ((c & 2) != 0) {
                 D.e0y = 1.f; D.e1y = 1.f;
@@ -242,18 +229,18 @@ __device__ __forceinline__ void decide(T xins, T yins, T zins, T in_sum, Cmp<T, 
         int ap, bp;
         bool af, bf;
         T p1 = xins + yins;
-        if (C.gt(p1, one)) { as = p1 - one; ap = 3; af = true; }
+        if (p1 > one) { as = p1 - one; ap = 3; af = true; }
         else { as = one - p1; ap = 4; af = false; }
         T p2 = xins + zins;
-        if (C.gt(p2, one)) { bs = p2 - one; bp = 5; bf = true; }
+        if (p2 > one) { bs = p2 - one; bp = 5; bf = true; }
         else { bs = one - p2; bp = 2; bf = false; }
         T p3 = yins + zins;
-        bool t3 = C.gt(p3, one);
+        bool t3 = p3 > one;
         score = t3 ? p3 - one : one - p3;
-        if (C.le(as, bs)) {
-            if (C.lt(as, score)) { ap = t3 ? 6 : 1; af = t3; }
+        if (as <= bs) {
+            if (as < score) { ap = t3 ? 6 : 1; af = t3; }
         } else {
-            if (C.lt(bs, score)) { bp = t3 ? 6 : 1; bf = t3; }
+            if (bs < score) { bp = t3 ? 6 : 1; bf = t3; }
         }
         if (af == bf) {
             if (af) {
@@ -284,14 +271,14 @@ __device__ __forceinline__ void decide(T xins, T yins, T zins, T in_sum, Cmp<T, 
 }
 
 
-// Octahedron extra points (opensimplex.py:535-700) from the six comparison
-// outcomes g1 = p1 > 1, g2 = p2 > 1, t3 = p3 > 1, ale = |p1-1| <= |p2-1|,
-// a_lt = |p1-1| < |p3-1|, b_lt = |p2-1| < |p3-1| (bit k of b).  Offsets are
-// in {-1, 0, 1, 2}; a block tabulates all 64 cases once (s_extra) and the
-// per-lane decision looks its case up.
-__device__ __forceinline__ uint32_t octa_case(int b)
+// The extra points' offsets of a case, o[0..2] and o[3..5], from the signs of
+// the comparisons' differences (1: negative).  Octahedron (opensimplex.py:
+// 535-700): bit 5 p1 - 1, 4 p2 - 1, 3 p3 - 1, 2 |p1-1| - |p2-1|, 1 |p1-1| -
+// |p3-1|, 0 |p2-1| - |p3-1|.  Offsets are in {-1, 0, 1, 2}; a block tabulates
+// every case once (s_extra) and the per-lane decision looks its case up.
+__device__ __forceinline__ void octa_case(int b, float *o)
 {
-    const bool g1 = b & 1, g2 = b & 2, t3 = b & 4, ale = b & 8, a_lt = b & 16, b_lt = b & 32;
+    const bool g1 = !(b & 32), g2 = !(b & 16), t3 = !(b & 8), ale = b & 4, a_lt = b & 2, b_lt = b & 1;
     const bool swa = ale && a_lt, swb = !ale && b_lt;
     const int oap = swa ? (t3 ? 6 : 1) : (g1 ? 3 : 4);
     const int obp = swb ? (t3 ? 6 : 1) : (g2 ? 5 : 2);
@@ -317,24 +304,23 @@ __device__ __forceinline__ uint32_t octa_case(int b)
         const bool qz = !qx && !qy;
         o1x = qx ? 2.f : 0.f; o1y = qy ? 2.f : 0.f; o1z = qz ? 2.f : 0.f;
     }
-    const float o[6] = {o0x, o0y, o0z, o1x, o1y, o1z};
-    uint32_t w = 0;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) w |= (uint32_t)((int)o[k] + 1) << (2 * k);
-    return w;
+    o[0] = o0x; o[1] = o0y; o[2] = o0z; o[3] = o1x; o[4] = o1y; o[5] = o1z;
 }
 
-// Tetrahedron extra points (opensimplex.py:302-533) from the comparison
-// outcomes, in the mirrored form the binary32 decision uses (region 1's
-// comparisons are region 0's with both sides negated): bit 0 x >= y, 1
-// z > y, 2 z > x, 3 wins > as, 4 wins > bs, 5 bs > as (as, bs the scores
-// the first three select), 6 region 1 (offsets t become 1 - t).
-__device__ __forceinline__ uint32_t tetra_case(int b)
+// Tetrahedra (opensimplex.py:302-533): bit 4 in_sum - 2 (clear: region 1), 3
+// x - y, 2 y - z, 1 x - z, 0 wins - the middle one of x, y, z.  The two scores
+// the reference compares with wins are the two largest (region 1: smallest),
+// so one of them is passed where the middle one is, and which of the two is
+// the larger (smaller) follows from the order.  Region 1's comparisons are
+// region 0's with both sides negated and its offsets t become 1 - t.
+__device__ __forceinline__ void tetra_case(int b, float *o)
 {
-    const bool xy = b & 1, zb = b & 2, za = b & 4, n1 = b & 8, n2 = b & 16, cnb = b & 32, r1 = b & 64;
+    const bool r1 = !(b & 16);
+    const bool xy = r1 == ((b & 8) != 0), zb = r1 != ((b & 4) != 0), za = r1 != ((b & 2) != 0);   // x >= y, z > y, z > x
+    const bool near = r1 == ((b & 1) != 0);
     const bool repb = xy && zb, repa = !xy && za;
+    const bool cnb = repb ? za : (repa ? !zb : !xy);
     const int ap = repa ? 4 : 1, bp = repb ? 4 : 2;
-    const bool near = n1 || n2;
     const int cn = cnb ? bp : ap;
     const int cf = ap | bp;
     const bool cn1 = (cn & 1) != 0, cn2 = (cn & 2) != 0, cn4 = (cn & 4) != 0;
@@ -345,16 +331,28 @@ __device__ __forceinline__ uint32_t tetra_case(int b)
     t[4] = near ? (cn2 ? 1.f : (cn1 ? 0.f : -1.f)) : ((cf & 2) ? 1.f : -1.f);
     t[2] = near ? (cn4 ? 1.f : 0.f) : ((cf & 4) ? 1.f : 0.f);
     t[5] = near ? (cn4 ? 1.f : -1.f) : ((cf & 4) ? 1.f : -1.f);
-    uint32_t w = 0;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) w |= (uint32_t)((int)(r1 ? 1.f - t[k] : t[k]) + 1) << (2 * k);
-    return w;
+    for (int k = 0; k < 6; ++k) o[k] = r1 ? 1.f - t[k] : t[k];
 }
 
-// Offset k of a case word: ((w >> 2k) & 3) - 1.
-__device__ __forceinline__ int word_offset(uint32_t w, int k)
+// Cases: [0, 64) octahedron, [64, 96) tetrahedra.
+constexpr int CASES = 96;
+__device__ __forceinline__ void extra_case(int i, float *o)
 {
-    return (int)((w >> (2 * k)) & 3u) - 1;
+    if (i < 64) octa_case(i, o); else tetra_case(i - 64, o);
+}
+
+// An extra point's offsets + 1 as steps of a hash address (bits 7-14): x at
+// bit 7, y at bit 16, z at bit 25, so that w, w >> 9 and w >> 18 each have
+// theirs at bit 7, nothing below it, and the rest above bit 14, which the
+// lookup masks away.
+__device__ __forceinline__ uint32_t pack_step(float ox, float oy, float oz)
+{
+    return (uint32_t)((int)ox + 1) << 7 | (uint32_t)((int)oy + 1) << 16 | (uint32_t)((int)oz + 1) << 25;
+}
+
+__device__ __forceinline__ int step_offset(uint32_t w, int axis)
+{
+    return (int)((w >> (7 + 9 * axis)) & 3u) - 1;
 }
 
 // The displacement offsets of an extra point o: o + (ox + oy + oz) / 3
@@ -368,94 +366,82 @@ __device__ __forceinline__ void extra_disp(float ox, float oy, float oz, float *
     E[2] = __fadd_rn(oz, s);
 }
 
-// Case word and displacement offsets of a decision from its six offsets
+// Step words and displacement offsets of a decision from its six offsets
 // (the binary64 path).
 __device__ __forceinline__ void pack_extra(Decision &D)
 {
-    const float o[6] = {D.e0x, D.e0y, D.e0z, D.e1x, D.e1y, D.e1z};
-    uint32_t w = 0;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) w |= (uint32_t)((int)o[k] + 1) << (2 * k);
-    D.w = w;
-    extra_disp(o[0], o[1], o[2], D.E);
-    extra_disp(o[3], o[4], o[5], D.E + 3);
+    D.w0 = pack_step(D.e0x, D.e0y, D.e0z);
+    D.w1 = pack_step(D.e1x, D.e1y, D.e1z);
+    extra_disp(D.e0x, D.e0y, D.e0z, D.E);
+    extra_disp(D.e1x, D.e1y, D.e1z, D.E + 3);
 }
 
-// Extra-point table of a block: [0, 64) octahedron cases, [64, 192)
-// tetrahedron cases.  Entry i is two float4s: the six displacement offsets
-// (E0x, E0y, E0z, E1x), (E1y, E1z, case word as bits, 0).
-__shared__ float4 s_extra[2 * 192];
+// Extra-point table of a block: case i's two float4s at i and CASES + i (so
+// that the lanes' different cases spread over the banks): the six displacement
+// offsets (E0x, E1x, E0y, E1y), (E0z, E1z, the two step words as bits),
+// in the order the paired operands take them.
+__shared__ float4 s_extra[2 * CASES];
 
 // Fill s_extra (the caller synchronises the block before use).
 __device__ __forceinline__ void init_extra_table()
 {
-    for (int i = threadIdx.x; i < 192; i += blockDim.x) {
-        const uint32_t w = i < 64 ? octa_case(i) : tetra_case(i - 64);
-        float E[6];
-        extra_disp((float)word_offset(w, 0), (float)word_offset(w, 1), (float)word_offset(w, 2), E);
-        extra_disp((float)word_offset(w, 3), (float)word_offset(w, 4), (float)word_offset(w, 5), E + 3);
-        s_extra[2 * i] = make_float4(E[0], E[1], E[2], E[3]);
-        s_extra[2 * i + 1] = make_float4(E[4], E[5], __uint_as_float(w), 0.0f);
+    for (int i = threadIdx.x; i < CASES; i += blockDim.x) {
+        float o[6], E[6];
+        extra_case(i, o);
+        extra_disp(o[0], o[1], o[2], E);
+        extra_disp(o[3], o[4], o[5], E + 3);
+        s_extra[i] = make_float4(E[0], E[3], E[1], E[4]);
+        s_extra[CASES + i] = make_float4(E[2], E[5], __uint_as_float(pack_step(o[0], o[1], o[2])),
+                                         __uint_as_float(pack_step(o[3], o[4], o[5])));
     }
 }
 
-// (offset k of a case word + 1) * 128: the offset's step in a hash address.
-__device__ __forceinline__ int word_step(uint32_t w, int k)
+// (bits << 1) | sign of d: one funnel shift per comparison.
+__device__ __forceinline__ uint32_t push_sign(uint32_t bits, float d)
 {
-    return (int)((k < 4 ? w << (7 - 2 * k) : w >> (2 * k - 7)) & 0x180u);
+    return __funnelshift_l(__float_as_uint(d), bits, 1);
 }
 
 // The same decision for the binary32 path without data-dependent branches
-// (lanes of a warp sit in different regions at high octaves).  Regions 0
-// and 1 are mirror images: region 1's comparisons are region 0's with both
-// sides negated (exact), its lattice-point codes are 7 - region 0's and its
-// offsets are 1 - region 0's; both tetrahedra and the octahedron are
-// evaluated and the region selects.  Every comparison evaluated records its
-// margin (a superset of those the branching form records), so a lane keeps
-// its binary32 decision only when all of them clear the margin.
-__device__ __forceinline__ int decide_sel(float x, float y, float z, float in_sum, Cmp<float, true> &C, int &region)
+// (lanes of a warp sit in different regions at high octaves): the sign of
+// each comparison's difference becomes a bit of the case number, for the
+// tetrahedra and the octahedron, and the region selects.  Every difference
+// is a margin (a superset of those the branching form compares), and a lane
+// keeps its binary32 decision only when all of them clear TAU, so ties and
+// the sign of a zero do not matter.  `m` is the smallest margin so far.
+// About 45 operations; comparisons, selects and masks of each outcome took 85.
+__device__ __forceinline__ int decide_sel(float x, float y, float z, float in_sum, float &m, int &region)
 {
-    const bool r0 = C.le(in_sum, 1.0f);
-    const bool r1 = !r0 && C.ge(in_sum, 2.0f);
-    // tetrahedron (region 0 form; s = -1 mirrors the comparisons for region 1)
-    const float s = r1 ? -1.0f : 1.0f;
-    const bool xy = C.ge(s * x, s * y);
-    const bool zb = C.gt(s * z, s * y);
-    const bool za = C.gt(s * z, s * x);
-    const bool repb = xy && zb, repa = !xy && za;
-    const float as = repa ? z : x, bs = repb ? z : y;
-    const float wins = (r1 ? 3.0f : 1.0f) - in_sum;
-    const bool n1 = C.gt(s * wins, s * as);
-    const bool n2 = C.gt(s * wins, s * bs);
-    const bool cnb = C.gt(s * bs, s * as);
-    // octahedron
-    const float p1 = x + y, p2 = x + z, p3 = y + z;
-    const bool g1 = C.gt(p1, 1.0f), g2 = C.gt(p2, 1.0f), t3 = C.gt(p3, 1.0f);
-    const float oas = g1 ? p1 - 1.0f : 1.0f - p1;
-    const float obs = g2 ? p2 - 1.0f : 1.0f - p2;
-    const float score = t3 ? p3 - 1.0f : 1.0f - p3;
-    const bool ale = C.le(oas, obs);
-    const bool a_lt = C.lt(oas, score), b_lt = C.lt(obs, score);
-    // the two extra points are a function of the region's comparison
-    // outcomes: one lookup in the block's table (tetrahedron or octahedron
-    // case, see tetra_case / octa_case)
-    const bool tet = r0 || r1;
-    const uint32_t ot = (g1 ? 1u : 0u) | (g2 ? 2u : 0u) | (t3 ? 4u : 0u) | (ale ? 8u : 0u) | (a_lt ? 16u : 0u) |
-                        (b_lt ? 32u : 0u);
-    const uint32_t tt = 64u + ((xy ? 1u : 0u) | (zb ? 2u : 0u) | (za ? 4u : 0u) | (n1 ? 8u : 0u) | (n2 ? 16u : 0u) |
-                               (cnb ? 32u : 0u) | (r1 ? 64u : 0u));
+    const float mn = fminf(x, y), mx = fmaxf(x, y);
+    const float mid = fmaxf(mn, fminf(mx, z));
+    m = fminf(m, fminf(fminf(mn, z), 1.0f - fmaxf(mx, z)));      // the cell: 0 < x, y, z < 1
+    const float e1 = in_sum - 1.0f, e2 = in_sum - 2.0f;
+    const bool r0 = e1 < 0.0f, r1 = e2 >= 0.0f;
+    const float dxy = x - y, dyz = y - z, dxz = x - z;
+    const float dw = ((r1 ? 3.0f : 1.0f) - in_sum) - mid;
+    const float d1 = e1 - z, d2 = e1 - y, d3 = e1 - x;            // x + y - 1, x + z - 1, y + z - 1
+    const float q12 = fabsf(d1) - fabsf(d2), q13 = fabsf(d1) - fabsf(d3), q23 = fabsf(d2) - fabsf(d3);
+    m = fminf(m, fminf(fabsf(e1), fabsf(e2)));
+    m = fminf(m, fminf(fabsf(dxy), fabsf(dyz)));
+    m = fminf(m, fminf(fabsf(dxz), fabsf(dw)));
+    m = fminf(m, fminf(fabsf(d1), fabsf(d2)));
+    m = fminf(m, fminf(fabsf(d3), fabsf(q12)));
+    m = fminf(m, fminf(fabsf(q13), fabsf(q23)));
+    uint32_t tt = push_sign(2u, e2), ot = push_sign(0u, d1);    // 2 << 5 = 64: the tetrahedra's cases
+    tt = push_sign(push_sign(push_sign(push_sign(tt, dxy), dyz), dxz), dw);
+    ot = push_sign(push_sign(push_sign(push_sign(push_sign(ot, d2), d3), q12), q13), q23);
     region = r0 ? 0 : (r1 ? 1 : 2);
-    return (int)(tet ? tt : ot);
+    return (int)(r0 || r1 ? tt : ot);
 }
 
 // Decision of a binary32-path lane from its case-table entry.
 __device__ __forceinline__ void case_decision(int ci, int region, Decision &D)
 {
-    const float4 *t = s_extra + 2 * ci;
-    const float4 a = t[0], b = t[1];
+    const float4 a = s_extra[ci], b = s_extra[CASES + ci];
     D.region = region;
-    D.w = __float_as_uint(b.z);
-    D.E[0] = a.x; D.E[1] = a.y; D.E[2] = a.z; D.E[3] = a.w; D.E[4] = b.x; D.E[5] = b.y;
+    D.w0 = __float_as_uint(b.z);
+    D.w1 = __float_as_uint(b.w);
+    D.E[0] = a.x; D.E[3] = a.y; D.E[1] = a.z; D.E[4] = a.w; D.E[2] = b.x; D.E[5] = b.y;
 }
 
 // opensimplex.py:18-21 in binary64
@@ -490,9 +476,7 @@ __device__ __noinline__ Cell decide_f64(double X, double Y, double Z, double s)
     double xb = __dadd_rn((double)xsb, sq), yb = __dadd_rn((double)ysb, sq), zb = __dadd_rn((double)zsb, sq);
     double xins = __dsub_rn(xs, (double)xsb), yins = __dsub_rn(ys, (double)ysb), zins = __dsub_rn(zs, (double)zsb);
     double in_sum = __dadd_rn(__dadd_rn(xins, yins), zins);
-    Cmp<double, false> C;
-    C.m = 0.f;
-    decide<double, false>(xins, yins, zins, in_sum, C, c.D);
+    decide(xins, yins, zins, in_sum, c.D);
     pack_extra(c.D);
     c.dxd = __dsub_rn(x, xb);
     c.dyd = __dsub_rn(y, yb);
@@ -518,11 +502,11 @@ struct Core {
 };
 
 // The decision from the split of x*scale into integers A (binary32, |A| <
-// 2^22) and fractions a (|a| < 1) for each axis; `big` = max |x*scale|.
+// 2^22; M = A + MAGIC) and fractions a (|a| < 1) for each axis; `big` = max |x*scale|.
 // Returns false when binary64 must decide.  The error analysis is at
 // decide_f32 (a within 3.1e-8 of x*scale - A).
-__device__ __forceinline__ bool decide_core(float Ax, float ax, float Ay, float ay, float Az, float az, float big,
-                                            Core &o)
+__device__ __forceinline__ bool decide_core(float Mx, float Ax, float ax, float My, float Ay, float ay, float Mz, float Az,
+                                            float az, float big, Core &o)
 {
     const float T = __fadd_rn(__fadd_rn(Ax, Ay), Az);
     const float q = floorf(__fmaf_rn(T, SIXTH, 1.0f / 12.0f));
@@ -531,19 +515,17 @@ __device__ __forceinline__ bool decide_core(float Ax, float ax, float Ay, float 
     const float bx = __fmaf_rn(-u, SIXTH, ax), by = __fmaf_rn(-u, SIXTH, ay), bz = __fmaf_rn(-u, SIXTH, az);
     const float fx = floorf(bx), fy = floorf(by), fz = floorf(bz);
     const float xins = __fsub_rn(bx, fx), yins = __fsub_rn(by, fy), zins = __fsub_rn(bz, fz);
-    const float xsbf = __fadd_rn(__fsub_rn(Ax, q), fx), ysbf = __fadd_rn(__fsub_rn(Ay, q), fy),
-                zsbf = __fadd_rn(__fsub_rn(Az, q), fz);
-    const int xi = __float_as_int(__fadd_rn(xsbf, MAGIC)), yi = __float_as_int(__fadd_rn(ysbf, MAGIC)),
-              zi = __float_as_int(__fadd_rn(zsbf, MAGIC));
+    // the cell's integers stay on MAGIC's grid (|A| < 2^22: exact)
+    const int xi = __float_as_int(__fadd_rn(__fsub_rn(Mx, q), fx)), yi = __float_as_int(__fadd_rn(__fsub_rn(My, q), fy)),
+              zi = __float_as_int(__fadd_rn(__fsub_rn(Mz, q), fz));
     o.xsb = xi - MAGIC_BITS; o.ysb = yi - MAGIC_BITS; o.zsb = zi - MAGIC_BITS;
     o.xb7 = xi << 7; o.yb7 = yi << 7; o.zb7 = zi << 7;
     o.fx = fx; o.fy = fy; o.fz = fz;
     o.G = __fadd_rn(r, __fadd_rn(__fadd_rn(fx, fy), fz));
-    Cmp<float, true> C;
-    C.m = fminf(fminf(fminf(xins, 1.0f - xins), fminf(yins, 1.0f - yins)), fminf(zins, 1.0f - zins));
     const float in_sum = __fadd_rn(__fadd_rn(xins, yins), zins);
-    o.ci = decide_sel(xins, yins, zins, in_sum, C, o.region);
-    return C.m >= TAU && big < PMAX;
+    float m = 1.0f;
+    o.ci = decide_sel(xins, yins, zins, in_sum, m, o.region);
+    return m >= TAU && big < PMAX;
 }
 
 // Binary32 path.  Returns false when binary64 must decide.
@@ -573,10 +555,11 @@ __device__ __forceinline__ bool decide_f32(float xh, float xl, float yh, float y
     ex = fmaf(xh, sl, ex); ey = fmaf(yh, sl, ey); ez = fmaf(zh, sl, ez);
     ex = fmaf(xl, sh, ex); ey = fmaf(yl, sh, ey); ez = fmaf(zl, sh, ez);
     float big = fmaxf(fabsf(px), fmaxf(fabsf(py), fabsf(pz)));
-    float Ax = (px + MAGIC) - MAGIC, Ay = (py + MAGIC) - MAGIC, Az = (pz + MAGIC) - MAGIC;
+    const float Mx = px + MAGIC, My = py + MAGIC, Mz = pz + MAGIC;
+    const float Ax = Mx - MAGIC, Ay = My - MAGIC, Az = Mz - MAGIC;
     float ax = (px - Ax) + ex, ay = (py - Ay) + ey, az = (pz - Az) + ez;
     Core o;
-    const bool ok = decide_core(Ax, ax, Ay, ay, Az, az, big, o);
+    const bool ok = decide_core(Mx, Ax, ax, My, Ay, ay, Mz, Az, az, big, o);
     c.xsb = o.xsb; c.ysb = o.ysb; c.zsb = o.zsb;
     c.xb7 = o.xb7; c.yb7 = o.yb7; c.zb7 = o.zb7;
     const float g = __fmul_rn(o.G, THIRD);
@@ -587,53 +570,82 @@ __device__ __forceinline__ bool decide_f32(float xh, float xl, float yh, float y
     return ok;
 }
 
-// One lattice contribution: attn^4 * (grad . d) if attn > 0.
-__device__ __forceinline__ float contrib(uint32_t w, float dx, float dy, float dz, bool on)
+// The table's word at an extra point (base: the cell's hash bases less one
+// step, w its step word).
+__device__ __forceinline__ uint32_t lk_extra(uint32_t lb, int xm, int ym, int zm, uint32_t w)
 {
-    float attn = fmaf(-dx, dx, fmaf(-dy, dy, fmaf(-dz, dz, 2.0f)));
-    attn = on ? fmaxf(attn, 0.0f) : 0.0f;
-    float a2 = attn * attn;
-    float gx = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7442)) - GBIAS;
-    float gy = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7443)) - GBIAS;
-    float gz = __uint_as_float((w & 0x7Fu) | 0x4B000000u) - GBIAS;
-    float dot = fmaf(gx, dx, fmaf(gy, dy, gz * dz));
-    return (a2 * a2) * dot;
+    const uint32_t hx = lk(lb, (int)((uint32_t)xm + w));
+    const uint32_t hy = lk(lb, (int)(hx + (uint32_t)ym + (w >> 9)));
+    return lk(lb, (int)(hy + (uint32_t)zm + (w >> 18)));
 }
 
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 
-__device__ __forceinline__ float gcomp(uint32_t w, uint32_t sel)
-{
-    return __uint_as_float(__byte_perm(w, 0x4B000000u, sel));
-}
-
 // Two lattice contributions at once in paired binary32 arithmetic (one
 // FFMA2/FMUL2/FADD2 does both): acc += attn^4 * (grad . d) for slots a and
-// b; ON (1 or 0) masks slots outside the region.  -attn = |d|^2 - 2 is
-// clamped at 0 before squaring, so only attn > 0 counts.
+// b; ON (1 or 0) masks slots outside the region (MASK).  -attn = |d|^2 - 2
+// is clamped at 0 before squaring, so only attn > 0 counts.
+template <bool MASK>
 __device__ __forceinline__ float2 contrib2(uint32_t wa, uint32_t wb, float2 DX, float2 DY, float2 DZ, float2 ON,
                                            float2 acc)
 {
-    float2 sq = __fmul2_rn(DZ, DZ);
-    sq = __ffma2_rn(DY, DY, sq);
-    sq = __ffma2_rn(DX, DX, sq);
-    float2 na = __fadd2_rn(sq, f2(-2.0f, -2.0f));
+    float2 na = __ffma2_rn(DZ, DZ, f2(-2.0f, -2.0f));
+    na = __ffma2_rn(DY, DY, na);
+    na = __ffma2_rn(DX, DX, na);
     na = f2(fminf(na.x, 0.0f), fminf(na.y, 0.0f));
-    na = __fmul2_rn(na, ON);
+    if (MASK) na = __fmul2_rn(na, ON);
     const float2 a2 = __fmul2_rn(na, na);
     const float2 a4 = __fmul2_rn(a2, a2);
-    const float2 nb = f2(-GBIAS, -GBIAS);
-    const float2 gx = __fadd2_rn(f2(gcomp(wa, 0x7442), gcomp(wb, 0x7442)), nb);
-    const float2 gy = __fadd2_rn(f2(gcomp(wa, 0x7443), gcomp(wb, 0x7443)), nb);
-    const float2 gz = __fadd2_rn(f2(__uint_as_float((wa & 0x7Fu) | 0x4B000000u),
-                                    __uint_as_float((wb & 0x7Fu) | 0x4B000000u)), nb);
+    const float2 gx = f2(grad_of(wa, 0), grad_of(wb, 0)), gy = f2(grad_of(wa, 1), grad_of(wb, 1)),
+                 gz = f2(grad_of(wa, 2), grad_of(wb, 2));
     float2 dot = __fmul2_rn(gz, DZ);
     dot = __ffma2_rn(gy, DY, dot);
     dot = __ffma2_rn(gx, DX, dot);
     return __ffma2_rn(a4, dot, acc);
 }
 
-// noise3d(x*s) * 103 for one vertex and octave.
+// The fixed corners that a lane of region g evaluates first: corner 0 | A1,
+// A2, A3 = (1,0,0), (0,1,0), (0,0,1) | B1, B2, B3 = (1,1,0), (1,0,1), (0,1,1).
+// Region 0: 0, A1, A2, A3; region 1: corner 0 (there (1,1,1)), B1, B2, B3; the
+// octahedron: A1, A2, A3, B1 (its B2 and B3 are a slot pair of their own).
+__device__ __forceinline__ int region_corner(int g, int x)
+{
+    return g == 2 ? x + 1 : (x == 0 ? 0 : (g == 1 ? 3 + x : x));
+}
+
+// Three times component a of corner c's displacement offset in region g.
+__device__ __forceinline__ int corner_thirds(int g, int c, int a)
+{
+    if (c == 0) return g == 1 ? 6 : 0;
+    if (c <= 3) return a == c - 1 ? 4 : 1;     // (4,1,1), (1,4,1), (1,1,4)
+    return a == 6 - c ? 2 : 5;                 // (5,5,2), (5,2,5), (2,5,5)
+}
+
+// Displacement offsets o + (ox + oy + oz)/3, negated, of the fixed corners
+// that a lane of each region evaluates (slots X1..X4 of noise_raw): entry
+// 4 q + region, q = 0: (X1x, X2x, X1y, X2y), 1: (X1z, X2z, X3x, X4x), 2: (X3y,
+// X4y, X3z, X4z).
+__shared__ float4 s_corner32[12];
+
+__device__ __forceinline__ void init_corner32_table(int g)
+{
+    if (g >= 3) return;
+    float v[4][3];
+    for (int x = 0; x < 4; ++x) {
+        const int c = region_corner(g, x);
+        for (int a = 0; a < 3; ++a) {
+            const int m = corner_thirds(g, c, a);
+            v[x][a] = m == 6 ? -2.0f : (m == 5 ? -(1.0f + 2.0f * THIRD) : (m == 4 ? -(1.0f + THIRD) : (m == 2 ? -(2.0f * THIRD) : (m == 1 ? -THIRD : 0.0f))));
+        }
+    }
+    s_corner32[g] = make_float4(v[0][0], v[1][0], v[0][1], v[1][1]);
+    s_corner32[4 + g] = make_float4(v[0][2], v[1][2], v[2][0], v[3][0]);
+    s_corner32[8 + g] = make_float4(v[2][1], v[3][1], v[2][2], v[3][2]);
+}
+
+// noise3d(x*s) * 103 for one vertex and octave.  A lane evaluates its
+// region's four or six fixed corners and the two extra points in four slot
+// pairs (X1..X4, the octahedron's X5 and X6, the extra points).
 template <bool TRACE>
 __device__ __forceinline__ float noise_raw(float xh, float xl, float yh, float yl, float zh, float zl,
                                            float sh, float sl, double X, double Y, double Z, double s,
@@ -645,52 +657,55 @@ __device__ __forceinline__ float noise_raw(float xh, float xl, float yh, float y
         ++nfb;
     }
     const int r = c.D.region;
-    const bool on0 = r != 2, onA = r != 1, onB = r != 0;
     // hash prefixes of the fixed slots
     uint32_t h0 = lk(lb, c.xb7), h1 = lk(lb, c.xb7 + 128);
     uint32_t h00 = lk(lb, (int)h0 + c.yb7), h01 = lk(lb, (int)h0 + c.yb7 + 128);
     uint32_t h10 = lk(lb, (int)h1 + c.yb7), h11 = lk(lb, (int)h1 + c.yb7 + 128);
     const int z0 = c.zb7, z1 = c.zb7 + 128;
     const float dx0 = c.dx0, dy0 = c.dy0, dz0 = c.dz0;
-    // slot 0: (0,0,0) in region 0, (1,1,1) in region 1
-    uint32_t w0 = lk(lb, r == 1 ? (int)h11 + z1 : (int)h00 + z0);
-    const float k0 = r == 1 ? 1.0f + 1.0f : 0.0f;   // o + sum(o)/3 with o = (1,1,1): 1 + 1
-    // mixed corners; displacement d = d0 - o - sum(o)/3
-    const float c1 = 1.0f + THIRD, c2 = 2.0f * THIRD, c3 = 1.0f + 2.0f * THIRD;
-    uint32_t w100 = lk(lb, (int)h10 + z0), w010 = lk(lb, (int)h01 + z0), w001 = lk(lb, (int)h00 + z1);
-    uint32_t w110 = lk(lb, (int)h11 + z0), w101 = lk(lb, (int)h10 + z1), w011 = lk(lb, (int)h01 + z1);
+    // corner 0: (0,0,0) in region 0, (1,1,1) in region 1
+    const bool r1 = r == 1, r2 = r == 2;
+    const uint32_t w0 = lk(lb, r1 ? (int)h11 + z1 : (int)h00 + z0);
+    const uint32_t w100 = lk(lb, (int)h10 + z0), w010 = lk(lb, (int)h01 + z0), w001 = lk(lb, (int)h00 + z1);
+    const uint32_t w110 = lk(lb, (int)h11 + z0), w101 = lk(lb, (int)h10 + z1), w011 = lk(lb, (int)h01 + z1);
     // extra points
     const Decision &D = c.D;
-    const uint32_t ew = D.w;
+    const uint32_t ew0 = D.w0, ew1 = D.w1;
     const int xm = c.xb7 - 128, ym = c.yb7 - 128, zm = c.zb7 - 128;
-    uint32_t we0 = lk(lb, (int)lk(lb, (int)lk(lb, xm + word_step(ew, 0)) + ym + word_step(ew, 1)) + zm + word_step(ew, 2));
-    uint32_t we1 = lk(lb, (int)lk(lb, (int)lk(lb, xm + word_step(ew, 3)) + ym + word_step(ew, 4)) + zm + word_step(ew, 5));
+    const uint32_t we0 = lk_extra(lb, xm, ym, zm, ew0), we1 = lk_extra(lb, xm, ym, zm, ew1);
+    const uint32_t wX1 = r2 ? w100 : w0, wX2 = r2 ? w010 : (r1 ? w110 : w100);
+    const uint32_t wX3 = r2 ? w001 : (r1 ? w101 : w010), wX4 = r2 ? w110 : (r1 ? w011 : w001);
+    const float4 k0 = s_corner32[r], k1 = s_corner32[4 + r], k2 = s_corner32[8 + r];
     const float2 X0 = f2(dx0, dx0), Y0 = f2(dy0, dy0), Z0 = f2(dz0, dz0);
-    const float fon0 = on0 ? 1.0f : 0.0f, fA = onA ? 1.0f : 0.0f, fB = onB ? 1.0f : 0.0f;
+    const float fr2 = r2 ? 1.0f : 0.0f;
+    const float2 none = f2(1.0f, 1.0f);
+    const float c2 = 2.0f * THIRD, c3 = 1.0f + 2.0f * THIRD;   // displacement d = d0 - o - sum(o)/3
     float2 acc = f2(0.0f, 0.0f);
-    acc = contrib2(w0, w100, __fadd2_rn(X0, f2(-k0, -c1)), __fadd2_rn(Y0, f2(-k0, -THIRD)),
-                   __fadd2_rn(Z0, f2(-k0, -THIRD)), f2(fon0, fA), acc);
-    acc = contrib2(w010, w001, __fadd2_rn(X0, f2(-THIRD, -THIRD)), __fadd2_rn(Y0, f2(-c1, -THIRD)),
-                   __fadd2_rn(Z0, f2(-THIRD, -c1)), f2(fA, fA), acc);
-    acc = contrib2(w110, w101, __fadd2_rn(X0, f2(-c3, -c3)), __fadd2_rn(Y0, f2(-c3, -c2)),
-                   __fadd2_rn(Z0, f2(-c2, -c3)), f2(fB, fB), acc);
-    acc = contrib2(w011, we0, __fadd2_rn(X0, f2(-c2, -D.E[0])), __fadd2_rn(Y0, f2(-c3, -D.E[1])),
-                   __fadd2_rn(Z0, f2(-c3, -D.E[2])), f2(fB, 1.0f), acc);
-    float v = (acc.x + acc.y) + contrib(we1, dx0 - D.E[3], dy0 - D.E[4], dz0 - D.E[5], true);
+    acc = contrib2<false>(wX1, wX2, __fadd2_rn(X0, f2(k0.x, k0.y)), __fadd2_rn(Y0, f2(k0.z, k0.w)),
+                          __fadd2_rn(Z0, f2(k1.x, k1.y)), none, acc);
+    acc = contrib2<false>(wX3, wX4, __fadd2_rn(X0, f2(k1.z, k1.w)), __fadd2_rn(Y0, f2(k2.x, k2.y)),
+                          __fadd2_rn(Z0, f2(k2.z, k2.w)), none, acc);
+    acc = contrib2<true>(w101, w011, __fadd2_rn(X0, f2(-c3, -c2)), __fadd2_rn(Y0, f2(-c2, -c3)),
+                         __fadd2_rn(Z0, f2(-c3, -c3)), f2(fr2, fr2), acc);
+    acc = contrib2<false>(we0, we1, __fadd2_rn(X0, f2(-D.E[0], -D.E[3])), __fadd2_rn(Y0, f2(-D.E[1], -D.E[4])),
+                          __fadd2_rn(Z0, f2(-D.E[2], -D.E[5])), none, acc);
+    const float v = acc.x + acc.y;
     if (TRACE) {
         tr[0] = c.xsb; tr[1] = c.ysb; tr[2] = c.zsb; tr[3] = r;
         int e[6];
-        for (int k = 0; k < 6; ++k) e[k] = word_offset(ew, k);
+        for (int k = 0; k < 6; ++k) e[k] = step_offset(k < 3 ? ew0 : ew1, k % 3);
         tr[4] = c.xsb + e[0]; tr[5] = c.ysb + e[1]; tr[6] = c.zsb + e[2];
         tr[7] = c.xsb + e[3]; tr[8] = c.ysb + e[4]; tr[9] = c.zsb + e[5];
         const int o[9][3] = {{r == 1, r == 1, r == 1}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {1, 1, 0},
                              {1, 0, 1}, {0, 1, 1}, {e[0], e[1], e[2]}, {e[3], e[4], e[5]}};
         const uint32_t w[9] = {w0, w100, w010, w001, w110, w101, w011, we0, we1};
+        const bool on0 = r != 2, onA = r != 1, onB = r != 0;
         const bool on[9] = {on0, onA, onA, onA, onB, onB, onB, true, true};
         for (int k = 0; k < 9; ++k) {
             int32_t *q = sl9 + 5 * k;
             q[0] = c.xsb + o[k][0]; q[1] = c.ysb + o[k][1]; q[2] = c.zsb + o[k][2];
-            q[3] = (int32_t)(((w[k] >> 16) & 0xFF) | (((w[k] >> 24) & 0xFF) << 8) | ((w[k] & 0x7F) << 16));
+            q[3] = 0;
+            for (int a = 0; a < 3; ++a) q[3] |= ((int)grad_of(w[k], a) + 16) << (8 * a);
             q[4] = on[k] ? 1 : 0;
         }
     }
@@ -773,17 +788,30 @@ __device__ __forceinline__ void anchor_third(int m, float &H, float &L)
     L = __fmul_rn((float)(N - 3 * q), C3L);
 }
 
-// Pair case table of a block: entry i (as s_extra) is four float4s: the two
-// extra points' offsets e + (ex + ey + ez)/3 anchored, hi parts
-// (E0x, E0y, E0z, E1x), (E1y, E1z, case word, 0), doubled lo parts
-// (E0x, E0y, E0z, E1x), (E1y, E1z, 0, 0).
-__shared__ float4 s_extra_p[4 * 192];
+// anchor_third(m) and its doubled lo part for m = -8..7 at entry m & 15.
+__shared__ float2 s_third[16];
 
-__device__ __forceinline__ void anchored_offsets(uint32_t w, float *H, float *L)
+__device__ __forceinline__ void init_third_table(int i)
+{
+    if (i >= 0 && i < 16) {
+        float H, L;
+        anchor_third(i < 8 ? i : i - 16, H, L);
+        s_third[i] = make_float2(H, 2.0f * L);
+    }
+}
+
+// Pair case table of a block: case i (as s_extra) has four float4s, CASES
+// apart: the two extra points' offsets e + (ex + ey + ez)/3 anchored, hi parts
+// (E0x, E1x, E0y, E1y), (E0z, E1z, the two step words), doubled lo parts
+// (E0x, E1x, E0y, E1y), (E0z, E1z, 0, 0).
+__shared__ float4 s_extra_p[4 * CASES];
+
+__device__ __forceinline__ void anchored_offsets(uint32_t w0, uint32_t w1, float *H, float *L)
 {
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
-        const int ox = word_offset(w, 3 * p), oy = word_offset(w, 3 * p + 1), oz = word_offset(w, 3 * p + 2);
+        const uint32_t w = p ? w1 : w0;
+        const int ox = step_offset(w, 0), oy = step_offset(w, 1), oz = step_offset(w, 2);
         const int t = ox + oy + oz;
         anchor_third(3 * ox + t, H[3 * p], L[3 * p]);
         anchor_third(3 * oy + t, H[3 * p + 1], L[3 * p + 1]);
@@ -793,14 +821,16 @@ __device__ __forceinline__ void anchored_offsets(uint32_t w, float *H, float *L)
 
 __device__ __forceinline__ void init_extra_table_pair(int i)
 {
-    if (i >= 0 && i < 192) {
-        const uint32_t w = i < 64 ? octa_case(i) : tetra_case(i - 64);
+    if (i >= 0 && i < CASES) {
+        float o[6];
+        extra_case(i, o);
+        const uint32_t w0 = pack_step(o[0], o[1], o[2]), w1 = pack_step(o[3], o[4], o[5]);
         float H[6], L[6];
-        anchored_offsets(w, H, L);
-        s_extra_p[4 * i] = make_float4(H[0], H[1], H[2], H[3]);
-        s_extra_p[4 * i + 1] = make_float4(H[4], H[5], __uint_as_float(w), 0.0f);
-        s_extra_p[4 * i + 2] = make_float4(2.0f * L[0], 2.0f * L[1], 2.0f * L[2], 2.0f * L[3]);
-        s_extra_p[4 * i + 3] = make_float4(2.0f * L[4], 2.0f * L[5], 0.0f, 0.0f);
+        anchored_offsets(w0, w1, H, L);
+        s_extra_p[i] = make_float4(H[0], H[3], H[1], H[4]);
+        s_extra_p[CASES + i] = make_float4(H[2], H[5], __uint_as_float(w0), __uint_as_float(w1));
+        s_extra_p[2 * CASES + i] = make_float4(2.0f * L[0], 2.0f * L[3], 2.0f * L[1], 2.0f * L[4]);
+        s_extra_p[3 * CASES + i] = make_float4(2.0f * L[2], 2.0f * L[5], 0.0f, 0.0f);
     }
 }
 
@@ -824,6 +854,18 @@ __device__ __forceinline__ void slot_disp(float X0H, float X0L2, float2 K, float
         H = h0;
         L2 = l2;
     }
+}
+
+// v times the sign of g.
+__device__ __forceinline__ float with_sign(float v, float g)
+{
+    return __uint_as_float(__float_as_uint(v) ^ (__float_as_uint(g) & 0x80000000u));
+}
+
+// The component that the gradient of a table word has its +-11 in.
+__device__ __forceinline__ float of_axis(uint32_t w, float x, float y, float z)
+{
+    return (w & (2u << 26)) ? z : ((w & (1u << 26)) ? y : x);
 }
 
 // Two lattice contributions (slots a, b in the lanes) in pair arithmetic,
@@ -887,8 +929,8 @@ __device__ __forceinline__ void contrib2_pair(uint32_t wa, uint32_t wb, float X0
     float2 l4 = fma2(h2, h2, f2(-h4.x, -h4.y));
     l4 = fma2(fma2(two, h2, l2), l2, l4);
     // grad . d as a pair (dh, dl), times DSC (see below)
-    const float4 ga = s_grad[wa & 31u], gb = s_grad[wb & 31u];
-    const float2 gx = f2(ga.x, gb.x), gy = f2(ga.y, gb.y), gz = f2(ga.z, gb.z);
+    const float2 gx = f2(grad_of(wa, 0), grad_of(wb, 0)), gy = f2(grad_of(wa, 1), grad_of(wb, 1)),
+                 gz = f2(grad_of(wa, 2), grad_of(wb, 2));
     float2 dh, dl;
     if (NORM) {
         // products exact as q + qe, summed with two-sums; DSC = 1
@@ -905,11 +947,9 @@ __device__ __forceinline__ void contrib2_pair(uint32_t wa, uint32_t wb, float X0
         // g_i = s_i (4 + 7 [i == a]), grad . hi = 4 (U + V) exactly, U =
         // sum s_i hi_i + 2 s_a hi_a (|U| < 8 on the grid: exact), V =
         // -s_a hi_a / 4; the lo parts' product in binary32.  DSC = 1/4.
-        const uint4 sa = s_gsign[wa & 31u], sb = s_gsign[wb & 31u];
-        const float2 sx = f2(__uint_as_float(__float_as_uint(Xh.x) ^ sa.x), __uint_as_float(__float_as_uint(Xh.y) ^ sb.x));
-        const float2 sy = f2(__uint_as_float(__float_as_uint(Yh.x) ^ sa.y), __uint_as_float(__float_as_uint(Yh.y) ^ sb.y));
-        const float2 sz = f2(__uint_as_float(__float_as_uint(Zh.x) ^ sa.z), __uint_as_float(__float_as_uint(Zh.y) ^ sb.z));
-        const float2 s_a = f2(sa.w == 0u ? sx.x : (sa.w == 1u ? sy.x : sz.x), sb.w == 0u ? sx.y : (sb.w == 1u ? sy.y : sz.y));
+        const float2 sx = f2(with_sign(Xh.x, gx.x), with_sign(Xh.y, gx.y)), sy = f2(with_sign(Yh.x, gy.x), with_sign(Yh.y, gy.y)),
+                     sz = f2(with_sign(Zh.x, gz.x), with_sign(Zh.y, gz.y));
+        const float2 s_a = f2(of_axis(wa, sx.x, sy.x, sz.x), of_axis(wb, sx.y, sy.y, sz.y));
         const float2 U = fma2(f2(2.0f, 2.0f), s_a, add2(add2(sx, sy), sz));
         const float2 V = mul2(f2(-0.25f, -0.25f), s_a);
         // a fast two-sum: where |U| < |V| (below 3/8) the sum, on the 2^-23
@@ -946,17 +986,12 @@ __device__ __forceinline__ void init_corner_table(int i)
     // X1..X4 per region in thirds m / 3 (hi), and the sign of the lo part
     if (i >= 0 && i < 12) {
         const int q = i / 3, g = i % 3;
-        // corner 0 | A1, A2, A3 | B1, B2, B3: region 0 (0, A1, A2, A3), region 1
-        // (corner (1,1,1) = 6/3, B1, B2, B3), octahedron (A1, A2, A3, B1)
         float v[2][4];
         for (int u = 0; u < 2; ++u) {
             const int x = 2 * (q / 2) + u;                   // slot X1..X4
-            const int c = g == 2 ? x + 1 : (x == 0 ? 0 : (g == 1 ? 3 + x : x));   // 0, A1-A3 = 1-3, B1-B3 = 4-6
+            const int c = region_corner(g, x);
             for (int a = 0; a < 3; ++a) {
-                int m = 0;
-                if (c == 0) m = g == 1 ? 6 : 0;
-                else if (c <= 3) m = a == c - 1 ? 4 : 1;     // (4,1,1), (1,4,1), (1,1,4)
-                else m = a == 6 - c ? 2 : 5;                 // (5,5,2), (5,2,5), (2,5,5)
+                const int m = corner_thirds(g, c, a);
                 v[u][a] = m == 6 ? 2.0f : (m == 5 ? T5H : (m == 4 ? T4H : (m == 2 ? T2H : (m == 1 ? T1H : 0.0f))));
             }
             v[u][3] = c == 0 ? 0.0f : (c <= 3 ? -C3L2 : C3L2);
@@ -969,10 +1004,11 @@ __device__ __forceinline__ void init_corner_table(int i)
 // x*scale = A + a1 + a2 + a3 for one axis: x = x1 + x2 + x3 and scale =
 // s1 + s2 + s3 exact binary32 triples; |x*scale| < 2^22 for A to be exact.
 __device__ __forceinline__ void coord_split(float x1, float x2, float x3, float s1, float s2, float s3, bool pow2,
-                                            float &A, float &a1, float &a2, float &a3)
+                                            float &p, float &M, float &A, float &a1, float &a2, float &a3)
 {
-    const float p = __fmul_rn(x1, s1);
-    A = __fsub_rn(__fadd_rn(p, MAGIC), MAGIC);
+    p = __fmul_rn(x1, s1);
+    M = __fadd_rn(p, MAGIC);
+    A = __fsub_rn(M, MAGIC);
     a1 = __fsub_rn(p, A);
     if (pow2) {                       // scale = s1, a power of two: exact scaling
         a2 = __fmul_rn(x2, s1);
@@ -1030,24 +1066,25 @@ __device__ __forceinline__ void noise_pair(float x1, float x2, float x3, float y
                                            float z2, float z3, const OctP &O, bool pow2, uint32_t lb, unsigned &nfb,
                                            float &vh, float &vl)
 {
-    float Ax, ax1, ax2, ax3, Ay, ay1, ay2, ay3, Az, az1, az2, az3;
-    coord_split(x1, x2, x3, O.s1, O.s2, O.s3, pow2, Ax, ax1, ax2, ax3);
-    coord_split(y1, y2, y3, O.s1, O.s2, O.s3, pow2, Ay, ay1, ay2, ay3);
-    coord_split(z1, z2, z3, O.s1, O.s2, O.s3, pow2, Az, az1, az2, az3);
+    float px, Mx, Ax, ax1, ax2, ax3, py, My, Ay, ay1, ay2, ay3, pz, Mz, Az, az1, az2, az3;
+    coord_split(x1, x2, x3, O.s1, O.s2, O.s3, pow2, px, Mx, Ax, ax1, ax2, ax3);
+    coord_split(y1, y2, y3, O.s1, O.s2, O.s3, pow2, py, My, Ay, ay1, ay2, ay3);
+    coord_split(z1, z2, z3, O.s1, O.s2, O.s3, pow2, pz, Mz, Az, az1, az2, az3);
     const float ax = __fadd_rn(ax1, ax2), ay = __fadd_rn(ay1, ay2), az = __fadd_rn(az1, az2);
-    const float big = fmaxf(fabsf(__fadd_rn(Ax, ax)), fmaxf(fabsf(__fadd_rn(Ay, ay)), fabsf(__fadd_rn(Az, az))));
+    const float big = fmaxf(fabsf(px), fmaxf(fabsf(py), fabsf(pz)));
     Core o;
     int region, xb7, yb7, zb7;
-    uint32_t ew;
+    uint32_t ew0, ew1;
     float X0H, X0L2, Y0H, Y0L2, Z0H, Z0L2;
     float EH[6], EL2[6];
-    if (decide_core(Ax, ax, Ay, ay, Az, az, big, o)) {
+    if (decide_core(Mx, Ax, ax, My, Ay, ay, Mz, Az, az, big, o)) {
         region = o.region;
         xb7 = o.xb7; yb7 = o.yb7; zb7 = o.zb7;
         // the fraction anchored, then dx0 = a - (f + G/3)
-        float GH, GL;
-        anchor_third((int)o.G, GH, GL);
-        const float GL2 = __fmul_rn(2.0f, GL);
+        // (-6 <= G <= 5: |a| < 0.51 here, so the skewed fractions a - (r + ax +
+        // ay + az) / 6 lie in (-1.6, 0.8) and their floors in -2..0, r in 0..5)
+        const float2 third = s_third[__float_as_uint(__fadd_rn(o.G, MAGIC)) & 15u];
+        const float GH = third.x, GL2 = third.y;
         const float FXH = __fsub_rn(__fadd_rn(ax, ANC), ANC), FYH = __fsub_rn(__fadd_rn(ay, ANC), ANC),
                     FZH = __fsub_rn(__fadd_rn(az, ANC), ANC);
         const float FXL = __fadd_rn(__fadd_rn(__fsub_rn(ax1, FXH), ax2), ax3);
@@ -1059,11 +1096,12 @@ __device__ __forceinline__ void noise_pair(float x1, float x2, float x3, float y
         X0L2 = __fmaf_rn(2.0f, FXL, -GL2);
         Y0L2 = __fmaf_rn(2.0f, FYL, -GL2);
         Z0L2 = __fmaf_rn(2.0f, FZL, -GL2);
-        const float4 *t = s_extra_p + 4 * o.ci;
-        const float4 t0 = t[0], t1 = t[1], t2 = t[2], t3 = t[3];
-        EH[0] = t0.x; EH[1] = t0.y; EH[2] = t0.z; EH[3] = t0.w; EH[4] = t1.x; EH[5] = t1.y;
-        ew = __float_as_uint(t1.z);
-        EL2[0] = t2.x; EL2[1] = t2.y; EL2[2] = t2.z; EL2[3] = t2.w; EL2[4] = t3.x; EL2[5] = t3.y;
+        const float4 *t = s_extra_p + o.ci;
+        const float4 t0 = t[0], t1 = t[CASES], t2 = t[2 * CASES], t3 = t[3 * CASES];
+        EH[0] = t0.x; EH[3] = t0.y; EH[1] = t0.z; EH[4] = t0.w; EH[2] = t1.x; EH[5] = t1.y;
+        ew0 = __float_as_uint(t1.z);
+        ew1 = __float_as_uint(t1.w);
+        EL2[0] = t2.x; EL2[3] = t2.y; EL2[1] = t2.z; EL2[4] = t2.w; EL2[2] = t3.x; EL2[5] = t3.y;
     } else {
         // the vertex as binary64 (the triple's sum is exact)
         const double X = (double)x1 + (double)x2 + (double)x3, Y = (double)y1 + (double)y2 + (double)y3,
@@ -1079,9 +1117,10 @@ __device__ __forceinline__ void noise_pair(float x1, float x2, float x3, float y
         Y0L2 = __fmul_rn(2.0f, L);
         anchor_f64(c.dzd, Z0H, L);
         Z0L2 = __fmul_rn(2.0f, L);
-        ew = c.D.w;
+        ew0 = c.D.w0;
+        ew1 = c.D.w1;
         float EL[6];
-        anchored_offsets(ew, EH, EL);
+        anchored_offsets(ew0, ew1, EH, EL);
         for (int k = 0; k < 6; ++k) EL2[k] = __fmul_rn(2.0f, EL[k]);
     }
     const bool r1 = region == 1, r2 = region == 2;
@@ -1093,8 +1132,7 @@ __device__ __forceinline__ void noise_pair(float x1, float x2, float x3, float y
     const uint32_t w100 = lk(lb, (int)h10 + zo0), w010 = lk(lb, (int)h01 + zo0), w001 = lk(lb, (int)h00 + zo1);
     const uint32_t w110 = lk(lb, (int)h11 + zo0), w101 = lk(lb, (int)h10 + zo1), w011 = lk(lb, (int)h01 + zo1);
     const int xm = xb7 - 128, ym = yb7 - 128, zm = zb7 - 128;
-    const uint32_t we0 = lk(lb, (int)lk(lb, (int)lk(lb, xm + word_step(ew, 0)) + ym + word_step(ew, 1)) + zm + word_step(ew, 2));
-    const uint32_t we1 = lk(lb, (int)lk(lb, (int)lk(lb, xm + word_step(ew, 3)) + ym + word_step(ew, 4)) + zm + word_step(ew, 5));
+    const uint32_t we0 = lk_extra(lb, xm, ym, zm, ew0), we1 = lk_extra(lb, xm, ym, zm, ew1);
     // fixed corners per lane (offsets o + (ox + oy + oz)/3 in thirds: A1 =
     // (1,0,0) -> (4,1,1)/3, A2 (1,4,1)/3, A3 (1,1,4)/3, B1 = (1,1,0) ->
     // (5,5,2)/3, B2 (5,2,5)/3, B3 (2,5,5)/3; corner 0: (0,0,0) or (2,2,2));
@@ -1122,9 +1160,9 @@ __device__ __forceinline__ void noise_pair(float x1, float x2, float x3, float y
     float e;
     two_sum1(AH.x, AH.y, vh, e);
     vl = __fadd_rn(e, __fadd_rn(AL.x, AL.y));
-    if (!NORM) {                      // the dot products carried a factor 1/4 (exact)
-        vh = __fmul_rn(vh, 4.0f);
-        vl = __fmul_rn(vl, 4.0f);
+    if (NORM) {                       // without NORM the dot products carry a factor 1/4 (exact)
+        vh = __fmul_rn(vh, 0.25f);
+        vl = __fmul_rn(vl, 0.25f);
     }
 }
 
@@ -1132,9 +1170,9 @@ __device__ __forceinline__ void noise_pair(float x1, float x2, float x3, float y
 // then renormalised (|rl| <= ulp(rh)/2).
 __device__ __forceinline__ void octave_accumulate(float vh, float vl, float amph, float ampl, float &rh, float &rl)
 {
-    constexpr float R103 = 1.0f / 103.0f;
+    constexpr float R103 = 4.0f / 103.0f;
     const float wq = __fmul_rn(vh, R103);
-    const float rem = __fmaf_rn(-wq, 103.0f, vh);                 // exact
+    const float rem = __fmaf_rn(-wq, 25.75f, vh);                 // exact
     const float wl = __fmul_rn(__fadd_rn(rem, vl), R103);
     const float s = __fadd_rn(1.0f, wq);                          // |wq| <= 1: fast two-sum
     const float lo = __fadd_rn(__fadd_rn(__fsub_rn(1.0f, s), wq), wl);
@@ -1192,10 +1230,7 @@ __device__ __forceinline__ unsigned long long pair_key(float h, float l)
     return ((unsigned long long)fkey(h) << 32) | (unsigned long long)fkey(l);
 }
 
-__device__ __forceinline__ uint32_t lane_base(const uint32_t *T)
-{
-    return (uint32_t)__cvta_generic_to_shared(T) + ((threadIdx.x & 31u) << 2);
-}
+__device__ __forceinline__ uint32_t lane_base() { return (threadIdx.x & 31u) << 2; }
 
 __global__ void __launch_bounds__(256) fbm_kernel(const double *__restrict__ xyz, int64_t n,
                                                   const int32_t *__restrict__ perm,
@@ -1203,11 +1238,12 @@ __global__ void __launch_bounds__(256) fbm_kernel(const double *__restrict__ xyz
                                                   double *__restrict__ out64, float *__restrict__ out32,
                                                   int accumulate, unsigned long long *nfb_out)
 {
-    extern __shared__ __align__(16) uint32_t smem[];
-    build_table(smem, perm, pgi);
+    build_table(perm, pgi);
+    init_grad_table();
     init_extra_table();
+    init_corner32_table((int)threadIdx.x);
     __syncthreads();
-    const uint32_t lb = lane_base(smem);
+    const uint32_t lb = lane_base();
     unsigned nfb = 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -1221,8 +1257,9 @@ __global__ void __launch_bounds__(256) fbm_kernel(const double *__restrict__ xyz
             float v = noise_raw<false>(xh, xl, yh, yl, zh, zl, P.s_hi[o], P.s_lo[o], X, Y, Z, P.s[o], lb,
                                        nfb, nullptr, nullptr);
             // (noise + 1) * 0.5 * strength * radius, noise = v / 103
-            acc += fmaf(v, P.amp[o] * (1.0f / 103.0f), P.amp[o]);
+            acc = fmaf(v, P.amp[o], acc);
         }
+        acc += P.base;
         if (out64) out64[i] = accumulate ? out64[i] + (double)acc : (double)acc;
         if (out32) out32[i] = accumulate ? out32[i] + acc : acc;
     }
@@ -1239,11 +1276,12 @@ __global__ void __launch_bounds__(256) trace_kernel(const double *__restrict__ x
                                                     int32_t *__restrict__ slots,
                                                     unsigned long long *nfb_out)
 {
-    extern __shared__ __align__(16) uint32_t smem[];
-    build_table(smem, perm, pgi);
+    build_table(perm, pgi);
+    init_grad_table();
     init_extra_table();
+    init_corner32_table((int)threadIdx.x);
     __syncthreads();
-    const uint32_t lb = lane_base(smem);
+    const uint32_t lb = lane_base();
     float sh, sl;
     split_f64(s, sh, sl);
     unsigned nfb = 0;
@@ -1368,10 +1406,11 @@ __device__ __forceinline__ void octave_value(const Triples &t, const OctP &O, bo
 // filled by the lower ones meanwhile).
 __device__ __forceinline__ void init_pair_tables()
 {
-    static_assert(PAIR_THREADS == 512, "threads 256-447, 448-459 and 480-503 fill the tables");
+    static_assert(PAIR_THREADS == 512, "threads 256-351, 448-459 and 480-495 fill the small tables");
+    init_grad_table();
     init_extra_table_pair((int)threadIdx.x - 256);
     init_corner_table((int)threadIdx.x - 448);
-    init_grad_table((int)threadIdx.x - 480);
+    init_third_table((int)threadIdx.x - 480);
 }
 
 // Octave o's constants of a planet descriptor or a launch's parameters.
@@ -1438,11 +1477,10 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) fbm_batch_kernel(const nx_fbm
                                                                     const __grid_constant__ FbmSplit split,
                                                                     unsigned long long *nfb_out)
 {
-    extern __shared__ __align__(16) uint32_t smem[];
     __shared__ unsigned long long s_mm[2][PAIR_WARPS];
     init_pair_tables();
     __syncthreads();
-    const uint32_t lb = lane_base(smem);
+    const uint32_t lb = lane_base();
     float2 *part = reinterpret_cast<float2 *>(smem + TABLE_WORDS);
     const int S = SPLIT ? split.S : 1, U = PAIR_THREADS / S, per = CHUNK / U;
     const int u0 = split.first[blockIdx.x], u1 = split.first[blockIdx.x + 1];
@@ -1458,7 +1496,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) fbm_batch_kernel(const nx_fbm
             kmn = ~0ull;
             kmx = 0ull;
             __syncthreads();
-            build_table_pair(smem, planets[p].perm, planets[p].pgi);
+            build_table(planets[p].perm, planets[p].pgi);
             __syncthreads();
             cur = p;
         }
@@ -1525,12 +1563,11 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) fbm_pair_kernel(const double 
                                                                    unsigned long long *minmax,
                                                                    unsigned long long *nfb_out)
 {
-    extern __shared__ __align__(16) uint32_t smem[];
     __shared__ unsigned long long s_mm[2][PAIR_WARPS];
-    build_table_pair(smem, perm, pgi);
+    build_table(perm, pgi);
     init_pair_tables();
     __syncthreads();
-    const uint32_t lb = lane_base(smem);
+    const uint32_t lb = lane_base();
     float2 *part = reinterpret_cast<float2 *>(smem + TABLE_WORDS);
     unsigned nfb = 0;
     unsigned long long kmn = ~0ull, kmx = 0ull;
@@ -1620,6 +1657,7 @@ NX_EXPORT int nx_fbm(const double *xyz_dev, int64_t n, const int32_t *perm_dev, 
     if (!elev_f64_dev && !elev_f32_dev) return nx::fail(NX_EINVAL, "nx_fbm: no output");
     FbmParams P;
     P.n_oct = n_octaves;
+    double base = 0.0;
     for (int o = 0; o < n_octaves; ++o) {
         double s = scale[o];
         float hi = (float)s;
@@ -1627,8 +1665,10 @@ NX_EXPORT int nx_fbm(const double *xyz_dev, int64_t n, const int32_t *perm_dev, 
         P.s_hi[o] = hi;
         P.s_lo[o] = lo;
         P.s[o] = s;
-        P.amp[o] = (float)(0.5 * strength[o] * radius);
+        P.amp[o] = (float)(0.5 * strength[o] * radius / 103.0);
+        base += 0.5 * strength[o] * radius;
     }
+    P.base = (float)base;
     int rc = configure_smem();
     if (rc) return rc;
     int grid = grid_for(n, 256, (const void *)fbm_kernel, TABLE_BYTES);

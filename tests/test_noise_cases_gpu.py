@@ -1,0 +1,64 @@
+"""The case tables of the binary32 decision: every order of the coordinates in every region, at and around its ties.
+
+Decisions are binary64's (a lane whose margin is below TAU = 4e-6 is decided there), so they are equal, not close."""
+import itertools
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from oracle import oracle as O  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+def _near_ties(rng, reach):
+    """Points whose position in the skewed cell is on, or `eps` off, one or two of the decision surfaces."""
+    base = rng.random((60_000, 3))
+    rows = [base]
+    x, y, z = base.T
+    one = np.ones_like(x)
+    planes = [lambda: (x, x, z), lambda: (x, y, y), lambda: (x, y, x),                      # equal coordinates
+              lambda: (x, y, one - x - y), lambda: (x, y, 2 - x - y),                       # the regions' borders
+              lambda: (x, one - x, z), lambda: (x, y, one - x), lambda: (x, y, one - y),    # sums of two are 1
+              lambda: (x, y, 2 - 2 * x - y), lambda: (x, 2 - 2 * y, y),                     # equal scores of the octahedron
+              lambda: (x, (one - x) / 2, (one - x) / 4), lambda: (x, (one - x - y) / 1, y)]  # wins equal to a score
+    for f in planes:
+        p = np.stack([np.broadcast_to(c, x.shape) for c in f()], 1)
+        p = p[((p >= 0) & (p <= 1)).all(1)][:4000]
+        for eps in (0.0, 1e-9, 1e-7, 3e-6, 5e-6, 1e-5, 1e-3):
+            rows.append(p + eps * rng.choice([-1.0, 0.0, 1.0], p.shape))
+    ins = np.concatenate(rows)
+    s = ins + rng.integers(-reach, reach + 1, ins.shape)
+    return s + s.sum(1, keepdims=True) / 3           # unskewed
+
+
+@pytest.mark.parametrize("reach", [0, 3, 40, 9000])
+def test_decisions_around_ties(reach):
+    from nixis_gb300 import opensimplex as osx
+    pts = _near_ties(np.random.default_rng(reach), reach)
+    perm, pgi = O.init(reach)
+    val, tr, sl, nfb = osx.noise3d_trace(pts, perm, pgi)
+    want, want_tr, _ = O.noise3d_batch(pts, perm, pgi, trace=True)
+    assert np.array_equal(tr.cpu().numpy(), want_tr)
+    np.testing.assert_allclose(val.cpu().numpy(), want, rtol=0, atol=2e-6)
+    if reach <= 40:          # both kinds of lanes (at large coordinates the offsets drown)
+        assert 0 < nfb < len(pts)
+    # all the orders of every region were among them
+    ins = np.mod(pts - pts.sum(1, keepdims=True) / 6, 1.0)
+    seen = {(int(r), tuple(np.argsort(i))) for r, i in zip(want_tr[:, 3], ins)}
+    assert seen == set(itertools.product((0, 1, 2), itertools.permutations(range(3))))
+
+
+@pytest.mark.parametrize("reach", [0, 40])
+def test_pair_values_around_ties(reach):
+    """0.5 (noise + 1) in pairs, as one octave (renormalised) and as one of small amplitude, to the path's 2e-13 of the
+    summed amplitudes."""
+    from nixis_gb300 import terrain
+    pts = _near_ties(np.random.default_rng(reach + 1), reach)
+    perm, pgi = O.init(5)
+    for strength in ([1.0], [1.0, 1.0 / 16]):
+        got, _ = terrain.fbm(torch.from_numpy(pts).cuda(), perm, pgi, [1.0] * len(strength), strength, 1.0)
+        want = (O.noise3d_batch(pts, perm, pgi) + 1.0) * 0.5 * sum(strength)
+        assert np.abs(got.cpu().numpy() - want).max() <= 2e-13 * sum(strength)
