@@ -237,8 +237,10 @@ typedef struct nx_tiling {
     int32_t cmax;              /* updatable vertices per tile (capacity) */
     const int32_t *counts;     /* ntiles x (rings + 1): members, then each ring's size */
     const int32_t *ids;        /* ntiles x nmax global vertex ids */
-    const uint16_t *lnbr;      /* ntiles x cmax x 6 local neighbour indices, 0xFFFF = none */
-    const float *ledge;        /* ntiles x cmax x 6 edge lengths, (hi, lo) pairs */
+    /* rows in groups of 32, per group three planes of 32 rows' slots (0, 1),
+     * (2, 3), (4, 5): ntiles x cmax / 32 x 3 x 32 x 2 */
+    const uint16_t *lnbr;      /* local neighbour indices; where there is none, the vertex itself */
+    const float *ledge;        /* edge lengths, (hi, lo) pairs */
 } nx_tiling;
 
 /* Host: sizes of the tiling of divisions k (tile: square side, or minus

@@ -32,3 +32,10 @@ int sm_count();
         cudaError_t _e = cudaGetLastError();                  \
         if (_e != cudaSuccess) return nx::check_cuda(_e, name); \
     } while (0)
+
+// Tile tables (nx_tiling) hold an updatable row's six slots as three 16-byte
+// pairs of edges and three words of neighbours, rows in groups of 32, a
+// group's three planes one after the other: slot pair x of row l is unit
+// tile_unit(l) + 32 x.  A warp's 32 rows of a plane are 512 and 128 bytes in
+// one piece, and the planes' addresses differ by constants.
+__host__ __device__ __forceinline__ int tile_unit(int l) { return (l >> 5) * 96 + (l & 31); }

@@ -423,13 +423,38 @@ __host__ __device__ __forceinline__ int tb_npass(int iters, int R)
 // Length of pass q: greedy, each later pass keeps at least one iteration.
 __host__ __device__ __forceinline__ int tb_len(int iters, int R, int np, int q)
 {
-    int done = 0;
-    for (int x = 0; x < q; ++x) {
-        int l = iters - done - (np - 1 - x);
-        done += l < R ? l : R;
-    }
-    int l = iters - done - (np - 1 - q);
+    // iterations made before pass q: q R, less what later passes keep
+    const int done = q * R < iters - (np - q) ? q * R : iters - (np - q);
+    const int l = iters - done - (np - 1 - q);
     return l < R ? l : R;
+}
+
+// A state row's 32 bytes, in one access where the rows are 32-byte aligned
+// (wide): half the requests of the load and store phases.
+__device__ __forceinline__ void load_row(const float4 *p, bool wide, float4 &x, float4 &y)
+{
+    if (wide) {
+        asm("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+            : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w), "=f"(y.x), "=f"(y.y), "=f"(y.z), "=f"(y.w)
+            : "l"(__cvta_generic_to_global(p)));
+    } else {
+        x = p[0];
+        y = p[1];
+    }
+}
+
+__device__ __forceinline__ void store_row(float4 *p, bool wide, float4 x, float4 y)
+{
+    if (wide) {
+        asm volatile("st.global.v8.f32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};"
+                     :
+                     : "f"(x.x), "f"(x.y), "f"(x.z), "f"(x.w), "f"(y.x), "f"(y.y), "f"(y.z), "f"(y.w),
+                       "l"(__cvta_generic_to_global(p))
+                     : "memory");
+    } else {
+        p[0] = x;
+        p[1] = y;
+    }
 }
 
 struct TbArgs {
@@ -441,6 +466,7 @@ struct TbArgs {
     int smem_c;            // rows of the shared tile tables (>= every tile's updatable count)
     float4 *st0;
     float4 *st1;
+    bool wide = false;     // both 32-byte aligned (set by launch_tb)
     nx_erosion_ctl *ctl;
     // Optional fusion of the rescale: a planet's first pass reads the raw
     // fBm pair sums (float2 per row) and rescales them to its starting
@@ -450,6 +476,7 @@ struct TbArgs {
     const float2 *raw = nullptr;
     const unsigned long long *minmax = nullptr;
     double elo = 0.0, ehi = 0.0;
+    float eloh = 0.0f, elol = 0.0f;   // elo as a pair
     float w0h = 0.0f, w0l = 0.0f;
 };
 
@@ -469,7 +496,9 @@ __host__ __device__ __forceinline__ size_t tb_table_bytes(int c) { return 48 * (
 // limit less the kernel's static shared memory (set by tb_prepare).
 static size_t TB_SMEM_MAX = 200 * 1024;
 
-// One vertex's tile-table entries: local neighbour indices and edge pairs.
+// One vertex's tile-table entries: local neighbour indices and edge pairs
+// (in global memory in groups of 32 rows, see tile_unit; in shared memory
+// row by row).
 struct TileRow {
     uint32_t p01, p23, p45;
     float4 d01, d23, d45;
@@ -483,8 +512,9 @@ __device__ __forceinline__ TileRow tile_row(const uint32_t *lnb, const float4 *l
         r.p01 = lnb[3 * l]; r.p23 = lnb[3 * l + 1]; r.p45 = lnb[3 * l + 2];
         r.d01 = led[3 * l]; r.d23 = led[3 * l + 1]; r.d45 = led[3 * l + 2];
     } else {
-        r.p01 = __ldg(lnb + 3 * l); r.p23 = __ldg(lnb + 3 * l + 1); r.p45 = __ldg(lnb + 3 * l + 2);
-        r.d01 = __ldg(led + 3 * l); r.d23 = __ldg(led + 3 * l + 1); r.d45 = __ldg(led + 3 * l + 2);
+        const int u = tile_unit(l);
+        r.p01 = __ldg(lnb + u); r.p23 = __ldg(lnb + u + 32); r.p45 = __ldg(lnb + u + 64);
+        r.d01 = __ldg(led + u); r.d23 = __ldg(led + u + 32); r.d45 = __ldg(led + u + 64);
     }
     return r;
 }
@@ -526,6 +556,16 @@ __device__ __forceinline__ void tb_update(int l, const TileRow &row, const float
 // registers per thread at or under 65536 / (MINB * THREADS); the per-vertex
 // arithmetic fits 48 registers without spills), so more warps hide the
 // latency of the table reads when the tiles' shared memory allows it.
+// Bound by issue (67 % of the slots; the rest waits for the tables in L2, for
+// the other warps at the barriers, and for the load phase).  Measured (GB300,
+// 24 iterations on 6,400,002 vertices, 24 of 900,002 twice, 12 on 40,000,002):
+// 2.38 / 0.925 / 7.04 ms; tables in groups of 32 rows 2.25 / 0.876 / 6.89;
+// prologue without the loop over earlier passes and binary64, state rows in
+// one access 2.19 / 0.85 / 6.70; alternating order of the rows 2.16 / 0.833 /
+// 6.57.  No gain: planes as long as the tile (the extra pointers cost the
+// registers that keep a row's loads together: 2.59), neighbour byte offsets
+// instead of indices, the next row or the next iteration's first row loaded
+// ahead (2.28), ring sizes in shared memory (2.21).
 template <int THREADS, bool PF, bool SMT = false, bool ONE = false, int MINB = 0>
 __global__ void __launch_bounds__(THREADS, MINB > 0 ? MINB : (PF ? 768 : 1024) / THREADS) erosion_tb_kernel(TbArgs a)
 {
@@ -547,7 +587,9 @@ __global__ void __launch_bounds__(THREADS, MINB > 0 ? MINB : (PF ? 768 : 1024) /
     const int32_t *cnt = TL.counts + (int64_t)tile * (TL.rings + 1);
     const int T = cnt[0];
     int NL = T;
-    for (int r = 1; r <= len; ++r) NL += cnt[r];
+#pragma unroll
+    for (int r = 1; r <= 8; ++r)                 // rings <= 8: loads side by side
+        if (r <= len) NL += cnt[r];
     // rescale per pass: growth is below 16x per iteration, so a max under
     // 2^(96 - 4R) stays under 2^96 through the pass
     const float m = __uint_as_float(__ldg(&c->maxbits[q % 3]));
@@ -573,16 +615,16 @@ __global__ void __launch_bounds__(THREADS, MINB > 0 ? MINB : (PF ? 768 : 1024) /
     const float4 *led = reinterpret_cast<const float4 *>(TL.ledge) + (int64_t)tile * TL.cmax * 3;
     const int C0 = NL - cnt[len];                // members + rings 1..len-1: the rows this pass updates
     if (SMT) {
-        // tables of rows [0, C0): edge pairs as float4s, neighbour indices as
-        // 16-byte units (the tile's slice starts 16-byte aligned: cmax*12 is a
-        // multiple of 16 and C0 < cmax leaves room to round up)
+        // tables of rows [0, C0), row by row
         float4 *sled = reinterpret_cast<float4 *>(sed + a.smem_n + (a.smem_n & 1));
-        uint4 *slnb = reinterpret_cast<uint4 *>(sled + 3 * a.smem_c);
-        for (int r = threadIdx.x; r < 3 * C0; r += THREADS) sled[r] = __ldg(led + r);
-        const uint4 *g = reinterpret_cast<const uint4 *>(lnb);
-        for (int r = threadIdx.x; r < (C0 * 3 + 3) / 4; r += THREADS) slnb[r] = __ldg(g + r);
+        uint32_t *slnb = reinterpret_cast<uint32_t *>(sled + 3 * a.smem_c);
+        for (int r = threadIdx.x; r < C0; r += THREADS) {
+            const TileRow w = tile_row<false>(lnb, led, r);
+            sled[3 * r] = w.d01; sled[3 * r + 1] = w.d23; sled[3 * r + 2] = w.d45;
+            slnb[3 * r] = w.p01; slnb[3 * r + 1] = w.p23; slnb[3 * r + 2] = w.p45;
+        }
         led = sled;
-        lnb = reinterpret_cast<const uint32_t *>(slnb);
+        lnb = slnb;
     }
     TileRow myrow;
     if (ONE) {
@@ -595,7 +637,6 @@ __global__ void __launch_bounds__(THREADS, MINB > 0 ? MINB : (PF ? 768 : 1024) /
     // the planet's first pass of a fused run starts from the raw fBm sums
     const bool fresh = a.raw != nullptr && q == 0;
     float4 ic = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    const float eloh = (float)a.elo, elol = (float)(a.elo - (double)(float)a.elo);
     if (fresh) {
         __shared__ float4 s_ic;
         if (threadIdx.x == 0) s_ic = init_consts(a.minmax, bm.x, a.elo, a.ehi);
@@ -613,13 +654,13 @@ __global__ void __launch_bounds__(THREADS, MINB > 0 ? MINB : (PF ? 768 : 1024) /
         if (fresh) {
             // the state erosion_init_kernel would have written
             const float2 g0 = a.raw[r0], g1 = a.raw[r1];
-            const float2 h0 = init_height(g0, ic, eloh, elol), h1 = init_height(g1, ic, eloh, elol);
+            const float2 h0 = init_height(g0, ic, a.eloh, a.elol), h1 = init_height(g1, ic, a.eloh, a.elol);
             x0 = make_float4(h0.x, h0.y, a.w0h, a.w0l);
             x1 = make_float4(h1.x, h1.y, a.w0h, a.w0l);
             y0 = y1 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         } else {
-            x0 = ist[2 * r0]; y0 = ist[2 * r0 + 1];
-            x1 = ist[2 * r1]; y1 = ist[2 * r1 + 1];
+            load_row(ist + 2 * r0, a.wide, x0, y0);
+            load_row(ist + 2 * r1, a.wide, x1, y1);
         }
         const Pair w0 = prain(__fmul_rn(x0.z, lam), __fmul_rn(x0.w, lam), rain);
         buf0[l0] = make_float4(__fmul_rn(x0.x, lam), __fmul_rn(x0.y, lam), w0.h, w0.l);
@@ -641,7 +682,15 @@ __global__ void __launch_bounds__(THREADS, MINB > 0 ? MINB : (PF ? 768 : 1024) /
         } else {
             TileRow nextrow;
             if (PF && (int)threadIdx.x < C) nextrow = tile_row<SMT>(lnb, led, threadIdx.x);
-            for (int l = threadIdx.x; l < C; l += THREADS) {
+            // every other iteration from the end, so that the rows read last are
+            // still in L1 (a tile's tables are 86 KB, L1 has ~18 KB per block)
+            int l = threadIdx.x, step = THREADS;
+            if (!PF && (mi & 1)) {
+                l += (C - 1) / THREADS * THREADS;
+                step = -THREADS;
+                if (l >= C) l -= THREADS;
+            }
+            for (; (unsigned)l < (unsigned)C; l += step) {
                 TileRow row;
                 if (PF) {
                     row = nextrow;
@@ -661,8 +710,7 @@ __global__ void __launch_bounds__(THREADS, MINB > 0 ? MINB : (PF ? 768 : 1024) /
         const float4 v = fin[l];
         const float2 sv = sed[l];
         const int64_t row = P.vbeg + ids[l];
-        ost[2 * row] = v;
-        ost[2 * row + 1] = make_float4(sv.x, sv.y, 0.0f, 0.0f);
+        store_row(ost + 2 * row, a.wide, v, make_float4(sv.x, sv.y, 0.0f, 0.0f));
         vmax = fmaxf(vmax, fmaxf(fabsf(v.x), fmaxf(fabsf(v.z), fabsf(sv.x))));
     }
     __shared__ float s_wmax[THREADS / 32];
@@ -778,7 +826,7 @@ __device__ __forceinline__ float2 scaled_pair(double v, int K)
     return K == 0 ? nxf::pair(v) : nxf::pair(ldexp(v, -K));
 }
 
-// Measured (GB300, 10,000,002 heights): 154 -> 78 us (400 MB).
+// Measured (GB300, 10,000,002 heights): 154 -> 89 us (400 MB).
 __global__ void erosion_load64_kernel(const double *__restrict__ h, const double *__restrict__ w,
                                       const double *__restrict__ s, int64_t n, const unsigned long long *__restrict__ mbits,
                                       float4 *__restrict__ st, nx_erosion_ctl *__restrict__ ctl)
@@ -1095,8 +1143,9 @@ static size_t tb_launch_smem(int maxnl, int maxc)
     return b;
 }
 
-static cudaError_t launch_tb(int64_t grid, size_t smem, cudaStream_t s, const TbArgs &ta)
+static cudaError_t launch_tb(int64_t grid, size_t smem, cudaStream_t s, TbArgs ta)
 {
+    ta.wide = (((uintptr_t)ta.st0 | (uintptr_t)ta.st1) & 31u) == 0;
     if (g_tb_variant == 1) {
         if (g_tb_threads == 256) erosion_tb_kernel<256, true><<<(unsigned)grid, 256, smem, s>>>(ta);
         else erosion_tb_kernel<384, true><<<(unsigned)grid, 384, smem, s>>>(ta);
@@ -1268,6 +1317,8 @@ static int run_batch(const nx_erosion_planet *planets_dev, const nx_erosion_plan
             ta.raw = fuse->raw;
             ta.minmax = fuse->minmax;
             ta.elo = fuse->elo;
+            ta.eloh = (float)ta.elo;
+            ta.elol = (float)(ta.elo - (double)ta.eloh);
             ta.ehi = fuse->ehi;
             ta.w0h = fuse->w0h;
             ta.w0l = fuse->w0l;

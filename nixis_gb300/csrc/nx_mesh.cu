@@ -1039,9 +1039,9 @@ __device__ bool inner_tile(int k, int B, int R, int f, int i0, int j0, int nmax,
         const int l = w / 3, q = w - 3 * l, p = at[l];
         // slots 2q, 2q + 1 of (-1, 0), (-1, 1), (0, 1), (1, 0), (1, -1), (0, -1)
         const int s0 = q == 0 ? -W : (q == 1 ? 1 : W - 1), s1 = q == 0 ? 1 - W : (q == 1 ? W : -1);
-        lnbr[w] = (uint32_t)map[p + s0] | ((uint32_t)map[p + s1] << 16);
+        lnbr[tile_unit(l) + 32 * q] = (uint32_t)map[p + s0] | ((uint32_t)map[p + s1] << 16);
         const float4 *e = reinterpret_cast<const float4 *>(edge) + 3 * (int64_t)list[l];
-        ledge[w] = e[q];
+        ledge[tile_unit(l) + 32 * q] = e[q];
     }
     return true;
 }
@@ -1247,8 +1247,9 @@ __global__ void __launch_bounds__(512) tile_rings_kernel(int k, int B, bool alig
                     loc = hfind(H, key, val, jv[u]);
                     if (loc < 0) { s_bad = 1; loc = q; }
                 }
-                lnbr[((int64_t)tile * cmax + q) * 6 + sl] = (uint16_t)loc;
-                reinterpret_cast<float2 *>(ledge)[((int64_t)tile * cmax + q) * 6 + sl] = ev[u];
+                const int64_t at = 2 * (tile * 3 * cmax + tile_unit(q) + 32 * (sl >> 1)) + (sl & 1);
+                lnbr[at] = (uint16_t)loc;
+                reinterpret_cast<float2 *>(ledge)[at] = ev[u];
             }
         }
     }
@@ -1270,8 +1271,7 @@ static_assert(sizeof(nx_tiling) == 48, "tiling descriptor layout");
 // distance `reach` of a point or square (see nx_tiling_shape).
 static int tile_caps(int64_t nm, int64_t cm, int32_t *nmax, int32_t *cmax)
 {
-    cm = (cm + 3) & ~(int64_t)3;                     // cm*12 B: 16-byte units
-    if (cm > nm) cm = nm & ~(int64_t)3;
+    cm = (cm + 31) & ~(int64_t)31;                   // whole groups of rows (tile_unit)
     if (nm > 4096) return nx::fail(NX_EINVAL, "nx_tiling_shape: tile too large (%lld local vertices)", (long long)nm);
     *nmax = (int32_t)nm;
     *cmax = (int32_t)cm;

@@ -1,0 +1,52 @@
+"""Blocked passes: state rows off a 32-byte boundary, every pass length, every variant that shares the tables' layout."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def run(m, h, iters, cfg, shift):
+    """Heights, water and sediment after `iters` iterations; state rows `shift` floats off a 512-byte boundary."""
+    import torch
+    from nixis_gb300 import autotune, erosion
+    was = autotune.current()
+    try:
+        if cfg is not None:
+            autotune.use(cfg)
+        r = erosion.ErosionRun(m.xyz, m.nbr, m.edge, iters=iters)
+        r.k = m.k
+        for name in ("st", "st_tmp"):
+            t = getattr(r, name)
+            setattr(r, name, torch.zeros(t.numel() + 8, dtype=t.dtype, device="cuda")[shift:shift + t.numel()].view(t.shape))
+        r.load(h)
+        if cfg is None:
+            r.steps(iters, rain=0.01)
+        else:
+            assert r.blocked(iters, 0.01)
+        out = [torch.empty(m.n, dtype=torch.float64, device="cuda") for _ in range(3)]
+        r.store(*out)
+        return out
+    finally:
+        autotune.use(was)
+
+
+@pytest.mark.parametrize("iters", [1, 4, 5, 7, 16, 33])
+@pytest.mark.parametrize("shift", [0, 4])
+def test_rows_of_any_alignment(shift, iters):
+    import torch
+    from nixis_gb300 import autotune, mesh
+    m = mesh.PlanetMesh(67)
+    g = torch.Generator().manual_seed(iters)
+    h = torch.rand(m.n, dtype=torch.float64, generator=g).cuda() * 100.0
+    for a, b in zip(run(m, h, iters, None, 0), run(m, h, iters, autotune.current(), shift)):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("side, rings, threads, variant", [(32, 4, 384, 4), (16, 2, 256, 0), (20, 3, 384, 1), (24, 8, 512, 0), (33, 1, 320, 4)])
+def test_rows_of_any_order(side, rings, threads, variant):
+    import torch
+    from nixis_gb300 import autotune, mesh
+    m = mesh.PlanetMesh(90)
+    h = torch.rand(m.n, dtype=torch.float64, generator=torch.Generator().manual_seed(side)).cuda()
+    cfg = autotune.TbConfig(side, rings, threads, variant)
+    for a, b in zip(run(m, h, 13, None, 0), run(m, h, 13, cfg, 0)):
+        assert torch.equal(a, b)

@@ -8,7 +8,9 @@ def lists(tl, side, rings):
     """Per tile its counts, ids, neighbour indices and edge lengths (what lies beyond the counts is not written)."""
     import torch
     cnt = tl.counts.view(tl.ntiles, rings + 1)
-    ids, lnbr, ledge = tl.ids.view(tl.ntiles, tl.nmax), tl.lnbr[: tl.ntiles * tl.cmax * 6].view(tl.ntiles, tl.cmax, 6), tl.ledge.view(tl.ntiles, tl.cmax, 12)
+    ids, group = tl.ids.view(tl.ntiles, tl.nmax), (tl.ntiles, tl.cmax // 32, 3, 32, -1)
+    lnbr = tl.lnbr[: tl.ntiles * tl.cmax * 6].view(group).transpose(2, 3).reshape(tl.ntiles, tl.cmax, 6)
+    ledge = tl.ledge.view(group).transpose(2, 3).reshape(tl.ntiles, tl.cmax, 12)
     n, c = cnt.sum(1), cnt.sum(1) - cnt[:, rings]
     seen = torch.arange(tl.nmax, device="cuda") < n[:, None]
     upd = torch.arange(tl.cmax, device="cuda") < c[:, None]
