@@ -451,9 +451,9 @@ def bench_ours(args):
         torch.cuda.synchronize()
         plains[key] = npl / (time.perf_counter() - t0)
     plain = {"value": plains["plain"], "unit": UNIT,
-             "what": "one planet at a time, one launch per octave and per erosion iteration, synchronised per planet"}
+             "what": "one planet at a time, one launch for the octaves and one per erosion iteration, synchronised per planet"}
     plain_blocked = {"value": plains["plain_blocked"], "unit": UNIT,
-                     "what": "one planet at a time, one launch per octave and per blocked erosion pass (the batch's "
+                     "what": "one planet at a time, one launch for the octaves and one per blocked erosion pass (the batch's "
                              "erosion kernel), synchronised per planet"}
     # (outside the timed regions) every batched planet equals the planet generated alone
     res = batch.results()

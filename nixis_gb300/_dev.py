@@ -55,6 +55,13 @@ def upload(arr, tdt):
     return t.to("cuda")
 
 
+def put(dst, src, stream=None):
+    """The bytes of a small numpy array (or ctypes structure) into the CUDA
+    tensor dst, in stream order; src may change as soon as this returns."""
+    a = np.frombuffer(src, np.uint8) if not isinstance(src, np.ndarray) else np.ascontiguousarray(src)
+    call("nx_upload", ptr(dst), ctypes.c_void_p(a.ctypes.data), a.nbytes, stream_handle(stream))
+
+
 def to_host(dst, src):
     """dst[...] = src for a numpy array and a CUDA tensor of its type; straight
     into a contiguous array (80 MB: 430 us; through a fresh array, whose pages

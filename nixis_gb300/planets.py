@@ -10,7 +10,7 @@ Two execution paths over the same kernels:
   schedule.  The whole sequence can be captured once as a CUDA graph and
   replayed.
 * ``generate_plain`` -- the plain per-planet GPU path: one planet at a time,
-  one launch per octave and per erosion iteration, synchronised per planet.
+  one launch for the octaves and one per erosion iteration, synchronised per planet.
 
 The fBm runs in pair precision (nx_fbm_pair), the rescale to metres and
 the erosion state in binary32 pairs, and heights come back in binary64:
@@ -31,7 +31,7 @@ from . import autotune as _autotune
 from . import climate as _climate
 from . import mesh as _mesh
 from . import opensimplex as _osx
-from ._lib import ErosionPlanet, FbmPlanet, InsoPlanet, call, lib
+from ._lib import NX_MAX_OCTAVES, ErosionPlanet, FbmPlanet, InsoPlanet, call, lib
 
 ALIGN = 256
 
@@ -385,7 +385,6 @@ class _PlainWork:
     def ensure(self, n):
         if n > self.n:
             self.raw = torch.empty((n, 2), dtype=torch.float32, device="cuda")
-            self.hm = torch.empty(n, dtype=torch.float64, device="cuda")
             self.st = torch.empty((n, 8), dtype=torch.float32, device="cuda")
             self.st_tmp = torch.empty((n, 8), dtype=torch.float32, device="cuda")
             self.ws = torch.zeros(int(lib().nx_erosion_workspace_size(n, 1)), dtype=torch.uint8, device="cuda")
@@ -405,9 +404,10 @@ _ZERO_KEY = (0x80000000 << 32) | 0x80000000
 
 
 def generate_plain(request, meshes=None, sync=True, out=None, blocked=False):
-    """One planet: a launch per octave, per erosion iteration (blocked=True:
-    per temporally blocked pass of the batches' setting); synchronised.
-    Same arithmetic as the batched path, so the same bits."""
+    """One planet: a launch for the octaves and per erosion iteration
+    (blocked=True: per temporally blocked pass of the batches' setting, the
+    first of them rescaling the octaves' sums); synchronised.  Same
+    arithmetic as the batched path, so the same bits."""
     r = request
     meshes = meshes if meshes is not None else _mesh.MeshCache()
     m = meshes.get(r.divisions)
@@ -416,22 +416,23 @@ def generate_plain(request, meshes=None, sync=True, out=None, blocked=False):
     w.ensure(n)
     s = _dev.stream_handle()
     perm, pgi = _osx.init(r.seed)
-    w.perm.copy_(torch.from_numpy(perm))
-    w.pgi.copy_(torch.from_numpy(pgi))
+    _dev.put(w.perm, perm)
+    _dev.put(w.pgi, pgi)
     scale, strength = r.octave_args()
-    w.minmax.copy_(torch.tensor([-1, 0], dtype=torch.int64))          # {~0, 0}
+    _dev.put(w.minmax, np.array([-1, 0], np.int64))          # {~0, 0}
     # the precision choice per octave follows the planet's largest amplitude, as in the batch
     amp_ref = max([abs(0.5 * a * r.radius) for a in strength], default=0.0)
-    for o in range(r.octaves):
-        sc = (ctypes.c_double * 1)(scale[o])
-        st = (ctypes.c_double * 1)(strength[o])
-        last = o == r.octaves - 1
-        call("nx_fbm_pair", _dev.ptr(m.xyz), n, _dev.ptr(w.perm), _dev.ptr(w.pgi), 1, sc, st, float(r.radius),
-             amp_ref, _dev.ptr(w.raw), None, 1 if o > 0 else 0, _dev.ptr(w.minmax) if last else None, None, s)
+    for o in range(0, r.octaves, NX_MAX_OCTAVES):
+        k = min(NX_MAX_OCTAVES, r.octaves - o)
+        sc = (ctypes.c_double * k)(*scale[o:o + k])
+        st = (ctypes.c_double * k)(*strength[o:o + k])
+        call("nx_fbm_pair", _dev.ptr(m.xyz), n, _dev.ptr(w.perm), _dev.ptr(w.pgi), k, sc, st, float(r.radius),
+             amp_ref, _dev.ptr(w.raw), None, 1 if o > 0 else 0, _dev.ptr(w.minmax) if o + k == r.octaves else None,
+             None, s)
     if r.octaves == 0:
         w.raw[:n].zero_()
         k = _ZERO_KEY - (1 << 64)
-        w.minmax.copy_(torch.tensor([k, k], dtype=torch.int64))
+        _dev.put(w.minmax, np.array([k, k], np.int64))
     # the rescale to metres and the initial state: the batch's kernel on one
     # planet (state in buffer 0, or in buffer iters & 1 for a blocked run)
     blocked = blocked and r.erosion_iters > 0
@@ -439,30 +440,30 @@ def generate_plain(request, meshes=None, sync=True, out=None, blocked=False):
     d.vbeg, d.n, d.nbr, d.edge, d.slot = 0, n, m.nbr.data_ptr(), m.edge.data_ptr(), 0
     d.iters = r.erosion_iters if blocked else 0
     d.rain = r.rain
-    w.init_desc.copy_(torch.frombuffer(bytearray(bytes(d)), dtype=torch.uint8))
-    call("nx_erosion_init_batch", _dev.ptr(w.init_desc), ctypes.byref(d), 1, _dev.ptr(w.raw), _dev.ptr(w.minmax),
-         float(r.elev_lo), float(r.elev_hi), float(r.water0), _dev.ptr(w.st), _dev.ptr(w.st_tmp), s)
+    heights = torch.empty(n, dtype=torch.float64, device="cuda") if out is None else out
     if blocked:
         tb = _autotune.current()
         _autotune.apply(tb)
         tl = m.tiling(tb.tile_side, tb.rings)
         d.tiling, d.ntiles, d.maxnl, d.maxc = tl.dev.data_ptr(), tl.ntiles, tl.maxnl, tl.maxc
-        w.init_desc.copy_(torch.frombuffer(bytearray(bytes(d)), dtype=torch.uint8))
+        _dev.put(w.init_desc, d)
         need = int(lib().nx_erosion_workspace_size(max(n, tl.ntiles * ALIGN), 1))
         if getattr(w, "ws_tb", None) is None or w.ws_tb.numel() < need:
             w.ws_tb = torch.zeros(need, dtype=torch.uint8, device="cuda")
         ws = w.ws_tb
         call("nx_erosion_ctl_init", _dev.ptr(ws), ws.numel(), 1, s)
-        call("nx_erosion_batch", _dev.ptr(w.init_desc), ctypes.byref(d), 1, _dev.ptr(w.st), _dev.ptr(w.st_tmp), None,
-             _dev.ptr(ws), ws.numel(), s)
+        call("nx_erosion_run_batch", _dev.ptr(w.init_desc), ctypes.byref(d), 1, _dev.ptr(w.raw), _dev.ptr(w.minmax),
+             float(r.elev_lo), float(r.elev_hi), float(r.water0), _dev.ptr(w.st), _dev.ptr(w.st_tmp),
+             _dev.ptr(heights), _dev.ptr(ws), ws.numel(), s)
     else:
+        _dev.put(w.init_desc, d)
+        call("nx_erosion_init_batch", _dev.ptr(w.init_desc), ctypes.byref(d), 1, _dev.ptr(w.raw), _dev.ptr(w.minmax),
+             float(r.elev_lo), float(r.elev_hi), float(r.water0), _dev.ptr(w.st), _dev.ptr(w.st_tmp), s)
         ws = w.ws
         call("nx_erosion_ctl_init", _dev.ptr(ws), ws.numel(), 1, s)
         call("nx_erosion_steps", _dev.ptr(m.nbr), _dev.ptr(m.edge), n, _dev.ptr(w.st), _dev.ptr(w.st_tmp),
              r.erosion_iters, ctypes.c_float(r.rain), _dev.ptr(w.planet), None, None, _dev.ptr(ws), ws.numel(), s)
-    hd = w.hm[:n] if out is None else out
-    call("nx_erosion_store", _dev.ptr(w.st), n, _dev.ptr(ws), _dev.ptr(hd), None, None, s)
-    heights = hd.clone() if out is None else hd
+        call("nx_erosion_store", _dev.ptr(w.st), n, _dev.ptr(ws), _dev.ptr(heights), None, None, s)
     ins = None
     if r.insolation:
         rot, tilts = _climate.annual_schedule(r.axial_tilt, r.days, r.days, r.hours)
