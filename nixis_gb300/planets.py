@@ -415,6 +415,11 @@ def generate_plain(request, meshes=None, sync=True, out=None, blocked=False):
     w = _plain
     w.ensure(n)
     s = _dev.stream_handle()
+    blocked = blocked and r.erosion_iters > 0
+    if blocked:
+        # (enqueued before the noise: its counts are waited for behind it)
+        tb = _autotune.current()
+        tl = m.tiling(tb.tile_side, tb.rings)
     perm, pgi = _osx.init(r.seed)
     _dev.put(w.perm, perm)
     _dev.put(w.pgi, pgi)
@@ -435,16 +440,13 @@ def generate_plain(request, meshes=None, sync=True, out=None, blocked=False):
         _dev.put(w.minmax, np.array([k, k], np.int64))
     # the rescale to metres and the initial state: the batch's kernel on one
     # planet (state in buffer 0, or in buffer iters & 1 for a blocked run)
-    blocked = blocked and r.erosion_iters > 0
     d = ErosionPlanet()
     d.vbeg, d.n, d.nbr, d.edge, d.slot = 0, n, m.nbr.data_ptr(), m.edge.data_ptr(), 0
     d.iters = r.erosion_iters if blocked else 0
     d.rain = r.rain
     heights = torch.empty(n, dtype=torch.float64, device="cuda") if out is None else out
     if blocked:
-        tb = _autotune.current()
         _autotune.apply(tb)
-        tl = m.tiling(tb.tile_side, tb.rings)
         d.tiling, d.ntiles, d.maxnl, d.maxc = tl.dev.data_ptr(), tl.ntiles, tl.maxnl, tl.maxc
         _dev.put(w.init_desc, d)
         need = int(lib().nx_erosion_workspace_size(max(n, tl.ntiles * ALIGN), 1))
