@@ -216,23 +216,24 @@ constexpr int DAY_GROUP = 8;
 // the breakpoints T: convex, so near a breakpoint it is the larger of the
 // two lines that meet there, and no comparison with T is needed.  With t =
 // a_h / |z| a value is |z| (P0 t + Q1).
-// Shared memory after the staged constants: the bucket table of SP + 1
-// float4s (SP a power of two > the days), the lines L[nf + 1] = (P0,
-// Q1) (exact sums rounded once), K[SP] the sorted tan_d, padded with +inf,
+// Shared memory after the staged constants: the bucket table of NB + 1
+// float4s (bucket_count), the lines L[nf + 1] = (P0,
+// Q1) (exact sums rounded once), K[SP] (SP a power of two > the days) the
+// sorted tan_d, padded with +inf,
 // with their cos_d.  Bucket b holds the t nearest to tmax (1 - (b /
-// SP)^2), tmax the largest tan_d: seasonal tilts go as a sine, so the
+// NB)^2), tmax the largest tan_d: seasonal tilts go as a sine, so the
 // breakpoints crowd at tmax as those t do, and hardly a bucket gets two
 // (with buckets of equal width in t the crowded ones held up to 14, and the
 // walk through them was a third of the instructions).  Bucket 0 takes all t
 // beyond tmax.  An entry is the lines of the bucket's two ends (p0, p0', q1,
-// q1') where its breakpoints lie within 2e-6 of each other; otherwise p0 is
+// q1') where its breakpoints lie within 2e-6 of each other (or 1e-9 tmax); otherwise p0 is
 // NaN, the two ends' line numbers follow, and a vertex takes the largest of
 // the lines between.  A bucket number one off by rounding changes a value by
 // no more than its rounding does, as the lines meet there.
 // Measured (GB300, a year of hourly positions, 10,000,002 vertices): 289 ->
-// 137 us (2.0 TB/s of the 28 B per vertex; issue-bound, 66 % of the issue
-// slots, 340 instructions per vertex with the search and the binary64 test
-// at 507); 9,002 vertices 63.6 -> 16.6 us (the blocks' start).
+// 137 us with the tables and the test in pairs, 111 us in a kernel of its own
+// (BREAK_THREADS); a month 224 -> 101 us with 256 buckets instead of 32;
+// 9,002 vertices 63.6 -> 16.6 us (the blocks' start).
 constexpr int SORT_MAX = 512;
 
 __host__ __device__ __forceinline__ int sort_pad(int n)
@@ -240,6 +241,15 @@ __host__ __device__ __forceinline__ int sort_pad(int n)
     int p = 1;
     while (p < n) p <<= 1;
     return p;
+}
+
+// Buckets of a schedule's table: as many as the padded days, 256 at least
+// (a month's breakpoints are spread over t, not crowded at tmax: with 32
+// buckets several share one).
+__host__ __device__ __forceinline__ int bucket_count(int n_tilt)
+{
+    const int sp = sort_pad(n_tilt + 1);
+    return sp < 256 ? 256 : sp;
 }
 
 // Exclusive prefix sums over the block of 64-bit integers (two per thread),
@@ -277,7 +287,7 @@ struct Breaks {
     const float4 *rot = nullptr;   // the rotations, two to an entry
     uint32_t bucket = 0;       // shared address of the table less what a bucket number's binary32 exponent adds
     int nf = -1;               // factored days
-    float sp = 0.0f;           // buckets
+    float nb = 0.0f;           // buckets
     float inv = 0.0f;          // 1 / tmax
     bool crowded = false;      // some bucket holds distinct breakpoints
 };
@@ -289,7 +299,7 @@ __device__ __forceinline__ Breaks stage_breakpoints(const InsoArgs &a, const flo
 {
     const int nd = __float_as_int(tt[a.n_tilt].y);
     const int nf = a.n_tilt - nd;
-    const int sp = sort_pad(a.n_tilt + 1);
+    const int sp = sort_pad(a.n_tilt + 1), nb = bucket_count(a.n_tilt);
     // bitonic sort of the factored days by tan (direct days, padding: +inf),
     // the cosine alongside
     for (int d = threadIdx.x; d < sp; d += blockDim.x) {
@@ -327,7 +337,7 @@ __device__ __forceinline__ Breaks stage_breakpoints(const InsoArgs &a, const flo
     bk.L = L;
     bk.bucket = (uint32_t)__cvta_generic_to_shared(bucket) - (0x4B000000u << 4);
     bk.nf = nf;
-    bk.sp = (float)sp;
+    bk.nb = (float)nb;
     auto tan_of = [&](int j) { return __uint_as_float(K[j].x); };
     const float tmax = nf > 0 ? tan_of(nf - 1) : 0.0f;
     bk.inv = tmax > 0.0f ? 1.0f / tmax : 0.0f;
@@ -337,11 +347,12 @@ __device__ __forceinline__ Breaks stage_breakpoints(const InsoArgs &a, const flo
         return c;
     };
     bool crowded = false;
-    for (int b = threadIdx.x; b <= sp; b += blockDim.x) {
-        const float w0 = ((float)b - 0.5f) / bk.sp, w1 = ((float)b + 0.5f) / bk.sp;
+    for (int b = threadIdx.x; b <= nb; b += blockDim.x) {
+        const float w0 = ((float)b - 0.5f) / bk.nb, w1 = ((float)b + 0.5f) / bk.nb;
         const int k0 = below(tmax * (1.0f - w1 * w1)), k1 = b > 0 && tmax > 0.0f ? below(tmax * (1.0f - w0 * w0)) : nf;
         const float2 l0 = L[k0], l1 = L[k1];
-        const bool simple = k1 - k0 <= 1 || tan_of(k1 - 1) - tan_of(k0) <= 2e-6f * tan_of(k1 - 1);
+        const float gap = k1 - k0 <= 1 ? 0.0f : tan_of(k1 - 1) - tan_of(k0);
+        const bool simple = gap <= 2e-6f * tan_of(max(k1 - 1, 0)) || gap <= 1e-9f * tmax;   // (or all at t = 0)
         bucket[b] = simple ? make_float4(l0.x, l1.x, l0.y, l1.y)
                            : make_float4(__int_as_float(0x7FFFFFFF), __int_as_float(k0), __int_as_float(k1), 0.0f);
         crowded = crowded || !simple;
@@ -363,7 +374,7 @@ __device__ __forceinline__ float pair_value(const Breaks &bk, float a, float c, 
 {
     // the bucket number, rounded to nearest, in the low bits of a binary32
     const float w = approx_sqrt(__saturatef(fmaf(-a, ti, 1.0f)));
-    const uint32_t at = (__float_as_uint(fmaf(w, bk.sp, 8388608.0f)) << 4) + bk.bucket;
+    const uint32_t at = (__float_as_uint(fmaf(w, bk.nb, 8388608.0f)) << 4) + bk.bucket;
     float4 e;
     asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(e.x), "=f"(e.y), "=f"(e.z), "=f"(e.w) : "r"(at));
     const float2 v2 = __ffma2_rn(make_float2(a, a), make_float2(e.x, e.y),
@@ -547,7 +558,7 @@ __device__ __forceinline__ float arc_sum(const InsoArgs &a, const Arcs &A, float
     return tot;
 }
 
-template <int HP>
+template <int HP, bool BREAKS>
 __device__ __forceinline__ float inso_vertex(const InsoArgs &a, double X, double Y, double Z, double r, float r2h,
                                              float r2l, float zmin, float inv_r, const float4 *tt = nullptr,
                                              const Breaks &bk = Breaks(), const Arcs &arc = Arcs())
@@ -557,7 +568,7 @@ __device__ __forceinline__ float inso_vertex(const InsoArgs &a, double X, double
     if (HP == ARCS && on_sphere) return arc_sum(a, arc, x, y, z) * inv_r;
     float tot = 0.0f, comp = 0.0f;          // Kahan over tilts
     const int nr = HP > 0 ? HP : a.n_rot;
-    if (on_sphere && HP > 0 && (HP & 1) == 0 && a.pairs) {
+    if (on_sphere && HP > 0 && (HP & 1) == 0 && (BREAKS || a.pairs)) {
         // u = A cos(theta) + B sin(theta) = k U(theta) with k = cos(tau) and
         // U = x cos(theta) - y sin(theta) the same for every day, so per day
         //   sum_h max(|C|, |u_h|) = |k| sum_h max(|C| / |k|, |U_h|)
@@ -565,14 +576,14 @@ __device__ __forceinline__ float inso_vertex(const InsoArgs &a, double X, double
         // day costs a max and an add per rotation pair.  Days with |k| near 0
         // take the direct form.
         float au[HP > 0 ? HP : 2];
-        if (!tt || bk.nf < 0) {
+        if (!BREAKS && (!tt || bk.nf < 0)) {
 #pragma unroll
             for (int h = 0; h < (HP > 0 ? HP : 2); ++h) {
                 const float2 q = a.rot[h];
                 au[h] = fabsf(fmaf(x, q.x, -(y * q.y)));
             }
         }
-        if (tt) {
+        if (BREAKS || tt) {
             // constants staged by the block: per day a shared load, one
             // multiply for the threshold, the max / add of each pair and one
             // paired multiply-add into the group's lanes; the days' C terms
@@ -585,7 +596,7 @@ __device__ __forceinline__ float inso_vertex(const InsoArgs &a, double X, double
                 comp = (tk - tot) - yk;
                 tot = tk;
             };
-            if (bk.nf >= 0) {
+            if (BREAKS || bk.nf >= 0) {
                 // each pair's line pair from its bucket of t = a_h / |z|
                 // (|z| kept off 0: 1e-20 r in its place changes no value)
                 const float ti = approx_rcp(fmaxf(az, zmin)) * bk.inv;
@@ -722,20 +733,28 @@ __device__ __forceinline__ Breaks stage_all(const InsoArgs &a, float4 *s_tilt)
     stage_tilts<HP>(a, s_tilt);
     if (a.n_tilt <= SORT_MAX) {
         // 16-byte units: the bucket table first, then the lines, then the rest
-        const int sp = sort_pad(a.n_tilt + 1);
         float4 *bucket = s_tilt + a.n_tilt + 1 + (a.n_tilt + 3) / 4;
-        float2 *L = reinterpret_cast<float2 *>(bucket + sp + 1);
+        float2 *L = reinterpret_cast<float2 *>(bucket + bucket_count(a.n_tilt) + 1);
         uint2 *K = reinterpret_cast<uint2 *>(L + a.n_tilt + 1);
         bk = stage_breakpoints(a, s_tilt, K, L, bucket);
     }
     return bk;
 }
 
-template <int HP>
-__global__ void __launch_bounds__(256, 4) insolation_kernel(InsoArgs a)
+// Threads of a block: two of 512 per SM for the breakpoints' tables (half as
+// many tables to build as with 256), in a kernel without the other forms,
+// whose registers it spilled: a year on 10,000,002 vertices 142 -> 111 us (2.5
+// TB/s of the 28 B per vertex), 40,000,002 521 -> 355 us.  One block of 768
+// is as fast on large spheres, 106 instead of 97 us where a bucket is crowded.
+constexpr int BREAK_THREADS = 512, BREAK_BLOCKS = 2;
+template <bool BREAKS>
+constexpr int INSO_THREADS = BREAKS ? BREAK_THREADS : 256;
+
+template <int HP, bool BREAKS>
+__device__ __forceinline__ void insolation_body(const InsoArgs &a)
 {
     extern __shared__ float4 s_tilt[];
-    const bool staged = HP > 0 && a.pairs && a.n_tilt <= TILT_STAGE_MAX;
+    const bool staged = BREAKS || (HP > 0 && a.pairs && a.n_tilt <= TILT_STAGE_MAX);
     Breaks bk;
     Arcs arc;
     if (staged) bk = stage_all<HP>(a, s_tilt);
@@ -750,7 +769,7 @@ __global__ void __launch_bounds__(256, 4) insolation_kernel(InsoArgs a)
         const double cx = X, cy = Y, cz = Z;
         const int64_t j = i + step;
         if (j < a.n) { X = a.xyz[3 * j]; Y = a.xyz[3 * j + 1]; Z = a.xyz[3 * j + 2]; }
-        const float tot = inso_vertex<HP>(a, cx, cy, cz, a.r, a.r2h, a.r2l, a.zmin, a.inv_r, staged ? s_tilt : nullptr,
+        const float tot = inso_vertex<HP, BREAKS>(a, cx, cy, cz, a.r, a.r2h, a.r2l, a.zmin, a.inv_r, staged ? s_tilt : nullptr,
                                           bk, arc);
         // the scale here instead of in a pass of its own over the sums (10 M
         // vertices: 11 us of 137)
@@ -759,14 +778,36 @@ __global__ void __launch_bounds__(256, 4) insolation_kernel(InsoArgs a)
     }
 }
 
+template <int HP, bool BREAKS = false>
+__global__ void __launch_bounds__(INSO_THREADS<BREAKS>, BREAKS ? BREAK_BLOCKS : 4) insolation_kernel(InsoArgs a)
+{
+    insolation_body<HP, BREAKS>(a);
+}
+
+// A short schedule's table as a kernel argument (a table of its own on the
+// device takes another launch, ~3 us).
+constexpr int ARG_POSITIONS = 496;
+struct InsoTable {
+    float2 t[ARG_POSITIONS];
+};
+
+template <int HP, bool BREAKS = false>
+__global__ void __launch_bounds__(INSO_THREADS<BREAKS>, BREAKS ? BREAK_BLOCKS : 4)
+    insolation_args_kernel(InsoArgs a, const __grid_constant__ InsoTable table)
+{
+    a.rot = table.t;
+    a.tilt = table.t + a.n_rot;
+    insolation_body<HP, BREAKS>(a);
+}
+
 // Many planets: planet p's vertices fill packed rows [vbeg, vbeg + n)
 // (vbeg a multiple of 256); one block covers 256 rows of one planet.
-template <int HP>
-__global__ void __launch_bounds__(256, 3) insolation_batch_kernel(InsoArgs a, const nx_inso_planet *__restrict__ P, int np,
+template <int HP, bool BREAKS = false>
+__global__ void __launch_bounds__(256, BREAKS ? 4 : 3) insolation_batch_kernel(InsoArgs a, const nx_inso_planet *__restrict__ P, int np,
                                                                int64_t total_rows)
 {
     extern __shared__ float4 s_tilt[];
-    const bool staged = HP > 0 && a.pairs && a.n_tilt <= TILT_STAGE_MAX;
+    const bool staged = BREAKS || (HP > 0 && a.pairs && a.n_tilt <= TILT_STAGE_MAX);
     Breaks bk;
     Arcs arc;
     if (staged) bk = stage_all<HP>(a, s_tilt);
@@ -792,7 +833,7 @@ __global__ void __launch_bounds__(256, 3) insolation_batch_kernel(InsoArgs a, co
         const int64_t i = blk * 256 + threadIdx.x - beg;
         if (i < 0 || i >= P[p].n) continue;
         const double *xyz = P[p].xyz;
-        a.out[beg + i] = inso_vertex<HP>(a, xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], r, r2h, r2l, zmin, inv_r,
+        a.out[beg + i] = inso_vertex<HP, BREAKS>(a, xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], r, r2h, r2l, zmin, inv_r,
                                          staged ? s_tilt : nullptr, bk, arc);
     }
 }
@@ -927,8 +968,8 @@ size_t tilt_smem(const InsoArgs &a)
     if (!a.pairs || a.n_tilt > TILT_STAGE_MAX) return 0;
     size_t b = sizeof(float4) * ((size_t)a.n_tilt + 1) + sizeof(int) * (size_t)a.n_tilt;
     if (a.n_tilt <= SORT_MAX) {    // the list rounded to 16 bytes, bucket table, lines, sorted days
-        const size_t sp = (size_t)sort_pad(a.n_tilt + 1), nt = (size_t)a.n_tilt;
-        b = sizeof(float4) * (nt + 1 + (nt + 3) / 4 + sp + 1) + sizeof(float2) * (nt + 1 + sp);
+        const size_t sp = (size_t)sort_pad(a.n_tilt + 1), nb = (size_t)bucket_count(a.n_tilt), nt = (size_t)a.n_tilt;
+        b = sizeof(float4) * (nt + 1 + (nt + 3) / 4 + nb + 1) + sizeof(float2) * (nt + 1 + sp);
     }
     return b;
 }
@@ -944,9 +985,13 @@ int grid_for(int64_t n, int per_sm = 8)
 // Blocks of a 12-pair launch: a block that sums by breakpoints sorts the
 // schedule first, so the grid is the resident blocks (4 per SM) and each
 // block takes many vertices.
-int grid_staged(int64_t n, const InsoArgs &a)
+// Whether a schedule is summed by breakpoints.
+bool breaks(const InsoArgs &a) { return a.pairs && a.n_rot == 12 && a.n_tilt <= SORT_MAX; }
+
+int grid_breaks(int64_t n)
 {
-    return grid_for(n, a.pairs && a.n_tilt <= SORT_MAX ? 4 : 8);
+    const int64_t g = (n + INSO_THREADS<true> - 1) / INSO_THREADS<true>, cap = (int64_t)nx::sm_count() * BREAK_BLOCKS;
+    return (int)(g < cap ? g : cap);
 }
 
 // Whether a schedule is summed by arcs.
@@ -992,11 +1037,11 @@ NX_EXPORT int nx_insolation_plan(const double *rot_deg, int n_rot, const double 
 }
 
 static int insolation_sums(const double *xyz_dev, int64_t n, double radius, const float *table_dev, int n_rot_entries,
-                           int pairs, int n_tilt, float scale, float *out_dev, int accumulate, void *stream)
+                           int pairs, int n_tilt, float scale, float *out_dev, int accumulate, void *stream, const float *table_host = nullptr)
 {
     if (n < 0 || n_rot_entries < 0 || n_tilt < 0) return nx::fail(NX_EINVAL, "nx_insolation: negative size");
     if (n == 0) return NX_OK;
-    if (!xyz_dev || !out_dev || ((n_rot_entries || n_tilt) && !table_dev))
+    if (!xyz_dev || !out_dev || ((n_rot_entries || n_tilt) && !table_dev && !table_host))
         return nx::fail(NX_EINVAL, "nx_insolation: null pointer");
     if (!(radius > 0.0)) return nx::fail(NX_EINVAL, "nx_insolation: radius must be > 0");
     cudaStream_t s = (cudaStream_t)stream;
@@ -1019,12 +1064,27 @@ static int insolation_sums(const double *xyz_dev, int64_t n, double radius, cons
     a.out = out_dev;
     a.accumulate = accumulate;
     a.scale = scale;
-    if (a.pairs && n_rot_entries == 12)
-        insolation_kernel<12><<<grid_staged(n, a), 256, tilt_smem(a), s>>>(a);
-    else if (use_arcs(a, n))
-        insolation_kernel<ARCS><<<grid_for(n, 4), 256, arc_smem(a.pairs ? 2 * a.n_rot : a.n_rot), s>>>(a);
-    else
+    const size_t arcs = arc_smem(a.pairs ? 2 * a.n_rot : a.n_rot);
+    if (table_host) {
+        InsoTable T;
+        memcpy(T.t, table_host, sizeof(float2) * (size_t)(n_rot_entries + n_tilt));
+        if (breaks(a))
+            insolation_args_kernel<12, true><<<grid_breaks(n), INSO_THREADS<true>, tilt_smem(a), s>>>(a, T);
+        else if (a.pairs && n_rot_entries == 12)
+            insolation_args_kernel<12><<<grid_for(n), 256, tilt_smem(a), s>>>(a, T);
+        else if (use_arcs(a, n))
+            insolation_args_kernel<ARCS><<<grid_for(n, 4), 256, arcs, s>>>(a, T);
+        else
+            insolation_args_kernel<0><<<grid_for(n), 256, 0, s>>>(a, T);
+    } else if (breaks(a)) {
+        insolation_kernel<12, true><<<grid_breaks(n), INSO_THREADS<true>, tilt_smem(a), s>>>(a);
+    } else if (a.pairs && n_rot_entries == 12) {
+        insolation_kernel<12><<<grid_for(n), 256, tilt_smem(a), s>>>(a);
+    } else if (use_arcs(a, n)) {
+        insolation_kernel<ARCS><<<grid_for(n, 4), 256, arcs, s>>>(a);
+    } else {
         insolation_kernel<0><<<grid_for(n), 256, 0, s>>>(a);
+    }
     NX_CHECK_LAUNCH("insolation_kernel");
     nx::note_launch(1);
     return NX_OK;
@@ -1048,11 +1108,13 @@ NX_EXPORT int nx_insolation_positions(const double *xyz_dev, int64_t n, double r
     int entries = 0, pairs = 0;
     int rc = nx_insolation_plan(rot_deg, n_rot, tilt_deg, n_tilt, table, &entries, &pairs);
     if (rc) return rc;
-    if (n_rot && n_tilt) {
+    const bool args = entries + n_tilt <= ARG_POSITIONS;
+    if (n_rot && n_tilt && !args) {
         rc = nx_upload(table_dev, table, (int64_t)sizeof(float) * 2 * (entries + n_tilt), stream);
         if (rc) return rc;
     }
-    return insolation_sums(xyz_dev, n, radius, table_dev, entries, pairs, n_tilt, (float)scale, out_dev, accumulate, stream);
+    return insolation_sums(xyz_dev, n, radius, table_dev, entries, pairs, n_tilt, (float)scale, out_dev, accumulate, stream,
+                           args ? table : nullptr);
 }
 
 // climate.calculate_seasonal_tilt(axial, climate.day2deg(year, d)) for days
@@ -1098,8 +1160,10 @@ NX_EXPORT int nx_insolation_batch(const nx_inso_planet *planets_dev, const nx_in
     a.accumulate = 0;
     a.scale = 1.0f;
     cudaStream_t s = (cudaStream_t)stream;
-    if (a.pairs && n_rot_entries == 12)
-        insolation_batch_kernel<12><<<grid_staged(total, a), 256, tilt_smem(a), s>>>(a, planets_dev, nplanets, total);
+    if (breaks(a))
+        insolation_batch_kernel<12, true><<<grid_for(total, 4), 256, tilt_smem(a), s>>>(a, planets_dev, nplanets, total);
+    else if (a.pairs && n_rot_entries == 12)
+        insolation_batch_kernel<12><<<grid_for(total), 256, tilt_smem(a), s>>>(a, planets_dev, nplanets, total);
     else if (use_arcs(a, total))
         insolation_batch_kernel<ARCS><<<grid_for(total, 4), 256, arc_smem(a.pairs ? 2 * a.n_rot : a.n_rot), s>>>(
             a, planets_dev, nplanets, total);

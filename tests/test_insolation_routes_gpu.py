@@ -5,6 +5,8 @@ to n/pi, each rounded once (4 roundings of 2^-25), three products (2^-24 each) a
 either end of the arc, whose term is then within 1e-6 of 0; by breakpoints the lines' sums are rounded once and 12 values
 of a few roundings each are added.
 """
+import math
+
 import numpy as np
 import pytest
 
@@ -56,3 +58,21 @@ def test_large_sphere_and_batch_rows_take_the_same_values():
         rot, tilts = climate.annual_schedule(r.axial_tilt, r.days, r.days, r.hours)
         want = climate.insolation_sum(mesh.PlanetMesh(r.divisions).xyz, 1.0, rot, tilts) * (climate.SOLAR_CONSTANT / (r.days * r.hours))
         assert torch.equal(got.insolation, want)
+
+
+@pytest.mark.parametrize("days", [1, 2, 7, 30, 127, 128, 255, 256, 300, 366, 400, 495, 511, 512, 513])
+def test_bucket_tables_of_any_length(days):
+    """Hourly positions over `days` days, days past the first year repeating (equal and nearly equal breakpoints), as
+    the sum of its terms one by one."""
+    import torch
+    from nixis_gb300 import climate, mesh
+    m = mesh.PlanetMesh(23)
+    rot, tilts = climate.annual_schedule(23.44, 365, days, 24)
+    got = climate.insolation_sum(m.xyz, 1.0, rot, tilts).double()
+    r, t = (torch.tensor(v, dtype=torch.float64, device="cuda") * (math.pi / 180) for v in (rot, tilts))
+    x, y, z = m.xyz.T
+    want = torch.zeros(m.n, dtype=torch.float64, device="cuda")
+    for tau in t:
+        u = (x[:, None] * r.cos() - y[:, None] * r.sin()) * tau.cos() + (z * tau.sin())[:, None]
+        want += u.clamp(min=0).sum(1)
+    assert (got - want).abs().max() <= 2e-6 * want.max()
