@@ -358,13 +358,8 @@ class PlanetBatch:
 
 
 def _tb_npass(iters, R):
-    """Passes of a temporally blocked run: ceil(iters/R), made = iters mod 2."""
-    if iters <= 0:
-        return 0
-    n = (iters + R - 1) // R
-    if (n ^ iters) & 1:
-        n += 1
-    return n
+    """Passes of a blocked run that starts from the raw sums."""
+    return (iters + R - 1) // R if iters > 0 else 0
 
 
 def generate_batched(requests, meshes=None):
