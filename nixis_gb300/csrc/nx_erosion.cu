@@ -544,7 +544,8 @@ __device__ __forceinline__ void tb_update(int l, const TileRow &row, const float
     }
     Pair hn, wn, sn;
     erode_finish(Pair{me.x, me.y}, Pair{me.z, me.w}, Pair{ms.x, ms.y}, A, L, hn, wn, sn);
-    const Pair wr = more ? prain(wn.h, wn.l, rain) : wn;
+    Pair wr = wn;
+    if (more) wr = prain(wn.h, wn.l, rain);
     nxt[l] = make_float4(hn.h, hn.l, wr.h, wr.l);
     sed[l] = make_float2(sn.h, sn.l);
 }
@@ -682,8 +683,11 @@ __global__ void __launch_bounds__(THREADS, MINB > 0 ? MINB : (PF ? 768 : 1024) /
         const float4 *cur = (mi & 1) ? buf1 : buf0;
         float4 *nxt = (mi & 1) ? buf0 : buf1;
         const bool more = mi + 1 < len;          // rain for the next iteration in the pass
+        // (no rain: adding 0 changes no value; 2.18 -> 2.14 ms for 24 iterations
+        // of 6,400,002 vertices)
+        const bool wet = more && rain != 0.0f;
         if (ONE) {
-            if ((int)threadIdx.x < C) tb_update(threadIdx.x, myrow, cur, nxt, sed, rain, more);
+            if ((int)threadIdx.x < C) tb_update(threadIdx.x, myrow, cur, nxt, sed, rain, wet);
         } else {
             TileRow nextrow;
             if (PF && (int)threadIdx.x < C) nextrow = tile_row<SMT>(lnb, led, threadIdx.x);
@@ -703,7 +707,7 @@ __global__ void __launch_bounds__(THREADS, MINB > 0 ? MINB : (PF ? 768 : 1024) /
                 } else {
                     row = tile_row<SMT>(lnb, led, l);
                 }
-                tb_update(l, row, cur, nxt, sed, rain, more);
+                tb_update(l, row, cur, nxt, sed, rain, wet);
             }
         }
         __syncthreads();
