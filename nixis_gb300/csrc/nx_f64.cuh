@@ -124,6 +124,48 @@ __device__ __forceinline__ double times(double a, int w)
     return __longlong_as_double((long long)(b | ((unsigned long long)sign << 32)));
 }
 
+// A factor b for mul: its significand in the top 53 bits of m (0: b outside
+// [2^-500, 2^500), products take the binary64 pipe).
+struct Factor {
+    double b;
+    unsigned long long m;
+    uint32_t hw;
+};
+
+__device__ __forceinline__ Factor factor(double b)
+{
+    const uint2 w = words(b);
+    const bool in = ((w.y >> 20) & 0x7FFu) - 523u < 1000u;
+    return Factor{b, in ? ((unsigned long long)((w.y & 0xFFFFFu) | 0x100000u) << 43) | ((unsigned long long)w.x << 11) : 0ull, w.y};
+}
+
+static __device__ __noinline__ double mul_slow(double a, double b) { return __dmul_rn(a, b); }
+
+// a * F.b, correctly rounded, without the binary64 pipe: the top 64 bits of
+// the significands' product round to 53 whatever the others are unless they
+// end in a half exactly (one in 2^11, then and outside the ranges the
+// binary64 product).  About 28 integer operations, half the pipe's 16 cycles
+// of a warp where the others are free.
+__device__ __forceinline__ double mul(double a, const Factor &F)
+{
+    const uint2 w = words(a);
+    const uint32_t e = (w.y >> 20) & 0x7FFu;
+    if (e - 523u < 1000u && F.m) {
+        const unsigned long long A = ((unsigned long long)((w.y & 0xFFFFFu) | 0x100000u) << 43) | ((unsigned long long)w.x << 11);
+        const unsigned long long hi = __umul64hi(A, F.m);            // in [2^62, 2^64)
+        const uint32_t top = (uint32_t)(hi >> 63);
+        const unsigned long long x = top ? hi : hi << 1;
+        if (((uint32_t)x & 0x7FFu) != 0x400u) {
+            const unsigned long long m = (x >> 11) + (((uint32_t)x >> 10) & 1u);
+            // (m's leading bit adds 1 to the exponent field)
+            const uint32_t field = e + ((F.hw >> 20) & 0x7FFu) - 1024u + top;
+            const unsigned long long b = m + ((unsigned long long)(field | ((w.y ^ F.hw) >> 20 & 0x800u)) << 52);
+            return __longlong_as_double((long long)b);
+        }
+    }
+    return mul_slow(a, F.b);
+}
+
 static __device__ __noinline__ double div_slow(double a, double b) { return __ddiv_rn(a, b); }
 static __device__ __noinline__ double sqrt_slow(double s) { return __dsqrt_rn(s); }
 

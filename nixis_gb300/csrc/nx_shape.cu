@@ -23,13 +23,14 @@
 // memory.  A division or square root costs one of them (nx_f64.cuh) instead
 // of about ten, comparisons and keys none (integers), operations of the
 // reference that change nothing (* 1.0, / 1.0, + 0.0) are left out, and the
-// whole shaping is four passes, ~14 binary64 operations a vertex: the two
+// whole shaping is four passes, ~11 binary64 operations a vertex: the two
 // masked ranges come from one pass over h1 (the land's values are the same
 // before and after the ocean's power curve), and the extremes of a monotone
 // map are the map of the extremes, so neither needs a pass of its own.
 // Measured (GB300, shape_heights of 6,400,002 heights): 975 -> 268 us (20
-// passes before); the two curve passes run the binary64 pipe at 81-83 %, the
-// pass with the scan at 61 %.
+// passes before); with the products put together from integers as well
+// (nxf::mul) 280 -> 250 us on another machine, a rescale 84 -> 67: the
+// binary64 pipe is then busy for 49-77 % of a pass, the integer one for 58-62.
 #include "nx_common.cuh"
 #include "nx_f64.cuh"
 
@@ -85,18 +86,19 @@ struct RescaleArgs {
 
 // One linear map ((v - from) / span) * width + to.
 struct Linear {
-    double from, width, to;
+    double from, to;
+    nxf::Factor width;
     nxf::Recip span;
     __device__ __forceinline__ double operator()(double v) const
     {
-        return __dadd_rn(__dmul_rn(nxf::div(__dsub_rn(v, from), span), width), to);
+        return __dadd_rn(nxf::mul(nxf::div(__dsub_rn(v, from), span), width), to);
     }
 };
 
 __device__ __forceinline__ Linear rescale_low(const RescaleArgs &a, double x_min, double x_max)
 {
     const double end = a.form == 0 ? x_max : a.mid, top = a.form == 0 ? a.upper : a.mid;
-    return Linear{x_min, __dsub_rn(top, a.lower), a.lower, nxf::recip(__dsub_rn(end, x_min))};
+    return Linear{x_min, a.lower, nxf::factor(__dsub_rn(top, a.lower)), nxf::recip(__dsub_rn(end, x_min))};
 }
 
 // find_percent_val (util.py:556-566)
@@ -198,7 +200,7 @@ __global__ void __launch_bounds__(THREADS) rescale_kernel(const double *__restri
     if (a.has_umin && a.u_min < x_min) x_min = a.u_min;
     if (a.has_umax && a.u_max > x_max) x_max = a.u_max;
     const Linear low = rescale_low(a, x_min, x_max);
-    const Linear high{a.mid, __dsub_rn(a.upper, a.mid), a.mid, nxf::recip(__dsub_rn(x_max, a.mid))};
+    const Linear high{a.mid, a.mid, nxf::factor(__dsub_rn(a.upper, a.mid)), nxf::recip(__dsub_rn(x_max, a.mid))};
     // v <= mid and v >= mid by keys (false for a NaN on either side)
     const bool no_mid = is_nan(a.mid);
     const u64 kmid = dkey(a.mid);
@@ -212,8 +214,9 @@ __global__ void __launch_bounds__(THREADS) rescale_kernel(const double *__restri
         const bool none = no_mid || is_nan(v), below = !none && k <= kmid;
         if (FORM == 1) {
             // the operands selected, so that warps on both sides run one path
-            const Linear both{nxf::pick(below, low.from, high.from), nxf::pick(below, low.width, high.width),
-                              nxf::pick(below, low.to, high.to),
+            const Linear both{nxf::pick(below, low.from, high.from), nxf::pick(below, low.to, high.to),
+                              nxf::Factor{nxf::pick(below, low.width.b, high.width.b),
+                                          below ? low.width.m : high.width.m, below ? low.width.hw : high.width.hw},
                               nxf::Recip{nxf::pick(below, low.span.b, high.span.b), below ? low.span.y1 : high.span.y1,
                                          below ? low.span.y2 : high.span.y2}};
             out[i] = both(v);
@@ -291,7 +294,8 @@ __device__ __forceinline__ Range range_of(const Run &r, u64 kmin, u64 kmax)
 // The map of power_rescale (util.py:223-248): ((v - lo) / range) ** power,
 // back to the range.
 struct Curve {
-    double lo, range, power;
+    double lo, power;
+    nxf::Factor range;
     nxf::Recip span;
     __device__ __forceinline__ double operator()(double v) const
     {
@@ -299,14 +303,14 @@ struct Curve {
         if (power == 2.0) t = __dmul_rn(t, t);
         else if (power == 0.5) t = nxf::sqrt(t);
         else if (power != 1.0) t = pow(__dadd_rn(t, 0.0), power);
-        return __dadd_rn(__dmul_rn(t, range), lo);
+        return __dadd_rn(nxf::mul(t, range), lo);
     }
 };
 
 __device__ __forceinline__ Curve curve_of(const Range &r, double power)
 {
     const double range = __dsub_rn(r.hi, r.lo);
-    return Curve{r.lo, range, power, nxf::recip(range)};
+    return Curve{r.lo, power, nxf::factor(range), nxf::recip(range)};
 }
 
 // All chunks' runs joined by one block; valid in thread 0.
@@ -437,11 +441,13 @@ __global__ void __launch_bounds__(THREADS) shape_curve_kernel(const double *__re
         const double v = h1[i];
         // the operands selected, so that a coast's warps run one path
         const bool wet = !dry && dkey(v) <= klev;
-        const double lo = nxf::pick(wet, sea.lo, land.lo), range = nxf::pick(wet, sea.range, land.range);
-        double t = nxf::div(__dsub_rn(v, lo), nxf::Recip{range, wet ? sea.span.y1 : land.span.y1, wet ? sea.span.y2 : land.span.y2});
+        const double lo = nxf::pick(wet, sea.lo, land.lo);
+        const nxf::Factor range{nxf::pick(wet, sea.range.b, land.range.b), wet ? sea.range.m : land.range.m,
+                                wet ? sea.range.hw : land.range.hw};
+        double t = nxf::div(__dsub_rn(v, lo), nxf::Recip{range.b, wet ? sea.span.y1 : land.span.y1, wet ? sea.span.y2 : land.span.y2});
         if (wet) t = nxf::sqrt(t);
-        else t = __dmul_rn(t, t);
-        const double r = __dsub_rn(__dadd_rn(__dmul_rn(t, range), lo), level);
+        else t = nxf::mul(t, nxf::factor(t));
+        const double r = __dsub_rn(__dadd_rn(nxf::mul(t, range), lo), level);
         h4[i] = r;
         const u64 q = dkey(r);
         nmin = umax(nmin, ~q);
