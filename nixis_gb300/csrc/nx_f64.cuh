@@ -166,6 +166,23 @@ __device__ __forceinline__ double mul(double a, const Factor &F)
     return mul_slow(a, F.b);
 }
 
+// a * a, as mul.
+__device__ __forceinline__ double square(double a)
+{
+    const uint2 w = words(a);
+    const uint32_t e = (w.y >> 20) & 0x7FFu;
+    if (e - 523u < 1000u) {
+        const unsigned long long A = ((unsigned long long)((w.y & 0xFFFFFu) | 0x100000u) << 43) | ((unsigned long long)w.x << 11);
+        const unsigned long long hi = __umul64hi(A, A);
+        const uint32_t top = (uint32_t)(hi >> 63);
+        const unsigned long long x = top ? hi : hi << 1;
+        if (((uint32_t)x & 0x7FFu) != 0x400u)
+            return __longlong_as_double((long long)((x >> 11) + (((uint32_t)x >> 10) & 1u) +
+                                                    ((unsigned long long)(2u * e - 1024u + top) << 52)));
+    }
+    return mul_slow(a, a);
+}
+
 static __device__ __noinline__ double div_slow(double a, double b) { return __ddiv_rn(a, b); }
 static __device__ __noinline__ double sqrt_slow(double s) { return __dsqrt_rn(s); }
 

@@ -41,13 +41,14 @@ __constant__ IcoHome c_home;
 
 // Point = normalise(w0*A + w1*B + w2*C), sums in the written order, no FMA.
 // GB300's two binary64 operations per SM and cycle bound the vertices: the
-// integer multiples come from integer products, the norm and the quotients
-// from one binary64 operation each (nx_f64.cuh), which leaves 15 a vertex of
-// about 58.  Measured (GB300, 4,900,002 vertices): 506 -> 173 us.
+// integer multiples and the squares come from integer products, the norm and
+// the quotients from one binary64 operation each (nx_f64.cuh), which leaves 12
+// a vertex of about 58.  Measured (GB300, 4,900,002 vertices): 506 -> 173 us;
+// with the squares, 10,000,002 vertices 363 -> 304.
 __device__ __forceinline__ void normalise(const double *p, double *out)
 {
     const double r = nxf::sqrt(
-        __dadd_rn(__dadd_rn(__dmul_rn(p[0], p[0]), __dmul_rn(p[1], p[1])), __dmul_rn(p[2], p[2])));
+        __dadd_rn(__dadd_rn(nxf::square(p[0]), nxf::square(p[1])), nxf::square(p[2])));
     const nxf::Recip R = nxf::recip(r);
     for (int c = 0; c < 3; ++c) out[c] = nxf::div(p[c], R);
 }
@@ -256,7 +257,7 @@ __device__ __forceinline__ double edge_len(const double *xyz, int64_t v, int64_t
     const double dx = __dsub_rn(xyz[3 * v], xyz[3 * j]);
     const double dy = __dsub_rn(xyz[3 * v + 1], xyz[3 * j + 1]);
     const double dz = __dsub_rn(xyz[3 * v + 2], xyz[3 * j + 2]);
-    return nxf::sqrt(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
+    return nxf::sqrt(__dadd_rn(__dadd_rn(nxf::square(dx), nxf::square(dy)), nxf::square(dz)));
 }
 
 __device__ __forceinline__ float2 edge_pair(double d) { return nxf::pair(d); }
@@ -446,10 +447,11 @@ __global__ void __launch_bounds__(256) ico_neighbours_kernel(int k, int64_t nv, 
 // one distance: a vertex computes its slots 2-4, (i, j+1), (i+1, j) and
 // (i+1, j-1), and writes each into its own row and the neighbour's opposite
 // slot (s + 3) mod 6.  Distances to vertices of edges and corners are
-// computed by both sides.  So 9 binary64 operations an edge, each edge once,
-// and no search for the reverse slot.  Measured (GB300, 4,900,002 vertices):
-// 359 us, against ~880 us for the general pair of passes before (the binary64
-// operations alone take 227 us).
+// computed by both sides.  So 6 binary64 operations an edge (the squares come
+// from integer products), each edge once, and no search for the reverse slot.
+// Measured (GB300, 4,900,002 vertices): 289 us, 359 us with the squares in
+// binary64 (the binary64 operations alone take 151 and 227 us), ~880 us for
+// the general pair of passes before.
 __global__ void __launch_bounds__(256) ico_edges_kernel(int k, int64_t nv, const double *__restrict__ xyz,
                                                         const int32_t *__restrict__ nbr, float2 *__restrict__ el,
                                                         int *__restrict__ info)
@@ -1386,7 +1388,7 @@ __device__ __forceinline__ void best_take(Best &b, const double *xyz, int64_t v,
 {
     if (v == b.i[0] || v == b.i[1] || v == b.i[2]) return;
     const double dx = __dsub_rn(qx, xyz[3 * v]), dy = __dsub_rn(qy, xyz[3 * v + 1]), dz = __dsub_rn(qz, xyz[3 * v + 2]);
-    const double d = nxf::sqrt(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
+    const double d = nxf::sqrt(__dadd_rn(__dadd_rn(nxf::square(dx), nxf::square(dy)), nxf::square(dz)));
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
         if (!(d < b.d[m] || (d == b.d[m] && v < b.i[m]))) continue;
