@@ -915,7 +915,9 @@ __device__ __forceinline__ int hinsert(const HashSet &H, int32_t *key, int32_t *
 {
     uint32_t h = hslot(H, v);
     for (uint32_t probe = 0; probe <= H.mask; ++probe) {
-        const int32_t old = atomicCAS(&key[h], -1, v);
+        // (most are there already: a read costs less than an exchange)
+        const int32_t seen = *reinterpret_cast<volatile int32_t *>(key + h);
+        const int32_t old = seen == -1 ? atomicCAS(&key[h], -1, v) : seen;
         if (old == -1) {
             const int idx = atomicAdd(cnt, 1);
             if (idx >= nmax) { val[h] = -1; return -1; }
@@ -958,7 +960,10 @@ __device__ __forceinline__ int square_distance(int i, int j, int B)
 // neighbour table that differs from the icosphere's in these rows is left to
 // the search (false).  Measured (GB300, divisions 700, 5,060 tiles of side 32
 // with 4 rings): the build 640 -> 290 us with the members found by the tiles
-// themselves; the searched tiles (about a third) take most of it.
+// themselves.  Bound by issue (69 % of the slots) and by the searched tiles
+// (about a third); rows by reciprocal, keys read before they are exchanged
+// and slots stored two at a time 329 -> 289 us on a slower machine, divisions
+// 1,000 585 -> 508.
 __device__ bool inner_tile(int k, int B, int R, int f, int i0, int j0, int nmax, const int32_t *__restrict__ nbr,
                            const float *__restrict__ edge, int32_t *__restrict__ tc, int32_t *__restrict__ tid,
                            uint32_t *__restrict__ lnbr, float4 *__restrict__ ledge, int *__restrict__ err, int32_t *sh)
@@ -970,19 +975,22 @@ __device__ bool inner_tile(int k, int B, int R, int f, int i0, int j0, int nmax,
     int32_t *cnt = reinterpret_cast<int32_t *>(map + ((np + 1) & ~1));     // [ring][chunk]
     __shared__ int s_base[10];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const uint32_t inv = 0xFFFFFFFFu / (uint32_t)W + 1u;
+    auto row_of = [&](int p) { return (int)__umulhi((uint32_t)p, inv); };     // p / W (p < 2^16)
     auto ring_of = [&](int p) {
-        const int a = p / W, d = p < np ? square_distance(a - R, p - a * W - R, B) : 99;
+        const int a = row_of(p), d = p < np ? square_distance(a - R, p - a * W - R, B) : 99;
         return d <= R ? d : 99;
     };
     const int64_t inner = 12 + (int64_t)30 * (k - 1) + (int64_t)f * ((int64_t)(k - 1) * (k - 2) / 2);
     auto id_of = [&](int p) {
-        const int64_t i = i0 + p / W - R, j = j0 + p % W - R;
+        const int a = row_of(p);
+        const int64_t i = i0 + a - R, j = j0 + p - a * W - R;
         return (int32_t)(inner + (i - 1) * (k - 1) - (i - 1) * i / 2 + j - 1);
     };
     bool same = true;
     for (int p = threadIdx.x; p < np; p += blockDim.x) {
         if (ring_of(p) >= R) continue;
-        const int32_t v = id_of(p), len = k - 1 - (i0 + p / W - R);
+        const int32_t v = id_of(p), len = k - 1 - (i0 + row_of(p) - R);
         const int2 *row = reinterpret_cast<const int2 *>(nbr + 6 * (int64_t)v);
         const int2 a = row[0], b = row[1], c = row[2];
         same = same && a.x == v - len - 1 && a.y == v - len && b.x == v + 1 && b.y == v + len && c.x == v + len - 1 && c.y == v - 1;
@@ -1220,39 +1228,48 @@ __global__ void __launch_bounds__(512) tile_rings_kernel(int k, int B, bool alig
     if (C0 > cmax) { if (threadIdx.x == 0) s_bad = 1; C0 = cmax; }
     __syncthreads();
     for (int q = threadIdx.x; q < NL; q += blockDim.x) tid[q] = list[q];
-    // four slots per thread per round, their global reads issued before any
-    // hash probe (independent loads in flight instead of a dependent chain)
-    constexpr int U = 4;
-    const int nslot = C0 * 6;
-    for (int w0 = threadIdx.x; w0 < nslot; w0 += U * blockDim.x) {
-        int32_t jv[U];
-        float2 ev[U];
+    // a missing neighbour (-1, pentagon slot) points at the vertex itself: the
+    // erosion update then sees equal heights and adds nothing
+    auto local = [&](int q, int32_t j) {
+        if (j < 0) return q;
+        const int loc = hfind(H, key, val, j);
+        if (loc < 0) { s_bad = 1; return q; }
+        return loc;
+    };
+    if (aligned) {
+        // two slots at a time, the global reads of two rounds issued before any
+        // hash probe
+        uint32_t *nb = reinterpret_cast<uint32_t *>(lnbr) + tile * 3 * cmax;
+        float4 *ed = reinterpret_cast<float4 *>(ledge) + tile * 3 * cmax;
+        constexpr int U = 2;
+        for (int w0 = threadIdx.x; w0 < 3 * C0; w0 += U * blockDim.x) {
+            int2 jv[U];
+            float4 ev[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int w = w0 + u * blockDim.x;
-            if (w < nslot) {
-                const int64_t g = 6 * (int64_t)list[w / 6] + w % 6;
-                jv[u] = nbr[g];
-                ev[u] = reinterpret_cast<const float2 *>(edge)[g];
+            for (int u = 0; u < U; ++u) {
+                const int w = w0 + u * blockDim.x;
+                if (w < 3 * C0) {
+                    const int64_t g = 3 * (int64_t)list[w / 3] + w % 3;
+                    jv[u] = reinterpret_cast<const int2 *>(nbr)[g];
+                    ev[u] = reinterpret_cast<const float4 *>(edge)[g];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int w = w0 + u * blockDim.x;
+                if (w < 3 * C0) {
+                    const int q = w / 3, at = tile_unit(q) + 32 * (w % 3);
+                    nb[at] = (uint32_t)local(q, jv[u].x) | ((uint32_t)local(q, jv[u].y) << 16);
+                    ed[at] = ev[u];
+                }
             }
         }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int w = w0 + u * blockDim.x;
-            if (w < nslot) {
-                const int q = w / 6, sl = w % 6;
-                // a missing neighbour (-1, pentagon slot) points at the vertex
-                // itself: the erosion update then sees equal heights and adds
-                // nothing
-                int loc = q;
-                if (jv[u] >= 0) {
-                    loc = hfind(H, key, val, jv[u]);
-                    if (loc < 0) { s_bad = 1; loc = q; }
-                }
-                const int64_t at = 2 * (tile * 3 * cmax + tile_unit(q) + 32 * (sl >> 1)) + (sl & 1);
-                lnbr[at] = (uint16_t)loc;
-                reinterpret_cast<float2 *>(ledge)[at] = ev[u];
-            }
+    } else {
+        for (int w = threadIdx.x; w < 6 * C0; w += blockDim.x) {
+            const int q = w / 6, sl = w % 6;
+            const int64_t g = 6 * (int64_t)list[q] + sl, at = 2 * (tile * 3 * cmax + tile_unit(q) + 32 * (sl >> 1)) + (sl & 1);
+            lnbr[at] = (uint16_t)local(q, nbr[g]);
+            reinterpret_cast<float2 *>(ledge)[at] = reinterpret_cast<const float2 *>(edge)[g];
         }
     }
     if (threadIdx.x == 0) {
@@ -1348,7 +1365,8 @@ NX_EXPORT int nx_tiling_build(int k, int tile, int rings, const int32_t *nbr_dev
     // hash keys + values, the local list (padded for sorting) and a scratch
     const size_t smem = sizeof(int32_t) * (2 * ((size_t)1 << hash_bits_for(nmax)) + 2 * (size_t)P2);
     NX_CHECK_CUDA(cudaFuncSetAttribute(tile_rings_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const bool aligned = (((uintptr_t)edge_dev | (uintptr_t)ledge_dev) & 15u) == 0 && ((uintptr_t)nbr_dev & 7u) == 0;
+    const bool aligned = (((uintptr_t)edge_dev | (uintptr_t)ledge_dev) & 15u) == 0 && ((uintptr_t)nbr_dev & 7u) == 0 &&
+                         ((uintptr_t)lnbr_dev & 3u) == 0;
     tile_rings_kernel<<<nt, 512, smem, s>>>(k, tile > 0 ? tile : 0, aligned, nbr_dev, edge_dev, nv, rings, nmax, cmax,
                                             counts_dev, ids_dev, lnbr_dev, ledge_dev, err_dev);
     NX_CHECK_LAUNCH("tile_rings_kernel");
