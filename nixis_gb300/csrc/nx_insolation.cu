@@ -415,9 +415,9 @@ __device__ __forceinline__ float pair_sum(const Breaks &bk, float x, float y, fl
 // Shared memory: the prefix sums P[n + 1] (exact sums rounded once), the
 // angles less the smallest one, ascending, an index F of NB = a power of two
 // >= n buckets (F[b] = angles below b 2 pi / NB), the rotations' order.
-// Measured (GB300, one tilt, 360 rotations): 110.8 -> 37.8 us for 2,500,002
-// vertices, 420 -> 111 us for 10,000,002 (2.5 TB/s of the 28 B per vertex;
-// instruction issue and the two gathers bound it).
+// Measured (GB300, one tilt, 360 rotations): 110.8 -> 35 us for 2,500,002
+// vertices, 420 -> 100 us for 10,000,002 (2.8 TB/s of the 28 B per vertex;
+// instruction issue and the two gathers bound it; see INSO_THREADS).
 // From ARC_MIN rotations on, and only for ARC_VERTICES vertices or
 // ARC_TERMS positions: below 128 rotations the maxima are as fast or faster
 // (30 tilts of 48 rotations, 625,002 vertices: 113 us against 131 us by
@@ -747,8 +747,12 @@ __device__ __forceinline__ Breaks stage_all(const InsoArgs &a, float4 *s_tilt)
 // TB/s of the 28 B per vertex), 40,000,002 521 -> 355 us.  One block of 768
 // is as fast on large spheres, 106 instead of 97 us where a bucket is crowded.
 constexpr int BREAK_THREADS = 512, BREAK_BLOCKS = 2;
-template <bool BREAKS>
-constexpr int INSO_THREADS = BREAKS ? BREAK_THREADS : 256;
+// By arcs: one block of 1,024 per SM where there are vertices for all of them,
+// blocks of 512 otherwise (a day of 360 rotations, with blocks of 256, 512
+// and 1,024: 10,000,002 vertices 119, 107, 103 us; 2,500,002 43.6, 39.6, 37.5;
+// 9,002 12.9, 12.9, 15.0).
+template <bool BREAKS, int HP>
+constexpr int INSO_THREADS = BREAKS ? BREAK_THREADS : (HP == ARCS ? 1024 : 256);
 
 template <int HP, bool BREAKS>
 __device__ __forceinline__ void insolation_body(const InsoArgs &a)
@@ -779,7 +783,7 @@ __device__ __forceinline__ void insolation_body(const InsoArgs &a)
 }
 
 template <int HP, bool BREAKS = false>
-__global__ void __launch_bounds__(INSO_THREADS<BREAKS>, BREAKS ? BREAK_BLOCKS : 4) insolation_kernel(InsoArgs a)
+__global__ void __launch_bounds__(INSO_THREADS<BREAKS, HP>, BREAKS ? BREAK_BLOCKS : (HP == ARCS ? 1 : 4)) insolation_kernel(InsoArgs a)
 {
     insolation_body<HP, BREAKS>(a);
 }
@@ -792,7 +796,7 @@ struct InsoTable {
 };
 
 template <int HP, bool BREAKS = false>
-__global__ void __launch_bounds__(INSO_THREADS<BREAKS>, BREAKS ? BREAK_BLOCKS : 4)
+__global__ void __launch_bounds__(INSO_THREADS<BREAKS, HP>, BREAKS ? BREAK_BLOCKS : (HP == ARCS ? 1 : 4))
     insolation_args_kernel(InsoArgs a, const __grid_constant__ InsoTable table)
 {
     a.rot = table.t;
@@ -990,7 +994,16 @@ bool breaks(const InsoArgs &a) { return a.pairs && a.n_rot == 12 && a.n_tilt <= 
 
 int grid_breaks(int64_t n)
 {
-    const int64_t g = (n + INSO_THREADS<true> - 1) / INSO_THREADS<true>, cap = (int64_t)nx::sm_count() * BREAK_BLOCKS;
+    const int64_t g = (n + BREAK_THREADS - 1) / BREAK_THREADS, cap = (int64_t)nx::sm_count() * BREAK_BLOCKS;
+    return (int)(g < cap ? g : cap);
+}
+
+int arc_threads(int64_t n) { return n >= (int64_t)nx::sm_count() * 1024 ? 1024 : 512; }
+
+int grid_arcs(int64_t n)
+{
+    const int t = arc_threads(n);
+    const int64_t g = (n + t - 1) / t, cap = (int64_t)nx::sm_count() * (1024 / t);
     return (int)(g < cap ? g : cap);
 }
 
@@ -1069,19 +1082,19 @@ static int insolation_sums(const double *xyz_dev, int64_t n, double radius, cons
         InsoTable T;
         memcpy(T.t, table_host, sizeof(float2) * (size_t)(n_rot_entries + n_tilt));
         if (breaks(a))
-            insolation_args_kernel<12, true><<<grid_breaks(n), INSO_THREADS<true>, tilt_smem(a), s>>>(a, T);
+            insolation_args_kernel<12, true><<<grid_breaks(n), BREAK_THREADS, tilt_smem(a), s>>>(a, T);
         else if (a.pairs && n_rot_entries == 12)
             insolation_args_kernel<12><<<grid_for(n), 256, tilt_smem(a), s>>>(a, T);
         else if (use_arcs(a, n))
-            insolation_args_kernel<ARCS><<<grid_for(n, 4), 256, arcs, s>>>(a, T);
+            insolation_args_kernel<ARCS><<<grid_arcs(n), arc_threads(n), arcs, s>>>(a, T);
         else
             insolation_args_kernel<0><<<grid_for(n), 256, 0, s>>>(a, T);
     } else if (breaks(a)) {
-        insolation_kernel<12, true><<<grid_breaks(n), INSO_THREADS<true>, tilt_smem(a), s>>>(a);
+        insolation_kernel<12, true><<<grid_breaks(n), BREAK_THREADS, tilt_smem(a), s>>>(a);
     } else if (a.pairs && n_rot_entries == 12) {
         insolation_kernel<12><<<grid_for(n), 256, tilt_smem(a), s>>>(a);
     } else if (use_arcs(a, n)) {
-        insolation_kernel<ARCS><<<grid_for(n, 4), 256, arcs, s>>>(a);
+        insolation_kernel<ARCS><<<grid_arcs(n), arc_threads(n), arcs, s>>>(a);
     } else {
         insolation_kernel<0><<<grid_for(n), 256, 0, s>>>(a);
     }
