@@ -783,7 +783,7 @@ __device__ __forceinline__ void insolation_body(const InsoArgs &a)
 }
 
 template <int HP, bool BREAKS = false>
-__global__ void __launch_bounds__(INSO_THREADS<BREAKS, HP>, BREAKS ? BREAK_BLOCKS : (HP == ARCS ? 1 : 4)) insolation_kernel(InsoArgs a)
+__global__ void __launch_bounds__(INSO_THREADS<BREAKS, HP>, BREAKS ? BREAK_BLOCKS : (HP == ARCS ? 1 : (HP == 12 ? 3 : 4))) insolation_kernel(InsoArgs a)
 {
     insolation_body<HP, BREAKS>(a);
 }
@@ -796,7 +796,7 @@ struct InsoTable {
 };
 
 template <int HP, bool BREAKS = false>
-__global__ void __launch_bounds__(INSO_THREADS<BREAKS, HP>, BREAKS ? BREAK_BLOCKS : (HP == ARCS ? 1 : 4))
+__global__ void __launch_bounds__(INSO_THREADS<BREAKS, HP>, BREAKS ? BREAK_BLOCKS : (HP == ARCS ? 1 : (HP == 12 ? 3 : 4)))
     insolation_args_kernel(InsoArgs a, const __grid_constant__ InsoTable table)
 {
     a.rot = table.t;
