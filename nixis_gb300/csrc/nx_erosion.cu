@@ -413,8 +413,9 @@ __device__ __forceinline__ double f32_scaled(float v, int K)
 // buffer 0, like the iteration-at-a-time path.
 
 // `any`: the first pass starts from the raw sums, so that there is no buffer
-// for it to start in and any number of passes ends in buffer 0.  Without the
-// pass made for the parity, and with equal lengths (below): 12 iterations on
+// for it to start in, or from the buffer that the number of passes asks for
+// (nx_erosion_run).  Without the pass made for the parity, and with equal
+// lengths (below): 12 iterations on
 // 40,000,002 vertices 6.60 -> 6.15 ms, 13 on 6,400,002 1.31 -> 1.19, 60 5.62
 // -> 5.57.
 __host__ __device__ __forceinline__ int tb_npass(int iters, int R, bool any = false)
@@ -472,6 +473,7 @@ struct TbArgs {
     float4 *st0;
     float4 *st1;
     bool wide = false;     // both 32-byte aligned (set by launch_tb)
+    bool any = false;      // passes of any number (tb_npass)
     nx_erosion_ctl *ctl;
     // Optional fusion of the rescale: a planet's first pass reads the raw
     // fBm pair sums (float2 per row) and rescales them to its starting
@@ -579,7 +581,7 @@ __global__ void __launch_bounds__(THREADS, MINB > 0 ? MINB : (PF ? 768 : 1024) /
     const int2 bm = a.blk_map[blockIdx.x];
     const nx_erosion_planet P = a.planets[bm.x];
     const int R = a.R;
-    const int np = tb_npass(P.iters, R, a.raw != nullptr);
+    const int np = tb_npass(P.iters, R, a.any);
     const int q = a.pass - P.t_start;            // the planet's own pass
     if (q < 0 || q >= np) return;
     const int len = tb_len(P.iters, np, q);
@@ -1289,7 +1291,7 @@ static int plan_batch(const nx_erosion_planet *planets_host, int np, bool allow_
 // rescale constants for the planets' first passes).
 static int run_batch(const nx_erosion_planet *planets_dev, const nx_erosion_planet *planets_host, int np,
                      float *st_dev, float *st_tmp, double *mass_dev, uint16_t *flow_dev, void *workspace,
-                     size_t ws_bytes, cudaStream_t s, bool allow_tb, const TbArgs *fuse = nullptr)
+                     size_t ws_bytes, cudaStream_t s, bool allow_tb, const TbArgs *fuse = nullptr, bool any = false)
 {
     if (np <= 0) return NX_OK;
     if (!planets_dev || !planets_host || !st_dev || !st_tmp || !workspace)
@@ -1300,12 +1302,12 @@ static int run_batch(const nx_erosion_planet *planets_dev, const nx_erosion_plan
     const bool tb = pl.tb;
     const int R = pl.R, maxnl = pl.maxnl, maxc = pl.maxc, max_it = pl.max_it;
     const int64_t nblk = pl.nblk, ntiles_all = pl.ntiles_all;
-    if (fuse && !tb) return nx::fail(NX_EINVAL, "erosion: fused steps need the blocked path");
+    if ((fuse || any) && !tb) return nx::fail(NX_EINVAL, "erosion: the run needs the blocked path");
     if (tb) {
         if (ws_bytes < nx_erosion_workspace_size((ntiles_all > nblk ? ntiles_all : nblk) * BLOCK, np))
             return nx::fail(NX_EINVAL, "erosion: workspace too small");
         Workspace w = carve(workspace, np, ntiles_all > nblk ? ntiles_all : nblk);
-        const bool any = fuse != nullptr;
+        any = any || fuse;
         erosion_tb_map_kernel<<<np, 256, 0, s>>>(planets_dev, np, R, any, w.blk_map);
         NX_CHECK_LAUNCH("erosion_tb_map_kernel");
         nx::note_launch(1);
@@ -1323,6 +1325,7 @@ static int run_batch(const nx_erosion_planet *planets_dev, const nx_erosion_plan
         ta.st0 = (float4 *)st_dev;
         ta.st1 = (float4 *)st_tmp;
         ta.ctl = w.ctl;
+        ta.any = any;
         if (fuse) {
             ta.raw = fuse->raw;
             ta.minmax = fuse->minmax;
@@ -1563,6 +1566,13 @@ NX_EXPORT int nx_erosion_batch(const nx_erosion_planet *planets_dev, const nx_er
 {
     return run_batch(planets_dev, planets_host, nplanets, st_dev, st_tmp_dev, mass_dev, nullptr, workspace, ws_bytes,
                      (cudaStream_t)stream, true);
+}
+
+NX_EXPORT int nx_erosion_run(const nx_erosion_planet *planets_dev, const nx_erosion_planet *planets_host, int nplanets,
+                             float *st_dev, float *st_tmp_dev, void *workspace, size_t ws_bytes, void *stream)
+{
+    return run_batch(planets_dev, planets_host, nplanets, st_dev, st_tmp_dev, nullptr, nullptr, workspace, ws_bytes,
+                     (cudaStream_t)stream, true, nullptr, true);
 }
 
 NX_EXPORT int nx_erosion_ctl_init(void *workspace, size_t ws_bytes, int nplanets, void *stream)

@@ -14,7 +14,7 @@ import torch
 from . import _dev
 from . import autotune as _autotune
 from . import mesh as _mesh
-from ._lib import ErosionPlanet, call, lib
+from ._lib import ErosionPlanet, NxError, call, lib
 
 RAIN = 0.3 / 320            # erosion.py:182
 EVAPORATION = 0.1 / 320     # erosion.py:205
@@ -127,11 +127,16 @@ class ErosionRun:
             return False
         ws[:32].copy_(self.ws[:32])
         self.planet.copy_(torch.frombuffer(bytearray(bytes(d)), dtype=torch.uint8))
-        # the state enters in buffer iters & 1 and ends in buffer 0
-        st = (self.st, self.st_tmp) if iters % 2 == 0 else (self.st_tmp, self.st)
+        # the state enters in the buffer that the number of passes asks for and ends in buffer 0
+        st = (self.st, self.st_tmp) if -(-iters // tb.rings) % 2 == 0 else (self.st_tmp, self.st)
         _autotune.apply(tb)
-        call("nx_erosion_batch", _dev.ptr(self.planet), ctypes.byref(d), 1, _dev.ptr(st[0]), _dev.ptr(st[1]), None,
-             _dev.ptr(ws), ws.numel(), _dev.stream_handle(self.stream))
+        try:
+            call("nx_erosion_run", _dev.ptr(self.planet), ctypes.byref(d), 1, _dev.ptr(st[0]), _dev.ptr(st[1]),
+                 _dev.ptr(ws), ws.numel(), _dev.stream_handle(self.stream))
+        except NxError as e:
+            if e.code != 1:                      # NX_EINVAL: refused before any launch, the tiles do not fit
+                raise
+            return False
         self.st, self.st_tmp = st
         self.ws = ws
         self.iters_done += iters
