@@ -1,6 +1,7 @@
 """Device-buffer plumbing: numpy arrays are copied to CUDA tensors and back;
 CUDA tensors are used in place (zero copy)."""
 import ctypes
+import mmap
 
 import numpy as np
 import torch
@@ -35,6 +36,16 @@ def is_host(a):
     return isinstance(a, np.ndarray)
 
 
+def _in_memory(a):
+    """Whether a numpy array's bytes are ordinary memory (not a mapped file,
+    which the GPU is not sent to)."""
+    while isinstance(a, np.ndarray):
+        if isinstance(a, np.memmap):
+            return False
+        a = a.base
+    return not isinstance(a, mmap.mmap)
+
+
 def upload(arr, tdt):
     """A CUDA tensor with the bytes of a contiguous numpy array, which the
     caller may change as soon as this returns.
@@ -43,14 +54,15 @@ def upload(arr, tdt):
     straight out of the array: the GPU reads pageable memory here at
     110-180 GB/s, and staging through pinned memory copies it once more on one
     core (24 MB: 147 us against 195, 80 MB: 466 against 627).  Only under
-    capture, where such a copy cannot be waited for, is it staged."""
+    capture, where such a copy cannot be waited for, and for a mapped file is it
+    staged."""
     if arr.nbytes <= UPLOAD_MAX:
         t = torch.empty(arr.shape, dtype=tdt, device="cuda")
         if arr.nbytes:
             call("nx_upload", ptr(t), ctypes.c_void_p(arr.ctypes.data), arr.nbytes, stream_handle())
         return t
     t = torch.from_numpy(arr)
-    if torch.cuda.is_current_stream_capturing():
+    if torch.cuda.is_current_stream_capturing() or not _in_memory(arr):
         return t.pin_memory().to("cuda", non_blocking=True)
     return t.to("cuda")
 
@@ -67,7 +79,8 @@ def to_host(dst, src):
     into a contiguous array (80 MB: 430 us; through a fresh array, whose pages
     have to be made first, 2,870)."""
     t = torch.empty(0, dtype=src.dtype).numpy().dtype
-    if dst.dtype == t and dst.flags.c_contiguous and dst.flags.writeable and tuple(dst.shape) == tuple(src.shape):
+    if (dst.dtype == t and dst.flags.c_contiguous and dst.flags.writeable and tuple(dst.shape) == tuple(src.shape)
+            and _in_memory(dst)):
         torch.from_numpy(dst).copy_(src)
     else:
         dst[...] = src.cpu().numpy()

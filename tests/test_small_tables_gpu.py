@@ -76,3 +76,18 @@ def test_schedules_by_arguments_and_by_table(n_rot, n_tilt):
     out = want.clone()
     climate.insolation_sum(m.xyz, 1.0, rot, tilt, out=out, accumulate=True)
     assert torch.equal(out, want + want)
+
+
+@gpu
+def test_mapped_files_go_through_staging(tmp_path):
+    """The same bytes from and into a memory-mapped file, also behind a plain view of it."""
+    a = np.random.default_rng(1).random(9000)
+    f = np.memmap(tmp_path / "x", np.float64, "w+", shape=a.shape)
+    f[:] = a
+    assert not _dev._in_memory(f) and not _dev._in_memory(np.asarray(f)[10:]) and _dev._in_memory(a[10:])
+    for src in (f, np.asarray(f)):
+        t = _dev.to_device(src, np.float64)
+        assert np.array_equal(t.cpu().numpy(), a)
+    out = np.memmap(tmp_path / "y", np.float64, "w+", shape=a.shape)
+    _dev.to_host(out, t)
+    assert np.array_equal(out, a)
