@@ -330,10 +330,11 @@ int nx_erosion_batch(const nx_erosion_planet *planets_dev, const nx_erosion_plan
                      void *stream);
 
 /* nx_erosion_batch by blocked passes only (NX_EINVAL where a planet has no
- * tiling that fits), ceil(iters / rings) of them: a planet's state starts in
- * st_dev, or in st_tmp_dev where that number is odd, and ends in st_dev. */
+ * tiling that fits, or `rings` is not what nx_erosion_tb_config set last),
+ * ceil(iters / rings) of them: a planet's state starts in st_dev, or in
+ * st_tmp_dev where that number is odd, and ends in st_dev. */
 int nx_erosion_run(const nx_erosion_planet *planets_dev, const nx_erosion_planet *planets_host, int nplanets,
-                   float *st_dev, float *st_tmp_dev, void *workspace, size_t ws_bytes, void *stream);
+                   int rings, float *st_dev, float *st_tmp_dev, void *workspace, size_t ws_bytes, void *stream);
 
 /* Serving: one launch that advances every listed planet (any order) by one
  * iteration, planet p at its own iteration t - t_start (planets outside

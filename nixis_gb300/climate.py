@@ -68,6 +68,7 @@ def _sum(verts, radius, rotations, tilts, out, accumulate, stream, scale=None):
         raise ValueError("out must be a float32 CUDA tensor of shape (N,)")
     if stream is not None:
         tdev.record_stream(stream)
+        xyz.record_stream(stream)
     if short:
         vp = ctypes.c_void_p
         call("nx_insolation_positions", _dev.ptr(xyz), n, float(radius), vp(rot.ctypes.data), len(rot),

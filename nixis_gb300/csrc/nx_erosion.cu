@@ -1291,7 +1291,7 @@ static int plan_batch(const nx_erosion_planet *planets_host, int np, bool allow_
 // rescale constants for the planets' first passes).
 static int run_batch(const nx_erosion_planet *planets_dev, const nx_erosion_planet *planets_host, int np,
                      float *st_dev, float *st_tmp, double *mass_dev, uint16_t *flow_dev, void *workspace,
-                     size_t ws_bytes, cudaStream_t s, bool allow_tb, const TbArgs *fuse = nullptr, bool any = false)
+                     size_t ws_bytes, cudaStream_t s, bool allow_tb, const TbArgs *fuse = nullptr, int rings = 0)
 {
     if (np <= 0) return NX_OK;
     if (!planets_dev || !planets_host || !st_dev || !st_tmp || !workspace)
@@ -1302,12 +1302,13 @@ static int run_batch(const nx_erosion_planet *planets_dev, const nx_erosion_plan
     const bool tb = pl.tb;
     const int R = pl.R, maxnl = pl.maxnl, maxc = pl.maxc, max_it = pl.max_it;
     const int64_t nblk = pl.nblk, ntiles_all = pl.ntiles_all;
-    if ((fuse || any) && !tb) return nx::fail(NX_EINVAL, "erosion: the run needs the blocked path");
+    if ((fuse || rings) && !tb) return nx::fail(NX_EINVAL, "erosion: the run needs the blocked path");
+    if (rings && R != rings) return nx::fail(NX_EINVAL, "erosion: passes are set to %d rings, not %d", R, rings);
     if (tb) {
         if (ws_bytes < nx_erosion_workspace_size((ntiles_all > nblk ? ntiles_all : nblk) * BLOCK, np))
             return nx::fail(NX_EINVAL, "erosion: workspace too small");
         Workspace w = carve(workspace, np, ntiles_all > nblk ? ntiles_all : nblk);
-        any = any || fuse;
+        const bool any = fuse || rings;
         erosion_tb_map_kernel<<<np, 256, 0, s>>>(planets_dev, np, R, any, w.blk_map);
         NX_CHECK_LAUNCH("erosion_tb_map_kernel");
         nx::note_launch(1);
@@ -1569,10 +1570,11 @@ NX_EXPORT int nx_erosion_batch(const nx_erosion_planet *planets_dev, const nx_er
 }
 
 NX_EXPORT int nx_erosion_run(const nx_erosion_planet *planets_dev, const nx_erosion_planet *planets_host, int nplanets,
-                             float *st_dev, float *st_tmp_dev, void *workspace, size_t ws_bytes, void *stream)
+                             int rings, float *st_dev, float *st_tmp_dev, void *workspace, size_t ws_bytes, void *stream)
 {
+    if (rings < 1) return nx::fail(NX_EINVAL, "nx_erosion_run: bad rings");
     return run_batch(planets_dev, planets_host, nplanets, st_dev, st_tmp_dev, nullptr, nullptr, workspace, ws_bytes,
-                     (cudaStream_t)stream, true, nullptr, true);
+                     (cudaStream_t)stream, true, nullptr, rings);
 }
 
 NX_EXPORT int nx_erosion_ctl_init(void *workspace, size_t ws_bytes, int nplanets, void *stream)

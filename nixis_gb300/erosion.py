@@ -131,14 +131,16 @@ class ErosionRun:
         st = (self.st, self.st_tmp) if -(-iters // tb.rings) % 2 == 0 else (self.st_tmp, self.st)
         _autotune.apply(tb)
         try:
-            call("nx_erosion_run", _dev.ptr(self.planet), ctypes.byref(d), 1, _dev.ptr(st[0]), _dev.ptr(st[1]),
+            call("nx_erosion_run", _dev.ptr(self.planet), ctypes.byref(d), 1, tb.rings, _dev.ptr(st[0]), _dev.ptr(st[1]),
                  _dev.ptr(ws), ws.numel(), _dev.stream_handle(self.stream))
         except NxError as e:
-            if e.code != 1:                      # NX_EINVAL: refused before any launch, the tiles do not fit
+            # NX_EINVAL: refused before any launch (the tiles do not fit, or
+            # another setting was applied meanwhile)
+            if e.code != 1:
                 raise
             return False
         self.st, self.st_tmp = st
-        self.ws = ws
+        self.ws, self.tiling = ws, tl            # (in use until the run's stream has passed them)
         self.iters_done += iters
         return True
 

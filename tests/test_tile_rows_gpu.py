@@ -50,3 +50,24 @@ def test_rows_of_any_order(side, rings, threads, variant):
     cfg = autotune.TbConfig(side, rings, threads, variant)
     for a, b in zip(run(m, h, 13, None, 0), run(m, h, 13, cfg, 0)):
         assert torch.equal(a, b)
+
+
+def test_passes_of_another_setting_are_refused():
+    """The buffer a state starts in follows from the rings, so a run for other rings than the setting's does nothing."""
+    import ctypes
+    import torch
+    from nixis_gb300 import _dev, _lib, autotune, erosion, mesh
+    m = mesh.PlanetMesh(40)
+    tb = autotune.current()
+    tl = m.tiling(tb.tile_side, tb.rings)
+    r = erosion.ErosionRun(m.xyz, m.nbr, m.edge)
+    r.load(torch.rand(m.n, dtype=torch.float64, device="cuda"))
+    was = r.st.clone()
+    autotune.apply(tb)
+    d = _lib.ErosionPlanet(0, m.n, m.nbr.data_ptr(), m.edge.data_ptr(), 7, 0.0, 0, 0, tl.dev.data_ptr(), tl.ntiles, tl.maxnl, tl.maxc)
+    ws = torch.zeros(int(_lib.lib().nx_erosion_workspace_size(max(m.n, 256 * tl.ntiles), 1)), dtype=torch.uint8, device="cuda")
+    for rings in (tb.rings + 1, 0):
+        with pytest.raises(_lib.NxError):
+            _lib.call("nx_erosion_run", _dev.ptr(r.planet), ctypes.byref(d), 1, rings, _dev.ptr(r.st), _dev.ptr(r.st_tmp), _dev.ptr(ws),
+                      ws.numel(), _dev.stream_handle())
+    assert torch.equal(r.st, was)
