@@ -5,6 +5,7 @@ State on the GPU is binary32 pairs (hi + lo) with a per-planet power-of-two
 scale (exact, see csrc/nx_erosion.cu); results are returned in the reference's float64
 arrays, updated in place like the reference.
 """
+import contextlib
 import ctypes
 import math
 
@@ -52,28 +53,34 @@ class ErosionRun:
         self.n = self.xyz.shape[0]
         self.nbr = _dev.to_device(neighbors, np.int32, (self.n, 6), "neighbors")
         n = self.n
-        # None: not the icosphere's own table, edges too long, or not worth finding out
-        self.k = (self._icosphere_divisions()
-                  if edge is None and iters >= BLOCKED_ITERS and iters * n >= BLOCKED_WORK else None)
-        if edge is None:
-            if self.k is None:
-                edge, err = _mesh.edge_lengths(self.xyz, self.nbr, stream=stream)
-            else:
-                edge = torch.empty((n, 6, 2), dtype=torch.float32, device="cuda")
-                err = torch.zeros(2, dtype=torch.int32, device="cuda")
-                call("nx_icosphere_edges", self.k, _dev.ptr(self.xyz), _dev.ptr(self.nbr), _dev.ptr(edge), _dev.ptr(err),
-                     _dev.stream_handle(stream))
-            err = err.cpu()
-            if err.numel() == 2 and not float(err.view(torch.float32)[1]) <= BLOCKED_EDGE:
-                self.k = None
-            if int(err[0]):
-                raise IndexError("neighbors holds an id outside [-1, N)")
+        with self._on_stream():
+            # None: not the icosphere's own table, edges too long, or not worth finding out
+            self.k = (self._icosphere_divisions()
+                      if edge is None and iters >= BLOCKED_ITERS and iters * n >= BLOCKED_WORK else None)
+            if edge is None:
+                if self.k is None:
+                    edge, err = _mesh.edge_lengths(self.xyz, self.nbr, stream=stream)
+                else:
+                    edge = torch.empty((n, 6, 2), dtype=torch.float32, device="cuda")
+                    err = torch.zeros(2, dtype=torch.int32, device="cuda")
+                    call("nx_icosphere_edges", self.k, _dev.ptr(self.xyz), _dev.ptr(self.nbr), _dev.ptr(edge), _dev.ptr(err),
+                         _dev.stream_handle(stream))
+                err = err.cpu()
+                if err.numel() == 2 and not float(err.view(torch.float32)[1]) <= BLOCKED_EDGE:
+                    self.k = None
+                if int(err[0]):
+                    raise IndexError("neighbors holds an id outside [-1, N)")
         self.edge = edge
         self.st = torch.empty((n, 8), dtype=torch.float32, device="cuda")    # (h, w, s as hi/lo pairs, 0, 0)
         self.st_tmp = torch.empty_like(self.st)
         self.ws = torch.zeros(int(lib().nx_erosion_workspace_size(n, 1)), dtype=torch.uint8, device="cuda")
         self.planet = torch.zeros(ctypes.sizeof(ErosionPlanet), dtype=torch.uint8, device="cuda")  # one descriptor
         self.iters_done = 0
+
+    def _on_stream(self):
+        """The run's stream as the current one, so that what the host reads
+        back is ordered behind the run's kernels."""
+        return torch.cuda.stream(self.stream) if self.stream is not None else contextlib.nullcontext()
 
     def _icosphere_divisions(self):
         """k if the neighbour table's face-interior rows are those of this
@@ -117,30 +124,31 @@ class ErosionRun:
         tb = _autotune.current()
         if self.k is None or iters < 1 or tb.variant not in (0, 1, 4, 5):
             return False
-        try:
-            tl = _mesh.MeshTiling(self, tb.tile_side, tb.rings, self.stream)
-            d = ErosionPlanet(0, self.n, self.nbr.data_ptr(), self.edge.data_ptr(), iters, float(rain), 0, 0,
-                              tl.dev.data_ptr(), tl.ntiles, tl.maxnl, tl.maxc)
-            ws = torch.empty(int(lib().nx_erosion_workspace_size(max(self.n, 256 * tl.ntiles), 1)), dtype=torch.uint8,
-                             device="cuda")
-        except RuntimeError:                     # too large a tile, or out of memory
-            return False
-        ws[:32].copy_(self.ws[:32])
-        self.planet.copy_(torch.frombuffer(bytearray(bytes(d)), dtype=torch.uint8))
-        # the state enters in the buffer that the number of passes asks for and ends in buffer 0
-        st = (self.st, self.st_tmp) if -(-iters // tb.rings) % 2 == 0 else (self.st_tmp, self.st)
-        _autotune.apply(tb)
-        try:
-            call("nx_erosion_run", _dev.ptr(self.planet), ctypes.byref(d), 1, tb.rings, _dev.ptr(st[0]), _dev.ptr(st[1]),
-                 _dev.ptr(ws), ws.numel(), _dev.stream_handle(self.stream))
-        except NxError as e:
-            # NX_EINVAL: refused before any launch (the tiles do not fit, or
-            # another setting was applied meanwhile)
-            if e.code != 1:
-                raise
-            return False
-        self.st, self.st_tmp = st
-        self.ws, self.tiling = ws, tl            # (in use until the run's stream has passed them)
+        with self._on_stream():
+            try:
+                tl = _mesh.MeshTiling(self, tb.tile_side, tb.rings, self.stream)
+                d = ErosionPlanet(0, self.n, self.nbr.data_ptr(), self.edge.data_ptr(), iters, float(rain), 0, 0,
+                                  tl.dev.data_ptr(), tl.ntiles, tl.maxnl, tl.maxc)
+                ws = torch.empty(int(lib().nx_erosion_workspace_size(max(self.n, 256 * tl.ntiles), 1)), dtype=torch.uint8,
+                                 device="cuda")
+            except RuntimeError:                     # too large a tile, or out of memory
+                return False
+            ws[:32].copy_(self.ws[:32])
+            self.planet.copy_(torch.frombuffer(bytearray(bytes(d)), dtype=torch.uint8))
+            # the state enters in the buffer that the number of passes asks for and ends in buffer 0
+            st = (self.st, self.st_tmp) if -(-iters // tb.rings) % 2 == 0 else (self.st_tmp, self.st)
+            _autotune.apply(tb)
+            try:
+                call("nx_erosion_run", _dev.ptr(self.planet), ctypes.byref(d), 1, tb.rings, _dev.ptr(st[0]), _dev.ptr(st[1]),
+                     _dev.ptr(ws), ws.numel(), _dev.stream_handle(self.stream))
+            except NxError as e:
+                # NX_EINVAL: refused before any launch (the tiles do not fit, or
+                # another setting was applied meanwhile)
+                if e.code != 1:
+                    raise
+                return False
+            self.st, self.st_tmp = st
+            self.ws, self.tiling = ws, tl            # (in use until the run's stream has passed them)
         self.iters_done += iters
         return True
 
@@ -159,7 +167,8 @@ class ErosionRun:
     def error(self):
         """The run's flag: 1 an id out of range, 2 or 3 a tiling that does
         not suit the passes (another setting was applied meanwhile)."""
-        return int(self.ws[:32].view(torch.int32)[6].item())
+        with self._on_stream():
+            return int(self.ws[:32].view(torch.int32)[6].item())
 
 
 def erosion_iteration3(verts, neighbors, r_buff, wat, sed):

@@ -71,3 +71,37 @@ def test_passes_of_another_setting_are_refused():
             _lib.call("nx_erosion_run", _dev.ptr(r.planet), ctypes.byref(d), 1, rings, _dev.ptr(r.st), _dev.ptr(r.st_tmp), _dev.ptr(ws),
                       ws.numel(), _dev.stream_handle())
     assert torch.equal(r.st, was)
+
+
+@pytest.mark.parametrize("turned", [False, True])
+def test_a_run_on_its_own_stream_reads_its_own_checks(turned, monkeypatch):
+    """The table's comparison and the edges' flag are read behind the run's kernels, which a busy stream delays."""
+    import torch
+    from nixis_gb300 import erosion, mesh
+    monkeypatch.setattr(erosion, "BLOCKED_WORK", 1)
+    m = mesh.PlanetMesh(50)
+    nbr = m.nbr.clone()
+    if turned:
+        nbr[-900] = nbr[-900].roll(1)
+    h = torch.rand(m.n, dtype=torch.float64, generator=torch.Generator().manual_seed(1)).cuda()
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    out = []
+    for stream in (None, s):
+        if stream is not None:
+            with torch.cuda.stream(stream):
+                torch.cuda._sleep(20_000_000)
+        r = erosion.ErosionRun(m.xyz, nbr, stream=stream, iters=9)
+        assert (r.k is None) == turned
+        torch.cuda.synchronize()
+        r.load(h)
+        torch.cuda.synchronize()
+        assert r.blocked(9, 0.01) != turned
+        if turned:
+            r.steps(9, rain=0.01)
+        assert r.error() == 0
+        torch.cuda.synchronize()
+        out.append(torch.empty_like(h))
+        r.store(out[-1])
+        torch.cuda.synchronize()
+    assert torch.equal(out[0], out[1])
