@@ -449,9 +449,11 @@ __global__ void __launch_bounds__(256) ico_neighbours_kernel(int k, int64_t nv, 
 // slot (s + 3) mod 6.  Distances to vertices of edges and corners are
 // computed by both sides.  So 6 binary64 operations an edge (the squares come
 // from integer products), each edge once, and no search for the reverse slot.
-// Measured (GB300, 4,900,002 vertices): 289 us, 359 us with the squares in
-// binary64 (the binary64 operations alone take 151 and 227 us), ~880 us for
-// the general pair of passes before.
+// Measured (GB300, 4,900,002 vertices): ~880 us for the general pair of
+// passes, 359 us here, 289 us with the squares from integers, 220 us with the
+// three distances side by side and slots 2 and 3 in one store (WIDE: rows
+// 16-byte aligned); the binary64 pipe is then busy for 82 % of it.
+template <bool WIDE>
 __global__ void __launch_bounds__(256) ico_edges_kernel(int k, int64_t nv, const double *__restrict__ xyz,
                                                         const int32_t *__restrict__ nbr, float2 *__restrict__ el,
                                                         int *__restrict__ info)
@@ -474,13 +476,19 @@ __global__ void __launch_bounds__(256) ico_edges_kernel(int k, int64_t nv, const
         interior_fij(v - inner, k, f, i, j);
         int32_t row[6];
         const unsigned in = interior_row(v, f, i, j, k, row);
-#pragma unroll
-        for (int s = 2; s < 5; ++s) {
-            const float2 d = edge_pair(edge_len(xyz, v, row[s]));
-            longest = fmaxf(longest, d.x);
-            el[6 * v + s] = d;
-            if (in & (1u << s)) el[6 * (int64_t)row[s] + (s + 3) % 6] = d;
+        const float2 d2 = edge_pair(edge_len(xyz, v, row[2])), d3 = edge_pair(edge_len(xyz, v, row[3])),
+                     d4 = edge_pair(edge_len(xyz, v, row[4]));
+        longest = fmaxf(longest, fmaxf(d2.x, fmaxf(d3.x, d4.x)));
+        if (WIDE) {
+            *reinterpret_cast<float4 *>(el + 6 * v + 2) = make_float4(d2.x, d2.y, d3.x, d3.y);
+        } else {
+            el[6 * v + 2] = d2;
+            el[6 * v + 3] = d3;
         }
+        el[6 * v + 4] = d4;
+        if (in & 4u) el[6 * (int64_t)row[2] + 5] = d2;
+        if (in & 8u) el[6 * (int64_t)row[3]] = d3;
+        if (in & 16u) el[6 * (int64_t)row[4] + 1] = d4;
         if ((in & 35u) != 35u) {
             if (!(in & 1u)) el[6 * v] = edge_pair(edge_len(xyz, v, row[0]));
             if (!(in & 2u)) el[6 * v + 1] = edge_pair(edge_len(xyz, v, row[1]));
@@ -651,7 +659,10 @@ NX_EXPORT int nx_icosphere_edges(int k, const double *xyz_dev, const int32_t *nb
     if (rc) return rc;
     if (!xyz_dev || !edge_dev) return nx::fail(NX_EINVAL, "nx_icosphere_edges: null pointer");
     const int64_t nv = (int64_t)10 * k * k + 2;
-    ico_edges_kernel<<<grid1d(nv), 256, 0, (cudaStream_t)stream>>>(k, nv, xyz_dev, nbr_dev, (float2 *)edge_dev, info_dev);
+    if (((uintptr_t)edge_dev & 15u) == 0)
+        ico_edges_kernel<true><<<grid1d(nv), 256, 0, (cudaStream_t)stream>>>(k, nv, xyz_dev, nbr_dev, (float2 *)edge_dev, info_dev);
+    else
+        ico_edges_kernel<false><<<grid1d(nv), 256, 0, (cudaStream_t)stream>>>(k, nv, xyz_dev, nbr_dev, (float2 *)edge_dev, info_dev);
     NX_CHECK_LAUNCH("ico_edges_kernel");
     nx::note_launch(1);
     return NX_OK;

@@ -54,3 +54,17 @@ def test_scaled_and_shuffled_vertices_have_exact_lengths():
         edge, _ = mesh.edge_lengths(xyz, nbr)
         hi = d.float()
         assert torch.equal(edge[..., 0], hi) and torch.equal(edge[..., 1], (d - hi.double()).float())
+
+
+@pytest.mark.parametrize("k", [2, 3, 17, 64])
+def test_edge_rows_of_any_alignment(k):
+    """Rows 8 bytes off a 16-byte boundary: the same pairs, nothing beside them."""
+    import torch
+    from nixis_gb300 import _dev, mesh
+    from nixis_gb300._lib import call
+    m = mesh.PlanetMesh(k)
+    buf = torch.full((m.edge.numel() + 4,), 7.0, dtype=torch.float32, device="cuda")
+    call("nx_icosphere_edges", k, _dev.ptr(m.xyz), _dev.ptr(m.nbr), _dev.ptr(buf[2:]), None, _dev.stream_handle())
+    assert torch.equal(buf[2:-2].view(m.edge.shape), m.edge)
+    assert torch.equal(m.edge, mesh.edge_lengths(m.xyz, m.nbr)[0])
+    assert (buf[:2] == 7.0).all() and (buf[-2:] == 7.0).all()
