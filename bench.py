@@ -407,7 +407,7 @@ def bench_ours(args):
                              "frac": fbm_tf / fp32_fma, "ms": fbm_ms,
                              "model": f"{FBM_ALG_FLOP} FLOP per vertex-octave (the reference's binary64 operations) x "
                                       f"{vo} vertex-octaves; peak = 152 SMs x 128 lanes x 2 x {sm_mhz:.0f} MHz (derived)",
-                             "note": "evaluated in float-float pairs (~2.4x the binary32 kernel's instructions) to stay "
+                             "note": "evaluated in float-float pairs (~2x the binary32 kernel's instructions) to stay "
                                      "within 1e-13 of binary64, which the erosion's flow choices need"}}
     issue = os.path.join(ROOT, "profiles", "fbm_issue.json")
     if os.path.exists(issue):
