@@ -775,8 +775,8 @@ __device__ __forceinline__ void insolation_body(const InsoArgs &a)
         if (j < a.n) { X = a.xyz[3 * j]; Y = a.xyz[3 * j + 1]; Z = a.xyz[3 * j + 2]; }
         const float tot = inso_vertex<HP, BREAKS>(a, cx, cy, cz, a.r, a.r2h, a.r2l, a.zmin, a.inv_r, staged ? s_tilt : nullptr,
                                           bk, arc);
-        // the scale here instead of in a pass of its own over the sums (10 M
-        // vertices: 11 us of 137)
+        // the scale here instead of in a pass of its own over the sums (11 us
+        // for 10 M vertices)
         const float v = __fmul_rn(tot, a.scale);
         a.out[i] = a.accumulate ? a.out[i] + v : v;
     }

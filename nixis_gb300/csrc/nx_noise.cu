@@ -1320,8 +1320,9 @@ __device__ __forceinline__ int chunk_planet(const nx_fbm_planet *P, int np, int 
 }
 
 // Threads of a pair block: one block of 512 per SM (128 registers a thread).
-// Measured (GB300, 12 octaves of 10,000,002 vertices): 3.13 ms, against 3.38
-// ms for two blocks of 256 (each with a table of its own), 3.63 ms for three
+// Measured (GB300, 12 octaves of 10,000,002 vertices, before the shorter
+// chains above, which take 2.75 ms now): 3.13 ms, against 3.38 ms for two
+// blocks of 256 (each with a table of its own), 3.63 ms for three
 // of 192, 3.74 ms for one of 640 and 3.90 ms for two of 320 (96 registers:
 // more warps, but longer dependent stretches).
 constexpr int PAIR_THREADS = 512;
