@@ -55,9 +55,10 @@ def _sum(verts, radius, rotations, tilts, out, accumulate, stream, scale=None):
     n = xyz.shape[0]
     rot = np.ascontiguousarray(rotations, np.float64)
     tilt = np.ascontiguousarray(tilts, np.float64)
-    short = len(rot) + len(tilt) <= MAX_POSITIONS
+    n_tilt = len(tilts)
+    short = len(rot) + n_tilt <= MAX_POSITIONS
     if short:
-        tdev = torch.empty(2 * (len(rot) + len(tilt)), dtype=torch.float32, device="cuda")
+        tdev = torch.empty(2 * (len(rot) + n_tilt), dtype=torch.float32, device="cuda")
     else:
         tab, nre, pairs = _plan(rot, tilt)
         tdev = _dev.to_device(tab, np.float32, name="table")
@@ -72,10 +73,10 @@ def _sum(verts, radius, rotations, tilts, out, accumulate, stream, scale=None):
     if short:
         vp = ctypes.c_void_p
         call("nx_insolation_positions", _dev.ptr(xyz), n, float(radius), vp(rot.ctypes.data), len(rot),
-             vp(tilt.ctypes.data), len(tilt), 1.0 if scale is None else float(scale), _dev.ptr(tdev), _dev.ptr(out),
+             vp(tilt.ctypes.data), n_tilt, 1.0 if scale is None else float(scale), _dev.ptr(tdev), _dev.ptr(out),
              1 if accumulate else 0, _dev.stream_handle(stream))
     else:
-        call("nx_insolation", _dev.ptr(xyz), n, float(radius), _dev.ptr(tdev), nre, pairs, len(tilt), _dev.ptr(out),
+        call("nx_insolation", _dev.ptr(xyz), n, float(radius), _dev.ptr(tdev), nre, pairs, n_tilt, _dev.ptr(out),
              1 if accumulate else 0, _dev.stream_handle(stream))
         if scale is not None:
             out.mul_(scale)
