@@ -455,11 +455,15 @@ __device__ __forceinline__ Arcs stage_arcs(const InsoArgs &a, void *smem)
         const float2 q = a.rot[i < a.n_rot ? i : i - a.n_rot];
         return i < a.n_rot ? q : make_float2(-q.x, -q.y);
     };
+    // (an angle that is no number has no place in the order: none of the
+    // tables, and the vertices go through the rotations one by one)
+    bool number = true;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const float2 q = rot(i);
         raw[i] = atan2f(q.y, q.x);
+        number = number && raw[i] == raw[i];
     }
-    __syncthreads();
+    if (!__syncthreads_and(number)) return A;
     bool ascending = true;
     for (int i = threadIdx.x; i + 1 < n; i += blockDim.x) ascending = ascending && raw[i] <= raw[i + 1];
     if (__syncthreads_and(ascending)) {
@@ -565,7 +569,7 @@ __device__ __forceinline__ float inso_vertex(const InsoArgs &a, double X, double
 {
     float x, y, z;
     const bool on_sphere = load_vertex(X, Y, Z, r, r2h, r2l, x, y, z);
-    if (HP == ARCS && on_sphere) return arc_sum(a, arc, x, y, z) * inv_r;
+    if (HP == ARCS && on_sphere && arc.n > 0) return arc_sum(a, arc, x, y, z) * inv_r;
     float tot = 0.0f, comp = 0.0f;          // Kahan over tilts
     const int nr = HP > 0 ? HP : a.n_rot;
     if (on_sphere && HP > 0 && (HP & 1) == 0 && (BREAKS || a.pairs)) {

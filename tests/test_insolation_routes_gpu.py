@@ -76,3 +76,17 @@ def test_bucket_tables_of_any_length(days):
         u = (x[:, None] * r.cos() - y[:, None] * r.sin()) * tau.cos() + (z * tau.sin())[:, None]
         want += u.clamp(min=0).sum(1)
     assert (got - want).abs().max() <= 2e-6 * want.max()
+
+
+@pytest.mark.parametrize("bad", [math.nan, math.inf])
+@pytest.mark.parametrize("where", [0, 77, 359])
+def test_a_rotation_that_is_no_number_lights_nothing(where, bad):
+    """It has no place among the sorted angles; the others' terms stay as they are rotation by rotation (120 at a time
+    is below the arcs' range).  2e-6 of the largest sum: two orders of summation in binary32."""
+    from nixis_gb300 import climate, mesh
+    m = mesh.PlanetMesh(17)
+    rot, tilts = [-180.0 + i for i in range(360)], [23.44, -7.5]
+    rot[where] = bad
+    got = climate.insolation_sum(m.xyz, 1.0, rot, tilts)
+    want = sum(climate.insolation_sum(m.xyz, 1.0, rot[q:q + 120], tilts) for q in (0, 120, 240))
+    assert (got - want).abs().max() <= 2e-6 * want.max()
