@@ -79,15 +79,26 @@ static_assert(sizeof(nx_fbm_planet) == 960, "fBm planet descriptor layout");
 constexpr int TABLE_WORDS = 256 * 32;
 constexpr int TABLE_BYTES = TABLE_WORDS * 4;
 
-// GRADIENTS_3D as binary32, per component and lane (entry 32 i + lane of
-// component c at s_gr[768 c + 32 i + lane]: no bank conflicts), in the order
-// of the component that is +-11: i = 8 axis + (0-7) (every gradient has one
-// +-11 and two +-4 components).  Three single loads a slot go straight into
-// the halves of the paired operands; one 16-byte load took moves to get there.
+// GRADIENTS_3D as binary32, a copy per lane (no bank conflicts).  Three
+// single loads a slot go straight into the halves of the paired operands; one
+// 16-byte load took moves to get there.  Two layouts of the same size:
+//  * binary32 kernels: the table's 72 numbers in its own order, number q of a
+//    lane at 32 q + lane, so that a gradient starts at any of them, as the
+//    reference's GRADIENTS_3D[index], [index + 1], [index + 2] do (init() makes
+//    multiples of 3 only, other tables need not);
+//  * AXIS, the pair kernels: component c of gradient i at 768 c + 32 i + lane,
+//    the gradients in the order of the component that is +-11, i = 8 axis +
+//    (0-7) (every gradient has one +-11 and two +-4 components); indices are
+//    rounded down to a multiple of 3.
 __shared__ float s_gr[3 * 768];
 
+template <bool AXIS>
 __device__ __forceinline__ void init_grad_table()
 {
+    if (!AXIS) {
+        for (int j = threadIdx.x; j < 72 * 32; j += blockDim.x) s_gr[j] = (float)c_grad3[j >> 5];
+        return;
+    }
     for (int j = threadIdx.x; j < 768; j += blockDim.x) {
         const int i = j >> 5, row = 3 * (i & 7) + (i >> 3);
         for (int c = 0; c < 3; ++c) s_gr[768 * c + j] = (float)c_grad3[3 * row + c];
@@ -96,21 +107,23 @@ __device__ __forceinline__ void init_grad_table()
 
 // The hash table (TABLE_WORDS), at the start of the block's dynamic memory.
 // A lane's word of an entry: perm in bits 7-14, and from bit 18 on the byte
-// offset of the entry's gradient in s_gr for this lane, 128 i + 4 lane (so
-// the gradient's axis is bits 26-27).
+// offset of the entry's gradient in s_gr for this lane, 128 i + 4 lane, i the
+// index itself or (AXIS) the gradient's place, whose axis is then bits 26-27.
 extern __shared__ __align__(16) uint32_t smem[];
 
 // A warp fills runs of 32 entries: each lane forms one entry's word (two
 // global reads a lane, all in flight together), then the 32 words go out one
 // by one to their 32 replicas, a conflict-free store each.
+template <bool AXIS>
 __device__ __forceinline__ void build_table(const int32_t *__restrict__ perm, const int32_t *__restrict__ pgi)
 {
     const uint32_t lane = threadIdx.x & 31;
     for (int k0 = (threadIdx.x >> 5) * 32; k0 < 256; k0 += blockDim.x) {
         const uint32_t p = (uint32_t)perm[k0 + lane] & 255u;
         int g = pgi[k0 + lane];
-        g = (g < 0 ? 0 : (g > 69 ? 69 : g)) / 3;
-        const uint32_t w = p << 7 | (uint32_t)(8 * (g % 3) + g / 3) << 23;
+        g = g < 0 ? 0 : (g > 69 ? 69 : g);
+        if (AXIS) g = 8 * (g / 3 % 3) + g / 9;
+        const uint32_t w = p << 7 | (uint32_t)g << 23;
 #pragma unroll 8
         for (int j = 0; j < 32; ++j) smem[32 * (k0 + j) + lane] = __shfl_sync(0xFFFFFFFFu, w, j) | lane << 18;
     }
@@ -126,9 +139,10 @@ __device__ __forceinline__ uint32_t lk(uint32_t lb, int a)
 }
 
 // Component c of the gradient of a table word.
+template <bool AXIS>
 __device__ __forceinline__ float grad_of(uint32_t w, int c)
 {
-    return *reinterpret_cast<const float *>(reinterpret_cast<const char *>(s_gr + 768 * c) + (w >> 16));
+    return *reinterpret_cast<const float *>(reinterpret_cast<const char *>(s_gr + (AXIS ? 768 : 32) * c) + (w >> 16));
 }
 
 // Split a binary64 into hi + lo binary32 with integer operations (no FP64
@@ -596,8 +610,8 @@ __device__ __forceinline__ float2 contrib2(uint32_t wa, uint32_t wb, float2 DX, 
     if (MASK) na = __fmul2_rn(na, ON);
     const float2 a2 = __fmul2_rn(na, na);
     const float2 a4 = __fmul2_rn(a2, a2);
-    const float2 gx = f2(grad_of(wa, 0), grad_of(wb, 0)), gy = f2(grad_of(wa, 1), grad_of(wb, 1)),
-                 gz = f2(grad_of(wa, 2), grad_of(wb, 2));
+    const float2 gx = f2(grad_of<false>(wa, 0), grad_of<false>(wb, 0)), gy = f2(grad_of<false>(wa, 1), grad_of<false>(wb, 1)),
+                 gz = f2(grad_of<false>(wa, 2), grad_of<false>(wb, 2));
     float2 dot = __fmul2_rn(gz, DZ);
     dot = __ffma2_rn(gy, DY, dot);
     dot = __ffma2_rn(gx, DX, dot);
@@ -705,7 +719,7 @@ __device__ __forceinline__ float noise_raw(float xh, float xl, float yh, float y
             int32_t *q = sl9 + 5 * k;
             q[0] = c.xsb + o[k][0]; q[1] = c.ysb + o[k][1]; q[2] = c.zsb + o[k][2];
             q[3] = 0;
-            for (int a = 0; a < 3; ++a) q[3] |= ((int)grad_of(w[k], a) + 16) << (8 * a);
+            for (int a = 0; a < 3; ++a) q[3] |= ((int)grad_of<false>(w[k], a) + 16) << (8 * a);
             q[4] = on[k] ? 1 : 0;
         }
     }
@@ -929,8 +943,8 @@ __device__ __forceinline__ void contrib2_pair(uint32_t wa, uint32_t wb, float X0
     float2 l4 = fma2(h2, h2, f2(-h4.x, -h4.y));
     l4 = fma2(fma2(two, h2, l2), l2, l4);
     // grad . d as a pair (dh, dl), times DSC (see below)
-    const float2 gx = f2(grad_of(wa, 0), grad_of(wb, 0)), gy = f2(grad_of(wa, 1), grad_of(wb, 1)),
-                 gz = f2(grad_of(wa, 2), grad_of(wb, 2));
+    const float2 gx = f2(grad_of<true>(wa, 0), grad_of<true>(wb, 0)), gy = f2(grad_of<true>(wa, 1), grad_of<true>(wb, 1)),
+                 gz = f2(grad_of<true>(wa, 2), grad_of<true>(wb, 2));
     float2 dh, dl;
     if (NORM) {
         // products exact as q + qe, summed with two-sums; DSC = 1
@@ -1238,8 +1252,8 @@ __global__ void __launch_bounds__(256) fbm_kernel(const double *__restrict__ xyz
                                                   double *__restrict__ out64, float *__restrict__ out32,
                                                   int accumulate, unsigned long long *nfb_out)
 {
-    build_table(perm, pgi);
-    init_grad_table();
+    build_table<false>(perm, pgi);
+    init_grad_table<false>();
     init_extra_table();
     init_corner32_table((int)threadIdx.x);
     __syncthreads();
@@ -1276,8 +1290,8 @@ __global__ void __launch_bounds__(256) trace_kernel(const double *__restrict__ x
                                                     int32_t *__restrict__ slots,
                                                     unsigned long long *nfb_out)
 {
-    build_table(perm, pgi);
-    init_grad_table();
+    build_table<false>(perm, pgi);
+    init_grad_table<false>();
     init_extra_table();
     init_corner32_table((int)threadIdx.x);
     __syncthreads();
@@ -1408,7 +1422,7 @@ __device__ __forceinline__ void octave_value(const Triples &t, const OctP &O, bo
 __device__ __forceinline__ void init_pair_tables()
 {
     static_assert(PAIR_THREADS == 512, "threads 256-351, 448-459 and 480-495 fill the small tables");
-    init_grad_table();
+    init_grad_table<true>();
     init_extra_table_pair((int)threadIdx.x - 256);
     init_corner_table((int)threadIdx.x - 448);
     init_third_table((int)threadIdx.x - 480);
@@ -1497,7 +1511,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) fbm_batch_kernel(const nx_fbm
             kmn = ~0ull;
             kmx = 0ull;
             __syncthreads();
-            build_table(planets[p].perm, planets[p].pgi);
+            build_table<true>(planets[p].perm, planets[p].pgi);
             __syncthreads();
             cur = p;
         }
@@ -1565,7 +1579,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) fbm_pair_kernel(const double 
                                                                    unsigned long long *nfb_out)
 {
     __shared__ unsigned long long s_mm[2][PAIR_WARPS];
-    build_table(perm, pgi);
+    build_table<true>(perm, pgi);
     init_pair_tables();
     __syncthreads();
     const uint32_t lb = lane_base();

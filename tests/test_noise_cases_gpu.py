@@ -62,3 +62,18 @@ def test_pair_values_around_ties(reach):
         got, _ = terrain.fbm(torch.from_numpy(pts).cuda(), perm, pgi, [1.0] * len(strength), strength, 1.0)
         want = (O.noise3d_batch(pts, perm, pgi) + 1.0) * 0.5 * sum(strength)
         assert np.abs(got.cpu().numpy() - want).max() <= 2e-13 * sum(strength)
+
+
+def test_gradients_that_start_anywhere():
+    """Tables whose entries are no multiples of 3: components index, index + 1 and index + 2 of the reference's table, in
+    binary32.  The path's 2e-6 times 16.1 / 12.3, the longest such gradient against the longest of init()'s."""
+    from nixis_gb300 import opensimplex as osx, terrain
+    rng = np.random.default_rng(2)
+    pts = rng.uniform(-30.0, 30.0, (50_000, 3))
+    perm, _ = O.init(3)
+    pgi = rng.integers(0, 70, 256).astype(np.int32)
+    want = O.noise3d_batch(pts, perm, pgi)
+    val = osx.noise3d_trace(pts, perm, pgi)[0].cpu().numpy()
+    np.testing.assert_allclose(val, want, rtol=0, atol=2.7e-6)
+    got = terrain.fbm(torch.from_numpy(pts).cuda(), perm, pgi, [1.0], [2.0], 1.0, out_dtype=torch.float32)[0]
+    np.testing.assert_allclose(got.cpu().numpy(), want + 1.0, rtol=0, atol=2.7e-6)
