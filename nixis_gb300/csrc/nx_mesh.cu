@@ -1462,10 +1462,16 @@ __global__ void __launch_bounds__(256) nearest3_kernel(int k, const double *__re
     __syncthreads();
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nq; p += (int64_t)gridDim.x * blockDim.x) {
         const double qx = q[3 * p], qy = q[3 * p + 1], qz = q[3 * p + 2];
-        // the query scaled to its largest component's binade
+        // the query scaled to its largest component's binade (below the smallest
+        // binade by a power of two, which only serves the location)
         const uint32_t ex = nxf::words(qx).y & 0x7FF00000u, ey = nxf::words(qy).y & 0x7FF00000u, ez = nxf::words(qz).y & 0x7FF00000u;
         const uint32_t e20 = max(ex, max(ey, ez));
-        const float x = scaled_chop(qx, e20), y = scaled_chop(qy, e20), z = scaled_chop(qz, e20);
+        float x = scaled_chop(qx, e20), y = scaled_chop(qy, e20), z = scaled_chop(qz, e20);
+        if (e20 == 0) {
+            x = (float)(qx * 0x1p1022);
+            y = (float)(qy * 0x1p1022);
+            z = (float)(qz * 0x1p1022);
+        }
         int bf = 0;
         float bw0 = 0.0f, bw1 = 0.0f, bw2 = 0.0f, bs = -INFINITY;
         for (int f = 0; f < 20; ++f) {
@@ -1514,11 +1520,15 @@ __global__ void __launch_bounds__(256) nearest3_kernel(int k, const double *__re
             // what it was)
             out = fminf(out, d);
         }
-        // a component is off by its truncation, below 2^-22 of the query: a
-        // distance by less than 2^-20
+        // A scaled query's components are below 2 and off by less than 2^-23, a
+        // vertex's by less than 2^-23 of itself, the vertex no longer than |q| +
+        // d; the subtraction, the three roundings of d^2 and the root add 3.5
+        // 2^-24 d: a distance is within 2^-23 (5.2 + 2.75 d), two of them within
+        // 1.3e-6 + 6.6e-7 d5 (a vertex left out at a larger distance than d5 is
+        // farther still by more than its own error grows).
         const float d3 = sqrtf(a[2]), d5 = sqrtf(out);
         Best b;
-        if (d5 > d3 + 4e-6f && a[3] < INFINITY) {
+        if (d5 > d3 + __fmaf_rn(7e-7f, d5, 4e-6f) && a[3] < INFINITY && e20 != 0) {
             for (int m = 0; m < 3; ++m) { b.d[m] = INFINITY; b.i[m] = -1; }
 #pragma unroll
             for (int m = 0; m < 4; ++m) best_take(b, xyz, id[m], qx, qy, qz);
