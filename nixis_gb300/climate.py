@@ -50,6 +50,22 @@ MAX_POSITIONS = 2000
 
 def _sum(verts, radius, rotations, tilts, out, accumulate, stream, scale=None):
     """insolation_sum, each sum times binary32 `scale`."""
+    if stream is None:
+        return _sum_here(verts, radius, rotations, tilts, out, accumulate, scale)
+    # what is uploaded, converted and scaled goes on the stream that reads it;
+    # a new result is the caller's stream's
+    if out is None:
+        out = torch.empty(len(verts), dtype=torch.float32, device="cuda")
+        accumulate = False
+        out.record_stream(stream)
+    if isinstance(verts, torch.Tensor) and verts.is_cuda:
+        verts.record_stream(stream)
+    with torch.cuda.stream(stream):
+        return _sum_here(verts, radius, rotations, tilts, out, accumulate, scale)
+
+
+def _sum_here(verts, radius, rotations, tilts, out, accumulate, scale):
+    """_sum on the current stream."""
     xyz = _dev.to_device(verts, np.float64, name="verts")
     _dev.check_vertices(xyz)
     n = xyz.shape[0]
@@ -67,17 +83,14 @@ def _sum(verts, radius, rotations, tilts, out, accumulate, stream, scale=None):
         accumulate = False
     if out.dtype != torch.float32 or out.shape != (n,) or not out.is_cuda:
         raise ValueError("out must be a float32 CUDA tensor of shape (N,)")
-    if stream is not None:
-        tdev.record_stream(stream)
-        xyz.record_stream(stream)
     if short:
         vp = ctypes.c_void_p
         call("nx_insolation_positions", _dev.ptr(xyz), n, float(radius), vp(rot.ctypes.data), len(rot),
              vp(tilt.ctypes.data), n_tilt, 1.0 if scale is None else float(scale), _dev.ptr(tdev), _dev.ptr(out),
-             1 if accumulate else 0, _dev.stream_handle(stream))
+             1 if accumulate else 0, _dev.stream_handle())
     else:
         call("nx_insolation", _dev.ptr(xyz), n, float(radius), _dev.ptr(tdev), nre, pairs, n_tilt, _dev.ptr(out),
-             1 if accumulate else 0, _dev.stream_handle(stream))
+             1 if accumulate else 0, _dev.stream_handle())
         if scale is not None:
             out.mul_(scale)
     return out

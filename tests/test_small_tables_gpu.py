@@ -91,3 +91,23 @@ def test_mapped_files_go_through_staging(tmp_path):
     out = np.memmap(tmp_path / "y", np.float64, "w+", shape=a.shape)
     _dev.to_host(out, t)
     assert np.array_equal(out, a)
+
+
+@gpu
+@pytest.mark.parametrize("busy", ["its own", "the caller's"])
+@pytest.mark.parametrize("days, hours", [(2000, 24), (6, 2400), (300, 24)])
+def test_a_schedule_on_another_stream(days, hours, busy):
+    """Table, sums and their scaling are in the order of the stream that was given, whichever of the two is held back."""
+    m = mesh.PlanetMesh(12)
+    want = climate.annual_insolation(m.xyz, 1.0, days=days, hours=hours, mean_wm2=True)
+    host = m.xyz.cpu().numpy()
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s if busy == "its own" else torch.cuda.current_stream()):
+        torch.cuda._sleep(200_000_000)
+    got = [climate.annual_insolation(v, 1.0, days=days, hours=hours, mean_wm2=True, stream=s) for v in (m.xyz, host)]
+    s.synchronize()
+    with torch.cuda.stream(s):
+        kept = [g.clone() for g in got]
+    torch.cuda.synchronize()
+    assert torch.equal(kept[0], want) and torch.equal(kept[1], want)
