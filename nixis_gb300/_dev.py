@@ -1,7 +1,6 @@
 """Device-buffer plumbing: numpy arrays are copied to CUDA tensors and back;
 CUDA tensors are used in place (zero copy)."""
 import ctypes
-import mmap
 
 import numpy as np
 import torch
@@ -37,13 +36,27 @@ def is_host(a):
 
 
 def _in_memory(a):
-    """Whether a numpy array's bytes are ordinary memory (not a mapped file,
-    which the GPU is not sent to)."""
-    while isinstance(a, np.ndarray):
-        if isinstance(a, np.memmap):
+    """Whether a numpy array's bytes are memory that numpy allocated: the base
+    of everything it is a view of, through memoryviews as well, owns its data.
+    Whatever else may lie behind an array (a mapped file, as np.memmap or
+    np.frombuffer of one or a checkpoint loaded with mmap; memory of another
+    process) is not told apart, and the GPU is not sent to it."""
+    while True:
+        if isinstance(a, np.ndarray):
+            if a.base is None:
+                return bool(a.flags.owndata)
+            a = a.base
+        elif isinstance(a, memoryview):
+            a = a.obj
+        else:
             return False
-        a = a.base
-    return not isinstance(a, mmap.mmap)
+
+
+def from_device(t):
+    """A CUDA tensor's values as a numpy array of its own memory."""
+    out = np.empty(tuple(t.shape), torch.empty(0, dtype=t.dtype).numpy().dtype)
+    torch.from_numpy(out).copy_(t)
+    return out
 
 
 def upload(arr, tdt):
@@ -54,8 +67,8 @@ def upload(arr, tdt):
     straight out of the array: the GPU reads pageable memory here at
     110-180 GB/s, and staging through pinned memory copies it once more on one
     core (24 MB: 147 us against 195, 80 MB: 466 against 627).  Only under
-    capture, where such a copy cannot be waited for, and for a mapped file is it
-    staged."""
+    capture, where such a copy cannot be waited for, and for memory that is not
+    numpy's own (_in_memory) is it staged."""
     if arr.nbytes <= UPLOAD_MAX:
         t = torch.empty(arr.shape, dtype=tdt, device="cuda")
         if arr.nbytes:

@@ -125,14 +125,14 @@ def brute_daily_insolation(verts, altitudes, radius, tilt, snapshot=False):
         raise NotImplementedError("insolation snapshots (PNG export) are not provided by nixis_gb300")
     host = _dev.is_host(verts)
     out = insolation_sum(verts, radius, np.arange(-180.0, 180.0), [float(tilt)])
-    return out.cpu().numpy() if host else out
+    return _dev.from_device(out) if host else out
 
 
 def calc_instant_insolation(verts, altitudes, radius, rotation, tilt):
     """climate.calc_instant_insolation (climate.py:492-500)."""
     host = _dev.is_host(verts)
     out = insolation_sum(verts, radius, [float(rotation)], [float(tilt)])
-    return out.cpu().numpy() if host else out
+    return _dev.from_device(out) if host else out
 
 
 def annual_schedule(axial_tilt=23.44, year_length=365, days=365, hours=24):
@@ -190,7 +190,7 @@ def calc_insolation_slice(radius, tilt):
     """climate.calc_insolation_slice (climate.py:503-533): float32 (181,),
     entry i the summed insolation of latitude i (i <= 90) or i - 181, over
     360 rotations of one degree."""
-    return _slice_tables(radius, [tilt])[0].cpu().numpy()
+    return _dev.from_device(_slice_tables(radius, [tilt])[0])
 
 
 def interpolate_insolation(verts, lookup_table, insolation, radius):
@@ -221,7 +221,7 @@ def calc_daily_insolation(verts, altitudes, radius, tilt):
     tab = _slice_tables(radius, [tilt])
     call("nx_interpolate_insolation", _dev.ptr(xyz), xyz.shape[0], float(radius), _dev.ptr(tab), 1, _dev.ptr(out), 0,
          _dev.stream_handle())
-    return out.cpu().numpy() if host else out
+    return _dev.from_device(out) if host else out
 
 
 def calc_yearly_insolation(points, height, radius, axial_tilt, snapshot=False):
@@ -238,7 +238,7 @@ def calc_yearly_insolation(points, height, radius, axial_tilt, snapshot=False):
     out = torch.empty(n, dtype=torch.float32, device="cuda")
     call("nx_interpolate_insolation", _dev.ptr(xyz), n, float(radius), _dev.ptr(tab), 360, _dev.ptr(out), 0,
          _dev.stream_handle())
-    return out.cpu().numpy() if host else out
+    return _dev.from_device(out) if host else out
 
 
 def assign_surface_temp(verts, altitudes, radius, tilt):
@@ -259,4 +259,4 @@ def assign_surface_temp(verts, altitudes, radius, tilt):
         raise ValueError("zero-size array to reduction operation minimum which has no identity")
     out = torch.empty(n, dtype=torch.float32, device="cuda")
     call("nx_surface_temp", _dev.ptr(xyz), n, float(radius), float(tilt), _dev.ptr(out), _dev.stream_handle())
-    return out.cpu().numpy() if host else out
+    return _dev.from_device(out) if host else out

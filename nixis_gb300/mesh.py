@@ -58,7 +58,7 @@ def create_mesh(divisions):
     """util.create_mesh: (points float64 (10k^2+2, 3), cells int32 (20k^2, 3))
     as numpy arrays (the reference returns numpy)."""
     xyz, tris = icosphere(divisions)
-    return xyz.cpu().numpy(), tris.cpu().numpy()
+    return _dev.from_device(xyz), _dev.from_device(tris)
 
 
 def _adjacency(t, stream=None):
@@ -89,7 +89,7 @@ def build_adjacency(triangles, stream=None):
     t = _dev.to_device(triangles, np.int32, name="triangles")
     adj, err = _adjacency(t, stream)
     _check_adjacency(int(err.item()))
-    return adj.cpu().numpy() if host else adj
+    return _dev.from_device(adj) if host else adj
 
 
 def sort_adjacency(adj, stream=None):

@@ -66,7 +66,7 @@ def noisearr3d(x, y, z, perm, perm_grad_index_3D):
     pts = np.stack([np.asarray(x, np.float64).ravel(), np.asarray(y, np.float64).ravel(),
                     np.asarray(z, np.float64).ravel()], axis=1)
     val, _, _, _ = noise3d_trace(pts, perm, perm_grad_index_3D)
-    return val.double().cpu().numpy()
+    return _dev.from_device(val.double())
 
 
 def noise3d(x, y, z, perm, perm_grad_index_3D):

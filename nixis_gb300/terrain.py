@@ -69,7 +69,7 @@ def sample_noise(verts, perm, pgi, n_roughness=1, n_strength=0.2, radius=1):
     (noise3d(v * n_roughness) + 1) * 0.5 * n_strength * radius."""
     host = _dev.is_host(verts)
     out, _ = fbm(verts, perm, pgi, [float(n_roughness)], [float(n_strength)], float(radius))
-    return out.cpu().numpy() if host else out
+    return _dev.from_device(out) if host else out
 
 
 def sample_octaves(verts, elevations, perm, pgi, n_octaves=1, n_init_roughness=1.5, n_init_strength=0.4,
@@ -82,7 +82,7 @@ def sample_octaves(verts, elevations, perm, pgi, n_octaves=1, n_init_roughness=1
     host = _dev.is_host(verts) if elevations is None else _dev.is_host(elevations)
     if elevations is None:
         out, _ = fbm(verts, perm, pgi, scale, strength, world_radius)
-        return out.cpu().numpy() if host else out
+        return _dev.from_device(out) if host else out
     if host:
         if elevations.dtype != np.float64 or not elevations.flags.c_contiguous:
             raise ValueError("elevations must be a C-contiguous float64 array")

@@ -69,7 +69,7 @@ def rescale(x, lower, upper, mid=None, mode=None, u_min=None, u_max=None, stream
          float(u_min if u_min is not None else 0.0), int(u_min is not None),
          float(u_max if u_max is not None else 0.0), int(u_max is not None), _dev.ptr(out), _dev.ptr(ws), ws.numel(),
          _dev.stream_handle(stream))
-    return out.cpu().numpy() if host else out
+    return _dev.from_device(out) if host else out
 
 
 def power_rescale(x, mask=None, mode=None, power=1.0, stream=None):
@@ -91,7 +91,7 @@ def power_rescale(x, mask=None, mode=None, power=1.0, stream=None):
     ws = _ws(n)
     call("nx_power_rescale", _dev.ptr(xd), n, _dev.ptr(md), m, float(power), _dev.ptr(out), _dev.ptr(ws), ws.numel(),
          _dev.stream_handle(stream))
-    return out.cpu().numpy() if host else out
+    return _dev.from_device(out) if host else out
 
 
 def find_percent_val(minval, maxval, percent):
@@ -110,7 +110,7 @@ def make_bool_elevation_mask(height, mask_elevation, stream=None):
     n = hd.numel()
     m = torch.empty(n, dtype=torch.uint8, device="cuda")
     call("nx_elevation_mask", _dev.ptr(hd), n, float(mask_elevation), _dev.ptr(m), _dev.stream_handle(stream))
-    return m.cpu().numpy().view(bool) if host else m.view(torch.bool)
+    return _dev.from_device(m).view(bool) if host else m.view(torch.bool)
 
 
 def shape_heights(height, min_alt=-4000.0, max_alt=8850.0, ocean_percent=55.0, stream=None):
@@ -129,7 +129,7 @@ def shape_heights(height, min_alt=-4000.0, max_alt=8850.0, ocean_percent=55.0, s
     call("nx_shape_heights", _dev.ptr(hd), n, float(min_alt), float(max_alt), float(ocean_percent), _dev.ptr(out),
          _dev.ptr(tmp), _dev.ptr(mask), _dev.ptr(level), _dev.ptr(ws), ws.numel(), _dev.stream_handle(stream))
     if host:
-        return out.cpu().numpy(), mask.cpu().numpy().view(bool), float(level.item())
+        return _dev.from_device(out), _dev.from_device(mask).view(bool), float(level.item())
     return out, mask.view(torch.bool), level
 
 
@@ -146,7 +146,7 @@ def make_ll_arr(width, height, radius, device=False, stream=None):
     _dev.require_cuda()
     out = torch.empty((int(height), int(width), 3), dtype=torch.float64, device="cuda")
     call("nx_make_ll", int(width), int(height), float(radius), _dev.ptr(out), _dev.stream_handle(stream))
-    return out if device else out.cpu().numpy()
+    return out if device else _dev.from_device(out)
 
 
 def query_nearest3(verts, neighbors, divisions, queries, stream=None):
@@ -167,7 +167,7 @@ def query_nearest3(verts, neighbors, divisions, queries, stream=None):
     call("nx_nearest3", int(divisions), _dev.ptr(xyz), _dev.ptr(nb), xyz.shape[0], _dev.ptr(q), q.shape[0],
          _dev.ptr(d), _dev.ptr(i), _dev.stream_handle(stream))
     d, i = d.reshape(shape), i.reshape(shape)
-    return (d.cpu().numpy(), i.cpu().numpy()) if host else (d, i)
+    return (_dev.from_device(d), _dev.from_device(i)) if host else (d, i)
 
 
 def _sample(dists, nbrs, colors, stream=None):
@@ -192,7 +192,7 @@ def make_gray_array(width, height, dists, nbrs, colors):
     """util.make_gray_array (util.py:342-366): per pixel the inverse-distance
     weighting of its 3 neighbours' colours, truncated to an integer and
     returned in the colours' dtype, shape (height, width)."""
-    v = _sample(dists, nbrs, colors).cpu().numpy().reshape(int(height), int(width))
+    v = _dev.from_device(_sample(dists, nbrs, colors)).reshape(int(height), int(width))
     return _as_dtype(v, colors)
 
 
@@ -209,5 +209,5 @@ def equirect_map(verts, neighbors, divisions, colors, width, height, radius, str
     query + make_gray_array); returns (height, width) in the colours' dtype."""
     ll = make_ll_arr(width, height, radius, device=True, stream=stream)
     d, i = query_nearest3(verts, neighbors, divisions, ll, stream=stream)
-    v = _sample(d, i, colors, stream=stream).cpu().numpy().reshape(int(height), int(width))
+    v = _dev.from_device(_sample(d, i, colors, stream=stream)).reshape(int(height), int(width))
     return _as_dtype(v, colors)

@@ -90,3 +90,27 @@ def test_mesh_eviction_prefers_meshes_no_arrived_request_needs():
     assert _victim(lru, refs, [100, 200, 400]) == 400
     assert _victim([300], refs, [100]) is None
     assert _victim(lru, {}, [999]) == 100            # none needed: least recently used
+
+
+def test_arrays_whose_memory_is_numpys_own(tmp_path):
+    import mmap
+    from multiprocessing import shared_memory
+    from nixis_gb300 import _dev
+    a = np.arange(24.0)
+    for own in (a, a[3:], a.reshape(4, 6).T, a.view(np.uint8), np.asarray(memoryview(a)), np.frombuffer(memoryview(a[1:])),
+                np.zeros(0), _dev.from_device(torch.arange(6.0).view(2, 3).T), _dev.from_device(torch.ones(4, dtype=torch.uint8)).view(bool)):
+        assert _dev._in_memory(own)
+    assert np.array_equal(_dev.from_device(torch.arange(6).view(2, 3).T), np.arange(6).reshape(2, 3).T)
+    (tmp_path / "f").write_bytes(bytes(80000))
+    torch.save(torch.zeros(9000, dtype=torch.float64), tmp_path / "t")
+    with open(tmp_path / "f", "r+b") as f:
+        mm = mmap.mmap(f.fileno(), 0)
+    shm = shared_memory.SharedMemory(create=True, size=80000)
+    others = [np.memmap(tmp_path / "f", np.float64, "r+"), np.asarray(np.memmap(tmp_path / "f", np.float64, "r+"))[5:],
+              np.frombuffer(mm), np.frombuffer(mm)[2:].reshape(-1, 2), np.asarray(memoryview(mm)), np.ndarray(10000, np.float64, mm),
+              np.ndarray(10000, np.float64, shm.buf), torch.from_file(str(tmp_path / "f"), size=10000, dtype=torch.float64).numpy(),
+              torch.load(tmp_path / "t", mmap=True).numpy()]
+    assert not any(_dev._in_memory(o) for o in others)
+    del others
+    shm.close()
+    shm.unlink()

@@ -8,7 +8,7 @@ import pytest
 
 torch = pytest.importorskip("torch")
 
-from nixis_gb300 import _dev, _lib, climate, mesh  # noqa: E402
+from nixis_gb300 import _dev, _lib, climate, mesh, util  # noqa: E402
 
 gpu = pytest.mark.gpu
 
@@ -111,3 +111,20 @@ def test_a_schedule_on_another_stream(days, hours, busy):
         kept = [g.clone() for g in got]
     torch.cuda.synchronize()
     assert torch.equal(kept[0], want) and torch.equal(kept[1], want)
+
+
+@gpu
+def test_bytes_of_a_mapping_go_through_staging(tmp_path):
+    """Arrays made of a mapping's buffer, past the size of an upload, in both directions."""
+    import mmap
+    a = np.random.default_rng(1).random(9000)
+    (tmp_path / "x").write_bytes(a.tobytes())
+    with open(tmp_path / "x", "r+b") as f:
+        mm = mmap.mmap(f.fileno(), 0)
+    for src in (np.frombuffer(mm), np.asarray(memoryview(mm)).view(np.float64)):
+        t = _dev.to_device(src, np.float64)
+        assert np.array_equal(t.cpu().numpy(), a)
+    _dev.to_host(np.frombuffer(mm), t + 1.0)
+    assert np.array_equal(np.frombuffer(mm), a + 1.0)
+    points, _ = util.create_mesh(4)              # (the library's own results need none)
+    assert _dev._in_memory(points)
