@@ -68,16 +68,16 @@ def upload(arr, tdt):
     Small tables go as kernel arguments (nothing waits).  The rest is copied
     straight out of the array: the GPU reads pageable memory here at
     110-180 GB/s, and staging through pinned memory copies it once more on one
-    core (24 MB: 147 us against 195, 80 MB: 466 against 627).  Only under
-    capture, where such a copy cannot be waited for, and for memory that is not
-    known (_in_memory) is it staged."""
+    core (24 MB: 147 us against 195, 80 MB: 466 against 627).  That copy waits
+    for the stream, so it is staged where the stream has work queued, under
+    capture, and for memory that is not known (_in_memory)."""
     if arr.nbytes <= UPLOAD_MAX:
         t = torch.empty(arr.shape, dtype=tdt, device="cuda")
         if arr.nbytes:
             call("nx_upload", ptr(t), ctypes.c_void_p(arr.ctypes.data), arr.nbytes, stream_handle())
         return t
     t = torch.from_numpy(arr)
-    if torch.cuda.is_current_stream_capturing() or not _in_memory(arr):
+    if torch.cuda.is_current_stream_capturing() or not _in_memory(arr) or not torch.cuda.current_stream().query():
         return t.pin_memory().to("cuda", non_blocking=True)
     return t.to("cuda")
 

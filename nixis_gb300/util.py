@@ -207,7 +207,10 @@ def equirect_map(verts, neighbors, divisions, colors, width, height, radius, str
     """A whole map on the GPU: pixel positions, nearest three vertices, and
     the gray weighting of `colors` (the reference's make_ll_arr + KD-tree
     query + make_gray_array); returns (height, width) in the colours' dtype."""
+    # (host arrays first, while the stream is idle: a direct copy waits for it)
+    xyz, nb, cd = (_dev.to_device(verts, np.float64, name="verts"), _dev.to_device(neighbors, np.int32, name="neighbors"),
+                   _dev.to_device(colors, np.float64, name="colors"))
     ll = make_ll_arr(width, height, radius, device=True, stream=stream)
-    d, i = query_nearest3(verts, neighbors, divisions, ll, stream=stream)
-    v = _dev.from_device(_sample(d, i, colors, stream=stream)).reshape(int(height), int(width))
+    d, i = query_nearest3(xyz, nb, divisions, ll, stream=stream)
+    v = _dev.from_device(_sample(d, i, cd, stream=stream)).reshape(int(height), int(width))
     return _as_dtype(v, colors)

@@ -128,3 +128,17 @@ def test_bytes_of_a_mapping_go_through_staging(tmp_path):
     assert np.array_equal(np.frombuffer(mm), a + 1.0)
     points, _ = util.create_mesh(4)              # (the library's own results need none)
     assert _dev._in_memory(points)
+
+
+@gpu
+def test_a_large_array_does_not_wait_for_a_busy_stream():
+    a = np.random.default_rng(2).random(300_000)
+    want = a.copy()
+    for _ in range(2):                           # (the first makes the page-locked buffer)
+        torch.cuda.synchronize()
+        torch.cuda._sleep(400_000_000)
+        t = _dev.to_device(a, np.float64)
+        busy = not torch.cuda.current_stream().query()
+    a[:] = 0.0
+    assert busy
+    assert np.array_equal(t.cpu().numpy(), want)
