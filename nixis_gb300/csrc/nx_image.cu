@@ -25,27 +25,28 @@ constexpr int LL_ROWS = 32;
 __global__ void __launch_bounds__(256) make_ll_kernel(int width, int height, double radius, double *__restrict__ out)
 {
     __shared__ double s_rc[LL_ROWS], s_z[LL_ROWS];           // radius cos(lat), radius sin(lat)
-    const int h0 = blockIdx.y * LL_ROWS;
-    if (threadIdx.x < LL_ROWS) {
-        const double latpercent = 180.0 / (double)(height - 1);
-        const double lat = fmax(__dsub_rn(90.0, __dmul_rn((double)(h0 + (int)threadIdx.x), latpercent)), -90.0);
-        const double a = __dmul_rn(lat, PI / 180);
-        s_rc[threadIdx.x] = __dmul_rn(radius, cos(a));
-        s_z[threadIdx.x] = __dmul_rn(radius, sin(a));
-    }
-    __syncthreads();
     const int w = blockIdx.x * 256 + threadIdx.x;
-    if (w >= width) return;
     const double lonpercent = 360.0 / (double)width;
     const double lon = fmax(__dadd_rn(-180.0, __dmul_rn((double)w, lonpercent)), -180.0);
     const double b = __dmul_rn(lon, PI / 180);
     const double cb = cos(b), sb = sin(b);
-    const int rows = min(LL_ROWS, height - h0);
-    for (int r = 0; r < rows; ++r) {
-        double *o = out + 3 * ((int64_t)(h0 + r) * width + w);
-        o[0] = __dmul_rn(s_rc[r], cb);
-        o[1] = __dmul_rn(s_rc[r], sb);
-        o[2] = s_z[r];
+    const double latpercent = 180.0 / (double)(height - 1);
+    for (int64_t h0 = (int64_t)blockIdx.y * LL_ROWS; h0 < height; h0 += (int64_t)gridDim.y * LL_ROWS) {
+        __syncthreads();
+        if (threadIdx.x < LL_ROWS) {
+            const double lat = fmax(__dsub_rn(90.0, __dmul_rn((double)(h0 + threadIdx.x), latpercent)), -90.0);
+            const double a = __dmul_rn(lat, PI / 180);
+            s_rc[threadIdx.x] = __dmul_rn(radius, cos(a));
+            s_z[threadIdx.x] = __dmul_rn(radius, sin(a));
+        }
+        __syncthreads();
+        const int rows = (int)(height - h0 < LL_ROWS ? height - h0 : LL_ROWS);
+        for (int r = 0; w < width && r < rows; ++r) {
+            double *o = out + 3 * ((h0 + r) * width + w);
+            o[0] = __dmul_rn(s_rc[r], cb);
+            o[1] = __dmul_rn(s_rc[r], sb);
+            o[2] = s_z[r];
+        }
     }
 }
 
@@ -89,9 +90,9 @@ int grid_for(int64_t n)
 NX_EXPORT int nx_make_ll(int width, int height, double radius, double *out_dev, void *stream)
 {
     if (width < 1 || height < 2 || !out_dev) return nx::fail(NX_EINVAL, "nx_make_ll: bad arguments");
-    // (a grid's y is at most 65,535 blocks: taller maps in parts of whole blocks)
-    const dim3 grid((unsigned)((width + 255) / 256), (unsigned)((height + LL_ROWS - 1) / LL_ROWS));
-    if (grid.y > 65535u) return nx::fail(NX_EINVAL, "nx_make_ll: more than %d rows", 65535 * LL_ROWS);
+    // (a grid's y is at most 65,535 blocks: taller maps by several blocks of rows each)
+    const int64_t yb = ((int64_t)height + LL_ROWS - 1) / LL_ROWS;
+    const dim3 grid((unsigned)((width + 255LL) / 256), (unsigned)(yb < 65535 ? yb : 65535));
     make_ll_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(width, height, radius, out_dev);
     NX_CHECK_LAUNCH("make_ll_kernel");
     nx::note_launch(1);

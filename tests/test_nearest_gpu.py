@@ -75,3 +75,14 @@ def test_queries_of_no_length_and_no_number():
     for bad in (float("nan"), float("inf")):
         d, i = util.query_nearest3(m.xyz, m.nbr, k, torch.tensor([[0.3, bad, 0.1]], dtype=torch.float64, device="cuda"))
         assert (i == -1).all() and torch.isinf(d).all()
+
+
+@pytest.mark.parametrize("size", [(1, 65535 * 32 + 1), (2, 65535 * 32 + 70)])
+def test_pixel_positions_of_maps_taller_than_a_grid(size):
+    import math
+    from nixis_gb300 import util
+    w, h = size
+    ll = util.make_ll_arr(w, h, 2.5, device=True)
+    for r in (0, 31, 32, h // 2, 65535 * 32 - 1, 65535 * 32, h - 1):
+        x, y, z = util.latlon2xyz(max(90.0 - r * (180.0 / (h - 1)), -90.0), -180.0, 2.5)
+        assert all(abs(u - v) <= 2 * math.ulp(2.5) for u, v in zip(ll[r, 0].tolist(), (x, y, z)))
