@@ -490,9 +490,15 @@ __global__ void __launch_bounds__(256) ico_edges_kernel(int k, int64_t nv, const
         if (in & 8u) el[6 * (int64_t)row[3]] = d3;
         if (in & 16u) el[6 * (int64_t)row[4] + 1] = d4;
         if ((in & 35u) != 35u) {
-            if (!(in & 1u)) el[6 * v] = edge_pair(edge_len(xyz, v, row[0]));
-            if (!(in & 2u)) el[6 * v + 1] = edge_pair(edge_len(xyz, v, row[1]));
-            if (!(in & 32u)) el[6 * v + 5] = edge_pair(edge_len(xyz, v, row[5]));
+            // (counted here too: a border vertex's row need not name this vertex)
+            auto border = [&](int slot) {
+                const float2 d = edge_pair(edge_len(xyz, v, row[slot]));
+                longest = fmaxf(longest, d.x);
+                el[6 * v + slot] = d;
+            };
+            if (!(in & 1u)) border(0);
+            if (!(in & 2u)) border(1);
+            if (!(in & 32u)) border(5);
         }
     }
     if (!info) return;

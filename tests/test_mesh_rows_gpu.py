@@ -68,3 +68,24 @@ def test_edge_rows_of_any_alignment(k):
     assert torch.equal(buf[2:-2].view(m.edge.shape), m.edge)
     assert torch.equal(m.edge, mesh.edge_lengths(m.xyz, m.nbr)[0])
     assert (buf[:2] == 7.0).all() and (buf[-2:] == 7.0).all()
+
+
+def test_the_longest_edge_counts_what_border_rows_leave_out(monkeypatch):
+    """A far vertex of a face's border that only face-interior rows name, in the slots that compute no other distance."""
+    import torch
+    from nixis_gb300 import erosion, mesh
+    monkeypatch.setattr(erosion, "BLOCKED_WORK", 1)
+    k = 40
+    m = mesh.PlanetMesh(k)
+    inner = 12 + 30 * (k - 1)
+    slots = {}
+    for slot in range(6):
+        for v in m.nbr[inner:, slot][m.nbr[inner:, slot] < inner].unique().tolist():
+            slots.setdefault(v, set()).add(slot)
+    v = next(v for v in sorted(slots) if v >= 12 and slots[v] <= {0, 1, 5})
+    nbr, xyz = m.nbr.clone(), m.xyz.clone()
+    nbr[:inner][nbr[:inner] == v] = -1
+    nbr[v] = -1
+    assert erosion.ErosionRun(xyz, nbr, iters=9).k == k
+    xyz[v] *= 9.0                                # 8 from its neighbours: too long for blocked passes
+    assert erosion.ErosionRun(xyz, nbr, iters=9).k is None
