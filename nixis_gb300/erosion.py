@@ -57,19 +57,22 @@ class ErosionRun:
             # None: not the icosphere's own table, edges too long, or not worth finding out
             self.k = (self._icosphere_divisions()
                       if edge is None and iters >= BLOCKED_ITERS and iters * n >= BLOCKED_WORK else None)
-            if edge is None:
-                if self.k is None:
-                    edge, err = _mesh.edge_lengths(self.xyz, self.nbr, stream=stream)
-                else:
-                    edge = torch.empty((n, 6, 2), dtype=torch.float32, device="cuda")
-                    err = torch.zeros(2, dtype=torch.int32, device="cuda")
-                    call("nx_icosphere_edges", self.k, _dev.ptr(self.xyz), _dev.ptr(self.nbr), _dev.ptr(edge), _dev.ptr(err),
-                         _dev.stream_handle(stream))
-                err = err.cpu()
-                if err.numel() == 2 and not float(err.view(torch.float32)[1]) <= BLOCKED_EDGE:
+            if edge is None and self.k is None:
+                edge, err = _mesh.edge_lengths(self.xyz, self.nbr, stream=stream)
+                bad = err.item()
+            elif edge is None:
+                edge = torch.empty((n, 6, 2), dtype=torch.float32, device="cuda")
+                info = torch.zeros(2, dtype=torch.int32, device="cuda")
+                call("nx_icosphere_edges", self.k, _dev.ptr(self.xyz), _dev.ptr(self.nbr), _dev.ptr(edge), _dev.ptr(info),
+                     _dev.stream_handle(stream))
+                info = info.cpu()
+                bad = int(info[0])
+                if not float(info.view(torch.float32)[1]) <= BLOCKED_EDGE:
                     self.k = None
-                if int(err[0]):
-                    raise IndexError("neighbors holds an id outside [-1, N)")
+            else:
+                bad = 0
+            if bad:
+                raise IndexError("neighbors holds an id outside [-1, N)")
         self.edge = edge
         self.st = torch.empty((n, 8), dtype=torch.float32, device="cuda")    # (h, w, s as hi/lo pairs, 0, 0)
         self.st_tmp = torch.empty_like(self.st)
@@ -121,8 +124,10 @@ class ErosionRun:
         is not known to be an icosphere's (see __init__) or the tiling does
         not fit."""
         iters = int(iters)
+        if self.k is None or iters < 1:
+            return False
         tb = _autotune.current()
-        if self.k is None or iters < 1 or tb.variant not in (0, 1, 4, 5):
+        if tb.variant not in (0, 1, 4, 5):
             return False
         with self._on_stream():
             try:

@@ -89,3 +89,18 @@ def test_load_and_store_keep_every_value():
         run.store(*out)
         for a, b in zip(v, out):
             assert ((a - b).abs() <= a.abs() * 2.0 ** -48).all()
+
+
+def test_short_runs_do_no_work_for_blocked_passes(monkeypatch):
+    """One iteration at a time, without asking for the setting of passes that are not made."""
+    import torch
+    from nixis_gb300 import autotune, erosion, mesh
+
+    def unwanted():
+        raise AssertionError("asked for")
+    monkeypatch.setattr(autotune, "current", unwanted)
+    m = mesh.PlanetMesh(20)
+    h = field(m, 2)
+    want = one_at_a_time(m.xyz, m.nbr, h, 3)
+    erosion.erode_terrain3(m.xyz, m.nbr, h, 3)
+    assert torch.equal(h, want)
