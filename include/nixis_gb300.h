@@ -336,6 +336,12 @@ int nx_erosion_batch(const nx_erosion_planet *planets_dev, const nx_erosion_plan
 int nx_erosion_run(const nx_erosion_planet *planets_dev, const nx_erosion_planet *planets_host, int nplanets,
                    int rings, float *st_dev, float *st_tmp_dev, void *workspace, size_t ws_bytes, void *stream);
 
+/* The same with a setting of its own (rings, threads, variant as
+ * nx_erosion_tb_config takes them), which no other call sees and none changes. */
+int nx_erosion_run_as(const nx_erosion_planet *planets_dev, const nx_erosion_planet *planets_host, int nplanets,
+                      int rings, int threads, int variant, float *st_dev, float *st_tmp_dev, void *workspace,
+                      size_t ws_bytes, void *stream);
+
 /* Serving: one launch that advances every listed planet (any order) by one
  * iteration, planet p at its own iteration t - t_start (planets outside
  * [0, iters) skip).  Control blocks are workspace slots [0, nslots);

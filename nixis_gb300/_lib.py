@@ -60,6 +60,7 @@ SIGNATURES = {
     "nx_erosion_ticks": (_i32, [_p, _p, _i32, _i32, _i32, _p, _p, _p, ctypes.c_size_t, _i32, _i32, _p]),
     "nx_erosion_passes": (_i32, [_p, _p, _i32, _i32, _i32, _p, _p, _p, ctypes.c_size_t, _i32, _i32, _p]),
     "nx_erosion_run": (_i32, [_p, _p, _i32, _i32, _p, _p, _p, ctypes.c_size_t, _p]),
+    "nx_erosion_run_as": (_i32, [_p, _p, _i32, _i32, _i32, _i32, _p, _p, _p, ctypes.c_size_t, _p]),
     "nx_erosion_npass": (_i32, [_i32]),
     "nx_shape_workspace_size": (ctypes.c_size_t, [_i64]),
     "nx_insolation_slices": (_i32, [_p, _i32, _d, _p, _p]),

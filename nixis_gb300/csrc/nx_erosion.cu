@@ -1124,59 +1124,65 @@ static int64_t planet_blocks(const nx_erosion_planet &P) { return (P.n + BLOCK -
 
 // Temporal blocking: rings of the tilings in use (all planets of a batch
 // share it) and a switch for comparisons.
-static int g_tb_rings = 4;
-static int g_tb_threads = 512;
-static int g_tb_variant = 0;
-static bool g_tb_enabled = true;
+struct TbSetting {
+    int rings, threads, variant;
+    bool enabled;
+};
+static TbSetting g_tb = {4, 512, 0, true};
 
-NX_EXPORT int nx_erosion_tb_config(int rings, int threads, int variant, int enabled)
+static int check_setting(const TbSetting &c, const char *who)
 {
-    if (rings < 1 || rings > 8) return nx::fail(NX_EINVAL, "nx_erosion_tb_config: rings must be in [1, 8]");
-    const bool ok = variant == 1 ? (threads == 256 || threads == 384)
-                  : (variant == 2 || variant == 3) ? (threads == 512 || threads == 1024)
-                  : variant == 0 ? (threads == 256 || threads == 512 || threads == 1024)
-                  : variant == 4 ? (threads == 256 || threads == 320 || threads == 384 || threads == 640)
-                  : variant == 5 ? threads == 256 : false;
-    if (!ok)
-        return nx::fail(NX_EINVAL, "nx_erosion_tb_config: threads %d do not go with variant %d", threads, variant);
-    g_tb_rings = rings;
-    g_tb_threads = threads;
-    g_tb_variant = variant;
-    g_tb_enabled = enabled != 0;
+    if (c.rings < 1 || c.rings > 8) return nx::fail(NX_EINVAL, "%s: rings must be in [1, 8]", who);
+    const int t = c.threads;
+    const bool ok = c.variant == 1 ? (t == 256 || t == 384)
+                  : (c.variant == 2 || c.variant == 3) ? (t == 512 || t == 1024)
+                  : c.variant == 0 ? (t == 256 || t == 512 || t == 1024)
+                  : c.variant == 4 ? (t == 256 || t == 320 || t == 384 || t == 640)
+                  : c.variant == 5 ? t == 256 : false;
+    if (!ok) return nx::fail(NX_EINVAL, "%s: threads %d do not go with variant %d", who, t, c.variant);
     return NX_OK;
 }
 
-// Shared memory of a launch of the configured variant.
-static size_t tb_launch_smem(int maxnl, int maxc)
+NX_EXPORT int nx_erosion_tb_config(int rings, int threads, int variant, int enabled)
+{
+    const TbSetting c = {rings, threads, variant, enabled != 0};
+    const int rc = check_setting(c, "nx_erosion_tb_config");
+    if (rc) return rc;
+    g_tb = c;
+    return NX_OK;
+}
+
+// Shared memory of a launch of a setting's variant.
+static size_t tb_launch_smem(const TbSetting &cfg, int maxnl, int maxc)
 {
     size_t b = tb_smem_bytes(maxnl + (maxnl & 1));
-    if (g_tb_variant == 2) b += tb_table_bytes(maxc);
+    if (cfg.variant == 2) b += tb_table_bytes(maxc);
     return b;
 }
 
-static cudaError_t launch_tb(int64_t grid, size_t smem, cudaStream_t s, TbArgs ta)
+static cudaError_t launch_tb(const TbSetting &cfg, int64_t grid, size_t smem, cudaStream_t s, TbArgs ta)
 {
     ta.wide = (((uintptr_t)ta.st0 | (uintptr_t)ta.st1) & 31u) == 0;
-    if (g_tb_variant == 1) {
-        if (g_tb_threads == 256) erosion_tb_kernel<256, true><<<(unsigned)grid, 256, smem, s>>>(ta);
+    if (cfg.variant == 1) {
+        if (cfg.threads == 256) erosion_tb_kernel<256, true><<<(unsigned)grid, 256, smem, s>>>(ta);
         else erosion_tb_kernel<384, true><<<(unsigned)grid, 384, smem, s>>>(ta);
-    } else if (g_tb_variant == 2) {
-        if (g_tb_threads == 512) erosion_tb_kernel<512, false, true><<<(unsigned)grid, 512, smem, s>>>(ta);
+    } else if (cfg.variant == 2) {
+        if (cfg.threads == 512) erosion_tb_kernel<512, false, true><<<(unsigned)grid, 512, smem, s>>>(ta);
         else erosion_tb_kernel<1024, false, true><<<(unsigned)grid, 1024, smem, s>>>(ta);
-    } else if (g_tb_variant == 3) {
-        if (g_tb_threads == 512) erosion_tb_kernel<512, false, false, true><<<(unsigned)grid, 512, smem, s>>>(ta);
+    } else if (cfg.variant == 3) {
+        if (cfg.threads == 512) erosion_tb_kernel<512, false, false, true><<<(unsigned)grid, 512, smem, s>>>(ta);
         else erosion_tb_kernel<1024, false, false, true><<<(unsigned)grid, 1024, smem, s>>>(ta);
-    } else if (g_tb_variant == 4) {
-        switch (g_tb_threads) {
+    } else if (cfg.variant == 4) {
+        switch (cfg.threads) {
         case 256: erosion_tb_kernel<256, false, false, false, 5><<<(unsigned)grid, 256, smem, s>>>(ta); break;
         case 320: erosion_tb_kernel<320, false, false, false, 4><<<(unsigned)grid, 320, smem, s>>>(ta); break;
         case 640: erosion_tb_kernel<640, false, false, false, 2><<<(unsigned)grid, 640, smem, s>>>(ta); break;
         default: erosion_tb_kernel<384, false, false, false, 3><<<(unsigned)grid, 384, smem, s>>>(ta); break;
         }
-    } else if (g_tb_variant == 5) {
+    } else if (cfg.variant == 5) {
         erosion_tb_kernel<256, false, false, false, 6><<<(unsigned)grid, 256, smem, s>>>(ta);
     } else {
-        switch (g_tb_threads) {
+        switch (cfg.threads) {
         case 256: erosion_tb_kernel<256, false><<<(unsigned)grid, 256, smem, s>>>(ta); break;
         case 1024: erosion_tb_kernel<1024, false><<<(unsigned)grid, 1024, smem, s>>>(ta); break;
         default: erosion_tb_kernel<512, false><<<(unsigned)grid, 512, smem, s>>>(ta); break;
@@ -1244,7 +1250,7 @@ struct BatchPlan {
     int64_t total = 0, nblk = 0, ntiles_all = 0;
 };
 
-static int plan_batch(const nx_erosion_planet *planets_host, int np, bool allow_tb, BatchPlan &pl)
+static int plan_batch(const nx_erosion_planet *planets_host, int np, bool allow_tb, const TbSetting &cfg, BatchPlan &pl)
 {
     pl = BatchPlan();
     for (int p = 0; p < np; ++p) {
@@ -1258,7 +1264,7 @@ static int plan_batch(const nx_erosion_planet *planets_host, int np, bool allow_
         if (P.vbeg + P.n > pl.total) pl.total = P.vbeg + P.n;
         pl.nblk += planet_blocks(P);
     }
-    bool tb = allow_tb && g_tb_enabled;
+    bool tb = allow_tb && cfg.enabled;
     for (int p = 0; p < np && tb; ++p) {
         const nx_erosion_planet &P = planets_host[p];
         if (P.iters == 0) {
@@ -1266,49 +1272,51 @@ static int plan_batch(const nx_erosion_planet *planets_host, int np, bool allow_
             continue;
         }
         if (!P.tiling || P.ntiles <= 0 || P.maxnl <= 0) { tb = false; break; }
-        if (g_tb_variant >= 2 && P.maxc <= 0)
+        if (cfg.variant >= 2 && P.maxc <= 0)
             return nx::fail(NX_EINVAL, "erosion: planet %d has no maxc (needed by blocked-kernel variant %d)", p,
-                            g_tb_variant);
-        if (g_tb_variant == 3 && P.maxc > g_tb_threads)
+                            cfg.variant);
+        if (cfg.variant == 3 && P.maxc > cfg.threads)
             return nx::fail(NX_EINVAL, "erosion: planet %d: tiles of %d updatable vertices exceed %d threads (variant 3)",
-                            p, P.maxc, g_tb_threads);
+                            p, P.maxc, cfg.threads);
         pl.ntiles_all += P.ntiles;
         if (P.maxnl > pl.maxnl) pl.maxnl = P.maxnl;
         if (P.maxc > pl.maxc) pl.maxc = P.maxc;
     }
     if (pl.maxnl == 0) tb = false;
     if (tb) {
-        pl.R = g_tb_rings;
+        pl.R = cfg.rings;
         int rc = tb_prepare();
         if (rc) return rc;
-        if (tb_launch_smem(pl.maxnl, pl.maxc) > (g_tb_variant == 2 ? TB_SMEM_MAX : 200 * 1024)) tb = false;
+        if (tb_launch_smem(cfg, pl.maxnl, pl.maxc) > (cfg.variant == 2 ? TB_SMEM_MAX : 200 * 1024)) tb = false;
     }
     pl.tb = tb;
     return NX_OK;
 }
 
-// fuse (blocked path only): the fusion fields of TbArgs (raw sums and
-// rescale constants for the planets' first passes).
+// cfg: the setting, taken once by the entry point (another thread may change it
+// meanwhile).  fuse (blocked path only): the fusion fields of TbArgs (raw sums and
+// rescale constants for the planets' first passes).  run: blocked passes of any
+// number, or nothing.
 static int run_batch(const nx_erosion_planet *planets_dev, const nx_erosion_planet *planets_host, int np,
                      float *st_dev, float *st_tmp, double *mass_dev, uint16_t *flow_dev, void *workspace,
-                     size_t ws_bytes, cudaStream_t s, bool allow_tb, const TbArgs *fuse = nullptr, int rings = 0)
+                     size_t ws_bytes, cudaStream_t s, bool allow_tb, const TbSetting &cfg,
+                     const TbArgs *fuse = nullptr, bool run = false)
 {
     if (np <= 0) return NX_OK;
     if (!planets_dev || !planets_host || !st_dev || !st_tmp || !workspace)
         return nx::fail(NX_EINVAL, "erosion: null pointer");
     BatchPlan pl;
-    int rc = plan_batch(planets_host, np, allow_tb && !mass_dev && !flow_dev, pl);
+    int rc = plan_batch(planets_host, np, allow_tb && !mass_dev && !flow_dev, cfg, pl);
     if (rc) return rc;
     const bool tb = pl.tb;
     const int R = pl.R, maxnl = pl.maxnl, maxc = pl.maxc, max_it = pl.max_it;
     const int64_t nblk = pl.nblk, ntiles_all = pl.ntiles_all;
-    if ((fuse || rings) && !tb) return nx::fail(NX_EINVAL, "erosion: the run needs the blocked path");
-    if (rings && R != rings) return nx::fail(NX_EINVAL, "erosion: passes are set to %d rings, not %d", R, rings);
+    if ((fuse || run) && !tb) return nx::fail(NX_EINVAL, "erosion: the run needs the blocked path");
     if (tb) {
         if (ws_bytes < nx_erosion_workspace_size((ntiles_all > nblk ? ntiles_all : nblk) * BLOCK, np))
             return nx::fail(NX_EINVAL, "erosion: workspace too small");
         Workspace w = carve(workspace, np, ntiles_all > nblk ? ntiles_all : nblk);
-        const bool any = fuse || rings;
+        const bool any = fuse || run;
         erosion_tb_map_kernel<<<np, 256, 0, s>>>(planets_dev, np, R, any, w.blk_map);
         NX_CHECK_LAUNCH("erosion_tb_map_kernel");
         nx::note_launch(1);
@@ -1337,14 +1345,14 @@ static int run_batch(const nx_erosion_planet *planets_dev, const nx_erosion_plan
             ta.w0h = fuse->w0h;
             ta.w0l = fuse->w0l;
         }
-        const size_t smem = tb_launch_smem(maxnl, maxc);
+        const size_t smem = tb_launch_smem(cfg, maxnl, maxc);
         for (int q = 0; q < maxpass; ++q) {
             int64_t grid = 0;
             for (int p = 0; p < np; ++p)
                 if (tb_npass(planets_host[p].iters, R, any) > q) grid += planets_host[p].ntiles;
             if (grid <= 0) break;
             ta.pass = q;
-            NX_CHECK_CUDA(launch_tb(grid, smem, s, ta));
+            NX_CHECK_CUDA(launch_tb(cfg, grid, smem, s, ta));
             nx::note_launch(1);
         }
         if (maxpass > 0) {
@@ -1460,6 +1468,7 @@ NX_EXPORT int nx_erosion_passes(const nx_erosion_planet *planets_dev, const nx_e
     if (nplanets <= 0 || npasses <= 0) return NX_OK;
     if (!planets_dev || !planets_host || !st_dev || !st_tmp_dev || !workspace || nslots <= 0)
         return nx::fail(NX_EINVAL, "nx_erosion_passes: bad arguments");
+    const TbSetting cfg = g_tb;
     int64_t ntiles = 0;
     int maxnl = 0, maxc = 0;
     for (int p = 0; p < nplanets; ++p) {
@@ -1468,24 +1477,24 @@ NX_EXPORT int nx_erosion_passes(const nx_erosion_planet *planets_dev, const nx_e
             return nx::fail(NX_EINVAL, "nx_erosion_passes: planet %d: bad descriptor", p);
         if (!P.tiling || P.ntiles <= 0 || P.maxnl <= 0)
             return nx::fail(NX_EINVAL, "nx_erosion_passes: planet %d has no tiling", p);
-        if (g_tb_variant >= 2 && P.maxc <= 0)
-            return nx::fail(NX_EINVAL, "nx_erosion_passes: planet %d has no maxc (needed by variant %d)", p, g_tb_variant);
-        if (g_tb_variant == 3 && P.maxc > g_tb_threads)
+        if (cfg.variant >= 2 && P.maxc <= 0)
+            return nx::fail(NX_EINVAL, "nx_erosion_passes: planet %d has no maxc (needed by variant %d)", p, cfg.variant);
+        if (cfg.variant == 3 && P.maxc > cfg.threads)
             return nx::fail(NX_EINVAL, "nx_erosion_passes: planet %d: tiles exceed %d threads (variant 3)", p,
-                            g_tb_threads);
+                            cfg.threads);
         ntiles += P.ntiles;
         if (P.maxnl > maxnl) maxnl = P.maxnl;
         if (P.maxc > maxc) maxc = P.maxc;
     }
     int rc = tb_prepare();
     if (rc) return rc;
-    if (tb_launch_smem(maxnl, maxc) > (g_tb_variant == 2 ? TB_SMEM_MAX : 200 * 1024))
+    if (tb_launch_smem(cfg, maxnl, maxc) > (cfg.variant == 2 ? TB_SMEM_MAX : 200 * 1024))
         return nx::fail(NX_EINVAL, "nx_erosion_passes: tiles too large");
     if (ws_bytes < nx_erosion_workspace_size(ntiles * BLOCK, nslots))
         return nx::fail(NX_EINVAL, "nx_erosion_passes: workspace too small");
     cudaStream_t s = (cudaStream_t)stream;
     Workspace w = carve(workspace, nslots, ntiles);
-    const int R = g_tb_rings;
+    const int R = cfg.rings;
     if (remap) {
         erosion_tb_map_kernel<<<nplanets, 256, 0, s>>>(planets_dev, nplanets, R, false, w.blk_map);
         NX_CHECK_LAUNCH("erosion_tb_map_kernel");
@@ -1502,14 +1511,14 @@ NX_EXPORT int nx_erosion_passes(const nx_erosion_planet *planets_dev, const nx_e
     ta.ctl = w.ctl;
     for (int q = 0; q < npasses; ++q) {
         ta.pass = pass + q;
-        NX_CHECK_CUDA(launch_tb(ntiles, tb_launch_smem(maxnl, maxc), s, ta));
+        NX_CHECK_CUDA(launch_tb(cfg, ntiles, tb_launch_smem(cfg, maxnl, maxc), s, ta));
         nx::note_launch(1);
     }
     return NX_OK;
 }
 
 // Passes a planet of `iters` iterations makes (temporally blocked runs).
-NX_EXPORT int nx_erosion_npass(int iters) { return tb_npass(iters, g_tb_rings); }
+NX_EXPORT int nx_erosion_npass(int iters) { return tb_npass(iters, g_tb.rings); }
 
 // After a planet's last iteration: its final scale exponent into K[0].
 NX_EXPORT int nx_erosion_finish(const nx_erosion_planet *planets_dev, int nplanets, void *workspace, void *stream)
@@ -1532,7 +1541,7 @@ NX_EXPORT int nx_erosion_finish_passes(const nx_erosion_planet *planets_dev, int
     if (nplanets <= 0) return NX_OK;
     if (!planets_dev || !workspace) return nx::fail(NX_EINVAL, "nx_erosion_finish_passes: null pointer");
     erosion_tb_rebase_kernel<<<(nplanets + 127) / 128, 128, 0, (cudaStream_t)stream>>>(
-        planets_dev, nplanets, g_tb_rings, false, (nx_erosion_ctl *)workspace);
+        planets_dev, nplanets, g_tb.rings, false, (nx_erosion_ctl *)workspace);
     NX_CHECK_LAUNCH("erosion_tb_rebase_kernel");
     nx::note_launch(1);
     return NX_OK;
@@ -1558,7 +1567,7 @@ NX_EXPORT int nx_erosion_steps(const int32_t *nbr_dev, const float *edge_dev, in
     // state enters in buffer 0; with an odd count the first iteration reads buffer 1
     if (iters & 1)
         NX_CHECK_CUDA(cudaMemcpyAsync(st_tmp_dev, st_dev, 2 * sizeof(float4) * (size_t)n, cudaMemcpyDeviceToDevice, s));
-    return run_batch(planet_dev, &P, 1, st_dev, st_tmp_dev, mass_dev, flow_dev, workspace, ws_bytes, s, false);
+    return run_batch(planet_dev, &P, 1, st_dev, st_tmp_dev, mass_dev, flow_dev, workspace, ws_bytes, s, false, g_tb);
 }
 
 NX_EXPORT int nx_erosion_batch(const nx_erosion_planet *planets_dev, const nx_erosion_planet *planets_host, int nplanets,
@@ -1566,15 +1575,27 @@ NX_EXPORT int nx_erosion_batch(const nx_erosion_planet *planets_dev, const nx_er
                                void *stream)
 {
     return run_batch(planets_dev, planets_host, nplanets, st_dev, st_tmp_dev, mass_dev, nullptr, workspace, ws_bytes,
-                     (cudaStream_t)stream, true);
+                     (cudaStream_t)stream, true, g_tb);
 }
 
 NX_EXPORT int nx_erosion_run(const nx_erosion_planet *planets_dev, const nx_erosion_planet *planets_host, int nplanets,
                              int rings, float *st_dev, float *st_tmp_dev, void *workspace, size_t ws_bytes, void *stream)
 {
-    if (rings < 1) return nx::fail(NX_EINVAL, "nx_erosion_run: bad rings");
+    const TbSetting cfg = g_tb;
+    if (rings != cfg.rings) return nx::fail(NX_EINVAL, "nx_erosion_run: passes are set to %d rings, not %d", cfg.rings, rings);
     return run_batch(planets_dev, planets_host, nplanets, st_dev, st_tmp_dev, nullptr, nullptr, workspace, ws_bytes,
-                     (cudaStream_t)stream, true, nullptr, rings);
+                     (cudaStream_t)stream, true, cfg, nullptr, true);
+}
+
+NX_EXPORT int nx_erosion_run_as(const nx_erosion_planet *planets_dev, const nx_erosion_planet *planets_host, int nplanets,
+                                int rings, int threads, int variant, float *st_dev, float *st_tmp_dev, void *workspace,
+                                size_t ws_bytes, void *stream)
+{
+    const TbSetting cfg = {rings, threads, variant, true};
+    const int rc = check_setting(cfg, "nx_erosion_run_as");
+    if (rc) return rc;
+    return run_batch(planets_dev, planets_host, nplanets, st_dev, st_tmp_dev, nullptr, nullptr, workspace, ws_bytes,
+                     (cudaStream_t)stream, true, cfg, nullptr, true);
 }
 
 NX_EXPORT int nx_erosion_ctl_init(void *workspace, size_t ws_bytes, int nplanets, void *stream)
@@ -1679,8 +1700,9 @@ NX_EXPORT int nx_erosion_run_batch(const nx_erosion_planet *planets_dev, const n
     int64_t total = 0;
     int rc = check_packed(planets_host, nplanets, &total);
     if (rc) return rc;
+    const TbSetting cfg = g_tb;
     BatchPlan pl;
-    rc = plan_batch(planets_host, nplanets, true, pl);
+    rc = plan_batch(planets_host, nplanets, true, cfg, pl);
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     if (!pl.tb) {
@@ -1688,7 +1710,7 @@ NX_EXPORT int nx_erosion_run_batch(const nx_erosion_planet *planets_dev, const n
                                    st_dev, st_tmp_dev, stream);
         if (rc) return rc;
         rc = run_batch(planets_dev, planets_host, nplanets, st_dev, st_tmp_dev, nullptr, nullptr, workspace, ws_bytes, s,
-                       true);
+                       true, cfg);
         if (rc) return rc;
         return nx_erosion_heights_batch(planets_dev, planets_host, nplanets, st_dev, workspace, heights_dev, stream);
     }
@@ -1713,7 +1735,7 @@ NX_EXPORT int nx_erosion_run_batch(const nx_erosion_planet *planets_dev, const n
     f.w0h = w0h;
     f.w0l = w0l;
     rc = run_batch(planets_dev, planets_host, nplanets, st_dev, st_tmp_dev, nullptr, nullptr, workspace, ws_bytes, s,
-                     true, &f);
+                   true, cfg, &f);
     if (rc) return rc;
     return nx_erosion_heights_batch(planets_dev, planets_host, nplanets, st_dev, workspace, heights_dev, stream);
 }
@@ -1826,7 +1848,7 @@ NX_EXPORT int nx_erosion_steps_noalloc(const int32_t *nbr_dev, const float *edge
     static_assert(256 + sizeof(nx_erosion_ctl) + 16 + NOALLOC_PARTIALS <= NOALLOC_HEAD + NOALLOC_PARTIALS,
                   "partials fit before the second state buffer");
     static_assert((NOALLOC_HEAD + NOALLOC_PARTIALS) % 256 == 0, "state buffer alignment");
-    rc = run_batch(desc, &P, 1, st_dev, st_tmp, mass_dev, nullptr, (void *)ctl, ws_bytes, s, false);
+    rc = run_batch(desc, &P, 1, st_dev, st_tmp, mass_dev, nullptr, (void *)ctl, ws_bytes, s, false, g_tb);
     if (rc) return rc;
     if (status_dev) {
         noalloc_status_kernel<<<1, 1, 0, s>>>(ctl, status_dev);

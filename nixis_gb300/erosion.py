@@ -142,14 +142,11 @@ class ErosionRun:
             self.planet.copy_(torch.frombuffer(bytearray(bytes(d)), dtype=torch.uint8))
             # the state enters in the buffer that the number of passes asks for and ends in buffer 0
             st = (self.st, self.st_tmp) if -(-iters // tb.rings) % 2 == 0 else (self.st_tmp, self.st)
-            _autotune.apply(tb)
             try:
-                call("nx_erosion_run", _dev.ptr(self.planet), ctypes.byref(d), 1, tb.rings, _dev.ptr(st[0]), _dev.ptr(st[1]),
-                     _dev.ptr(ws), ws.numel(), _dev.stream_handle(self.stream))
+                call("nx_erosion_run_as", _dev.ptr(self.planet), ctypes.byref(d), 1, tb.rings, tb.threads, tb.variant,
+                     _dev.ptr(st[0]), _dev.ptr(st[1]), _dev.ptr(ws), ws.numel(), _dev.stream_handle(self.stream))
             except NxError as e:
-                # NX_EINVAL: refused before any launch (the tiles do not fit, or
-                # another setting was applied meanwhile)
-                if e.code != 1:
+                if e.code != 1:                      # NX_EINVAL: refused before any launch (the tiles do not fit)
                     raise
                 return False
             self.st, self.st_tmp = st
@@ -171,7 +168,7 @@ class ErosionRun:
 
     def error(self):
         """The run's flag: 1 an id out of range, 2 or 3 a tiling that does
-        not suit the passes (another setting was applied meanwhile)."""
+        not suit the passes."""
         with self._on_stream():
             return int(self.ws[:32].view(torch.int32)[6].item())
 

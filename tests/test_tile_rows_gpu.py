@@ -105,3 +105,32 @@ def test_a_run_on_its_own_stream_reads_its_own_checks(turned, monkeypatch):
         r.store(out[-1])
         torch.cuda.synchronize()
     assert torch.equal(out[0], out[1])
+
+
+def test_a_run_leaves_the_setting_of_others_alone(monkeypatch):
+    """A drop-in run takes its setting with it: batches and servers on other threads go on with the one they applied."""
+    import ctypes
+    import torch
+    from nixis_gb300 import _lib, autotune, erosion, mesh
+    monkeypatch.setattr(erosion, "BLOCKED_WORK", 1)
+    m = mesh.PlanetMesh(50)
+    h = torch.rand(m.n, dtype=torch.float64, generator=torch.Generator().manual_seed(4)).cuda()
+    was = autotune.current()
+    run = erosion.ErosionRun(m.xyz, m.nbr, iters=9).load(h)
+    try:
+        autotune.apply(autotune.TbConfig(16, 2, 256, 0))
+        assert run.blocked(9, erosion.RAIN)
+        assert _lib.lib().nx_erosion_npass(8) == 4
+    finally:
+        autotune.apply(was)
+    got = torch.empty_like(h)
+    run.store(got)
+    one = erosion.ErosionRun(m.xyz, m.nbr).load(h)
+    one.steps(9, rain=erosion.RAIN)
+    want = torch.empty_like(h)
+    one.store(want)
+    assert run.error() == 0 and torch.equal(got, want)
+    d = _lib.ErosionPlanet()
+    for rings, threads, variant in ((0, 256, 0), (9, 256, 0), (4, 384, 0), (4, 256, 7)):
+        with pytest.raises(_lib.NxError):
+            _lib.call("nx_erosion_run_as", None, ctypes.byref(d), 1, rings, threads, variant, None, None, None, 0, None)
