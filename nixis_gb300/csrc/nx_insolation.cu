@@ -97,9 +97,10 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e)
 }
 
 // A vertex in binary32 and whether it lies on the sphere of radius r
-// (| |v|^2 - r^2 | <= 1e-12 r^2): the difference in pairs, within 2^-44 r^2;
-// in binary64 for a radius or coordinate outside the pairs' range (a
-// coordinate of 0 among them).
+// (| |v|^2 - r^2 | <= 1e-12 r^2): the difference in pairs, within 2^-44 (6e-14)
+// of r^2; in binary64 where that does not decide (2e-13 about the bound), and
+// for a radius or coordinate outside the pairs' range (a coordinate of 0 among
+// them).
 __device__ __forceinline__ bool load_vertex(double X, double Y, double Z, double r, float r2h, float r2l, float &x,
                                             float &y, float &z)
 {
@@ -120,7 +121,8 @@ __device__ __forceinline__ bool load_vertex(double X, double Y, double Z, double
         x = signed_sum(xh, xl, hx);
         y = signed_sum(yh, yl, hy);
         z = signed_sum(zh, zl, hz);
-        return fabsf(__fadd_rn(__fsub_rn(s2, r2h), low)) <= 1e-12f * r2h;
+        const float over = fabsf(__fadd_rn(__fsub_rn(s2, r2h), low)) - 1e-12f * r2h;
+        if (fabsf(over) > 2e-13f * r2h) return over < 0.0f;
     }
     x = (float)X;
     y = (float)Y;

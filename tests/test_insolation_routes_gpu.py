@@ -90,3 +90,30 @@ def test_a_rotation_that_is_no_number_lights_nothing(where, bad):
     got = climate.insolation_sum(m.xyz, 1.0, rot, tilts)
     want = sum(climate.insolation_sum(m.xyz, 1.0, rot[q:q + 120], tilts) for q in (0, 120, 240))
     assert (got - want).abs().max() <= 2e-6 * want.max()
+
+
+@pytest.mark.parametrize("rotations", [24, 7, 360])
+def test_vertices_at_the_bound_of_the_sphere_test(rotations):
+    """| |v|^2 - r^2 | within 8e-14 r^2 of its bound of 1e-12 r^2: the formula is the one that binary64 picks, so a sum has
+    the bits of a vertex well inside the bound (the same binary32 coordinates) or of a radius well off (the same binary32
+    reciprocal)."""
+    import torch
+    from nixis_gb300 import climate
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    n, r = 200_000, 1.25
+    v = torch.randn(n, 3, dtype=torch.float64, device="cuda", generator=gen)
+    v = v / v.norm(dim=1, keepdim=True) * r
+    sign = torch.where(torch.arange(n, device="cuda") % 2 == 0, 1.0, -1.0).double()
+    off = sign * (1e-12 + (torch.rand(n, dtype=torch.float64, device="cuda", generator=gen) - 0.5) * 1.6e-13)
+    at, inside = v * (1 + off / 2)[:, None], v * (1 + 0.2 * off)[:, None]
+    # |at|^2 / r^2 - 1 as the kernel's binary64 forms it, but for two roundings (2e-16, left out below)
+    over = ((at[:, 0] * at[:, 0] + at[:, 1] * at[:, 1] + at[:, 2] * at[:, 2]) / (r * r) - 1).abs() - 1e-12
+    clear = (over.abs() > 2e-15) & (at.float() == inside.float()).all(1)
+    assert clear.float().mean() > 0.9
+    rot, tilts = [-180.0 + 360.0 / rotations * i for i in range(rotations)], [23.44, -11.0, 3.0]
+    got = climate.insolation_sum(at, r, rot, tilts)
+    on = climate.insolation_sum(inside, r, rot, tilts)
+    far = climate.insolation_sum(at, r * (1 + 1e-9), rot, tilts)
+    assert (on != far).float().mean() > 0.2
+    want = torch.where(over < 0, on, far)
+    assert torch.equal(got[clear], want[clear])
