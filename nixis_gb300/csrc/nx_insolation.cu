@@ -318,19 +318,25 @@ __device__ __forceinline__ Breaks stage_breakpoints(const InsoArgs &a, const flo
             }
             __syncthreads();
         }
-    // prefix sums of cos and of cos * tan: each thread a run of the days
+    auto tan_of = [&](int j) { return __uint_as_float(K[j].x); };
+    const float tmax = nf > 0 ? tan_of(nf - 1) : 0.0f;
+    // prefix sums of cos (2^-20 at least: exact in units of 2^-44) and of cos *
+    // tan, whose unit is 2^-53 of the power of two above the largest of them (so
+    // 512 of them stay below 2^63): each thread a run of the days
+    const int top = (int)(__float_as_uint(fminf(tmax, 1.0f)) >> 23) - 126, up = min(53 - top, 126);
+    const float in = __uint_as_float((uint32_t)(127 + up) << 23), out = __uint_as_float((uint32_t)(127 - up) << 23);
     const int per = (sp + (int)blockDim.x - 1) / (int)blockDim.x;
     const int j0 = min(nf, (int)threadIdx.x * per), j1 = min(nf, j0 + per);
     auto term = [&](int j, long long &u, long long &v) {
-        const float c = __uint_as_float(K[j].y), t = __uint_as_float(K[j].x), p = __fmul_rn(c, t);
+        const float c = __uint_as_float(K[j].y), t = tan_of(j), p = __fmul_rn(c, t);
         u += to_fixed(c);
-        v += to_fixed(p) + to_fixed(__fmaf_rn(c, t, -p));
+        v += __float2ll_rn(p * in) + __float2ll_rn(__fmaf_rn(c, t, -p) * in);
     };
     long long u = 0, v = 0, tu, tv;
     for (int j = j0; j < j1; ++j) term(j, u, v);
     block_scan2(u, v, tu, tv);
     for (int j = j0; j < j1; ++j) {
-        L[j] = make_float2(from_fixed(u), from_fixed(tv - v));
+        L[j] = make_float2(from_fixed(u), __ll2float_rn(tv - v) * out);
         term(j, u, v);
     }
     if (threadIdx.x == 0) L[nf] = make_float2(from_fixed(tu), 0.0f);
@@ -340,8 +346,6 @@ __device__ __forceinline__ Breaks stage_breakpoints(const InsoArgs &a, const flo
     bk.bucket = (uint32_t)__cvta_generic_to_shared(bucket) - (0x4B000000u << 4);
     bk.nf = nf;
     bk.nb = (float)nb;
-    auto tan_of = [&](int j) { return __uint_as_float(K[j].x); };
-    const float tmax = nf > 0 ? tan_of(nf - 1) : 0.0f;
     bk.inv = tmax > 0.0f ? 1.0f / tmax : 0.0f;
     auto below = [&](float t) {
         int c = 0;
