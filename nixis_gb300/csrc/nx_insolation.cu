@@ -400,14 +400,16 @@ __device__ __forceinline__ float pair_value(const Breaks &bk, float a, float c, 
 template <int HP, bool CROWDED>
 __device__ __forceinline__ float pair_sum(const Breaks &bk, float x, float y, float c, float ti)
 {
-    float s0 = 0.0f, s1 = 0.0f;
+    // (four short sums: with two of six each the roundings were as large as the
+    // values' own)
+    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
     for (int h = 0; h < HP; h += 2) {
         const float4 q = bk.rot[h / 2];
-        s0 += pair_value<CROWDED>(bk, fabsf(fmaf(x, q.x, -(y * q.y))), c, ti);
-        s1 += pair_value<CROWDED>(bk, fabsf(fmaf(x, q.z, -(y * q.w))), c, ti);
+        s[h % 4] += pair_value<CROWDED>(bk, fabsf(fmaf(x, q.x, -(y * q.y))), c, ti);
+        s[h % 4 + 1] += pair_value<CROWDED>(bk, fabsf(fmaf(x, q.z, -(y * q.w))), c, ti);
     }
-    return s0 + s1;
+    return (s[0] + s[1]) + (s[2] + s[3]);
 }
 
 // Arcs (HP = ARCS).  x cos(theta) - y sin(theta) = rho cos(theta + phi), phi

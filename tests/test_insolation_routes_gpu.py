@@ -138,3 +138,21 @@ def test_years_of_small_tilts_at_the_poles(axial):
     for tau in t:
         want += ((x[:, None] * r.cos() - y[:, None] * r.sin()) * tau.cos() + (z * tau.sin())[:, None]).clamp(min=0).sum(1)
     assert ((got - want).abs() <= 5e-7 * want).all()
+
+
+@pytest.mark.parametrize("axial, allowed", [(23.44, 5.27e-8), (1.0, 5.67e-8), (0.01, 4.94e-8)])
+def test_a_years_error_is_no_larger_than_of_sums_in_binary64(axial, allowed):
+    """Root mean square error over a sphere, against the one measured where the days' sums were kept in binary64 and
+    looked up by their counts (the form that the tables of lines replaced)."""
+    import torch
+    from nixis_gb300 import climate, mesh
+    xyz = mesh.icosphere(60, with_tris=False)[0]
+    rot, tilts = climate.annual_schedule(axial, 365, 365, 24)
+    got = climate.insolation_sum(xyz, 1.0, rot, tilts).double()
+    r, t = (torch.tensor(v, dtype=torch.float64, device="cuda") * (math.pi / 180) for v in (rot, tilts))
+    x, y, z = xyz.T
+    u = x[:, None] * r.cos() - y[:, None] * r.sin()
+    want = torch.zeros_like(got)
+    for tau in t:
+        want += (u * tau.cos() + (z * tau.sin())[:, None]).clamp(min=0).sum(1)
+    assert (got - want).norm() <= allowed * want.norm()
