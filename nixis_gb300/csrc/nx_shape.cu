@@ -47,23 +47,28 @@ constexpr int PER_THREAD = 8;
 constexpr int CHUNK = THREADS * PER_THREAD;   // elements per summary
 constexpr u64 NONE = ~0ull;
 
-// Ordered key of a binary64 (-0 taken as +0, as the reference's
-// comparisons see them equal; below NONE, which a NaN's would be).
+__device__ __forceinline__ u64 umin(u64 a, u64 b) { return a < b ? a : b; }
+
+// Ordered key of a binary64, from 0 for -infinity on: -0 taken as +0, as the
+// reference's comparisons see them equal; every NaN, whatever its sign, one
+// key above +infinity's (and below NONE).
+constexpr u64 KEY_FIRST = 0x000FFFFFFFFFFFFFull, KEY_NAN = 0xFFF0000000000001ull - KEY_FIRST;
+
 __device__ __forceinline__ u64 dkey(double v)
 {
     const u64 b = nxf::bits(v);
-    if (b == 0x8000000000000000ull) return b;
+    if (b == 0x8000000000000000ull) return b - KEY_FIRST;
     const u64 k = (b & 0x8000000000000000ull) ? ~b : (b | 0x8000000000000000ull);
-    return k == NONE ? NONE - 1 : k;
+    return umin(k - KEY_FIRST, KEY_NAN);
 }
 
-__device__ __forceinline__ double dunkey(u64 k)
+__device__ __forceinline__ double dunkey(u64 q)
 {
+    const u64 k = q + KEY_FIRST;
     const u64 b = (k & 0x8000000000000000ull) ? (k & ~0x8000000000000000ull) : ~k;
     return __longlong_as_double((long long)b);
 }
 
-__device__ __forceinline__ u64 umin(u64 a, u64 b) { return a < b ? a : b; }
 __device__ __forceinline__ u64 umax(u64 a, u64 b) { return a > b ? a : b; }
 __device__ __forceinline__ bool is_nan(double v) { return (nxf::bits(v) << 1) > 0xFFE0000000000000ull; }
 

@@ -54,3 +54,20 @@ def test_shaping_equals_the_oracle(kind, n):
             with np.errstate(all="ignore"):
                 want = O.power_rescale(x, m.astype(np.uint8), mode, power)
             assert ulps(util.power_rescale(x, m, mode, power), want) <= 4, (mode, power)
+
+
+def test_the_sign_of_a_nan_does_not_matter():
+    """A NaN of either sign is np.max's result and not np.min's, so what lies below `mid` keeps its values."""
+    from nixis_gb300 import util
+    x = np.random.default_rng(4).normal(size=5000)
+    x[17] = np.nan
+    y = x.copy()
+    y.view(np.uint64)[17] ^= np.uint64(1 << 63)
+    for args, nans in (({}, 5000), ({"mid": 0.25}, 1 + (x > 0.25).sum()), ({"mid": 0.25, "mode": "lower"}, 1),
+                       ({"mid": -0.25, "mode": "upper"}, 1 + (x > -0.25).sum())):
+        a, b = util.rescale(x, -1.0, 2.0, **args), util.rescale(y, -1.0, 2.0, **args)
+        assert np.array_equal(a, b, equal_nan=True) and np.isnan(a).sum() == nans
+    m = np.random.default_rng(5).random(5000) < 0.5
+    for mode in (0, 1):
+        assert np.array_equal(util.power_rescale(x, m, mode, 2.0), util.power_rescale(y, m, mode, 2.0), equal_nan=True)
+    assert np.array_equal(util.make_bool_elevation_mask(x, 0.1), util.make_bool_elevation_mask(y, 0.1))
