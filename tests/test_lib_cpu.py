@@ -132,3 +132,9 @@ def test_hexagonal_tiles_cover_each_face_point_once_and_are_all_used(rho):
         assert nm.value >= 3 * (rho + R) ** 2 + 3 * (rho + R) + 1 and cm.value % 4 == 0
     for bad in (-1, -65, 0, 1):
         assert L.nx_tiling_shape(100, bad, 4, ctypes.byref(nt), ctypes.byref(nm), ctypes.byref(cm)) != 0
+
+
+def test_settings_tuned_on_the_old_tile_tables_are_not_taken_over():
+    """The version is part of the tuner's key; 1.1.0 had the tables row by row."""
+    from nixis_gb300 import _lib
+    assert _lib.lib().nx_version() > 10100
