@@ -283,12 +283,11 @@ __device__ __forceinline__ void block_scan2(long long &u, long long &v, long lon
 __device__ __forceinline__ long long to_fixed(float v) { return __float2ll_rn(v * 0x1p44f); }
 __device__ __forceinline__ float from_fixed(long long v) { return __ll2float_rn(v) * 0x1p-44f; }
 
-// Breakpoint tables of a block (stage_breakpoints), or nf < 0 for none.
+// Breakpoint tables of a block (stage_breakpoints).
 struct Breaks {
     const float2 *L = nullptr;
     const float4 *rot = nullptr;   // the rotations, two to an entry
     uint32_t bucket = 0;       // shared address of the table less what a bucket number's binary32 exponent adds
-    int nf = -1;               // factored days
     float nb = 0.0f;           // buckets
     float inv = 0.0f;          // 1 / tmax
     bool crowded = false;      // some bucket holds distinct breakpoints
@@ -344,7 +343,6 @@ __device__ __forceinline__ Breaks stage_breakpoints(const InsoArgs &a, const flo
     Breaks bk;
     bk.L = L;
     bk.bucket = (uint32_t)__cvta_generic_to_shared(bucket) - (0x4B000000u << 4);
-    bk.nf = nf;
     bk.nb = (float)nb;
     bk.inv = tmax > 0.0f ? 1.0f / tmax : 0.0f;
     auto below = [&](float t) {
@@ -580,17 +578,18 @@ __device__ __forceinline__ float inso_vertex(const InsoArgs &a, double X, double
     if (HP == ARCS && on_sphere && arc.n > 0) return arc_sum(a, arc, x, y, z) * inv_r;
     float tot = 0.0f, comp = 0.0f;          // Kahan over tilts
     const int nr = HP > 0 ? HP : a.n_rot;
-    if (on_sphere && HP > 0 && (HP & 1) == 0 && (BREAKS || a.pairs)) {
+    if constexpr (HP > 0) {
+    if (on_sphere) {
         // u = A cos(theta) + B sin(theta) = k U(theta) with k = cos(tau) and
         // U = x cos(theta) - y sin(theta) the same for every day, so per day
         //   sum_h max(|C|, |u_h|) = |k| sum_h max(|C| / |k|, |U_h|)
         // (exact in real arithmetic): |U_h| is formed once per vertex and a
         // day costs a max and an add per rotation pair.  Days with |k| near 0
         // take the direct form.
-        float au[HP > 0 ? HP : 2];
-        if (!BREAKS && (!tt || bk.nf < 0)) {
+        float au[HP];
+        if (!BREAKS) {
 #pragma unroll
-            for (int h = 0; h < (HP > 0 ? HP : 2); ++h) {
+            for (int h = 0; h < HP; ++h) {
                 const float2 q = a.rot[h];
                 au[h] = fabsf(fmaf(x, q.x, -(y * q.y)));
             }
@@ -608,19 +607,18 @@ __device__ __forceinline__ float inso_vertex(const InsoArgs &a, double X, double
                 comp = (tk - tot) - yk;
                 tot = tk;
             };
-            if (BREAKS || bk.nf >= 0) {
+            if constexpr (BREAKS) {
                 // each pair's line pair from its bucket of t = a_h / |z|
                 // (|z| kept off 0: 1e-20 r in its place changes no value)
                 const float ti = approx_rcp(fmaxf(az, zmin)) * bk.inv;
-                tot = (bk.crowded ? pair_sum<(HP > 0 ? HP : 2), true>(bk, x, y, az, ti)
-                                  : pair_sum<(HP > 0 ? HP : 2), false>(bk, x, y, az, ti));
+                tot = bk.crowded ? pair_sum<HP, true>(bk, x, y, az, ti) : pair_sum<HP, false>(bk, x, y, az, ti);
             } else {
             auto day = [&](int d, float2 g) {
                 const float4 k = tt[d];
                 const float c = az * k.y;
                 float2 acc = make_float2(fmaxf(c, au[0]), fmaxf(c, au[1]));
 #pragma unroll
-                for (int h = 2; h < (HP > 0 ? HP : 2); h += 2)
+                for (int h = 2; h < HP; h += 2)
                     acc = __fadd2_rn(acc, make_float2(fmaxf(c, au[h]), fmaxf(c, au[h + 1])));
                 return __ffma2_rn(make_float2(k.x, k.x), acc, g);
             };
@@ -645,7 +643,7 @@ __device__ __forceinline__ float inso_vertex(const InsoArgs &a, double X, double
                 const float A = x * t.x, B = -(y * t.x), C = z * t.y, aC = fabsf(C);
                 float s = 0.0f;
 #pragma unroll
-                for (int h = 0; h < (HP > 0 ? HP : 2); ++h) {
+                for (int h = 0; h < HP; ++h) {
                     const float2 q = a.rot[h];
                     s += fmaxf(aC, fabsf(fmaf(A, q.x, B * q.y)));
                 }
@@ -662,14 +660,14 @@ __device__ __forceinline__ float inso_vertex(const InsoArgs &a, double X, double
                 const float c = __fdividef(aC, ak);
                 float2 acc = make_float2(0.0f, 0.0f);
 #pragma unroll
-                for (int h = 0; h < (HP > 0 ? HP : 2); h += 2)
+                for (int h = 0; h < HP; h += 2)
                     acc = __fadd2_rn(acc, make_float2(fmaxf(c, au[h]), fmaxf(c, au[h + 1])));
                 s = fmaf(ak, acc.x + acc.y, (float)HP * C);
             } else {
                 const float A = x * t.x, B = -(y * t.x);
                 s = 0.0f;
 #pragma unroll
-                for (int h = 0; h < (HP > 0 ? HP : 2); ++h) {
+                for (int h = 0; h < HP; ++h) {
                     const float2 q = a.rot[h];
                     s += fmaxf(aC, fabsf(fmaf(A, q.x, B * q.y)));
                 }
@@ -682,30 +680,17 @@ __device__ __forceinline__ float inso_vertex(const InsoArgs &a, double X, double
         }
         return tot * inv_r;
     }
-    if (on_sphere) {
-        float2 rt[HP > 0 ? HP : 1];
-        if (HP > 0) {
-#pragma unroll
-            for (int h = 0; h < (HP > 0 ? HP : 1); ++h) rt[h] = a.rot[h];
-        }
+    } else if (on_sphere) {
         for (int d = 0; d < a.n_tilt; ++d) {
             const float2 t = a.tilt[d];
             const float A = x * t.x, B = -(y * t.x), C = z * t.y;
             float s = 0.0f;
             if (a.pairs) {
                 const float aC = fabsf(C);
-                if (HP > 0) {
-#pragma unroll
-                    for (int h = 0; h < (HP > 0 ? HP : 1); ++h) {
-                        float u = fmaf(A, rt[h].x, B * rt[h].y);
-                        s += fmaxf(aC, fabsf(u));
-                    }
-                } else {
-                    for (int h = 0; h < nr; ++h) {
-                        float2 q = a.rot[h];
-                        float u = fmaf(A, q.x, B * q.y);
-                        s += fmaxf(aC, fabsf(u));
-                    }
+                for (int h = 0; h < nr; ++h) {
+                    float2 q = a.rot[h];
+                    float u = fmaf(A, q.x, B * q.y);
+                    s += fmaxf(aC, fabsf(u));
                 }
                 s = fmaf((float)nr, C, s);
             } else {
@@ -741,16 +726,12 @@ __device__ __forceinline__ float inso_vertex(const InsoArgs &a, double X, double
 template <int HP>
 __device__ __forceinline__ Breaks stage_all(const InsoArgs &a, float4 *s_tilt)
 {
-    Breaks bk;
     stage_tilts<HP>(a, s_tilt);
-    if (a.n_tilt <= SORT_MAX) {
-        // 16-byte units: the bucket table first, then the lines, then the rest
-        float4 *bucket = s_tilt + a.n_tilt + 1 + (a.n_tilt + 3) / 4;
-        float2 *L = reinterpret_cast<float2 *>(bucket + bucket_count(a.n_tilt) + 1);
-        uint2 *K = reinterpret_cast<uint2 *>(L + a.n_tilt + 1);
-        bk = stage_breakpoints(a, s_tilt, K, L, bucket);
-    }
-    return bk;
+    // 16-byte units: the bucket table first, then the lines, then the rest
+    float4 *bucket = s_tilt + a.n_tilt + 1 + (a.n_tilt + 3) / 4;
+    float2 *L = reinterpret_cast<float2 *>(bucket + bucket_count(a.n_tilt) + 1);
+    uint2 *K = reinterpret_cast<uint2 *>(L + a.n_tilt + 1);
+    return stage_breakpoints(a, s_tilt, K, L, bucket);
 }
 
 // Threads of a block: two of 512 per SM for the breakpoints' tables (half as
@@ -770,11 +751,12 @@ template <int HP, bool BREAKS>
 __device__ __forceinline__ void insolation_body(const InsoArgs &a)
 {
     extern __shared__ float4 s_tilt[];
-    const bool staged = BREAKS || (HP > 0 && a.pairs && a.n_tilt <= TILT_STAGE_MAX);
+    const bool staged = BREAKS || (HP > 0 && a.n_tilt <= TILT_STAGE_MAX);
     Breaks bk;
     Arcs arc;
-    if (staged) bk = stage_all<HP>(a, s_tilt);
-    if (HP == ARCS) arc = stage_arcs(a, s_tilt);
+    if constexpr (BREAKS) bk = stage_all<HP>(a, s_tilt);
+    else if (HP > 0 && staged) stage_tilts<HP>(a, s_tilt);
+    if constexpr (HP == ARCS) arc = stage_arcs(a, s_tilt);
     // the next vertex is read while this one is summed (32 warps' 768 bytes
     // each are too few in flight per SM for the memory's latency)
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
@@ -823,11 +805,12 @@ __global__ void __launch_bounds__(256, BREAKS ? 4 : 3) insolation_batch_kernel(I
                                                                int64_t total_rows)
 {
     extern __shared__ float4 s_tilt[];
-    const bool staged = BREAKS || (HP > 0 && a.pairs && a.n_tilt <= TILT_STAGE_MAX);
+    const bool staged = BREAKS || (HP > 0 && a.n_tilt <= TILT_STAGE_MAX);
     Breaks bk;
     Arcs arc;
-    if (staged) bk = stage_all<HP>(a, s_tilt);
-    if (HP == ARCS) arc = stage_arcs(a, s_tilt);
+    if constexpr (BREAKS) bk = stage_all<HP>(a, s_tilt);
+    else if (HP > 0 && staged) stage_tilts<HP>(a, s_tilt);
+    if constexpr (HP == ARCS) arc = stage_arcs(a, s_tilt);
     // rows only go up: walk to the next planet, and form a planet's radius
     // constants (binary64) once
     int p = -1;
@@ -998,12 +981,13 @@ int grid_for(int64_t n, int per_sm = 8)
     return (int)(g < 1 ? 1 : g);
 }
 
-// Blocks of a 12-pair launch: a block that sums by breakpoints sorts the
-// schedule first, so the grid is the resident blocks (4 per SM) and each
-// block takes many vertices.
-// Whether a schedule is summed by breakpoints.
+// Whether a schedule is summed by breakpoints (short ones as kernel arguments
+// always are: 12 pairs leave room for 484 days).
+static_assert(ARG_POSITIONS - 12 <= SORT_MAX, "no args kernel for longer schedules of 12 pairs");
 bool breaks(const InsoArgs &a) { return a.pairs && a.n_rot == 12 && a.n_tilt <= SORT_MAX; }
 
+// A block that sums by breakpoints sorts the schedule first, so the grid is the
+// resident blocks and each takes many vertices.
 int grid_breaks(int64_t n)
 {
     const int64_t g = (n + BREAK_THREADS - 1) / BREAK_THREADS, cap = (int64_t)nx::sm_count() * BREAK_BLOCKS;
@@ -1095,8 +1079,6 @@ static int insolation_sums(const double *xyz_dev, int64_t n, double radius, cons
         memcpy(T.t, table_host, sizeof(float2) * (size_t)(n_rot_entries + n_tilt));
         if (breaks(a))
             insolation_args_kernel<12, true><<<grid_breaks(n), BREAK_THREADS, tilt_smem(a), s>>>(a, T);
-        else if (a.pairs && n_rot_entries == 12)
-            insolation_args_kernel<12><<<grid_for(n), 256, tilt_smem(a), s>>>(a, T);
         else if (use_arcs(a, n))
             insolation_args_kernel<ARCS><<<grid_arcs(n), arc_threads(n), arcs, s>>>(a, T);
         else

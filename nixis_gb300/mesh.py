@@ -198,8 +198,7 @@ class MeshTiling:
         dev = "cuda"
         self.counts = torch.zeros(self.ntiles * (rings + 1), dtype=torch.int32, device=dev)
         self.ids = torch.empty(self.ntiles * self.nmax, dtype=torch.int32, device=dev)
-        # (+8: the shared-table kernel copies whole 16-byte units past a tile's last row)
-        self.lnbr = torch.empty(self.ntiles * self.cmax * 6 + 8, dtype=torch.int16, device=dev)
+        self.lnbr = torch.empty(self.ntiles * self.cmax * 6, dtype=torch.int16, device=dev)
         self.ledge = torch.empty(self.ntiles * self.cmax * 12, dtype=torch.float32, device=dev)
         err = torch.zeros(3, dtype=torch.int32, device=dev)
         call("nx_tiling_build", mesh.k, tile_side, rings, _dev.ptr(mesh.nbr), _dev.ptr(mesh.edge), _dev.ptr(self.counts),
