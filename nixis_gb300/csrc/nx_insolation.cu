@@ -97,15 +97,17 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e)
 }
 
 // A vertex in binary32 and whether it lies on the sphere of radius r
-// (| |v|^2 - r^2 | <= 1e-12 r^2): the difference in pairs, within 2^-44 (6e-14)
-// of r^2; in binary64 where that does not decide (2e-13 about the bound), and
-// for a radius or coordinate outside the pairs' range (a coordinate of 0 among
-// them).
+// (| |v|^2 - r^2 | <= 1e-12 r^2): yes where the difference in pairs, within
+// 2^-44 (6e-14) of r^2, is below 8e-13 r^2; otherwise, and for a radius or
+// coordinate outside the pairs' range (a coordinate of 0 among them), as
+// binary64 has it.  JOIN: for sums over a schedule's positions one by one.
+template <bool JOIN>
 __device__ __forceinline__ bool load_vertex(double X, double Y, double Z, double r, float r2h, float r2l, float &x,
                                             float &y, float &z)
 {
     const uint32_t hx = (uint32_t)__double2hiint(X), hy = (uint32_t)__double2hiint(Y), hz = (uint32_t)__double2hiint(Z);
     const uint32_t ax = hx & 0x7FFFFFFFu, ay = hy & 0x7FFFFFFFu, az = hz & 0x7FFFFFFFu;
+    bool on = false;
     if (min(ax, min(ay, az)) >= (983u << 20) && max(ax, max(ay, az)) < (1084u << 20) && r2h > 0.0f) {
         float xh, xl, yh, yl, zh, zl;
         split_abs(ax, (uint32_t)__double2loint(X), xh, xl);
@@ -121,14 +123,24 @@ __device__ __forceinline__ bool load_vertex(double X, double Y, double Z, double
         x = signed_sum(xh, xl, hx);
         y = signed_sum(yh, yl, hy);
         z = signed_sum(zh, zl, hz);
-        const float over = fabsf(__fadd_rn(__fsub_rn(s2, r2h), low)) - 1e-12f * r2h;
-        if (fabsf(over) > 2e-13f * r2h) return over < 0.0f;
+        on = fabsf(__fadd_rn(__fsub_rn(s2, r2h), low)) <= 8e-13f * r2h;
     }
-    x = (float)X;
-    y = (float)Y;
-    z = (float)Z;
-    const double rho2 = X * X + Y * Y + Z * Z, r2 = r * r;
-    return fabs(rho2 - r2) <= 1e-12 * r2;
+    if (!on) {
+        x = (float)X;
+        y = (float)Y;
+        z = (float)Z;
+        const double rho2 = X * X + Y * Y + Z * Z, r2 = r * r;
+        on = fabs(rho2 - r2) <= 1e-12 * r2;
+    }
+    if (JOIN) {
+        // one way out, which the compiler does not see behind: with two it made
+        // the loops over a schedule twice, with half the loads in flight (2,500
+        // days of 9,002 vertices 605 us instead of 321)
+        int o = on;
+        asm volatile("" : "+f"(x), "+f"(y), "+f"(z), "+r"(o));
+        return o != 0;
+    }
+    return on;
 }
 
 // climate.py:419-442 for a vertex off the sphere of radius r (binary32).
@@ -400,12 +412,14 @@ __device__ __forceinline__ float pair_sum(const Breaks &bk, float x, float y, fl
 {
     // (four short sums: with two of six each the roundings were as large as the
     // values' own)
-    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float s[4];
 #pragma unroll
     for (int h = 0; h < HP; h += 2) {
         const float4 q = bk.rot[h / 2];
-        s[h % 4] += pair_value<CROWDED>(bk, fabsf(fmaf(x, q.x, -(y * q.y))), c, ti);
-        s[h % 4 + 1] += pair_value<CROWDED>(bk, fabsf(fmaf(x, q.z, -(y * q.w))), c, ti);
+        const float u = pair_value<CROWDED>(bk, fabsf(fmaf(x, q.x, -(y * q.y))), c, ti);
+        const float v = pair_value<CROWDED>(bk, fabsf(fmaf(x, q.z, -(y * q.w))), c, ti);
+        s[h % 4] = h < 4 ? u : s[h % 4] + u;
+        s[h % 4 + 1] = h < 4 ? v : s[h % 4 + 1] + v;
     }
     return (s[0] + s[1]) + (s[2] + s[3]);
 }
@@ -574,7 +588,7 @@ __device__ __forceinline__ float inso_vertex(const InsoArgs &a, double X, double
                                              const Breaks &bk = Breaks(), const Arcs &arc = Arcs())
 {
     float x, y, z;
-    const bool on_sphere = load_vertex(X, Y, Z, r, r2h, r2l, x, y, z);
+    const bool on_sphere = load_vertex<!BREAKS && HP != ARCS>(X, Y, Z, r, r2h, r2l, x, y, z);
     if (HP == ARCS && on_sphere && arc.n > 0) return arc_sum(a, arc, x, y, z) * inv_r;
     float tot = 0.0f, comp = 0.0f;          // Kahan over tilts
     const int nr = HP > 0 ? HP : a.n_rot;
@@ -747,7 +761,7 @@ constexpr int BREAK_THREADS = 512, BREAK_BLOCKS = 2;
 template <bool BREAKS, int HP>
 constexpr int INSO_THREADS = BREAKS ? BREAK_THREADS : (HP == ARCS ? 1024 : 256);
 
-template <int HP, bool BREAKS>
+template <int HP, bool BREAKS, bool AHEAD>
 __device__ __forceinline__ void insolation_body(const InsoArgs &a)
 {
     extern __shared__ float4 s_tilt[];
@@ -757,16 +771,20 @@ __device__ __forceinline__ void insolation_body(const InsoArgs &a)
     if constexpr (BREAKS) bk = stage_all<HP>(a, s_tilt);
     else if (HP > 0 && staged) stage_tilts<HP>(a, s_tilt);
     if constexpr (HP == ARCS) arc = stage_arcs(a, s_tilt);
-    // the next vertex is read while this one is summed (32 warps' 768 bytes
-    // each are too few in flight per SM for the memory's latency)
+    // AHEAD: the next vertex is read while this one is summed (32 warps' 768
+    // bytes each are too few in flight per SM for the memory's latency: one
+    // position on 10,000,002 vertices 74 -> 62 us); sums over more positions
+    // than a launch's arguments hold are better off with the registers (2,500
+    // days of 2,500,002 vertices 9.36 -> 8.98 ms)
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     double X = 0.0, Y = 0.0, Z = 0.0;
-    if (i < a.n) { X = a.xyz[3 * i]; Y = a.xyz[3 * i + 1]; Z = a.xyz[3 * i + 2]; }
+    if (AHEAD && i < a.n) { X = a.xyz[3 * i]; Y = a.xyz[3 * i + 1]; Z = a.xyz[3 * i + 2]; }
     for (; i < a.n; i += step) {
+        if (!AHEAD) { X = a.xyz[3 * i]; Y = a.xyz[3 * i + 1]; Z = a.xyz[3 * i + 2]; }
         const double cx = X, cy = Y, cz = Z;
         const int64_t j = i + step;
-        if (j < a.n) { X = a.xyz[3 * j]; Y = a.xyz[3 * j + 1]; Z = a.xyz[3 * j + 2]; }
+        if (AHEAD && j < a.n) { X = a.xyz[3 * j]; Y = a.xyz[3 * j + 1]; Z = a.xyz[3 * j + 2]; }
         const float tot = inso_vertex<HP, BREAKS>(a, cx, cy, cz, a.r, a.r2h, a.r2l, a.zmin, a.inv_r, staged ? s_tilt : nullptr,
                                           bk, arc);
         // the scale here instead of in a pass of its own over the sums (11 us
@@ -779,7 +797,7 @@ __device__ __forceinline__ void insolation_body(const InsoArgs &a)
 template <int HP, bool BREAKS = false>
 __global__ void __launch_bounds__(INSO_THREADS<BREAKS, HP>, BREAKS ? BREAK_BLOCKS : (HP == ARCS ? 1 : (HP == 12 ? 3 : 4))) insolation_kernel(InsoArgs a)
 {
-    insolation_body<HP, BREAKS>(a);
+    insolation_body<HP, BREAKS, BREAKS || HP == ARCS>(a);
 }
 
 // A short schedule's table as a kernel argument (a table of its own on the
@@ -795,7 +813,7 @@ __global__ void __launch_bounds__(INSO_THREADS<BREAKS, HP>, BREAKS ? BREAK_BLOCK
 {
     a.rot = table.t;
     a.tilt = table.t + a.n_rot;
-    insolation_body<HP, BREAKS>(a);
+    insolation_body<HP, BREAKS, true>(a);
 }
 
 // Many planets: planet p's vertices fill packed rows [vbeg, vbeg + n)

@@ -156,3 +156,20 @@ def test_a_years_error_is_no_larger_than_of_sums_in_binary64(axial, allowed):
     for tau in t:
         want += (u * tau.cos() + (z * tau.sin())[:, None]).clamp(min=0).sum(1)
     assert (got - want).norm() <= allowed * want.norm()
+
+
+@pytest.mark.parametrize("rotations, days", [(24, 2048), (24, 2049), (7, 700), (100, 90)])
+def test_long_schedules_day_by_day(rotations, days):
+    """Past the breakpoints' 512 days, past the 2,048 staged ones, and by single rotations, vertices on the sphere and off."""
+    import torch
+    from nixis_gb300 import climate, mesh
+    xyz = mesh.icosphere(9, with_tris=False)[0]
+    rot, tilts = climate.annual_schedule(23.44, days, days, rotations)
+    r, t = (torch.tensor(v, dtype=torch.float64, device="cuda") * (math.pi / 180) for v in (rot, tilts))
+    x, y, z = xyz.T
+    want = torch.zeros(xyz.shape[0], dtype=torch.float64, device="cuda")
+    for tau in t:
+        want += ((x[:, None] * r.cos() - y[:, None] * r.sin()) * tau.cos() + (z * tau.sin())[:, None]).clamp(min=0).sum(1)
+    assert (climate.insolation_sum(xyz, 1.0, rot, tilts).double() - want).abs().max() <= 2e-6 * want.max()
+    off = climate.insolation_sum(xyz, 1.0 + 1e-9, rot, tilts).double()
+    assert (off - want).abs().max() <= 1e-5 * want.max()
