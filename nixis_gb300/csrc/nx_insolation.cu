@@ -438,12 +438,17 @@ __device__ __forceinline__ float pair_sum(const Breaks &bk, float x, float y, fl
 // Measured (GB300, one tilt, 360 rotations): 110.8 -> 35 us for 2,500,002
 // vertices, 420 -> 100 us for 10,000,002 (2.8 TB/s of the 28 B per vertex;
 // instruction issue and the two gathers bound it; see INSO_THREADS).
-// From ARC_MIN rotations on, and only for ARC_VERTICES vertices or
-// ARC_TERMS positions: below 128 rotations the maxima are as fast or faster
-// (30 tilts of 48 rotations, 625,002 vertices: 113 us against 131 us by
-// arcs; of 96: 205 against 131 us, but 22.6 against 35 us for 9,002
-// vertices), and on a small sphere a block's sorting and prefix sums show
-// (128 rotations, 9,002 vertices: 6.3 against 8.3 us; 625,002: 14.5 us both).
+// From ARC_MIN rotations on, for ARC_VERTICES vertices or ARC_TERMS positions:
+// a sum by arcs has a few roundings whatever its rotations (5e-8 of the norm
+// for one-degree days, 5e-7 by maxima), and its time hardly depends on them,
+// but a block's sorting and prefix sums take ~5 us.  By arcs / by maxima, us
+// (GB300, 9,002, 256,002, 625,002 and 2,500,002 vertices): 128 rotations 7.0 /
+// 2.8, 11.5 / 6.4, 14.9 / 11.1, 31.1 / 36.2; 360 8.0 / 3.7, 12.1 / 10.3, 15.6 /
+// 21.3, 31.8 / 75.9; 700 12.4 / 21.8, 16.4 / 48.7, 19.5 / 104, 35.8 / 372; of 48
+// rotations, 30 tilts, 20.3 / 9.5, 43.3 / 37.8, 88.2 / 87.9, 249 / 331.  So large
+// spheres and long days gain time by arcs, a one-degree day on a small one
+// pays 4 us for the smaller error, and fewer rotations than ARC_MIN have
+// little error to lose.
 constexpr int ARCS = -1;
 constexpr int ARC_MIN = 128;
 constexpr int64_t ARC_VERTICES = 1 << 18;

@@ -1437,10 +1437,7 @@ __device__ __forceinline__ OctP oct_of(const nx_fbm_planet &P, int o)
     return O;
 }
 
-// The sum over P's octaves at vertex i, added to (rh, rl).  SPLIT: the block
-// evaluates one step's PAIR_THREADS / S vertices from `first` on; the sum is
-// valid in threads below PAIR_THREADS / S (vertex first + thread), the octaves
-// summed there in order, so the bits do not depend on S.
+// The sum over P's octaves at one vertex, added to (rh, rl).
 template <typename P_t>
 __device__ __forceinline__ void sum_octaves(const P_t &P, int n_oct, const Triples &t, bool pow2, uint32_t lb,
                                             unsigned &nfb, float &rh, float &rl)
@@ -1453,6 +1450,9 @@ __device__ __forceinline__ void sum_octaves(const P_t &P, int n_oct, const Tripl
     }
 }
 
+// The same by a whole block for one step's PAIR_THREADS / S vertices from
+// `first` on: the sum is valid in threads below PAIR_THREADS / S (vertex first +
+// thread), the octaves summed there in order, so the bits do not depend on S.
 template <typename P_t>
 __device__ __forceinline__ void sum_split(const P_t &P, int n_oct, const double *__restrict__ xyz, int64_t first,
                                           int64_t last, int S, bool pow2, uint32_t lb, float2 *part, unsigned &nfb,
@@ -1553,8 +1553,8 @@ struct FbmPairParams {
 };
 
 // One planet, the pair path: the octaves of P (any subset of a planet's
-// octaves: the plain path launches one per octave, accumulate = 1 after
-// the first) added to the running pair sums in out2 (float2 per vertex),
+// octaves: the plain path launches NX_MAX_OCTAVES at a time, accumulate = 1
+// after the first) added to the running pair sums in out2 (float2 per vertex),
 // and/or written as binary64 (out64, = hi + lo exactly; accumulate adds to
 // it).  minmax (optional): ordered keys of the resulting pair sums.
 //

@@ -24,12 +24,18 @@ CAPACITY = 0.2 / 320        # erosion.py:207
 
 # A run over an icosphere's own neighbour table takes the temporally blocked
 # passes from this many vertex-iterations on, and from BLOCKED_ITERS
-# iterations (ErosionRun.blocked).  They save ~14 us per million
-# vertex-iterations and cost the tiling (53 us per million vertices) and
-# ~300 us of host work.  Measured (GB300, erode_terrain3 one iteration at a
-# time against blocked, us): 10,000,002 vertices x 4 iterations 2721 / 2731,
-# x 8 3929 / 3172, x 50 16648 / 9895; 2,500,002 x 8 1216 / 1207, x 16
-# 1881 / 1546; 625,002 x 25 842 / 973, x 50 1359 / 1347; 100,002 x 50 623 / 882.
+# iterations (ErosionRun.blocked).  They cost the tiling and ~300 us of host
+# work, and save 16 us per million vertex-iterations where the state and the
+# tables are larger than L2 (from ~800,000 vertices on), 2-6 below.  The line
+# is where they pay at every size.  Measured (GB300, erode_terrain3 one
+# iteration at a time against blocked, us), at it: 36,002 vertices x 1,000
+# 6,420 / 4,733; 100,002 x 336 2,840 / 2,490; 225,002 x 150 1,787 / 1,480;
+# 256,002 x 132 1,667 / 1,644; 400,002 x 84 1,466 / 1,417; 625,002 x 54 1,391 /
+# 1,330; 1,024,002 x 33 1,613 / 1,308; 6,400,002 x 6 2,101 / 1,840; 10,000,002 x
+# 5 2,940 / 2,444; below it: 256,002 x 50 765 / 983, 400,002 x 50 973 / 1,058,
+# 1,024,002 x 16 924 / 941, 2,500,002 x 5 939 / 1,006 (from 1,000,000 vertices on
+# they would pay from 2e7 on: 1,600,002 x 12 1,049 / 1,023, 2,500,002 x 8 1,152 /
+# 1,102, 6,400,002 x 3 1,581 / 1,547).
 # A pass rescales its planet before its iterations, not between them, for a
 # growth below 16 per iteration: water grows by up to 2 + 6 d, so edges
 # longer than BLOCKED_EDGE (a sphere in metres) go one iteration at a time.
