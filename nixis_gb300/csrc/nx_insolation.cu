@@ -412,16 +412,16 @@ __device__ __forceinline__ float pair_sum(const Breaks &bk, float x, float y, fl
 {
     // (four short sums: with two of six each the roundings were as large as the
     // values' own)
-    float s[4];
+    float2 s[2];
 #pragma unroll
     for (int h = 0; h < HP; h += 2) {
         const float4 q = bk.rot[h / 2];
-        const float u = pair_value<CROWDED>(bk, fabsf(fmaf(x, q.x, -(y * q.y))), c, ti);
-        const float v = pair_value<CROWDED>(bk, fabsf(fmaf(x, q.z, -(y * q.w))), c, ti);
-        s[h % 4] = h < 4 ? u : s[h % 4] + u;
-        s[h % 4 + 1] = h < 4 ? v : s[h % 4 + 1] + v;
+        const float2 u = make_float2(pair_value<CROWDED>(bk, fabsf(fmaf(x, q.x, -(y * q.y))), c, ti),
+                                     pair_value<CROWDED>(bk, fabsf(fmaf(x, q.z, -(y * q.w))), c, ti));
+        s[h / 2 % 2] = h < 4 ? u : __fadd2_rn(s[h / 2 % 2], u);
     }
-    return (s[0] + s[1]) + (s[2] + s[3]);
+    const float2 t = __fadd2_rn(s[0], s[1]);
+    return t.x + t.y;
 }
 
 // Arcs (HP = ARCS).  x cos(theta) - y sin(theta) = rho cos(theta + phi), phi
@@ -594,7 +594,7 @@ __device__ __forceinline__ float inso_vertex(const InsoArgs &a, double X, double
 {
     float x, y, z;
     const bool on_sphere = load_vertex<!BREAKS && HP != ARCS>(X, Y, Z, r, r2h, r2l, x, y, z);
-    if (HP == ARCS && on_sphere && arc.n > 0) return arc_sum(a, arc, x, y, z) * inv_r;
+    if (HP == ARCS && on_sphere) return arc_sum(a, arc, x, y, z) * inv_r;
     float tot = 0.0f, comp = 0.0f;          // Kahan over tilts
     const int nr = HP > 0 ? HP : a.n_rot;
     if constexpr (HP > 0) {
@@ -783,6 +783,17 @@ __device__ __forceinline__ void insolation_body(const InsoArgs &a)
     // days of 2,500,002 vertices 9.36 -> 8.98 ms)
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    // the scale here instead of in a pass of its own over the sums (11 us for
+    // 10 M vertices)
+    auto put = [&](int64_t at, float sum) {
+        const float v = __fmul_rn(sum, a.scale);
+        a.out[at] = a.accumulate ? a.out[at] + v : v;
+    };
+    if (HP == ARCS && arc.n == 0) {
+        for (; i < a.n; i += step)
+            put(i, inso_vertex<0, false>(a, a.xyz[3 * i], a.xyz[3 * i + 1], a.xyz[3 * i + 2], a.r, a.r2h, a.r2l, a.zmin, a.inv_r));
+        return;
+    }
     double X = 0.0, Y = 0.0, Z = 0.0;
     if (AHEAD && i < a.n) { X = a.xyz[3 * i]; Y = a.xyz[3 * i + 1]; Z = a.xyz[3 * i + 2]; }
     for (; i < a.n; i += step) {
@@ -790,12 +801,7 @@ __device__ __forceinline__ void insolation_body(const InsoArgs &a)
         const double cx = X, cy = Y, cz = Z;
         const int64_t j = i + step;
         if (AHEAD && j < a.n) { X = a.xyz[3 * j]; Y = a.xyz[3 * j + 1]; Z = a.xyz[3 * j + 2]; }
-        const float tot = inso_vertex<HP, BREAKS>(a, cx, cy, cz, a.r, a.r2h, a.r2l, a.zmin, a.inv_r, staged ? s_tilt : nullptr,
-                                          bk, arc);
-        // the scale here instead of in a pass of its own over the sums (11 us
-        // for 10 M vertices)
-        const float v = __fmul_rn(tot, a.scale);
-        a.out[i] = a.accumulate ? a.out[i] + v : v;
+        put(i, inso_vertex<HP, BREAKS>(a, cx, cy, cz, a.r, a.r2h, a.r2l, a.zmin, a.inv_r, staged ? s_tilt : nullptr, bk, arc));
     }
 }
 
@@ -824,7 +830,7 @@ __global__ void __launch_bounds__(INSO_THREADS<BREAKS, HP>, BREAKS ? BREAK_BLOCK
 // Many planets: planet p's vertices fill packed rows [vbeg, vbeg + n)
 // (vbeg a multiple of 256); one block covers 256 rows of one planet.
 template <int HP, bool BREAKS = false>
-__global__ void __launch_bounds__(256, BREAKS ? 4 : 3) insolation_batch_kernel(InsoArgs a, const nx_inso_planet *__restrict__ P, int np,
+__global__ void __launch_bounds__(256, HP == 12 && !BREAKS ? 3 : 4) insolation_batch_kernel(InsoArgs a, const nx_inso_planet *__restrict__ P, int np,
                                                                int64_t total_rows)
 {
     extern __shared__ float4 s_tilt[];
@@ -834,30 +840,39 @@ __global__ void __launch_bounds__(256, BREAKS ? 4 : 3) insolation_batch_kernel(I
     if constexpr (BREAKS) bk = stage_all<HP>(a, s_tilt);
     else if (HP > 0 && staged) stage_tilts<HP>(a, s_tilt);
     if constexpr (HP == ARCS) arc = stage_arcs(a, s_tilt);
-    // rows only go up: walk to the next planet, and form a planet's radius
-    // constants (binary64) once
-    int p = -1;
-    int64_t beg = 0, next = 0;
-    double r = 1.0;
-    float r2h = 0.0f, r2l = 0.0f, zmin = 0.0f, inv_r = 1.0f;
-    for (int64_t blk = blockIdx.x; blk * 256 < total_rows; blk += gridDim.x) {
-        if (p < 0 || blk * 256 >= next) {
-            do {
-                ++p;
-                next = p + 1 < np ? P[p + 1].vbeg : INT64_MAX;
-            } while (blk * 256 >= next);
-            beg = P[p].vbeg;
-            r = P[p].radius;
-            radius_pair(r, r2h, r2l);
-            inv_r = (float)(1.0 / r);
-            zmin = (float)(1e-20 * r);
+    auto rows = [&](auto vertex) {
+        // rows only go up: walk to the next planet, and form a planet's radius
+        // constants (binary64) once
+        int p = -1;
+        int64_t beg = 0, next = 0;
+        double r = 1.0;
+        float r2h = 0.0f, r2l = 0.0f, zmin = 0.0f, inv_r = 1.0f;
+        for (int64_t blk = blockIdx.x; blk * 256 < total_rows; blk += gridDim.x) {
+            if (p < 0 || blk * 256 >= next) {
+                do {
+                    ++p;
+                    next = p + 1 < np ? P[p + 1].vbeg : INT64_MAX;
+                } while (blk * 256 >= next);
+                beg = P[p].vbeg;
+                r = P[p].radius;
+                radius_pair(r, r2h, r2l);
+                inv_r = (float)(1.0 / r);
+                zmin = (float)(1e-20 * r);
+            }
+            const int64_t i = blk * 256 + threadIdx.x - beg;
+            if (i < 0 || i >= P[p].n) continue;
+            const double *v = P[p].xyz + 3 * i;
+            a.out[beg + i] = vertex(v[0], v[1], v[2], r, r2h, r2l, zmin, inv_r);
         }
-        const int64_t i = blk * 256 + threadIdx.x - beg;
-        if (i < 0 || i >= P[p].n) continue;
-        const double *xyz = P[p].xyz;
-        a.out[beg + i] = inso_vertex<HP, BREAKS>(a, xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], r, r2h, r2l, zmin, inv_r,
-                                         staged ? s_tilt : nullptr, bk, arc);
-    }
+    };
+    if (HP == ARCS && arc.n == 0)
+        rows([&](double x, double y, double z, double r, float r2h, float r2l, float zmin, float inv_r) {
+            return inso_vertex<0, false>(a, x, y, z, r, r2h, r2l, zmin, inv_r);
+        });
+    else
+        rows([&](double x, double y, double z, double r, float r2h, float r2l, float zmin, float inv_r) {
+            return inso_vertex<HP, BREAKS>(a, x, y, z, r, r2h, r2l, zmin, inv_r, staged ? s_tilt : nullptr, bk, arc);
+        });
 }
 
 // ---------------------------------------------------------------------------
