@@ -1041,11 +1041,12 @@ int grid_arcs(int64_t n)
     return (int)(g < cap ? g : cap);
 }
 
-// Whether a schedule is summed by arcs.
-bool use_arcs(const InsoArgs &a, int64_t vertices)
+// Whether a schedule is summed by arcs (radius: on spheres whose squares are
+// binary32 numbers, 2^-20 to 2^60).
+bool use_arcs(const InsoArgs &a, int64_t vertices, bool radius)
 {
     const int n = a.pairs ? 2 * a.n_rot : a.n_rot;
-    return n >= ARC_MIN && n <= ARC_MAX && (vertices >= ARC_VERTICES || n * a.n_tilt >= ARC_TERMS);
+    return radius && n >= ARC_MIN && n <= ARC_MAX && (vertices >= ARC_VERTICES || n * a.n_tilt >= ARC_TERMS);
 }
 
 }  // namespace
@@ -1117,7 +1118,7 @@ static int insolation_sums(const double *xyz_dev, int64_t n, double radius, cons
         memcpy(T.t, table_host, sizeof(float2) * (size_t)(n_rot_entries + n_tilt));
         if (breaks(a))
             insolation_args_kernel<12, true><<<grid_breaks(n), BREAK_THREADS, tilt_smem(a), s>>>(a, T);
-        else if (use_arcs(a, n))
+        else if (use_arcs(a, n, a.r2h > 0.0f))
             insolation_args_kernel<ARCS><<<grid_arcs(n), arc_threads(n), arcs, s>>>(a, T);
         else
             insolation_args_kernel<0><<<grid_for(n), 256, 0, s>>>(a, T);
@@ -1125,7 +1126,7 @@ static int insolation_sums(const double *xyz_dev, int64_t n, double radius, cons
         insolation_kernel<12, true><<<grid_breaks(n), BREAK_THREADS, tilt_smem(a), s>>>(a);
     } else if (a.pairs && n_rot_entries == 12) {
         insolation_kernel<12><<<grid_for(n), 256, tilt_smem(a), s>>>(a);
-    } else if (use_arcs(a, n)) {
+    } else if (use_arcs(a, n, a.r2h > 0.0f)) {
         insolation_kernel<ARCS><<<grid_arcs(n), arc_threads(n), arcs, s>>>(a);
     } else {
         insolation_kernel<0><<<grid_for(n), 256, 0, s>>>(a);
@@ -1184,11 +1185,15 @@ NX_EXPORT int nx_insolation_batch(const nx_inso_planet *planets_dev, const nx_in
     if (!planets_dev || !planets_host || !out_dev || !table_dev || n_rot_entries <= 0 || n_tilt <= 0)
         return nx::fail(NX_EINVAL, "nx_insolation_batch: bad arguments");
     int64_t total = 0;
+    bool radius = true;
     for (int p = 0; p < nplanets; ++p) {
         const nx_inso_planet &P = planets_host[p];
         if (P.vbeg % 256 || P.n < 0 || (P.n > 0 && !P.xyz) || !(P.radius > 0) || P.vbeg < total)
             return nx::fail(NX_EINVAL, "nx_insolation_batch: planet %d: rows must be packed, 256-aligned", p);
         total = P.vbeg + P.n;
+        float h, l;
+        radius_pair(P.radius, h, l);
+        radius = radius && h > 0.0f;
     }
     InsoArgs a;
     a.xyz = nullptr;
@@ -1209,7 +1214,7 @@ NX_EXPORT int nx_insolation_batch(const nx_inso_planet *planets_dev, const nx_in
         insolation_batch_kernel<12, true><<<grid_for(total, 4), 256, tilt_smem(a), s>>>(a, planets_dev, nplanets, total);
     else if (a.pairs && n_rot_entries == 12)
         insolation_batch_kernel<12><<<grid_for(total), 256, tilt_smem(a), s>>>(a, planets_dev, nplanets, total);
-    else if (use_arcs(a, total))
+    else if (use_arcs(a, total, radius))
         insolation_batch_kernel<ARCS><<<grid_for(total, 4), 256, arc_smem(a.pairs ? 2 * a.n_rot : a.n_rot), s>>>(
             a, planets_dev, nplanets, total);
     else

@@ -173,3 +173,24 @@ def test_long_schedules_day_by_day(rotations, days):
     assert (climate.insolation_sum(xyz, 1.0, rot, tilts).double() - want).abs().max() <= 2e-6 * want.max()
     off = climate.insolation_sum(xyz, 1.0 + 1e-9, rot, tilts).double()
     assert (off - want).abs().max() <= 1e-5 * want.max()
+
+
+@pytest.mark.parametrize("radius", [1e-30, 1e-19, 1e19, 1e25])
+def test_spheres_whose_squares_are_no_binary32_numbers(radius):
+    """A one-degree day as the sum of three parts of 120 rotations (below the arcs' range), alone and in a batch; 2e-6 of
+    the largest sum (two orders of summation in binary32)."""
+    import ctypes
+    import torch
+    from nixis_gb300 import _dev, _lib, climate, mesh
+    xyz = mesh.icosphere(20, with_tris=False)[0] * radius
+    rot, tilts = [-180.0 + i for i in range(360)], [11.0]
+    want = sum(climate.insolation_sum(xyz, radius, rot[q:q + 120], tilts) for q in (0, 120, 240))
+    assert (climate.insolation_sum(xyz, radius, rot, tilts) - want).abs().max() <= 2e-6 * want.max()
+    tab, nre, pairs = climate._plan(rot, tilts)
+    table, out = torch.from_numpy(tab).cuda(), torch.empty(xyz.shape[0], dtype=torch.float32, device="cuda")
+    d = (_lib.InsoPlanet * 1)()
+    d[0].xyz, d[0].n, d[0].vbeg, d[0].radius = xyz.data_ptr(), xyz.shape[0], 0, radius
+    dev = torch.frombuffer(bytearray(bytes(d)), dtype=torch.uint8).cuda()
+    _lib.call("nx_insolation_batch", _dev.ptr(dev), ctypes.cast(d, ctypes.c_void_p), 1, _dev.ptr(table), nre, pairs, 1, _dev.ptr(out),
+              _dev.stream_handle())
+    assert (out - want).abs().max() <= 2e-6 * want.max()
