@@ -480,9 +480,11 @@ __device__ __forceinline__ Arcs stage_arcs(const InsoArgs &a, void *smem)
         const float2 q = a.rot[i < a.n_rot ? i : i - a.n_rot];
         return i < a.n_rot ? q : make_float2(-q.x, -q.y);
     };
-    // (an angle that is no number has no place in the order: none of the
-    // tables, and the vertices go through the rotations one by one)
+    // (an angle that is no number has no place in the order, and a tilt that is
+    // none no arc: none of the tables, and the vertices go through the rotations
+    // one by one)
     bool number = true;
+    for (int d = threadIdx.x; d < a.n_tilt; d += blockDim.x) number = number && a.tilt[d].x == a.tilt[d].x;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const float2 q = rot(i);
         raw[i] = atan2f(q.y, q.x);

@@ -194,3 +194,18 @@ def test_spheres_whose_squares_are_no_binary32_numbers(radius):
     _lib.call("nx_insolation_batch", _dev.ptr(dev), ctypes.cast(d, ctypes.c_void_p), 1, _dev.ptr(table), nre, pairs, 1, _dev.ptr(out),
               _dev.stream_handle())
     assert (out - want).abs().max() <= 2e-6 * want.max()
+
+
+@pytest.mark.parametrize("bad", [math.nan, math.inf])
+@pytest.mark.parametrize("rotations", [128, 129])
+def test_a_tilt_that_is_no_number_gives_what_the_rotations_one_by_one_give(rotations, bad):
+    """Three tilts by arcs (their 384 positions reach the rule's 360), each alone by maxima: no number in pairs, where both
+    sides of a maximum are none, 0 otherwise.  2e-6 of the largest sum."""
+    import torch
+    from nixis_gb300 import climate, mesh
+    xyz = mesh.icosphere(9, with_tris=False)[0]
+    rot, tilts = [-180.0 + 360.0 / rotations * i for i in range(rotations)], [20.0, bad, -7.0]
+    got = climate.insolation_sum(xyz, 1.0, rot, tilts)
+    want = sum(climate.insolation_sum(xyz, 1.0, rot, [t]) for t in tilts)
+    assert torch.equal(got.isnan(), want.isnan()) and bool(want.isnan().all()) == (rotations == 128)
+    assert rotations == 128 or (got - want).abs().max() <= 2e-6 * want.max()
