@@ -53,11 +53,13 @@ def _in_memory(a):
 
 
 def from_device(t):
-    """A CUDA tensor's values as a numpy array, in torch's memory (its base is
-    marked as such): the driver program at 256,002 vertices takes 3.0 ms so and
-    4.8 ms with arrays made by numpy, whose pages cost more to make."""
+    """A CUDA tensor's values as a numpy array, in torch's memory: the driver
+    program at 256,002 vertices takes 3.0 ms so and 4.8 ms with arrays made by
+    numpy, whose pages cost more to make.  Where upload would ask, the array's
+    base is marked as such."""
     a = (t.cpu() if t.is_cuda else t.clone()).numpy()
-    a.base._nx_host = True
+    if a.nbytes > UPLOAD_MAX:
+        a.base._nx_host = True
     return a
 
 

@@ -100,7 +100,8 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e)
 // (| |v|^2 - r^2 | <= 1e-12 r^2): yes where the difference in pairs, within
 // 2^-44 (6e-14) of r^2, is below 8e-13 r^2; otherwise, and for a radius or
 // coordinate outside the pairs' range (a coordinate of 0 among them), as
-// binary64 has it.  JOIN: for sums over a schedule's positions one by one.
+// binary64 has it.  JOIN: the answer is hidden as well (in the kernel by
+// breakpoints it costs 3 us of a year's 106 on 10,000,002 vertices).
 template <bool JOIN>
 __device__ __forceinline__ bool load_vertex(double X, double Y, double Z, double r, float r2h, float r2l, float &x,
                                             float &y, float &z)
@@ -132,22 +133,24 @@ __device__ __forceinline__ bool load_vertex(double X, double Y, double Z, double
         const double rho2 = X * X + Y * Y + Z * Z, r2 = r * r;
         on = fabs(rho2 - r2) <= 1e-12 * r2;
     }
+    // One way out, which the compiler does not see behind.  With two it made
+    // the loops over a schedule twice, with half the loads in flight (2,500 days
+    // of 9,002 vertices 605 us instead of 317); without the coordinates here it
+    // made the loop of vertices off the sphere half as fast again (24 positions
+    // of 10 tilts on 400,002 of them 171 us instead of 128).
     if (JOIN) {
-        // one way out, which the compiler does not see behind: with two it made
-        // the loops over a schedule twice, with half the loads in flight (2,500
-        // days of 9,002 vertices 605 us instead of 321)
         int o = on;
         asm volatile("" : "+f"(x), "+f"(y), "+f"(z), "+r"(o));
         return o != 0;
     }
+    asm volatile("" : "+f"(x), "+f"(y), "+f"(z));
     return on;
 }
 
-// climate.py:419-442 for a vertex off the sphere of radius r (binary32).
-__device__ __forceinline__ float general_term(float x, float y, float z, float inv_r, float ct, float st, float cr, float sr)
+// climate.py:419-442 for a vertex off the sphere of radius r (binary32),
+// turned to (rx, ry, z).
+__device__ __forceinline__ float general_term(float rx, float ry, float z, float inv_r, float ct, float st)
 {
-    float rx = x * cr - y * sr;
-    float ry = x * sr + y * cr;
     float tx = rx * ct + z * st;
     float ty = ry;
     float tz = z * ct - rx * st;
@@ -595,7 +598,7 @@ __device__ __forceinline__ float inso_vertex(const InsoArgs &a, double X, double
                                              const Breaks &bk = Breaks(), const Arcs &arc = Arcs())
 {
     float x, y, z;
-    const bool on_sphere = load_vertex<!BREAKS && HP != ARCS>(X, Y, Z, r, r2h, r2l, x, y, z);
+    const bool on_sphere = load_vertex<!BREAKS>(X, Y, Z, r, r2h, r2l, x, y, z);
     if (HP == ARCS && on_sphere) return arc_sum(a, arc, x, y, z) * inv_r;
     float tot = 0.0f, comp = 0.0f;          // Kahan over tilts
     const int nr = HP > 0 ? HP : a.n_rot;
@@ -730,10 +733,13 @@ __device__ __forceinline__ float inso_vertex(const InsoArgs &a, double X, double
     for (int d = 0; d < a.n_tilt; ++d) {
         const float2 t = a.tilt[d];
         float s = 0.0f;
+#pragma unroll 6
         for (int h = 0; h < nr; ++h) {
-            float2 q = a.rot[h];
-            s += general_term(x, y, z, inv_r, t.x, t.y, q.x, q.y);
-            if (a.pairs) s += general_term(x, y, z, inv_r, t.x, t.y, -q.x, -q.y);
+            // (a pair's other rotation turns to the opposite point)
+            const float2 q = a.rot[h];
+            const float rx = x * q.x - y * q.y, ry = x * q.y + y * q.x;
+            s += general_term(rx, ry, z, inv_r, t.x, t.y);
+            if (HP > 0 || a.pairs) s += general_term(-rx, -ry, z, inv_r, t.x, t.y);
         }
         float yk = s - comp;
         float tk = tot + yk;

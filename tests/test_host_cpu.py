@@ -98,7 +98,7 @@ def test_arrays_whose_memory_is_numpys_own(tmp_path):
     from nixis_gb300 import _dev
     a = np.arange(24.0)
     for own in (a, a[3:], a.reshape(4, 6).T, a.view(np.uint8), np.asarray(memoryview(a)), np.frombuffer(memoryview(a[1:])),
-                np.zeros(0), _dev.from_device(torch.arange(6.0).view(2, 3).T), _dev.from_device(torch.ones(4, dtype=torch.uint8)).view(bool)):
+                np.zeros(0), _dev.from_device(torch.arange(6000.0).view(2, 3000).T), _dev.from_device(torch.ones(20000, dtype=torch.uint8)).view(bool)):
         assert _dev._in_memory(own)
     assert np.array_equal(_dev.from_device(torch.arange(6).view(2, 3).T), np.arange(6).reshape(2, 3).T)
     (tmp_path / "f").write_bytes(bytes(80000))

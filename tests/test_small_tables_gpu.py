@@ -126,7 +126,7 @@ def test_bytes_of_a_mapping_go_through_staging(tmp_path):
         assert np.array_equal(t.cpu().numpy(), a)
     _dev.to_host(np.frombuffer(mm), t + 1.0)
     assert np.array_equal(np.frombuffer(mm), a + 1.0)
-    points, _ = util.create_mesh(4)              # (the library's own results need none)
+    points, _ = util.create_mesh(10)             # (the library's own results need none)
     assert _dev._in_memory(points)
 
 
