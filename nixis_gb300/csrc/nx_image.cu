@@ -18,35 +18,35 @@ constexpr double PI = 3.141592653589793;
 // util.latlon2xyz (util.py:79-88).  A block takes LL_ROWS rows of 256 columns:
 // a column's sine and cosine are computed once per block, a row's once per
 // block row, instead of all four per pixel (binary64 sines and cosines, ~40
-// operations each on a pipe of two per SM and cycle).  Measured (GB300, 1024 x
-// 512 pixels): 103 -> 16 us.
-constexpr int LL_ROWS = 32;
-
-__global__ void __launch_bounds__(256) make_ll_kernel(int width, int height, double radius, double *__restrict__ out)
+// operations each on a pipe of two per SM and cycle).  32 rows, or 4 where 32
+// would leave three SMs in four without a block.  PART: rows from `base` on.
+// Measured (GB300): 1,024 x 512 pixels 103 -> 14.4 us; 256 x 128 pixels 8.9 us
+// one by one, 13.4 in blocks of 32 rows and 8.1 of 4, 400 x 200 24.2, 14.3, 8.1.
+template <int LL_ROWS, bool PART>
+__global__ void __launch_bounds__(256) make_ll_kernel(int width, int height, int base, double radius, double *__restrict__ out)
 {
     __shared__ double s_rc[LL_ROWS], s_z[LL_ROWS];           // radius cos(lat), radius sin(lat)
+    const int h0 = (PART ? base : 0) + blockIdx.y * LL_ROWS;
+    if (threadIdx.x < LL_ROWS) {
+        const double latpercent = 180.0 / (double)(height - 1);
+        const double lat = fmax(__dsub_rn(90.0, __dmul_rn((double)(h0 + (int)threadIdx.x), latpercent)), -90.0);
+        const double a = __dmul_rn(lat, PI / 180);
+        s_rc[threadIdx.x] = __dmul_rn(radius, cos(a));
+        s_z[threadIdx.x] = __dmul_rn(radius, sin(a));
+    }
+    __syncthreads();
     const int w = blockIdx.x * 256 + threadIdx.x;
+    if (w >= width) return;
     const double lonpercent = 360.0 / (double)width;
     const double lon = fmax(__dadd_rn(-180.0, __dmul_rn((double)w, lonpercent)), -180.0);
     const double b = __dmul_rn(lon, PI / 180);
     const double cb = cos(b), sb = sin(b);
-    const double latpercent = 180.0 / (double)(height - 1);
-    for (int64_t h0 = (int64_t)blockIdx.y * LL_ROWS; h0 < height; h0 += (int64_t)gridDim.y * LL_ROWS) {
-        __syncthreads();
-        if (threadIdx.x < LL_ROWS) {
-            const double lat = fmax(__dsub_rn(90.0, __dmul_rn((double)(h0 + threadIdx.x), latpercent)), -90.0);
-            const double a = __dmul_rn(lat, PI / 180);
-            s_rc[threadIdx.x] = __dmul_rn(radius, cos(a));
-            s_z[threadIdx.x] = __dmul_rn(radius, sin(a));
-        }
-        __syncthreads();
-        const int rows = (int)(height - h0 < LL_ROWS ? height - h0 : LL_ROWS);
-        for (int r = 0; w < width && r < rows; ++r) {
-            double *o = out + 3 * ((h0 + r) * width + w);
-            o[0] = __dmul_rn(s_rc[r], cb);
-            o[1] = __dmul_rn(s_rc[r], sb);
-            o[2] = s_z[r];
-        }
+    const int rows = min(LL_ROWS, height - h0);
+    for (int r = 0; r < rows; ++r) {
+        double *o = out + 3 * ((int64_t)(h0 + r) * width + w);
+        o[0] = __dmul_rn(s_rc[r], cb);
+        o[1] = __dmul_rn(s_rc[r], sb);
+        o[2] = s_z[r];
     }
 }
 
@@ -90,12 +90,22 @@ int grid_for(int64_t n)
 NX_EXPORT int nx_make_ll(int width, int height, double radius, double *out_dev, void *stream)
 {
     if (width < 1 || height < 2 || !out_dev) return nx::fail(NX_EINVAL, "nx_make_ll: bad arguments");
-    // (a grid's y is at most 65,535 blocks: taller maps by several blocks of rows each)
-    const int64_t yb = ((int64_t)height + LL_ROWS - 1) / LL_ROWS;
-    const dim3 grid((unsigned)((width + 255LL) / 256), (unsigned)(yb < 65535 ? yb : 65535));
-    make_ll_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(width, height, radius, out_dev);
-    NX_CHECK_LAUNCH("make_ll_kernel");
-    nx::note_launch(1);
+    const cudaStream_t s = (cudaStream_t)stream;
+    const int64_t xb = (width + 255LL) / 256;
+    auto grid = [&](int64_t h, int rows) { return dim3((unsigned)xb, (unsigned)((h + rows - 1) / rows)); };
+    // (a grid's y is at most 65,535 blocks: taller maps in parts)
+    const int64_t part = 65535LL * 32;
+    for (int64_t base = 0; base < height; base += part) {
+        const int64_t h = height - base < part ? height - base : part;
+        if (height > part)
+            make_ll_kernel<32, true><<<grid(h, 32), 256, 0, s>>>(width, height, (int)base, radius, out_dev);
+        else if (xb * ((h + 31) / 32) < nx::sm_count() / 4)
+            make_ll_kernel<4, false><<<grid(h, 4), 256, 0, s>>>(width, height, 0, radius, out_dev);
+        else
+            make_ll_kernel<32, false><<<grid(h, 32), 256, 0, s>>>(width, height, 0, radius, out_dev);
+        NX_CHECK_LAUNCH("make_ll_kernel");
+        nx::note_launch(1);
+    }
     return NX_OK;
 }
 
