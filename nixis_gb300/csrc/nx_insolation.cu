@@ -459,17 +459,24 @@ constexpr int ARC_TERMS = 360;
 constexpr int ARC_MAX = 1024;
 constexpr float TWO_PI = 6.28318531f;
 
+// Rotations without pairs keep their prefix sums as the integers they are formed
+// as, and a vertex's products with their rest: a difference of rounded sums is
+// off by what the largest sum is, which a vertex lit in a few rotations would
+// show (129 to 1,023 rotations, up to 40 of them lit: 4-30 times the error of
+// those terms added one by one; as integers no more than theirs).  The maxima of
+// pairs cancel in the same way as rounded sums do, so pairs keep those.
 struct Arcs {
-    const float2 *P = nullptr;
+    const float2 *P = nullptr;     // pairs
+    const longlong2 *Q = nullptr;  // no pairs: units of 2^-44
     const float *ang = nullptr;
     const int *F = nullptr;
     int n = 0, nb = 0;
     float base = 0.0f, scale = 0.0f;
 };
 
-__host__ __device__ __forceinline__ size_t arc_smem(int n)
+__host__ __device__ __forceinline__ size_t arc_smem(int n, int pairs)
 {
-    return sizeof(float2) * ((size_t)n + 1) + sizeof(float) * (2 * (size_t)n + 1) + sizeof(int) * (size_t)(sort_pad(n) + n + 1);
+    return (pairs ? sizeof(float2) : sizeof(longlong2)) * ((size_t)n + 1) + sizeof(float) * (2 * (size_t)n + 1) + sizeof(int) * (size_t)(sort_pad(n) + n + 1);
 }
 
 __device__ __forceinline__ Arcs stage_arcs(const InsoArgs &a, void *smem)
@@ -477,7 +484,8 @@ __device__ __forceinline__ Arcs stage_arcs(const InsoArgs &a, void *smem)
     Arcs A;
     const int n = a.pairs ? 2 * a.n_rot : a.n_rot, nb = sort_pad(n);
     float2 *P = reinterpret_cast<float2 *>(smem);
-    float *ang = reinterpret_cast<float *>(P + n + 1), *raw = ang + n;
+    longlong2 *Q = reinterpret_cast<longlong2 *>(smem);
+    float *ang = a.pairs ? reinterpret_cast<float *>(P + n + 1) : reinterpret_cast<float *>(Q + n + 1), *raw = ang + n;
     int *order = reinterpret_cast<int *>(raw + n + 1), *F = order + n;
     auto rot = [&](int i) {
         const float2 q = a.rot[i < a.n_rot ? i : i - a.n_rot];
@@ -520,11 +528,15 @@ __device__ __forceinline__ Arcs stage_arcs(const InsoArgs &a, void *smem)
     block_scan2(u, v, tu, tv);
     for (int j = j0; j < j1; ++j) {
         const float2 q = rot(order[j]);
-        P[j] = make_float2(from_fixed(u), from_fixed(v));
+        if (a.pairs) P[j] = make_float2(from_fixed(u), from_fixed(v));
+        else Q[j] = make_longlong2(u, v);
         u += to_fixed(q.x);
         v += to_fixed(q.y);
     }
-    if (threadIdx.x == 0) P[n] = make_float2(from_fixed(tu), from_fixed(tv));
+    if (threadIdx.x == 0) {
+        if (a.pairs) P[n] = make_float2(from_fixed(tu), from_fixed(tv));
+        else Q[n] = make_longlong2(tu, tv);
+    }
     __syncthreads();
     for (int b = threadIdx.x; b <= nb; b += blockDim.x) {
         const float edge = (float)b * (TWO_PI / (float)nb);
@@ -538,6 +550,7 @@ __device__ __forceinline__ Arcs stage_arcs(const InsoArgs &a, void *smem)
     }
     __syncthreads();
     A.P = P;
+    A.Q = Q;
     A.ang = ang;
     A.F = F;
     A.n = n;
@@ -562,28 +575,49 @@ __device__ __forceinline__ float arc_sum(const InsoArgs &a, const Arcs &A, float
     for (int d = 0; d < a.n_tilt; ++d) {
         const float2 t = a.tilt[d];
         const float C = z * t.y, den = fabsf(t.x) * rho;
-        float2 S = make_float2(0.0f, 0.0f);
-        int cnt = 0;
+        int lo = 0, hi = 0, turns = 0;         // rotations [lo, hi), and all of them once more
         if (C >= den) {
-            S = A.P[A.n];
-            cnt = A.n;
+            hi = A.n;
         } else if (C > -den) {
             const float alpha = acosf(__fdividef(-C, den));
             float a0 = (t.x < 0.0f ? phi + 0.5f * TWO_PI : phi) - alpha - A.base;
             a0 -= TWO_PI * floorf(a0 * (1.0f / TWO_PI));
             const float a1 = a0 + 2.0f * alpha;
-            const int lo = arc_find(A, a0), hi = arc_find(A, a1 < TWO_PI ? a1 : a1 - TWO_PI);
+            turns = a1 >= TWO_PI ? 1 : 0;
+            lo = arc_find(A, a0);
+            hi = arc_find(A, turns ? a1 - TWO_PI : a1);
+        }
+        const float cnt = (float)(hi - lo + turns * A.n);
+        float s;
+        if (a.pairs) {
             const float2 l = A.P[lo], h = A.P[hi];
-            S = make_float2(h.x - l.x, h.y - l.y);
-            cnt = hi - lo;
-            if (a1 >= TWO_PI) {
+            float2 S = make_float2(h.x - l.x, h.y - l.y);
+            if (turns) {
                 const float2 w = A.P[A.n];
                 S.x += w.x;
                 S.y += w.y;
-                cnt += A.n;
             }
+            s = fmaf(t.x, fmaf(x, S.x, -(y * S.y)), C * cnt);
+        } else {
+            const longlong2 l = A.Q[lo], h = A.Q[hi];
+            long long u = h.x - l.x, v = h.y - l.y;
+            if (turns) {
+                const longlong2 w = A.Q[A.n];
+                u += w.x;
+                v += w.y;
+            }
+            // t.x (x Sx - y Sy) + z t.y cnt in pairs
+            const float Sx = from_fixed(u), Sy = -from_fixed(v);
+            const float px = __fmul_rn(x, Sx), py = __fmul_rn(y, Sy), p = __fmul_rn(C, cnt);
+            float q, qe, r, re;
+            two_sum(px, py, q, qe);
+            qe += __fmaf_rn(x, Sx, -px) + __fmaf_rn(y, Sy, -py);
+            const float g = __fmul_rn(t.x, q);
+            two_sum(g, p, r, re);
+            re += __fmaf_rn(t.x, q, -g) + __fmaf_rn(C, cnt, -p);
+            s = r + fmaf(t.x, qe, fmaf(__fmaf_rn(z, t.y, -C), cnt, re));
         }
-        const float s = fmaxf(fmaf(t.x, fmaf(x, S.x, -(y * S.y)), C * (float)cnt), 0.0f);
+        s = fmaxf(s, 0.0f);
         const float yk = s - comp;
         const float tk = tot + yk;
         comp = (tk - tot) - yk;
@@ -1120,7 +1154,7 @@ static int insolation_sums(const double *xyz_dev, int64_t n, double radius, cons
     a.out = out_dev;
     a.accumulate = accumulate;
     a.scale = scale;
-    const size_t arcs = arc_smem(a.pairs ? 2 * a.n_rot : a.n_rot);
+    const size_t arcs = arc_smem(a.pairs ? 2 * a.n_rot : a.n_rot, a.pairs);
     if (table_host) {
         InsoTable T;
         memcpy(T.t, table_host, sizeof(float2) * (size_t)(n_rot_entries + n_tilt));
@@ -1223,7 +1257,7 @@ NX_EXPORT int nx_insolation_batch(const nx_inso_planet *planets_dev, const nx_in
     else if (a.pairs && n_rot_entries == 12)
         insolation_batch_kernel<12><<<grid_for(total), 256, tilt_smem(a), s>>>(a, planets_dev, nplanets, total);
     else if (use_arcs(a, total, radius))
-        insolation_batch_kernel<ARCS><<<grid_for(total, 4), 256, arc_smem(a.pairs ? 2 * a.n_rot : a.n_rot), s>>>(
+        insolation_batch_kernel<ARCS><<<grid_for(total, 4), 256, arc_smem(a.pairs ? 2 * a.n_rot : a.n_rot, a.pairs), s>>>(
             a, planets_dev, nplanets, total);
     else
         insolation_batch_kernel<0><<<grid_for(total), 256, 0, s>>>(a, planets_dev, nplanets, total);

@@ -209,3 +209,25 @@ def test_a_tilt_that_is_no_number_gives_what_the_rotations_one_by_one_give(rotat
     want = sum(climate.insolation_sum(xyz, 1.0, rot, [t]) for t in tilts)
     assert torch.equal(got.isnan(), want.isnan()) and bool(want.isnan().all()) == (rotations == 128)
     assert rotations == 128 or (got - want).abs().max() <= 2e-6 * want.max()
+
+
+@pytest.mark.parametrize("rotations", [361, 511, 1023])
+@pytest.mark.parametrize("tilt", [23.44, 75.0])
+def test_vertices_lit_in_few_rotations_without_pairs(rotations, tilt):
+    """Near where night lasts all day, by arcs.  Tolerance (stated): binary32 terms of three products of two or three
+    rounded factors are within 6 2^-24 of themselves each, and a rotation misplaced at an end of the arc (an angle's
+    cosine is off by 2^-23, twice) adds at most 4 2^-24: (6 m + 8) 2^-24 for a vertex lit in m rotations."""
+    import torch
+    from nixis_gb300 import climate
+    rng = np.random.default_rng(7)
+    t = math.radians(tilt)
+    z = -math.cos(t) * (1.0 + rng.uniform(-1e-3, 1e-3, 6000))
+    at = rng.uniform(-math.pi, math.pi, len(z))
+    v = np.stack([np.sqrt(1.0 - z * z) * np.cos(at), np.sqrt(1.0 - z * z) * np.sin(at), z], axis=1)
+    rot = [-180.0 + 360.0 / rotations * i for i in range(rotations)]
+    got = climate.insolation_sum(torch.from_numpy(v).cuda(), 1.0, rot, [tilt]).double().cpu().numpy()
+    r = np.radians(rot)
+    u = (v[:, :1] * np.cos(r) - v[:, 1:2] * np.sin(r)) * math.cos(t) + v[:, 2:] * math.sin(t)
+    lit = (u > 0.0).sum(1)
+    assert ((lit >= 1) & (lit <= 8)).sum() > 100
+    assert (np.abs(got - np.maximum(u, 0.0).sum(1)) <= (6 * lit + 8) * 2.0 ** -24)[lit <= 60].all()
