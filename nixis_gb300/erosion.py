@@ -210,10 +210,12 @@ def _run_inplace(verts, neighbors, h, w, s, iters, rain, with_fields):
             if a is not None and tuple(a.shape) != (0,):
                 raise ValueError(f"{name}: expected shape (0,), got {tuple(a.shape)}")
         return
+    # (host fields before the run zeroes its workspace: a busy stream has them staged)
+    hd, wd, sd = (_dev.to_device(a, np.float64) if host and a is not None else a for a in (h, w, s))
     run = ErosionRun(verts, neighbors, iters=iters)
-    hd = _dev.to_device(h, np.float64, (run.n,), "heights")
-    wd = _dev.to_device(w, np.float64, (run.n,), "water") if w is not None else None
-    sd = _dev.to_device(s, np.float64, (run.n,), "sediment") if s is not None else None
+    hd = _dev.to_device(hd, np.float64, (run.n,), "heights")
+    wd = _dev.to_device(wd, np.float64, (run.n,), "water") if w is not None else None
+    sd = _dev.to_device(sd, np.float64, (run.n,), "sediment") if s is not None else None
     run.load(hd, wd, sd)
     done = run.blocked(iters, rain)
     if done and run.error() > 1:

@@ -142,3 +142,19 @@ def test_a_large_array_does_not_wait_for_a_busy_stream():
     a[:] = 0.0
     assert busy
     assert np.array_equal(t.cpu().numpy(), want)
+
+
+@gpu
+def test_a_call_on_an_idle_stream_stages_nothing(monkeypatch):
+    """Host fields of a drop-in erosion are copied before the run's own work is on the stream."""
+    from nixis_gb300 import erosion
+    points, cells = util.create_mesh(20)
+    nbr = util.build_adjacency(cells)
+    util.sort_adjacency(nbr)
+    staged = []
+    pin = torch.Tensor.pin_memory
+    monkeypatch.setattr(torch.Tensor, "pin_memory", lambda t, *a: staged.append(t.shape) or pin(t, *a))
+    torch.cuda.synchronize()
+    height = points[:, 2] * 100.0
+    erosion.erode_terrain3(points, nbr, height, num_iter=3)
+    assert staged == []
