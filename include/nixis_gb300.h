@@ -70,6 +70,10 @@ int nx_perm_init(int64_t seed, int32_t *perm, int32_t *pgi);
  * part of the graph. */
 int nx_upload(void *dst_dev, const void *src_host, int64_t bytes, void *stream);
 
+/* 1 where `stream` has nothing queued and is not being captured, otherwise 0.
+ * Leaves captures on other threads as they are. */
+int nx_stream_idle(void *stream);
+
 /* ------------------------------------------------------------------ */
 /* Noise                                                               */
 /* ------------------------------------------------------------------ */

@@ -21,6 +21,7 @@ SIGNATURES = {
     "nx_version": (_i32, []),
     "nx_launch_count": (_u64, []),
     "nx_upload": (_i32, [_p, _p, _i64, _p]),
+    "nx_stream_idle": (_i32, [_p]),
     "nx_perm_init": (_i32, [_i64, _p, _p]),
     "nx_fbm": (_i32, [_p, _i64, _p, _p, _i32, _p, _p, _d, _p, _p, _i32, _p, _p]),
     "nx_sample_octaves": (_i32, [_p, _i64, _p, _p, _i32, _d, _d, _d, _d, _d, _p, _p, _i32, _p]),

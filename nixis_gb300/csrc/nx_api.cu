@@ -125,3 +125,21 @@ NX_EXPORT int nx_upload(void *dst_dev, const void *src_host, int64_t bytes, void
     }
     return NX_OK;
 }
+
+// (the question is one that a capture on another thread forbids by default: the
+// calling thread's interaction with captures is relaxed meanwhile)
+NX_EXPORT int nx_stream_idle(void *stream)
+{
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    bool idle = cudaStreamIsCapturing((cudaStream_t)stream, &capture) == cudaSuccess &&
+                capture == cudaStreamCaptureStatusNone;
+    if (idle && cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess) {
+        idle = cudaStreamQuery((cudaStream_t)stream) == cudaSuccess;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+    } else {
+        idle = false;
+    }
+    if (!idle) cudaGetLastError();
+    return idle ? 1 : 0;
+}

@@ -158,3 +158,38 @@ def test_a_call_on_an_idle_stream_stages_nothing(monkeypatch):
     height = points[:, 2] * 100.0
     erosion.erode_terrain3(points, nbr, height, num_iter=3)
     assert staged == []
+
+
+@gpu
+def test_the_question_whether_a_stream_is_idle_leaves_captures_whole():
+    """Asked while another thread captures, of a busy stream, and of the captured one."""
+    import threading
+    idle = _lib.lib().nx_stream_idle
+    x, got = torch.zeros(8, device="cuda"), []
+    graph, s, busy = torch.cuda.CUDAGraph(), torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=s):
+        x.add_(1.0)
+        other = threading.Thread(target=lambda: got.append(idle(None)))
+        other.start()
+        other.join()
+        got.append(idle(s.cuda_stream))
+    assert got == [1, 0]
+    graph.replay()
+    torch.cuda.synchronize()
+    assert x.eq(1.0).all()
+    with torch.cuda.stream(busy):
+        torch.cuda._sleep(100_000_000)
+    assert idle(busy.cuda_stream) == 0
+    busy.synchronize()
+    assert idle(busy.cuda_stream) == 1
+
+
+@gpu
+def test_the_handle_is_the_current_streams():
+    s = torch.cuda.Stream()
+    for _ in range(2):
+        assert _dev.stream_handle().value == (torch.cuda.current_stream().cuda_stream or None)
+        with torch.cuda.stream(s):
+            assert _dev.stream_handle().value == s.cuda_stream
+    assert _dev.stream_handle(s).value == s.cuda_stream
