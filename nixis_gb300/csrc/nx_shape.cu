@@ -49,23 +49,28 @@ constexpr u64 NONE = ~0ull;
 
 __device__ __forceinline__ u64 umin(u64 a, u64 b) { return a < b ? a : b; }
 
-// Ordered key of a binary64, from 0 for -infinity on: -0 taken as +0, as the
-// reference's comparisons see them equal; every NaN, whatever its sign, one
-// key above +infinity's (and below NONE).
-constexpr u64 KEY_FIRST = 0x000FFFFFFFFFFFFFull, KEY_NAN = 0xFFF0000000000001ull - KEY_FIRST;
+// Ordered key of a binary64: -0 taken as +0, as the reference's comparisons see
+// them equal; every NaN, whatever its sign, one key above +infinity's (and below
+// NONE).  Those three are found by the high word and leave the others the two
+// operations of the sign (shape_heights of 6,400,002 heights 248.5 us; with
+// 64-bit comparisons for every key 251.5).
+constexpr u64 KEY_SIGN = 0x8000000000000000ull, KEY_NAN = 0xFFF0000000000001ull;
 
 __device__ __forceinline__ u64 dkey(double v)
 {
     const u64 b = nxf::bits(v);
-    if (b == 0x8000000000000000ull) return b - KEY_FIRST;
-    const u64 k = (b & 0x8000000000000000ull) ? ~b : (b | 0x8000000000000000ull);
-    return umin(k - KEY_FIRST, KEY_NAN);
+    const unsigned hi = (unsigned)(b >> 32);
+    u64 k = b ^ ((u64)((long long)b >> 63) | KEY_SIGN);
+    if (hi == 0x80000000u || hi + hi >= 0xFFE00000u) {
+        if (b == KEY_SIGN) k = KEY_SIGN;
+        if ((b & ~KEY_SIGN) > 0x7FF0000000000000ull) k = KEY_NAN;
+    }
+    return k;
 }
 
-__device__ __forceinline__ double dunkey(u64 q)
+__device__ __forceinline__ double dunkey(u64 k)
 {
-    const u64 k = q + KEY_FIRST;
-    const u64 b = (k & 0x8000000000000000ull) ? (k & ~0x8000000000000000ull) : ~k;
+    const u64 b = (k & KEY_SIGN) ? (k & ~KEY_SIGN) : ~k;
     return __longlong_as_double((long long)b);
 }
 
