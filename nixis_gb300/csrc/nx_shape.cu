@@ -129,9 +129,7 @@ struct Ws {
     u64 pad;
 };
 
-// np.min and np.max: both are NaN where a value is.
-__device__ __forceinline__ double min_of(u64 kmin, u64 kmax) { return dunkey(kmax == KEY_NAN ? KEY_NAN : kmin); }
-__device__ __forceinline__ double ext_min(const Extremes &e) { return min_of(~e.nmin, e.max); }
+__device__ __forceinline__ double ext_min(const Extremes &e) { return dunkey(~e.nmin); }
 __device__ __forceinline__ double ext_max(const Extremes &e) { return dunkey(e.max); }
 
 // Fold every thread's keys into e: one pair of atomics per block.
@@ -204,12 +202,12 @@ __global__ void __launch_bounds__(THREADS) minmax_kernel(const double *__restric
     fold_extremes(nmin, max, &w->in);
     if (!SHAPE || !last_block(&w->blocks) || threadIdx.x) return;
     const volatile Extremes *e = &w->in;
-    const double x_min = min_of(~e->nmin, e->max), x_max = dunkey(e->max);
+    const double x_min = dunkey(~e->nmin), x_max = dunkey(e->max);
     w->base = rescale_low(a, x_min, x_max);
     const u64 p = dkey(w->base(x_min)), q = dkey(w->base(x_max));
     w->kmin = umin(p, q);
     w->kmax = umax(p, q);
-    w->level = percent_val(min_of(w->kmin, w->kmax), dunkey(w->kmax), percent);
+    w->level = percent_val(dunkey(w->kmin), dunkey(w->kmax), percent);
     if (level_out) *level_out = w->level;
 }
 
@@ -302,10 +300,9 @@ __device__ __forceinline__ Run join_block(Run r)
 }
 
 // power_rescale's range from the whole run and np.min / np.max of the field
-// (keys).  Where those are NaN no comparison holds and both ends stay NaN.
+// (keys).
 __device__ __forceinline__ Range range_of(const Run &r, u64 kmin, u64 kmax)
 {
-    if (kmax == KEY_NAN) return Range{dunkey(KEY_NAN), dunkey(KEY_NAN)};
     u64 hi = umax(kmin, r.rest);
     if (r.min != NONE && r.first >= kmax) hi = umax(hi, r.first);
     return Range{dunkey(umin(kmax, r.min)), dunkey(hi)};
