@@ -49,21 +49,23 @@ constexpr u64 NONE = ~0ull;
 
 __device__ __forceinline__ u64 umin(u64 a, u64 b) { return a < b ? a : b; }
 
-// Ordered key of a binary64: -0 taken as +0, as the reference's comparisons see
-// them equal; every NaN, whatever its sign, one key above +infinity's (and below
-// NONE).  Those three are found by the high word and leave the others the two
-// operations of the sign (shape_heights of 6,400,002 heights 248.5 us; with
-// 64-bit comparisons for every key 251.5).
-constexpr u64 KEY_SIGN = 0x8000000000000000ull, KEY_NAN = 0xFFF0000000000001ull;
+// Ordered key of a binary64, below NONE: -0 taken as +0, as the reference's
+// comparisons see them equal.  A NaN with its sign bit set, as 0 / 0 gives, is
+// smaller than all numbers, so the minimum is NaN with it; any other NaN comes
+// right below 0, so in a field on both sides of 0 it is neither extreme.  -0 and
+// NaNs are found by the high word and leave the others the two operations of the
+// sign (shape_heights of 6,400,002 heights 246.4 us; with 64-bit comparisons for
+// every key 251.5).
+constexpr u64 KEY_SIGN = 0x8000000000000000ull, KEY_NAN = 0x7FF7FFFFFFFFFFFFull;
 
 __device__ __forceinline__ u64 dkey(double v)
 {
     const u64 b = nxf::bits(v);
     const unsigned hi = (unsigned)(b >> 32);
     u64 k = b ^ ((u64)((long long)b >> 63) | KEY_SIGN);
-    if (hi == 0x80000000u || hi + hi >= 0xFFE00000u) {
+    if (hi == 0x80000000u || (hi < 0x80000000u && hi >= 0x7FF00000u)) {
         if (b == KEY_SIGN) k = KEY_SIGN;
-        if ((b & ~KEY_SIGN) > 0x7FF0000000000000ull) k = KEY_NAN;
+        if ((long long)b > 0x7FF0000000000000ll) k = KEY_NAN;
     }
     return k;
 }
@@ -399,7 +401,7 @@ __global__ void __launch_bounds__(THREADS) shape_base_kernel(const double *__res
             const double v = low(h[i]);
             h1[i] = v;
             q = dkey(v);
-            mask[i] = !dry && q <= klev ? 1 : 0;
+            mask[i] = !dry && q <= klev && q != KEY_NAN ? 1 : 0;
         }
         s_key[slot(k)] = q;
     }
@@ -408,7 +410,7 @@ __global__ void __launch_bounds__(THREADS) shape_base_kernel(const double *__res
     for (int k = 0; k < PER_THREAD; ++k) {
         const u64 q = s_key[slot(threadIdx.x * PER_THREAD + k)];
         if (q == NONE) continue;
-        if (!dry && q <= klev) append(sea, q);
+        if (!dry && q <= klev && q != KEY_NAN) append(sea, q);
         else append(land, q);
     }
     sea = join_block(sea);
@@ -433,8 +435,7 @@ __global__ void __launch_bounds__(THREADS) shape_base_kernel(const double *__res
     const Range r1 = range_of(sea, w->kmin, w->kmax);
     w->range[1] = r1;
     // np.min / np.max of h2: the land as it is, the ocean's ends through the
-    // curve (monotone for a positive range; otherwise it gives NaN, the
-    // largest key)
+    // curve (monotone for a positive range; otherwise it gives NaN)
     u64 k2min = land.min, k2max = land.min == NONE ? 0ull : umax(land.rest, land.first);
     if (sea.min != NONE) {
         const Curve curve = curve_of(r1, 0.5);
@@ -457,7 +458,8 @@ __global__ void __launch_bounds__(THREADS) shape_curve_kernel(const double *__re
     for (int64_t i = (int64_t)blockIdx.x * THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * THREADS) {
         const double v = h1[i];
         // the operands selected, so that a coast's warps run one path
-        const bool wet = !dry && dkey(v) <= klev;
+        const u64 k = dkey(v);
+        const bool wet = !dry && k <= klev && k != KEY_NAN;
         const double lo = nxf::pick(wet, sea.lo, land.lo);
         const nxf::Factor range{nxf::pick(wet, sea.range.b, land.range.b), wet ? sea.range.m : land.range.m,
                                 wet ? sea.range.hw : land.range.hw};

@@ -56,18 +56,32 @@ def test_shaping_equals_the_oracle(kind, n):
             assert ulps(util.power_rescale(x, m, mode, power), want) <= 4, (mode, power)
 
 
-def test_the_sign_of_a_nan_does_not_matter():
-    """A NaN of either sign is np.max's result and not np.min's, so what lies below `mid` keeps its values."""
+@pytest.mark.parametrize("field", [[5.0, 7.0, 6.0], [-5.0, -7.0, -6.0], [-1.0, 2.0, 0.5]])
+@pytest.mark.parametrize("at", [0, 2, 3])
+def test_nans_by_their_sign(field, at):
+    """A negative NaN is the smallest key, so the minimum is NaN; a positive one counts as a number right below 0."""
     from nixis_gb300 import util
-    x = np.random.default_rng(4).normal(size=5000)
-    x[17] = np.nan
+    x = np.insert(field, at, np.nan)
     y = x.copy()
-    y.view(np.uint64)[17] ^= np.uint64(1 << 63)
-    for args, nans in (({}, 5000), ({"mid": 0.25}, 1 + (x > 0.25).sum()), ({"mid": 0.25, "mode": "lower"}, 1),
-                       ({"mid": -0.25, "mode": "upper"}, 1 + (x > -0.25).sum())):
-        a, b = util.rescale(x, -1.0, 2.0, **args), util.rescale(y, -1.0, 2.0, **args)
-        assert np.array_equal(a, b, equal_nan=True) and np.isnan(a).sum() == nans
-    m = np.random.default_rng(5).random(5000) < 0.5
-    for mode in (0, 1):
-        assert np.array_equal(util.power_rescale(x, m, mode, 2.0), util.power_rescale(y, m, mode, 2.0), equal_nan=True)
-    assert np.array_equal(util.make_bool_elevation_mask(x, 0.1), util.make_bool_elevation_mask(y, 0.1))
+    y.view(np.uint64)[at] ^= np.uint64(1 << 63)
+    number = ~np.isnan(x)
+    lo, hi = min(min(field), 0.0), max(max(field), 0.0)
+    assert np.allclose(util.rescale(x, 0.0, 1.0), (x - lo) / (hi - lo), rtol=1e-15, equal_nan=True)
+    assert np.isnan(util.rescale(y, 0.0, 1.0)).all()
+    above = number & (x > 0.6)
+    for v in (x, y):
+        assert np.array_equal(util.rescale(v, 0.0, 1.0, mid=0.6)[above], ((x - 0.6) / (max(hi, 0.0) - 0.6) * 0.4 + 0.6)[above])
+    assert np.array_equal(np.isnan(util.rescale(y, 0.0, 1.0, mid=0.6)), ~above)
+    everywhere = np.ones(4, bool)
+    assert np.array_equal(np.isnan(util.power_rescale(x, everywhere, 1, 2.0)), ~number)
+    assert np.isnan(util.power_rescale(y, everywhere, 1, 2.0)).all()
+    assert np.array_equal(np.isnan(util.shape_heights(x)[0]), ~number) and np.isnan(util.shape_heights(y)[0]).all()
+
+
+@pytest.mark.parametrize("field, nans", [([0.0, 1.0, 0.99, 0.98], [0]), ([1.0, 0.0, 0.01, 0.02], [0, 1, 2, 3]), ([0.0, 1.0], [0, 1]),
+                                         ([0.0, 0.8, 0.9, 1.0], [0])])
+def test_a_single_vertex_of_ocean_or_land(field, nans):
+    """Its curve is 0 / 0, the minimum of the last rescale: no number there and in the ocean, the land is mapped."""
+    from nixis_gb300 import util
+    h, _, level = util.shape_heights(np.array(field))
+    assert np.flatnonzero(np.isnan(h)).tolist() == nans and level == 3067.5
