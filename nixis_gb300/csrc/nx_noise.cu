@@ -1047,11 +1047,15 @@ __device__ __forceinline__ void anchor_pair(float h, float l, float &H, float &L
     L = __fadd_rn(__fsub_rn(h, H), l);
 }
 
-// A binary64 value in [-2, 2) anchored (binary64 decision path).
+// A displacement anchored (binary64 decision path).  It lies in [-2, 2) unless
+// the coordinate is past binary64's integers; beyond 4 no lattice point of the
+// cell is near and 4 does as well, while larger ones' low parts are not small
+// and their squares (contrib2_pair) would stay where attn is 0.
 __device__ __forceinline__ void anchor_f64(double d, float &H, float &L)
 {
-    const float h = __double2float_rn(d);
-    anchor_pair(h, __double2float_rn(__dsub_rn(d, (double)h)), H, L);
+    const float h = __double2float_rn(d), l = __double2float_rn(__dsub_rn(d, (double)h));
+    const bool far = fabsf(h) > 4.0f && fabsf(h) < 0x1p66f;       // (an infinite coordinate stays no number)
+    anchor_pair(far ? copysignf(4.0f, h) : h, far ? 0.0f : l, H, L);
 }
 
 // Per-octave constants of the pair path.

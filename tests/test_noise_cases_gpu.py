@@ -77,3 +77,15 @@ def test_gradients_that_start_anywhere():
     np.testing.assert_allclose(val, want, rtol=0, atol=2.7e-6)
     got = terrain.fbm(torch.from_numpy(pts).cuda(), perm, pgi, [1.0], [2.0], 1.0, out_dtype=torch.float32)[0]
     np.testing.assert_allclose(got.cpu().numpy(), want + 1.0, rtol=0, atol=2.7e-6)
+
+
+@pytest.mark.parametrize("octaves, x", [(1, 1e17), (4, 1e16), (4, 1e17), (12, 1e15), (12, 1e16)])
+def test_coordinates_past_the_integers(octaves, x):
+    """No lattice point is near there, so an octave adds half its strength and no more."""
+    from nixis_gb300 import opensimplex, terrain
+    perm, pgi = opensimplex.init(5)
+    strength = [0.5 ** o for o in range(octaves)]
+    got = terrain.fbm(np.full((3, 3), x), perm, pgi, [2.0 ** o for o in range(octaves)], strength, 1.0)[0]
+    assert torch.equal(got, torch.full_like(got, 0.5 * sum(strength)))
+    for x in (np.inf, -np.inf, np.nan):
+        assert terrain.fbm(np.full((3, 3), x), perm, pgi, [1.0, 2.0], [1.0, 0.5], 1.0)[0].isnan().all()
